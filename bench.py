@@ -925,7 +925,7 @@ def cpu_reference_run(nprocs, steps, warmup):
     try:
         import oracle as O
         import build as B
-        have_ref = os.path.exists(B.harness_path(Q, 1, True)) or os.path.isdir(B.REF)
+        have_ref = os.path.exists(B.harness_path(Q, 1, True)) or B.have_reference()
     except Exception:
         have_ref = False
     if have_ref:
@@ -985,7 +985,7 @@ def cpu_reference_extras():
     }
     for case, _ in runs.values():
         per = any(b == "periodic" for b in case.mesh.spec.boundary)
-        if not (os.path.exists(B.harness_path(case.params.q, case.mesh.spec.max_level, per)) or os.path.isdir(B.REF)):
+        if not (os.path.exists(B.harness_path(case.params.q, case.mesh.spec.max_level, per)) or B.have_reference()):
             return {"unavailable": "the reference harness is not built"}
     out = {}
     with tempfile.TemporaryDirectory() as td:

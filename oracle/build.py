@@ -46,6 +46,12 @@ from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 REF = os.environ.get("MT_REFERENCE_DIR", "/root/reference")
+
+
+def have_reference() -> bool:
+    """Whether the reference checkout holds its sources (an empty folder does not)."""
+    return os.path.isfile(os.path.join(REF, "header", "LBM_Manager.hpp"))
+
 REF_TUS = [
     "LBM_Manager.cpp",
     "LBM_Simulator.cpp",
@@ -166,7 +172,7 @@ def _shim_header(q: int, L: int, periodic: bool = False) -> str:
 
 def build_refharness(q: int, L: int, force: bool = False, periodic: bool = False) -> str:
     out = harness_path(q, L, periodic)
-    if not os.path.isdir(REF):
+    if not have_reference():
         if os.path.exists(out):
             return out
         raise FileNotFoundError("reference checkout not present and no prebuilt harness")
@@ -201,7 +207,7 @@ def build_refharness(q: int, L: int, force: bool = False, periodic: bool = False
 
 def build_all(harness: bool = True) -> None:
     build_oracle_lib()
-    if harness and os.path.isdir(REF):
+    if harness and have_reference():
         for q, L in HARNESS_VARIANTS:
             build_refharness(q, L)
         for q, L in PERIODIC_VARIANTS:
