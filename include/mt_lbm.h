@@ -306,14 +306,17 @@ int mt_case_status(mt_ctx *ctx, int32_t case_id);
  * 256 only; the other slots are left unwritten). */
 int mt_case_tune(mt_ctx *ctx, int32_t case_id, int32_t *best_block, float *ms_per_candidate);
 /* Forms of the multi-level fused brick pass (no reference counterpart):
- * 0: one cell per lane step at 8 resident 128-thread blocks per SM (FP32: 7),
+ * for FP32 / FP16 / BF16 storage
+ * 0: a lane gathers, collides and stores two x-adjacent cells together (packed
+ *    FP32 arithmetic) at 6 resident 128-thread blocks per SM (16-bit D3Q19: 7),
  *    the default;
- * 3: the lane's two cells in one unrolled sequence, so that the second
- *    cell's gathers overlap the first cell's collision, at 6 blocks;
- * for FP32 / FP16 / BF16 storage also
- * 1: the two cells together in packed FP32 pair arithmetic at 4 blocks,
- * 2: form 0 at 6 blocks with more registers per thread.
- * Forms 0, 2 and 3 compute the same values bit for bit. */
+ * 2, 3: form 0 at other numbers of resident blocks (16 bits 7 and 8, D3Q19 8
+ *    and 9; FP32 5 and 7);
+ * 1: one cell per lane step;
+ * for FP64
+ * 0: one cell per lane step, the default;
+ * 3: the lane's two cells in one unrolled sequence.
+ * All forms of a storage compute the same values bit for bit. */
 #define MT_BRICK_FORMS 4
 /* Project autotuner of the multi-level fused brick pass: times each brick
  * level's pass in each of its forms on the case's own bricks, without

@@ -18,12 +18,41 @@ namespace mt {
 // ----------------------------------------------------------------------------
 // build kernels
 // ----------------------------------------------------------------------------
-__global__ void k_tag_cells(const uint64_t *raw, const uint8_t *set, int64_t nraw, const uint64_t *key, int64_t n,
-                            uint32_t *tag, int8_t *bcidx)
+// sorted raw keys (with repeats): a cell starts where the key changes (low
+// half), a brick where the key's brick part does (high half)
+__global__ void k_starts(const uint64_t *key, int64_t n, int shift, unsigned long long *flag)
+{
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    unsigned long long v = 0;
+    if (i == 0 || key[i] != key[i - 1]) v |= 1ull;
+    if (i == 0 || (key[i] >> shift) != (key[i - 1] >> shift)) v |= 1ull << 32;
+    flag[i] = v;
+}
+
+// c = inclusive scan of the starts: cell rank and brick of sorted key i
+__global__ void k_fill_bricks(const uint64_t *key, const unsigned long long *c, int64_t n, int low, uint64_t *bkey,
+                              unsigned long long *bmask, int32_t *bstart, int32_t *slot)
+{
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    if (i > 0 && c[i] == c[i - 1]) return;
+    const int64_t r = (int64_t)(c[i] & 0xffffffffull) - 1, b = (int64_t)(c[i] >> 32) - 1;
+    const int m = (int)((key[i] >> low) & 63);
+    slot[r] = (int32_t)(64 * b + m);
+    atomicOr(bmask + b, 1ull << m);
+    if (i == 0 || (c[i] >> 32) != (c[i - 1] >> 32)) {
+        bkey[b] = key[i] >> (low + 6);
+        bstart[b] = (int32_t)r;
+    }
+}
+
+__global__ void k_tag_cells(const uint64_t *raw, const uint8_t *set, int64_t nraw, const LevelMap map, uint32_t *tag,
+                            int8_t *bcidx)
 {
     int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nraw) return;
-    int64_t i = find_key(key, n, raw[j]);
+    int64_t i = map.find(raw[j]);
     if (i < 0) return;
     const uint8_t s = set[j];
     uint32_t bit;
@@ -39,34 +68,53 @@ __global__ void k_tag_cells(const uint64_t *raw, const uint8_t *set, int64_t nra
     atomicOr(&tag[i], bit);
 }
 
+// slot of the cell at key + e_k, or -1 (also for slots without a cell): from
+// the neighbour bricks where they are exact, else by the key of
+// Morton_Assist::find_neighbor
 template <int Q>
-__global__ void k_neighbors(MortonGeom g, int level, const uint64_t *key, int64_t n, int32_t *nbr)
+__global__ void k_neighbors(MortonGeom g, int level, const LevelMap map, const int32_t *__restrict__ bnbr, int64_t n,
+                            int32_t *nbr)
 {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint64_t k0 = key[i];
+    const int64_t b = i >> 6;
+    const int m = (int)(i & 63);
+    const bool here = (map.bmask[b] >> m) & 1;
+    const uint64_t k0 = map.key(i);
+    const int x = (m & 1) | ((m >> 2) & 2), y = ((m >> 1) & 1) | ((m >> 3) & 2), z = ((m >> 2) & 1) | ((m >> 4) & 2);
 #pragma unroll
     for (int k = 1; k < Q; ++k) {
-        const uint64_t nk = find_neighbor(g, k0, level, ex(k), ey(k), ez(k));
-        nbr[(int64_t)(k - 1) * n + i] = (int32_t)find_key(key, n, nk);
+        int32_t out = -1;
+        if (here && bnbr) {
+            const int nx = x + ex(k), ny = y + ey(k), nz = z + ez(k);
+            const int s = ((nx >> 2) + 1) + 3 * ((ny >> 2) + 1) + 9 * ((nz >> 2) + 1);
+            const int ax = nx & 3, ay = ny & 3, az = nz & 3;
+            const int mm = (ax & 1) | ((ax & 2) << 2) | ((ay & 1) << 1) | ((ay & 2) << 3) | ((az & 1) << 2) | ((az & 2) << 4);
+            const int32_t bb = __ldg(bnbr + 27 * b + s);
+            if (bb >= 0 && ((map.bmask[bb] >> mm) & 1)) out = 64 * bb + mm;
+        } else if (here) {
+            out = (int32_t)map.find(find_neighbor(g, k0, level, ex(k), ey(k), ez(k)));
+        }
+        nbr[(int64_t)(k - 1) * n + i] = out;
     }
 }
 
-__global__ void k_dis_rows(const uint64_t *key, int64_t n, const uint64_t *dkey, int64_t nd, int32_t *disrow,
-                           uint32_t *tag)
+__global__ void k_dis_rows(const LevelMap map, const int32_t *slot, int64_t nc, const uint64_t *dkey, int64_t nd,
+                           int32_t *disrow, uint32_t *tag)
 {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    int64_t r = find_key(dkey, nd, key[i]);
+    int64_t r0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r0 >= nc) return;
+    const int64_t i = slot[r0];
+    int64_t r = find_key(dkey, nd, map.key(i));
     disrow[i] = (int32_t)r;
     if (r >= 0) tag[i] |= TAG_IB;
 }
 
-__global__ void k_dis_check(const uint64_t *dkey, int64_t nd, const uint64_t *key, int64_t n, int *err)
+__global__ void k_dis_check(const uint64_t *dkey, int64_t nd, const LevelMap map, int *err)
 {
     int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (r >= nd) return;
-    if (find_key(key, n, dkey[r]) < 0) atomicOr(err, DEVERR_DIS_NOT_FINEST);
+    if (map.find(dkey[r]) < 0) atomicOr(err, DEVERR_DIS_NOT_FINEST);
 }
 
 // children of a coarse cell on the fine level, in the order of
@@ -90,17 +138,17 @@ MT_HD void children(const MortonGeom &g, uint64_t code, int fine, uint64_t *ch)
 // F2C sources need every child stored and skip children listed in dis;
 // ghost sources write only children in ghost_overlap_C2F and not in dis.
 __global__ void k_expl_children(MortonGeom g, int fine, const int32_t *src, int64_t nsrc, int64_t nf2c,
-                                const uint64_t *ckey, const uint64_t *fkey, const uint32_t *ftag, int64_t nf,
-                                const uint64_t *dkey, int64_t nd, int32_t *child, int *err)
+                                const LevelMap cmap, const LevelMap fmap, const uint32_t *ftag, const uint64_t *dkey, int64_t nd,
+                                int32_t *child, int *err)
 {
     int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nsrc) return;
     uint64_t ch[8];
-    children(g, ckey[src[j]], fine, ch);
+    children(g, cmap.key(src[j]), fine, ch);
     for (int m = 0; m < 8; ++m) {
         int32_t out = -1;
         const bool in_dis = find_key(dkey, nd, ch[m]) >= 0;
-        const int64_t fi = find_key(fkey, nf, ch[m]);
+        const int64_t fi = fmap.find(ch[m]);
         if (!in_dis) {
             if (j < nf2c) {
                 if (fi < 0)
@@ -115,64 +163,25 @@ __global__ void k_expl_children(MortonGeom g, int fine, const int32_t *src, int6
     }
 }
 
-__global__ void k_coal_children(MortonGeom g, int fine, const int32_t *src, int64_t nsrc, const uint64_t *ckey,
-                                const uint64_t *fkey, int64_t nf, int32_t *child, int *err)
+__global__ void k_coal_children(MortonGeom g, int fine, const int32_t *src, int64_t nsrc, const LevelMap cmap,
+                                const LevelMap fmap, int32_t *child, int *err)
 {
     int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nsrc) return;
     uint64_t ch[8];
-    children(g, ckey[src[j]], fine, ch);
+    children(g, cmap.key(src[j]), fine, ch);
     for (int m = 0; m < 8; ++m) {
-        const int64_t fi = find_key(fkey, nf, ch[m]);
+        const int64_t fi = fmap.find(ch[m]);
         if (fi < 0) atomicOr(err, DEVERR_MISSING_CHILD);
         child[(int64_t)m * nsrc + j] = (int32_t)fi;
     }
 }
 
-// ---- 4x4x4 bricks of a level (fused schedule) --------------------------------
-__global__ void k_brick_flags(const uint64_t *key, int64_t n, int shift, int32_t *flag)
+// ---- the fused pass's tables over a level's bricks -----------------------------
+__global__ void k_brick_cls(const uint32_t *tag, int64_t n, int ib_level, uint8_t *bcls)
 {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    flag[i] = (i == 0 || (key[i] >> shift) != (key[i - 1] >> shift)) ? 1 : 0;
-}
-
-// cell index at position h of brick b's 6x6x6 neighbourhood (local
-// coordinates h % 6 - 1, h / 6 % 6 - 1, h / 36 - 1), or -1
-__global__ void k_brick_halo(int64_t nb, const int32_t *bstart, const unsigned long long *bmask,
-                             const int32_t *bnbr, int32_t *halo)
-{
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= 216 * nb) return;
-    const int64_t b = t / 216;
-    const int h = (int)(t - 216 * b);
-    const int nx = h % 6 - 1, ny = (h / 6) % 6 - 1, nz = h / 36 - 1;
-    const int sl = ((nx >> 2) + 1) + 3 * ((ny >> 2) + 1) + 9 * ((nz >> 2) + 1);
-    const int ax = nx & 3, ay = ny & 3, az = nz & 3;
-    const int mm = (ax & 1) | ((ax & 2) << 2) | ((ay & 1) << 1) | ((ay & 2) << 3) | ((az & 1) << 2) | ((az & 2) << 4);
-    const int32_t s = bnbr[27 * b + sl];
-    int32_t out = -1;
-    if (s >= 0) {
-        const unsigned long long nm = bmask[s];
-        if ((nm >> mm) & 1ull) out = bstart[s] + __popcll(nm & ((1ull << mm) - 1ull));
-    }
-    halo[t] = out;
-}
-
-// cb = inclusive scan of the flags: brick of cell i is cb[i] - 1
-__global__ void k_brick_fill(const uint64_t *key, const uint32_t *tag, int64_t n, int shift, int low,
-                             const int32_t *cb, int ib_level, int32_t *bstart, uint64_t *bkey,
-                             unsigned long long *bmask, uint8_t *bcls)
-{
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int64_t b = cb[i] - 1;
-    const int m = (int)((key[i] >> low) & 63);
-    if (i == 0 || cb[i] != cb[i - 1]) {
-        bstart[b] = (int32_t)i;
-        bkey[b] = key[i] >> shift;
-    }
-    atomicOr(bmask + b, 1ull << m);
     const uint32_t t = tag[i];
     // stream covers lat_f then overlap_C2F, and a C2F cell's fcol = f copy
     // comes after the collision (Collision_Manager.cpp:45-52)
@@ -183,21 +192,42 @@ __global__ void k_brick_fill(const uint64_t *key, const uint32_t *tag, int64_t n
         cls = 4;  // direct-forcing band: stream only, collided after the forcing
     else if ((t & TAG_LATF) && !(ib_level && (t & TAG_IB)))
         cls = 1;
-    bcls[64 * b + m] = cls;
+    bcls[i] = cls;
 }
 
 // cells whose streamed f a coarser level's coalescence reads: stream +
 // collide with f stored (class 3)
-__global__ void k_brick_mark(const int32_t *child, int64_t count, const int32_t *cb, const uint64_t *key, int low,
-                             uint8_t *bcls)
+__global__ void k_brick_mark(const int32_t *child, int64_t count, uint8_t *bcls)
 {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= count) return;
     const int32_t ci = child[t];
-    if (ci < 0) return;
-    const int64_t b = cb[ci] - 1;
-    const int m = (int)((key[ci] >> low) & 63);
-    if (bcls[64 * b + m] == 1) bcls[64 * b + m] = 3;
+    if (ci >= 0 && bcls[ci] == 1) bcls[ci] = 3;
+}
+
+// one warp per brick, two cells per lane
+template <int Q>
+__global__ void k_brick_flag(int64_t nb, const uint8_t *__restrict__ bcls, const int32_t *__restrict__ nbr,
+                             uint8_t *bflag)
+{
+    const int64_t b = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (b >= nb) return;
+    const int lane = threadIdx.x & 31;
+    bool work = false, whole = true, one = true;
+    for (int h = 0; h < 2; ++h) {
+        const int64_t i = 64 * b + lane + 32 * h;
+        const int cls = bcls[i];
+        one &= cls == 1;
+        if (!cls) continue;
+        work = true;
+        for (int k = 1; k < Q; ++k) whole &= nbr[(int64_t)(k - 1) * (64 * nb) + i] >= 0;
+    }
+    const unsigned all = 0xffffffffu;
+    work = __any_sync(all, work);
+    whole = __all_sync(all, whole);
+    one = __all_sync(all, one);
+    if (lane == 0)
+        bflag[b] = (uint8_t)((work ? BRICK_WORK : 0) | (whole ? BRICK_COMPLETE : 0) | (one ? BRICK_UNIFORM : 0));
 }
 
 // neighbour bricks: Morton_Assist::find_neighbor applied to the corner cell
@@ -218,6 +248,10 @@ __global__ void k_brick_nbrs(MortonGeom g, int level, const uint64_t *bkey, int6
     bnbr[t] = (int32_t)find_key(bkey, nb, nk >> shift);
 }
 
+struct BrickHasWork {
+    const uint8_t *flag;
+    __host__ __device__ bool operator()(const int32_t &b) const { return (flag[b] & BRICK_WORK) != 0; }
+};
 struct TagHas {
     const uint32_t *tag;
     uint32_t bit;
@@ -298,11 +332,11 @@ static int build_level(Ctx &ctx, Case &c, int l)
     const int Q = c.d.q;
     const bool on_dev = lv.draw_keys != nullptr;
     const int64_t nraw = on_dev ? lv.ndraw : (int64_t)lv.raw_keys.size();
-    lv.n = 0;
+    lv.n = lv.ncell = lv.nbrick = 0;
     if (nraw > 0) {
         uint64_t *d_raw = nullptr, *d_sorted = nullptr;
         uint8_t *d_set = nullptr;
-        int *d_num = nullptr;
+        unsigned long long *d_start = nullptr, *d_scan = nullptr;
         if (on_dev) {
             d_raw = lv.draw_keys;
             d_set = lv.draw_set;
@@ -315,32 +349,58 @@ static int build_level(Ctx &ctx, Case &c, int l)
             MT_CUDA(ctx, cudaMemcpyAsync(d_raw, lv.raw_keys.data(), 8 * nraw, cudaMemcpyHostToDevice, ctx.stream));
             MT_CUDA(ctx, cudaMemcpyAsync(d_set, lv.raw_set.data(), nraw, cudaMemcpyHostToDevice, ctx.stream));
         }
+        lv.low = 3 * (c.d.max_level - l);
         MT_CUDA(ctx, cudaMallocAsync(&d_sorted, 8 * nraw, ctx.stream));
-        MT_CUDA(ctx, cudaMallocAsync(&d_num, sizeof(int), ctx.stream));
+        MT_CUDA(ctx, cudaMallocAsync(&d_start, 8 * nraw, ctx.stream));
+        MT_CUDA(ctx, cudaMallocAsync(&d_scan, 8 * nraw, ctx.stream));
         size_t t1 = 0, t2 = 0;
         MT_CUDA(ctx, cub::DeviceRadixSort::SortKeys(nullptr, t1, d_raw, d_sorted, (int)nraw, 0, 64, ctx.stream));
-        MT_CUDA(ctx, cudaMallocAsync(&lv.key, 8 * nraw, ctx.stream));
-        MT_CUDA(ctx, cub::DeviceSelect::Unique(nullptr, t2, d_sorted, lv.key, d_num, (int)nraw, ctx.stream));
+        MT_CUDA(ctx, cub::DeviceScan::InclusiveSum(nullptr, t2, d_start, d_scan, (int)nraw, ctx.stream));
         void *tmp = nullptr;
         MT_CUDA(ctx, cudaMallocAsync(&tmp, std::max(t1, t2), ctx.stream));
         MT_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, t1, d_raw, d_sorted, (int)nraw, 0, 64, ctx.stream));
-        MT_CUDA(ctx, cub::DeviceSelect::Unique(tmp, t2, d_sorted, lv.key, d_num, (int)nraw, ctx.stream));
-        int h_num = 0;
-        MT_CUDA(ctx, cudaMemcpyAsync(&h_num, d_num, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
+        k_starts<<<grid_for(nraw, 256), 256, 0, ctx.stream>>>(d_sorted, nraw, lv.low + 6, d_start);
+        MT_LAUNCHED(ctx);
+        MT_CUDA(ctx, cub::DeviceScan::InclusiveSum(tmp, t2, d_start, d_scan, (int)nraw, ctx.stream));
+        unsigned long long h_num = 0;
+        MT_CUDA(ctx, cudaMemcpyAsync(&h_num, d_scan + (nraw - 1), 8, cudaMemcpyDeviceToHost, ctx.stream));
         MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
-        lv.n = h_num;
+        const int64_t nc = (int64_t)(h_num & 0xffffffffull), nb = (int64_t)(h_num >> 32);
+        if (64 * nb >= ((int64_t)1 << 31))
+            return set_err(ctx, MT_ERR_MESH, "a level holds more than 2^31 cell slots (64 per 4x4x4 brick in use)");
+        lv.ncell = nc;
+        lv.nbrick = nb;
+        lv.n = 64 * nb;
         const int64_t n = lv.n;
+        MT_CUDA(ctx, cudaMallocAsync(&lv.slot, 4 * nc, ctx.stream));
+        MT_CUDA(ctx, cudaMallocAsync(&lv.bkey, 8 * nb, ctx.stream));
+        MT_CUDA(ctx, cudaMallocAsync(&lv.bmask, 8 * nb, ctx.stream));
+        MT_CUDA(ctx, cudaMallocAsync(&lv.bstart, 4 * nb, ctx.stream));
+        MT_CUDA(ctx, cudaMemsetAsync(lv.bmask, 0, 8 * nb, ctx.stream));
+        k_fill_bricks<<<grid_for(nraw, 256), 256, 0, ctx.stream>>>(d_sorted, d_scan, nraw, lv.low, lv.bkey,
+                                                                   (unsigned long long *)lv.bmask, lv.bstart, lv.slot);
+        MT_LAUNCHED(ctx);
         MT_CUDA(ctx, cudaMallocAsync(&lv.tag, 4 * n, ctx.stream));
         MT_CUDA(ctx, cudaMemsetAsync(lv.tag, 0, 4 * n, ctx.stream));
         MT_CUDA(ctx, cudaMallocAsync(&lv.bcidx, n, ctx.stream));
         MT_CUDA(ctx, cudaMemsetAsync(lv.bcidx, 0xff, n, ctx.stream));
-        k_tag_cells<<<grid_for(nraw, 256), 256, 0, ctx.stream>>>(d_raw, d_set, nraw, lv.key, n, lv.tag, lv.bcidx);
+        k_tag_cells<<<grid_for(nraw, 256), 256, 0, ctx.stream>>>(d_raw, d_set, nraw, lv.map(), lv.tag, lv.bcidx);
         MT_LAUNCHED(ctx);
+        // neighbour bricks, where the periodic wraps fall on brick boundaries
+        bool exact = true;
+        for (int a = 0; a < 3; ++a) exact &= !(c.d.periodic[a] && ((c.d.extent0[a] << l) % 4) != 0);
+        if (exact) {
+            MT_CUDA(ctx, cudaMallocAsync(&lv.bnbr, 4 * 27 * nb, ctx.stream));
+            k_brick_nbrs<<<grid_for(27 * nb, 256), 256, 0, ctx.stream>>>(c.geom, l, lv.bkey, nb, lv.low + 6, lv.low,
+                                                                         lv.bnbr);
+            MT_LAUNCHED(ctx);
+        }
         cudaFreeAsync(tmp, ctx.stream);
         cudaFreeAsync(d_raw, ctx.stream);
         cudaFreeAsync(d_sorted, ctx.stream);
+        cudaFreeAsync(d_start, ctx.stream);
+        cudaFreeAsync(d_scan, ctx.stream);
         cudaFreeAsync(d_set, ctx.stream);
-        cudaFreeAsync(d_num, ctx.stream);
     }
     const int64_t n = lv.n;
     if (n == 0) return MT_OK;
@@ -348,9 +408,9 @@ static int build_level(Ctx &ctx, Case &c, int l)
     MT_CUDA(ctx, cudaMemsetAsync(lv.disrow, 0xff, 4 * n, ctx.stream));
     MT_CUDA(ctx, cudaMallocAsync(&lv.nbr, 4 * n * (Q - 1), ctx.stream));
     if (Q == 19)
-        k_neighbors<19><<<grid_for(n, 128), 128, 0, ctx.stream>>>(c.geom, l, lv.key, n, lv.nbr);
+        k_neighbors<19><<<grid_for(n, 128), 128, 0, ctx.stream>>>(c.geom, l, lv.map(), lv.bnbr, n, lv.nbr);
     else
-        k_neighbors<27><<<grid_for(n, 128), 128, 0, ctx.stream>>>(c.geom, l, lv.key, n, lv.nbr);
+        k_neighbors<27><<<grid_for(n, 128), 128, 0, ctx.stream>>>(c.geom, l, lv.map(), lv.bnbr, n, lv.nbr);
     MT_LAUNCHED(ctx);
     {
         int rc = amr_dispatch(c, [&](auto *tag) {
@@ -405,10 +465,11 @@ int amr_build(Ctx &ctx, Case &c)
         }
         Level &fl = c.lv[L];
         if (fl.n > 0) {
-            k_dis_rows<<<grid_for(fl.n, 256), 256, 0, ctx.stream>>>(fl.key, fl.n, c.dis_key, c.ndis, fl.disrow, fl.tag);
+            k_dis_rows<<<grid_for(fl.ncell, 256), 256, 0, ctx.stream>>>(fl.map(), fl.slot, fl.ncell, c.dis_key, c.ndis,
+                                                                        fl.disrow, fl.tag);
             MT_LAUNCHED(ctx);
         }
-        k_dis_check<<<grid_for(c.ndis, 256), 256, 0, ctx.stream>>>(c.dis_key, c.ndis, fl.key, fl.n, c.dev_err);
+        k_dis_check<<<grid_for(c.ndis, 256), 256, 0, ctx.stream>>>(c.dis_key, c.ndis, fl.map(), c.dev_err);
         MT_LAUNCHED(ctx);
         int rc = select_indices(ctx, fl.n, IbLatf{fl.tag}, &fl.iblist, &fl.nib);
         if (rc) return rc;
@@ -469,14 +530,14 @@ int amr_build(Ctx &ctx, Case &c)
         if (fl.nexpl) {
             MT_CUDA(ctx, cudaMallocAsync(&fl.expl_child, 4 * 8 * fl.nexpl, ctx.stream));
             k_expl_children<<<grid_for(fl.nexpl, 128), 128, 0, ctx.stream>>>(
-                c.geom, l, fl.expl_src, fl.nexpl, fl.nexpl_f2c, cl.key, fl.key, fl.tag, fl.n, c.dis_key, c.ndis,
+                c.geom, l, fl.expl_src, fl.nexpl, fl.nexpl_f2c, cl.map(), fl.map(), fl.tag, c.dis_key, c.ndis,
                 fl.expl_child, c.dev_err);
             MT_LAUNCHED(ctx);
         }
         if (cl.nlist[1]) {
             MT_CUDA(ctx, cudaMallocAsync(&cl.coal_child, 4 * 8 * cl.nlist[1], ctx.stream));
             k_coal_children<<<grid_for(cl.nlist[1], 128), 128, 0, ctx.stream>>>(
-                c.geom, l, cl.list[1], cl.nlist[1], cl.key, fl.key, fl.n, cl.coal_child, c.dev_err);
+                c.geom, l, cl.list[1], cl.nlist[1], cl.map(), fl.map(), cl.coal_child, c.dev_err);
             MT_LAUNCHED(ctx);
         }
     }
@@ -504,17 +565,15 @@ void amr_drop_fused(Case &c)
     }
     for (int l = 0; l < kMaxLevels; ++l) {
         Level &lv = c.lv[l];
-        void *ptrs[] = {lv.fused_list, lv.bstart, lv.bmask, lv.bnbr, lv.bcls, lv.bhalo};
+        void *ptrs[] = {lv.fused_list, lv.bcls, lv.bflag, lv.blist};
         for (void *p : ptrs)
             if (p) cudaFree(p);
         lv.fused_list = nullptr;
         lv.nfused = 0;
-        lv.bstart = nullptr;
-        lv.bmask = nullptr;
-        lv.bnbr = nullptr;
         lv.bcls = nullptr;
-        lv.bhalo = nullptr;
-        lv.nbrick = 0;
+        lv.bflag = nullptr;
+        lv.blist = nullptr;
+        lv.nblist = 0;
         lv.bricks = false;
     }
 }
@@ -523,9 +582,9 @@ void amr_free(Case &c)
 {
     for (int l = 0; l < kMaxLevels; ++l) {
         Level &lv = c.lv[l];
-        void *ptrs[] = {lv.key, lv.tag, lv.bcidx, lv.disrow, lv.nbr, lv.f, lv.fcol, lv.rho, lv.u,
+        void *ptrs[] = {lv.slot, lv.bkey, lv.tag, lv.bcidx, lv.disrow, lv.nbr, lv.f, lv.fcol, lv.rho, lv.u,
                         lv.collide_list, lv.stream_list, lv.iblist, lv.expl_src, lv.expl_child, lv.coal_child,
-                        lv.fcol_alt, lv.fused_list, lv.bstart, lv.bmask, lv.bnbr, lv.bcls, lv.bhalo,
+                        lv.fcol_alt, lv.fused_list, lv.bstart, lv.bmask, lv.bnbr, lv.bcls, lv.bflag, lv.blist,
                         lv.band, lv.collide_nb, lv.draw_keys, lv.draw_set, lv.expl_prev, lv.info_prev};
         for (void *p : ptrs)
             if (p) cudaFree(p);
@@ -714,61 +773,30 @@ static int record_fused_step(Ctx &ctx, Case &c)
     return MT_OK;
 }
 
-// Bricks of level l, when they reproduce the neighbour table exactly: every
-// periodic axis spans a multiple of 4 cells at this level (the wrap then
-// falls on a brick boundary).
+// The fused pass's tables of level l, where the neighbour bricks are exact.
 static int build_bricks(Ctx &ctx, Case &c, int l)
 {
     Level &lv = c.lv[l];
     const int L = c.d.max_level;
-    for (int a = 0; a < 3; ++a)
-        if (c.d.periodic[a] && ((c.d.extent0[a] << l) % 4) != 0) return MT_OK;
-    const int64_t n = lv.n;
+    const int64_t n = lv.n, nb = lv.nbrick;
+    if (!lv.bnbr) return MT_OK;
     if (n * c.d.q >= ((int64_t)1 << 32)) return MT_OK;  // the brick pass uses 32-bit element offsets
-    const int low = 3 * (L - l), shift = low + 6;
-    int32_t *flag = nullptr, *cb = nullptr;
-    MT_CUDA(ctx, cudaMallocAsync(&flag, 4 * n, ctx.stream));
-    MT_CUDA(ctx, cudaMallocAsync(&cb, 4 * n, ctx.stream));
-    k_brick_flags<<<grid_for(n, 256), 256, 0, ctx.stream>>>(lv.key, n, shift, flag);
-    MT_LAUNCHED(ctx);
-    size_t tb = 0;
-    MT_CUDA(ctx, cub::DeviceScan::InclusiveSum(nullptr, tb, flag, cb, (int)n, ctx.stream));
-    void *tmp = nullptr;
-    MT_CUDA(ctx, cudaMallocAsync(&tmp, tb, ctx.stream));
-    MT_CUDA(ctx, cub::DeviceScan::InclusiveSum(tmp, tb, flag, cb, (int)n, ctx.stream));
-    int32_t nb = 0;
-    MT_CUDA(ctx, cudaMemcpyAsync(&nb, cb + (n - 1), 4, cudaMemcpyDeviceToHost, ctx.stream));
-    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
-    uint64_t *bkey = nullptr;
-    MT_CUDA(ctx, cudaMallocAsync(&lv.bstart, 4 * (size_t)nb, ctx.stream));
-    MT_CUDA(ctx, cudaMallocAsync(&lv.bmask, 8 * (size_t)nb, ctx.stream));
-    MT_CUDA(ctx, cudaMallocAsync(&lv.bnbr, 4 * 27 * (size_t)nb, ctx.stream));
-    MT_CUDA(ctx, cudaMallocAsync(&lv.bcls, 64 * (size_t)nb, ctx.stream));
-    MT_CUDA(ctx, cudaMallocAsync(&bkey, 8 * (size_t)nb, ctx.stream));
-    MT_CUDA(ctx, cudaMemsetAsync(lv.bmask, 0, 8 * (size_t)nb, ctx.stream));
-    MT_CUDA(ctx, cudaMemsetAsync(lv.bcls, 0, 64 * (size_t)nb, ctx.stream));
+    MT_CUDA(ctx, cudaMallocAsync(&lv.bcls, n, ctx.stream));
+    MT_CUDA(ctx, cudaMallocAsync(&lv.bflag, nb, ctx.stream));
     const int ib_level = (l == L && l > 0) ? 1 : 0;
-    k_brick_fill<<<grid_for(n, 256), 256, 0, ctx.stream>>>(lv.key, lv.tag, n, shift, low, cb, ib_level, lv.bstart,
-                                                           bkey, (unsigned long long *)lv.bmask, lv.bcls);
+    k_brick_cls<<<grid_for(n, 256), 256, 0, ctx.stream>>>(lv.tag, n, ib_level, lv.bcls);
     MT_LAUNCHED(ctx);
     if (l > 0 && c.lv[l - 1].coal_child && c.lv[l - 1].nlist[1]) {
         const int64_t cnt = 8 * c.lv[l - 1].nlist[1];
-        k_brick_mark<<<grid_for(cnt, 256), 256, 0, ctx.stream>>>(c.lv[l - 1].coal_child, cnt, cb, lv.key, low,
-                                                                 lv.bcls);
+        k_brick_mark<<<grid_for(cnt, 256), 256, 0, ctx.stream>>>(c.lv[l - 1].coal_child, cnt, lv.bcls);
         MT_LAUNCHED(ctx);
     }
-    k_brick_nbrs<<<grid_for(27 * (int64_t)nb, 256), 256, 0, ctx.stream>>>(c.geom, l, bkey, nb, shift, low, lv.bnbr);
+    if (c.d.q == 19)
+        k_brick_flag<19><<<grid_for(32 * nb, 128), 128, 0, ctx.stream>>>(nb, lv.bcls, lv.nbr, lv.bflag);
+    else
+        k_brick_flag<27><<<grid_for(32 * nb, 128), 128, 0, ctx.stream>>>(nb, lv.bcls, lv.nbr, lv.bflag);
     MT_LAUNCHED(ctx);
-    MT_CUDA(ctx, cudaMallocAsync(&lv.bhalo, 4 * 216 * (size_t)nb, ctx.stream));
-    k_brick_halo<<<grid_for(216 * (int64_t)nb, 256), 256, 0, ctx.stream>>>(nb, lv.bstart,
-                                                                          (const unsigned long long *)lv.bmask,
-                                                                          lv.bnbr, lv.bhalo);
-    MT_LAUNCHED(ctx);
-    cudaFreeAsync(tmp, ctx.stream);
-    cudaFreeAsync(flag, ctx.stream);
-    cudaFreeAsync(cb, ctx.stream);
-    cudaFreeAsync(bkey, ctx.stream);
-    lv.nbrick = nb;
+    if (int rc = select_indices(ctx, nb, BrickHasWork{lv.bflag}, &lv.blist, &lv.nblist)) return rc;
     lv.bricks = true;
     return MT_OK;
 }
@@ -959,7 +987,7 @@ int batch_bricks(Ctx &ctx, BatchRec &R, const std::vector<Case *> &cs, int l, co
     };
     std::vector<std::vector<Case *>> groups;
     for (Case *c : cs) {
-        if (!c->lv[l].bricks || c->lv[l].nbrick >= kBatchOwnBricks) continue;
+        if (!c->lv[l].bricks || c->lv[l].nblist >= kBatchOwnBricks) continue;
         bool placed = false;
         for (auto &g : groups)
             if (g[0]->d.q == c->d.q && g[0]->d.collision == c->d.collision &&
@@ -980,8 +1008,11 @@ int batch_bricks(Ctx &ctx, BatchRec &R, const std::vector<Case *> &cs, int l, co
                 Case &c = *g[k];
                 Level &lv = c.lv[l];
                 BrickSlot &sl = d.slot[d.nslots];
-                sl.halo = lv.bhalo;
+                sl.list = lv.blist;
+                sl.nbr = lv.bnbr;
+                sl.mask = (const unsigned long long *)lv.bmask;
                 sl.cls = lv.bcls;
+                sl.flag = lv.bflag;
                 sl.fcol = lv.fcol;
                 sl.f = lv.f;
                 sl.fnext = lv.fcol_alt;
@@ -993,7 +1024,7 @@ int batch_bricks(Ctx &ctx, BatchRec &R, const std::vector<Case *> &cs, int l, co
                 sl.fall = (l == 0 && c.d.bc_mode == MT_BC_NEQ) ? 1 : 0;
                 sl.macros = c.macros_now;
                 sl.acc = (l == c.d.max_level && lv.nband) ? c.acc : nullptr;
-                d.off[d.nslots + 1] = d.off[d.nslots] + lv.nbrick;
+                d.off[d.nslots + 1] = d.off[d.nslots] + lv.nblist;
                 ++d.nslots;
             }
             d.total = d.off[d.nslots];
@@ -1036,7 +1067,7 @@ int batch_lbm_kernel(Ctx &ctx, BatchRec &R, const std::vector<Case *> &all, int 
             Batch &B = *R.b;
             cudaStream_t main = ctx.stream;
             std::vector<Case *> own;
-            auto batched = [&](const Case *c) { return c->lv[l].bricks && c->lv[l].nbrick < kBatchOwnBricks; };
+            auto batched = [&](const Case *c) { return c->lv[l].bricks && c->lv[l].nblist < kBatchOwnBricks; };
             for (Case *c : cs)
                 if (!batched(c) || (l == c->d.max_level && l > 0)) own.push_back(c);
             const int P = (int)std::min<size_t>(B.pool.size(), own.size());
@@ -1256,7 +1287,7 @@ int amr_get(Ctx &ctx, Case &c, int level, double *h_f, double *h_fcol)
     if (int rc = amr_sync_f(ctx, c)) return rc;
     Level &lv = c.lv[level];
     if (!lv.n) return MT_OK;
-    const size_t nb = sizeof(double) * (size_t)c.d.q * (size_t)lv.n;
+    const size_t nb = sizeof(double) * (size_t)c.d.q * (size_t)lv.ncell;
     double *d = nullptr;
     MT_CUDA(ctx, cudaMallocAsync(&d, nb, ctx.stream));
     int rc = MT_OK;
@@ -1280,7 +1311,7 @@ int amr_set(Ctx &ctx, Case &c, int level, const double *h_f, const double *h_fco
     c.prev_stale = true;
     Level &lv = c.lv[level];
     if (!lv.n) return MT_OK;
-    const size_t nb = sizeof(double) * (size_t)c.d.q * (size_t)lv.n;
+    const size_t nb = sizeof(double) * (size_t)c.d.q * (size_t)lv.ncell;
     double *d = nullptr;
     MT_CUDA(ctx, cudaMallocAsync(&d, nb, ctx.stream));
     int rc = MT_OK;
@@ -1303,24 +1334,122 @@ int amr_macros(Ctx &ctx, Case &c, int level, double *h_rho, double *h_u)
     Level &lv = c.lv[level];
     if (!lv.n) return MT_OK;
     double *d = nullptr;
-    MT_CUDA(ctx, cudaMallocAsync(&d, sizeof(double) * 4 * lv.n, ctx.stream));
+    MT_CUDA(ctx, cudaMallocAsync(&d, sizeof(double) * 4 * lv.ncell, ctx.stream));
     int rc = amr_dispatch(c, [&](auto *tag) {
         using S = std::remove_pointer_t<decltype(tag)>;
-        return AmrOps<S>::macros_out(ctx, c, level, d, d + lv.n);
+        return AmrOps<S>::macros_out(ctx, c, level, d, d + lv.ncell);
     });
     if (!rc) {
-        if (h_rho) MT_CUDA(ctx, cudaMemcpyAsync(h_rho, d, sizeof(double) * lv.n, cudaMemcpyDeviceToHost, ctx.stream));
-        if (h_u) MT_CUDA(ctx, cudaMemcpyAsync(h_u, d + lv.n, sizeof(double) * 3 * lv.n, cudaMemcpyDeviceToHost, ctx.stream));
+        if (h_rho) MT_CUDA(ctx, cudaMemcpyAsync(h_rho, d, sizeof(double) * lv.ncell, cudaMemcpyDeviceToHost, ctx.stream));
+        if (h_u) MT_CUDA(ctx, cudaMemcpyAsync(h_u, d + lv.ncell, sizeof(double) * 3 * lv.ncell, cudaMemcpyDeviceToHost, ctx.stream));
     }
     MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
     cudaFreeAsync(d, ctx.stream);
     return rc;
 }
 
-__global__ void k_find(const uint64_t *key, int64_t n, const uint64_t *q, int64_t nq, int64_t *out)
+// rank (position in key order) of a slot
+__device__ __forceinline__ int64_t rank_of(const LevelMap &map, const int32_t *bstart, int64_t i)
+{
+    const unsigned long long m = map.bmask[i >> 6];
+    return bstart[i >> 6] + __popcll(m & ((1ull << (i & 63)) - 1ull));
+}
+
+__global__ void k_find(const LevelMap map, const int32_t *bstart, const uint64_t *q, int64_t nq, int64_t *out)
 {
     int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j < nq) out[j] = find_key(key, n, q[j]);
+    if (j >= nq) return;
+    const int64_t i = map.find(q[j]);
+    out[j] = i < 0 ? -1 : rank_of(map, bstart, i);
+}
+
+// keys and tags of a level's cells in key order
+__global__ void k_cells_out(const LevelMap map, const int32_t *slot, const uint32_t *tag, int64_t nc, uint64_t *key,
+                            uint32_t *tg)
+{
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= nc) return;
+    const int64_t i = slot[r];
+    key[r] = map.key(i);
+    tg[r] = tag[i];
+}
+
+// the neighbour table by ranks
+__global__ void k_nbr_out(const LevelMap map, const int32_t *bstart, const int32_t *slot, int64_t nc, const int32_t *nbr,
+                          int links, int32_t *out)
+{
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= nc) return;
+    const int64_t i = slot[r], n = 64 * map.nb;
+    for (int k = 0; k < links; ++k) {
+        const int32_t j = nbr[k * n + i];
+        out[k * nc + r] = j < 0 ? -1 : (int32_t)rank_of(map, bstart, j);
+    }
+}
+
+// rows of 64-bit values between slots and key order
+__global__ void k_rows_move(const int32_t *slot, int64_t nc, int64_t n, int rows, long long *by_slot, long long *by_rank,
+                            int to_rank)
+{
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= nc) return;
+    const int64_t i = slot[r];
+    for (int a = 0; a < rows; ++a) {
+        if (to_rank)
+            by_rank[a * nc + r] = by_slot[a * n + i];
+        else
+            by_slot[a * n + i] = by_rank[a * nc + r];
+    }
+}
+
+int amr_get_keys(Ctx &ctx, Case &c, int level, uint64_t *h_keys, uint32_t *h_tags)
+{
+    Level &lv = c.lv[level];
+    const int64_t nc = lv.ncell;
+    if (!nc) return MT_OK;
+    uint64_t *d = nullptr;
+    MT_CUDA(ctx, cudaMallocAsync(&d, 12 * nc, ctx.stream));
+    uint32_t *t = (uint32_t *)(d + nc);
+    k_cells_out<<<grid_for(nc, 256), 256, 0, ctx.stream>>>(lv.map(), lv.slot, lv.tag, nc, d, t);
+    MT_LAUNCHED(ctx);
+    if (h_keys) MT_CUDA(ctx, cudaMemcpyAsync(h_keys, d, 8 * nc, cudaMemcpyDeviceToHost, ctx.stream));
+    if (h_tags) MT_CUDA(ctx, cudaMemcpyAsync(h_tags, t, 4 * nc, cudaMemcpyDeviceToHost, ctx.stream));
+    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
+    cudaFreeAsync(d, ctx.stream);
+    return MT_OK;
+}
+
+int amr_get_neighbors(Ctx &ctx, Case &c, int level, int32_t *h_nbr)
+{
+    Level &lv = c.lv[level];
+    const int64_t nc = lv.ncell;
+    const int links = c.d.q - 1;
+    if (!nc) return MT_OK;
+    int32_t *d = nullptr;
+    MT_CUDA(ctx, cudaMallocAsync(&d, 4 * nc * links, ctx.stream));
+    k_nbr_out<<<grid_for(nc, 256), 256, 0, ctx.stream>>>(lv.map(), lv.bstart, lv.slot, nc, lv.nbr, links, d);
+    MT_LAUNCHED(ctx);
+    MT_CUDA(ctx, cudaMemcpyAsync(h_nbr, d, 4 * nc * links, cudaMemcpyDeviceToHost, ctx.stream));
+    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
+    cudaFreeAsync(d, ctx.stream);
+    return MT_OK;
+}
+
+int amr_df_force_field(Ctx &ctx, Case &c, int64_t *h, bool get)
+{
+    Level &lv = c.lv[c.d.max_level];
+    const int64_t nc = lv.ncell;
+    if (!nc) return MT_OK;
+    const size_t bytes = sizeof(long long) * 3 * (size_t)nc;
+    long long *d = nullptr;
+    MT_CUDA(ctx, cudaMallocAsync(&d, bytes, ctx.stream));
+    if (!get) MT_CUDA(ctx, cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, ctx.stream));
+    k_rows_move<<<grid_for(nc, 256), 256, 0, ctx.stream>>>(lv.slot, nc, lv.n, 3, c.acc, d, get ? 1 : 0);
+    MT_LAUNCHED(ctx);
+    if (get) MT_CUDA(ctx, cudaMemcpyAsync(h, d, bytes, cudaMemcpyDeviceToHost, ctx.stream));
+    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
+    cudaFreeAsync(d, ctx.stream);
+    return MT_OK;
 }
 
 int amr_find(Ctx &ctx, Case &c, int level, const uint64_t *h_keys, int64_t nq, int64_t *h_idx)
@@ -1332,7 +1461,7 @@ int amr_find(Ctx &ctx, Case &c, int level, const uint64_t *h_keys, int64_t nq, i
     MT_CUDA(ctx, cudaMallocAsync(&dq, 8 * nq, ctx.stream));
     MT_CUDA(ctx, cudaMallocAsync(&dout, 8 * nq, ctx.stream));
     MT_CUDA(ctx, cudaMemcpyAsync(dq, h_keys, 8 * nq, cudaMemcpyHostToDevice, ctx.stream));
-    k_find<<<grid_for(nq, 256), 256, 0, ctx.stream>>>(lv.key, lv.n, dq, nq, dout);
+    k_find<<<grid_for(nq, 256), 256, 0, ctx.stream>>>(lv.map(), lv.bstart, dq, nq, dout);
     MT_LAUNCHED(ctx);
     MT_CUDA(ctx, cudaMemcpyAsync(h_idx, dout, 8 * nq, cudaMemcpyDeviceToHost, ctx.stream));
     MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));

@@ -39,8 +39,8 @@ __global__ void k_init_eq(int64_t n, const uint32_t *tag, double rho0, double ux
     for (int k = 0; k < Q; ++k) {
         const double v = solid ? 0. : feq_ref<Q>(k, rho0, ux, uy, uz);
         const C s = stored_f64<S>(sh, v, k);
-        T::st(f, k * n + i, s);
-        T::st(fcol, k * n + i, s);
+        T::st(f, at<Q>(k, i), s);
+        T::st(fcol, at<Q>(k, i), s);
     }
     rho[i] = (C)(solid ? 1. : rho0);
     u[i] = (C)(solid ? 0. : ux);
@@ -60,7 +60,7 @@ __global__ void k_macros(const int32_t *list, int64_t nl, int64_t n, const S *f,
     const int64_t i = list[j];
     C d[Q];
 #pragma unroll
-    for (int k = 0; k < Q; ++k) d[k] = full_sh<S>(sh, T::ld(f, k * n + i), k);
+    for (int k = 0; k < Q; ++k) d[k] = full_sh<S>(sh, T::ld(f, at<Q>(k, i)), k);
     C r, x, y, z;
     macros_g<Q, C>(d, r, x, y, z);
     rho[i] = r;
@@ -69,66 +69,43 @@ __global__ void k_macros(const int32_t *list, int64_t nl, int64_t n, const S *f,
     u[2 * n + i] = z;
 }
 
-// post-collision populations of one cell from its f (already in the compute
-// type C) and its macros: Collision_LBGK::collide (Collision_Manager.cpp:13-53)
-// or Collision_Cumulant::collide (Collision_Cumulant.cpp:22-159), stored into
-// fcol[k * n + i].  Shared by the phase kernel and the fused pull + collide
-// kernels so both schedules run the same arithmetic.
-template <int Q, class S, int COLL, class I = int64_t>
-__device__ __forceinline__ void collide_store(const typename Store<S>::C *d, typename Store<S>::C r,
-                                              typename Store<S>::C x, typename Store<S>::C y,
-                                              typename Store<S>::C z, double tau, S *fcol, I n, I i, const Shift &sh)
-{
-    using T = Store<S>;
-    using C = typename T::C;
-    if constexpr (COLL == MT_COLL_LBGK) {
-        if constexpr (!T::shifted) {
-#pragma unroll
-            for (int k = 0; k < Q; ++k) {
-                const double fk = d[k];
-                fcol[(I)k * n + i] = fk - (fk - feq_ref<Q>(k, r, x, y, z)) / tau;
-            }
-        } else {
-            const float om = (float)(1.0 / tau);
-            const float uu = 1.5f * (x * x + y * y + z * z);
-#pragma unroll
-            for (int k = 0; k < Q; ++k) {
-                const float eu = ex(k) * x + ey(k) * y + ez(k) * z;
-                const float wk = (float)w<Q>(k);
-                // deviations from the shift s_k = w_k + dw_k:
-                // feq - s = w ((rho - 1) + rho (3 eu + 4.5 eu^2 - 1.5 u^2)) - dw
-                const float dfeq = wk * ((r - 1.f) + r * (3.f * eu + 4.5f * eu * eu - uu)) - sh.dw[k];
-                const float s = d[k] - sh.v[k];
-                T::st(fcol, (I)k * n + i, fmaf(om, dfeq - s, s));
-            }
-        }
-    } else if constexpr (Q == 27) {
-        C o[27];
-        cumulant_collide<C>(d, r, x, y, z, (C)(1. / tau), o);
-#pragma unroll
-        for (int k = 0; k < 27; ++k) T::st(fcol, (I)k * n + i, stored_sh<S>(sh, o[k], k));
-    }
-}
-
-// The macros of d (rho, u into r, x, y, z) and its collision stored into
-// out: the reduced-precision D3Q27 cumulant takes the macros from the
-// collision's own first chimera pass (cumulant_macros_collide); every other
-// form computes them with macros_g and then collides (collide_store).
+// The macros (rho, u into r, x, y, z) of one cell from its stored values d (in
+// the compute type; overwritten) and its post-collision populations into
+// out[at(k, i)]: LBM_Manager::calculateMacros with Collision_LBGK::collide
+// (Collision_Manager.cpp:13-53) or Collision_Cumulant::collide
+// (Collision_Cumulant.cpp:22-159).  Shared by every kernel that collides one
+// cell; the reduced storages run the arithmetic of the packed pairs
+// (mt_pack2.cuh), so a cell's result does not depend on the kernel.
 template <int Q, class S, int COLL, class I>
-__device__ __forceinline__ void macros_collide_store(const typename Store<S>::C *d, typename Store<S>::C &r,
+__device__ __forceinline__ void macros_collide_store(typename Store<S>::C *d, typename Store<S>::C &r,
                                                      typename Store<S>::C &x, typename Store<S>::C &y,
-                                                     typename Store<S>::C &z, double tau, S *out, I n, I i,
+                                                     typename Store<S>::C &z, double tau, S *out, I i,
                                                      const Shift &sh)
 {
     using T = Store<S>;
-    if constexpr (COLL == MT_COLL_CUMULANT && Q == 27 && T::shifted) {
-        float o[27];
-        cumulant_macros_collide(d, r, x, y, z, (float)(1. / tau), o);
+    if constexpr (T::shifted) {
+        const float om = (float)(1.0 / tau);
+        if constexpr (COLL == MT_COLL_LBGK) {
+            p2::lbgk<Q, float>(d, r, x, y, z, om, sh);
+        } else {
+            p2::cumulant<float, false>(d, r, x, y, z, om, sh);
+        }
 #pragma unroll
-        for (int k = 0; k < 27; ++k) T::st(out, (I)k * n + i, stored_sh<S>(sh, o[k], k));
+        for (int k = 0; k < Q; ++k) T::st(out, at<Q>(k, i), d[k]);
     } else {
-        macros_g<Q, typename T::C>(d, r, x, y, z);
-        collide_store<Q, S, COLL>(d, r, x, y, z, tau, out, n, i, sh);
+        macros_g<Q, double>(d, r, x, y, z);
+        if constexpr (COLL == MT_COLL_LBGK) {
+#pragma unroll
+            for (int k = 0; k < Q; ++k) {
+                const double fk = d[k];
+                out[at<Q>(k, i)] = fk - (fk - feq_ref<Q>(k, r, x, y, z)) / tau;
+            }
+        } else if constexpr (Q == 27) {
+            double o[27];
+            cumulant_collide<double>(d, r, x, y, z, 1. / tau, o);
+#pragma unroll
+            for (int k = 0; k < 27; ++k) out[at<Q>(k, i)] = o[k];
+        }
     }
 }
 
@@ -145,14 +122,13 @@ __global__ void k_collide(const int32_t *list, int64_t nl, int64_t n, double tau
     const int64_t i = list[j];
     C d[Q];
 #pragma unroll
-    for (int k = 0; k < Q; ++k) d[k] = full_sh<S>(sh, T::ld(f, k * n + i), k);
+    for (int k = 0; k < Q; ++k) d[k] = T::ld(f, at<Q>(k, i));
     C r, x, y, z;
-    macros_collide_store<Q, S, COLL>(d, r, x, y, z, tau, fcol, n, i, sh);
+    macros_collide_store<Q, S, COLL>(d, r, x, y, z, tau, fcol, i, sh);
     rho[i] = r;
     u[i] = x;
     u[n + i] = y;
     u[2 * n + i] = z;
-    
 }
 
 // fcol = f on overlap_C2F (Collision_Manager.cpp:45-52)
@@ -163,7 +139,7 @@ __global__ void k_copy_fcol(const int32_t *list, int64_t nl, int64_t n, const S 
     if (j >= nl) return;
     const int64_t i = list[j];
 #pragma unroll
-    for (int k = 0; k < Q; ++k) fcol[k * n + i] = f[k * n + i];
+    for (int k = 0; k < Q; ++k) fcol[at<Q>(k, i)] = f[at<Q>(k, i)];
 }
 
 // ABPatternPull::stream (Stream_Manager.cpp:43-76): a missing neighbour keeps f
@@ -174,12 +150,12 @@ __global__ void k_stream(const int32_t *list, int64_t nl, int64_t n, int textboo
     const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nl) return;
     const int64_t i = list[j];
-    f[i] = fcol[i];
+    f[at<Q>(0, i)] = fcol[at<Q>(0, i)];
 #pragma unroll
     for (int k = 1; k < Q; ++k) {
         const int kk = textbook ? inv(k) : k;
         const int32_t s = nbr[(int64_t)(kk - 1) * n + i];
-        if (s >= 0) f[k * n + i] = fcol[k * n + s];
+        if (s >= 0) f[at<Q>(k, i)] = fcol[at<Q>(k, s)];
     }
 }
 
@@ -210,7 +186,7 @@ __global__ void k_explosion(const int32_t *__restrict__ src, const int32_t *__re
     const int64_t i = src[j];
     C d[Q];
 #pragma unroll
-    for (int k = 0; k < Q; ++k) d[k] = full_sh<S>(csh, T::ld(cfcol, k * nc + i), k);
+    for (int k = 0; k < Q; ++k) d[k] = full_sh<S>(csh, T::ld(cfcol, at<Q>(k, i)), k);
     if (cprev) {
 #pragma unroll
         for (int k = 0; k < Q; ++k) d[k] = C(1.5) * d[k] - C(0.5) * full_sh<S>(csh, T::ld(cprev, k * ns + j), k);
@@ -222,8 +198,8 @@ __global__ void k_explosion(const int32_t *__restrict__ src, const int32_t *__re
     for (int k = 0; k < Q; ++k) {
         const C fe = feq_heluo_g<Q, C>(k, r, x, y, z);
         const C v = stored_sh<S>(fsh, fe + (C)scale * (d[k] - fe), k);
-        T::st(ffcol, k * nf + ch, v);
-        if (both) T::st(ffcol2, k * nf + ch, v);
+        T::st(ffcol, at<Q>(k, ch), v);
+        if (both) T::st(ffcol2, at<Q>(k, ch), v);
     }
 }
 
@@ -236,7 +212,7 @@ __global__ void k_expl_save(const int32_t *__restrict__ src, int64_t ns, const S
     if (j >= ns) return;
     const int64_t i = src[j];
 #pragma unroll
-    for (int k = 0; k < Q; ++k) prev[k * ns + j] = cfcol[k * nc + i];
+    for (int k = 0; k < Q; ++k) prev[k * ns + j] = cfcol[at<Q>(k, i)];
 }
 
 // AMR_transDDF_coalescence (LBM_Manager.cpp:1131-1169)
@@ -257,7 +233,7 @@ __global__ void k_coalescence(const int32_t *list, const int32_t *child, int64_t
     for (int k = 0; k < Q; ++k) {
         C s = 0;
 #pragma unroll
-        for (int m = 0; m < 8; ++m) s += full_sh<S>(fsh, T::ld(ff, k * nf + ch[m]), k);
+        for (int m = 0; m < 8; ++m) s += full_sh<S>(fsh, T::ld(ff, at<Q>(k, ch[m])), k);
         a[k] = s / (C)8.0;
     }
     C r, x, y, z;
@@ -265,7 +241,7 @@ __global__ void k_coalescence(const int32_t *list, const int32_t *child, int64_t
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
         const C fe = feq_heluo_g<Q, C>(k, r, x, y, z);
-        T::st(cf, k * nc + i, stored_sh<S>(csh, fe + (C)scale * (a[k] - fe), k));
+        T::st(cf, at<Q>(k, i), stored_sh<S>(csh, fe + (C)scale * (a[k] - fe), k));
     }
 }
 
@@ -294,7 +270,7 @@ __global__ void k_coal_collide(const int32_t *__restrict__ list, const int32_t *
     for (int k = 0; k < Q; ++k) {
         C s = 0;
 #pragma unroll
-        for (int m = 0; m < 8; ++m) s += full_sh<S>(fsh, T::ld(ff, k * nf + ch[m]), k);
+        for (int m = 0; m < 8; ++m) s += full_sh<S>(fsh, T::ld(ff, at<Q>(k, ch[m])), k);
         a[k] = s / (C)8.0;
     }
     C r, x, y, z;
@@ -303,12 +279,12 @@ __global__ void k_coal_collide(const int32_t *__restrict__ list, const int32_t *
     for (int k = 0; k < Q; ++k) {
         const C fe = feq_heluo_g<Q, C>(k, r, x, y, z);
         const C st = stored_sh<S>(csh, fe + (C)scale * (a[k] - fe), k);
-        T::st(cf, k * nc + i, st);
+        T::st(cf, at<Q>(k, i), st);
         S sv;
         T::st(&sv, 0, st);
-        a[k] = full_sh<S>(csh, T::cv(sv), k);
+        a[k] = T::cv(sv);
     }
-    macros_collide_store<Q, S, COLL>(a, r, x, y, z, tau, cfnext, nc, i, csh);
+    macros_collide_store<Q, S, COLL>(a, r, x, y, z, tau, cfnext, i, csh);
     if (macros) {
         rho[i] = r;
         u[i] = x;
@@ -340,14 +316,14 @@ __global__ void k_bc_neq(const int32_t *list, int64_t nl, int b, int64_t n, cons
             const int32_t nb = k == 0 ? (int32_t)i : nbr[(int64_t)(k - 1) * n + i];
             if (nb < 0) {
                 atomicOr(err, DEVERR_MISSING_BC_NBR);
-                tmp[t * nl + j] = (double)full_sh<S>(sh, T::ld(f, k * n + i), k);
+                tmp[t * nl + j] = (double)full_sh<S>(sh, T::ld(f, at<Q>(k, i)), k);
                 continue;
             }
             const C fw = feq_g<Q, C>(k, rho[i], (C)ubx, (C)uby, (C)ubz);
             const C fn = feq_g<Q, C>(k, rho[nb], u[nb], u[n + nb], u[2 * n + nb]);
-            tmp[t * nl + j] = (double)(fw + full_sh<S>(sh, T::ld(f, k * n + nb), k) - fn);
+            tmp[t * nl + j] = (double)(fw + full_sh<S>(sh, T::ld(f, at<Q>(k, nb)), k) - fn);
         } else {
-            T::st(f, k * n + i, stored_sh<S>(sh, (C)tmp[t * nl + j], k));
+            T::st(f, at<Q>(k, i), stored_sh<S>(sh, (C)tmp[t * nl + j], k));
         }
     }
 }
@@ -376,14 +352,14 @@ __global__ void k_bc_neq_all(const int32_t *list, const int8_t *setb, int64_t nl
             const int32_t nb = k == 0 ? (int32_t)i : nbr[(int64_t)(k - 1) * n + i];
             if (nb < 0) {
                 atomicOr(err, DEVERR_MISSING_BC_NBR);
-                tmp[t * nl + j] = (double)full_sh<S>(sh, T::ld(f, k * n + i), k);
+                tmp[t * nl + j] = (double)full_sh<S>(sh, T::ld(f, at<Q>(k, i)), k);
                 continue;
             }
             const C fw = feq_g<Q, C>(k, rho[i], (C)ub.u[b][0], (C)ub.u[b][1], (C)ub.u[b][2]);
             const C fn = feq_g<Q, C>(k, rho[nb], u[nb], u[n + nb], u[2 * n + nb]);
-            tmp[t * nl + j] = (double)(fw + full_sh<S>(sh, T::ld(f, k * n + nb), k) - fn);
+            tmp[t * nl + j] = (double)(fw + full_sh<S>(sh, T::ld(f, at<Q>(k, nb)), k) - fn);
         } else {
-            T::st(f, k * n + i, stored_sh<S>(sh, (C)tmp[t * nl + j], k));
+            T::st(f, at<Q>(k, i), stored_sh<S>(sh, (C)tmp[t * nl + j], k));
         }
     }
 }
@@ -409,13 +385,13 @@ __global__ void k_bc_inout(const int32_t *list, int64_t nl, int east, int64_t n,
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
         if (east) {
-            const S v = fcol[k * n + nb];
-            fcol[k * n + i] = v;
-            f[k * n + i] = v;
+            const S v = fcol[at<Q>(k, nb)];
+            fcol[at<Q>(k, i)] = v;
+            f[at<Q>(k, i)] = v;
         } else {
             const C v = stored_sh<S>(sh, feq_g<Q, C>(k, (C)rho0, (C)ubx, (C)uby, (C)ubz), k);
-            T::st(fcol, k * n + i, v);
-            T::st(f, k * n + i, v);
+            T::st(fcol, at<Q>(k, i), v);
+            T::st(f, at<Q>(k, i), v);
         }
     }
 }
@@ -445,7 +421,7 @@ __global__ void k_bc_hh(const int32_t *list, int64_t nl, int east, int64_t n, in
     for (int k = 0; k < 19; ++k) {
         const int m = textbook ? k : inv(k);
         const int32_t src = m == 0 ? (int32_t)i : nbr[(int64_t)((textbook ? inv(m) : m) - 1) * n + i];
-        g[k] = full_sh<S>(sh, src >= 0 ? T::ld(fcol, (int64_t)m * n + src) : T::ld(f, (int64_t)m * n + i), m);
+        g[k] = full_sh<S>(sh, src >= 0 ? T::ld(fcol, at<19>(m, src)) : T::ld(f, at<19>(m, i)), m);
     }
     const C sgn = textbook ? C(1) : C(-1);
     if (!east) {
@@ -469,13 +445,13 @@ __global__ void k_bc_hh(const int32_t *list, int64_t nl, int east, int64_t n, in
 #pragma unroll
         for (int t = 0; t < 5; ++t) {
             const int k = in_e[t], m = textbook ? k : inv(k);
-            g[k] = full_sh<S>(sh, T::ld(f, (int64_t)m * n + nb), m);
+            g[k] = full_sh<S>(sh, T::ld(f, at<19>(m, nb)), m);
         }
     }
 #pragma unroll
     for (int k = 0; k < 19; ++k) {
         const int m = textbook ? k : inv(k);
-        T::st(f, (int64_t)m * n + i, stored_sh<S>(sh, g[k], m));
+        T::st(f, at<19>(m, i), stored_sh<S>(sh, g[k], m));
     }
 }
 
@@ -490,10 +466,9 @@ __global__ void k_bc_wall_collide(const int32_t *list, int64_t nl, int64_t n, do
     const int64_t i = list[j];
     C d[19];
 #pragma unroll
-    for (int k = 0; k < 19; ++k) d[k] = full_sh<S>(sh, T::ld(f, (int64_t)k * n + i), k);
+    for (int k = 0; k < 19; ++k) d[k] = T::ld(f, at<19>(k, i));
     C r, x, y, z;
-    macros_g<19, C>(d, r, x, y, z);
-    collide_store<19, S, MT_COLL_LBGK>(d, r, x, y, z, tau, fcol, n, i, sh);
+    macros_collide_store<19, S, MT_COLL_LBGK>(d, r, x, y, z, tau, fcol, i, sh);
 }
 
 // D3Q19_BC_Strategy::initial_Feq (D3Q19_BC_Manager.hpp:157-167) on one
@@ -511,8 +486,8 @@ __global__ void k_bc_set_eq(const int32_t *list, int64_t nl, int64_t n, double r
     for (int k = 0; k < Q; ++k) {
         const double v = feq_ref<Q>(k, rho0, ux, uy, uz);
         const C st = stored_f64<S>(sh, v, k);
-        T::st(f, k * n + i, st);
-        T::st(fcol, k * n + i, st);
+        T::st(f, at<Q>(k, i), st);
+        T::st(fcol, at<Q>(k, i), st);
     }
 }
 
@@ -530,7 +505,7 @@ __device__ __forceinline__ void ib_cell(int64_t i, int64_t n, const double *dr, 
 {
     using T = Store<S>;
     using C = typename T::C;
-    auto FC = [&](int k, int64_t idx) { return full_sh<S>(sh, T::ld(fcol, k * n + idx), k); };
+    auto FC = [&](int k, int64_t idx) { return full_sh<S>(sh, T::ld(fcol, at<Q>(k, idx)), k); };
     g[0] = FC(0, i);
     fx = 0;
     fy = 0;
@@ -616,7 +591,7 @@ __global__ void k_ib_treat(const int32_t *list, int64_t nl, int64_t n, const int
     C g[Q], fx, fy, fz;
     ib_cell<Q, FH, S>(i, n, dr, nbr, fcol, rho[i], g, fx, fy, fz, sh);
 #pragma unroll
-    for (int k = 0; k < Q; ++k) T::st(f, k * n + i, stored_sh<S>(sh, g[k], k));
+    for (int k = 0; k < Q; ++k) T::st(f, at<Q>(k, i), stored_sh<S>(sh, g[k], k));
     force[j] = (double)fx;
     force[nl + j] = (double)fy;
     force[2 * nl + j] = (double)fz;
@@ -639,28 +614,13 @@ template <int Q, class S>
 __device__ __forceinline__ void pull_src(int64_t i, int64_t n, const int32_t *src, const S *__restrict__ fcol,
                                          S *__restrict__ f, S *v)
 {
-    v[0] = fcol[i];
+    v[0] = fcol[at<Q>(0, i)];
 #pragma unroll
-    for (int k = 1; k < Q; ++k) v[k] = src[k] >= 0 ? fcol[k * n + src[k]] : f[k * n + i];
-    f[i] = v[0];
-#pragma unroll
-    for (int k = 1; k < Q; ++k)
-        if (src[k] >= 0) f[k * n + i] = v[k];
-}
-
-// pull_src with 32-bit element offsets (Q * n < 2^32)
-template <int Q, class S>
-__device__ __forceinline__ void pull_src32(uint32_t i, uint32_t n, const int32_t *src, const S *__restrict__ fcol,
-                                           S *__restrict__ f, S *v)
-{
-    v[0] = fcol[i];
+    for (int k = 1; k < Q; ++k) v[k] = src[k] >= 0 ? fcol[at<Q>(k, src[k])] : f[at<Q>(k, i)];
+    f[at<Q>(0, i)] = v[0];
 #pragma unroll
     for (int k = 1; k < Q; ++k)
-        v[k] = src[k] >= 0 ? fcol[(uint32_t)k * n + (uint32_t)src[k]] : f[(uint32_t)k * n + i];
-    f[i] = v[0];
-#pragma unroll
-    for (int k = 1; k < Q; ++k)
-        if (src[k] >= 0) f[(uint32_t)k * n + i] = v[k];
+        if (src[k] >= 0) f[at<Q>(k, i)] = v[k];
 }
 
 template <int Q, class S>
@@ -691,10 +651,10 @@ __global__ void k_pull_collide(const int32_t *__restrict__ list, int64_t nl, int
         S v[Q];
         pull_cell<Q, S>(i, n, textbook, nbr, fcol, f, v);
 #pragma unroll
-        for (int k = 0; k < Q; ++k) d[k] = full_sh<S>(sh, T::cv(v[k]), k);
+        for (int k = 0; k < Q; ++k) d[k] = T::cv(v[k]);
     }
     C r, x, y, z;
-    macros_collide_store<Q, S, COLL>(d, r, x, y, z, tau, fnext, n, i, sh);
+    macros_collide_store<Q, S, COLL>(d, r, x, y, z, tau, fnext, i, sh);
     if (macros) {
         rho[i] = r;
         u[i] = x;
@@ -716,61 +676,118 @@ __global__ void k_pull_copy(const int32_t *__restrict__ list, int64_t nl, int64_
     S v[Q];
     pull_cell<Q, S>(i, n, textbook, nbr, fcol, f, v);
 #pragma unroll
-    for (int k = 0; k < Q; ++k) fnext[k * n + i] = v[k];
+    for (int k = 0; k < Q; ++k) fnext[at<Q>(k, i)] = v[k];
 }
 
-// The fused pass over 4x4x4 bricks, one brick per warp (two cells per lane,
-// local Morton index lane and lane + 32).  halo[216 * b + h] holds the cell
-// index of position h = hx + 6 hy + 36 hz of the brick's 6x6x6 neighbourhood
-// (local coordinates hx - 1, hy - 1, hz - 1; -1 = no cell), resolved once
-// from the bricks' starts and occupancy masks; the warp stages it in shared
-// memory, so a cell's Q - 1 source indices are shared-memory reads at fixed
-// offsets.  The brick neighbours come from Morton_Assist::find_neighbor on a
-// corner cell, so each source is the cell the reference's find() returns.
-// Resident blocks per SM of each form and storage: brick_min_blocks.
-// bcls: 1 stream + collide, 3 the same with the streamed f stored, 2 stream
-// (f stored) + copy, 4 a direct-forcing band cell (stream; collided after
-// the forcing).  The streamed f of class-1 cells is read by nothing in
+// The fused pass over a level's 4x4x4 bricks, one warp per brick that has work.
+// A cell's sources lie in its own brick and the 26 around it: the warp reads
+// those 27 brick numbers once (108 B per brick; a table of every cell's
+// sources would be 4 (Q - 1) B per cell) and each source slot follows from
+// the cell's local coordinates.  The brick neighbours come from
+// Morton_Assist::find_neighbor on a corner cell, so each source is the cell the
+// reference's find() returns.
+// Classes (bcls): 1 stream + collide, 3 the same with the streamed f stored, 2
+// stream (f stored) + copy, 4 a direct-forcing band cell (stream; collided
+// after the forcing).  The streamed f of class-1 cells is read by nothing in
 // the coarse step (their next collision is computed here, a missing link's
 // f never changes), so it is stored only when `fall` is set or when the
 // state leaves the fused schedule (k_brick_pull).
 // When `macros` is set (the level's last substep of the coarse step) the
 // macros of the streamed f are written too: they are what the all-level
 // calculateMacros at the end of the coarse step computes.
+struct BrickTab {
+    const int32_t *__restrict__ list, *__restrict__ nbr;
+    const unsigned long long *__restrict__ mask;
+    const uint8_t *__restrict__ cls, *__restrict__ flag;
+};
 
-// The part of a brick cell's pass after its gather: v holds the streamed f
-// of cell i (class cls), present(k) says whether link k had a source cell
-// (a missing one keeps f, which is then not stored again).
-template <int Q, class S, int COLL, class P>
-__device__ __forceinline__ void brick_finish(uint32_t i, int cls, const S *v, P present, uint32_t n,
-                                             S *__restrict__ f, S *__restrict__ fnext, double tau,
-                                             typename Store<S>::C *__restrict__ rho,
-                                             typename Store<S>::C *__restrict__ u, int macros, int fall,
-                                             long long *__restrict__ acc, const Shift &sh)
+// a warp's neighbourhood in shared memory: where each neighbour brick's
+// populations start (an absent one: the brick's own, never used as a source)
+// and, for bricks with a missing source, its occupancy
+struct BrickHood {
+    uint32_t off[27];
+    unsigned long long mask[27];
+};
+template <int Q>
+__device__ __forceinline__ void brick_hood(int32_t b, int lane, const BrickTab &t, bool complete, BrickHood &h)
+{
+    if (lane < 27) {
+        const int32_t e = __ldg(t.nbr + 27 * (int64_t)b + lane);
+        h.off[lane] = (uint32_t)(e >= 0 ? e : b) * (64u * Q);
+        if (!complete) h.mask[lane] = e >= 0 ? __ldg(t.mask + e) : 0ull;
+    }
+    __syncwarp();
+}
+
+// one axis of a source position, v = local coordinate + offset in -1..4: bits
+// 0-5 its share of the local Morton index, bits 6 and up of the neighbour's
+// number; the three axes' shares add
+template <int A> __device__ __forceinline__ int axis_pos(int v)
+{
+    constexpr int step = A == 0 ? 1 : (A == 1 ? 3 : 9);
+    return ((((v >> 2) + 1) * step) << 6) | ((v & 1) << A) | ((v & 2) << (A + 2));
+}
+
+// the streamed populations of one cell (local Morton index m)
+template <int Q, class S>
+__device__ __forceinline__ void brick_gather(uint32_t i, int textbook, bool complete, const BrickHood &h,
+                                             const S *__restrict__ fcol, const S *__restrict__ f, S *v)
+{
+    const int m = (int)(i & 63u);
+    const int x = (m & 1) | ((m >> 2) & 2), y = ((m >> 1) & 1) | ((m >> 3) & 2), z = ((m >> 2) & 1) | ((m >> 4) & 2);
+    int px[3], py[3], pz[3];
+#pragma unroll
+    for (int d = -1; d <= 1; ++d) {
+        const int s = textbook ? -d : d;
+        px[1 + d] = axis_pos<0>(x + s);
+        py[1 + d] = axis_pos<1>(y + s);
+        pz[1 + d] = axis_pos<2>(z + s);
+    }
+    v[0] = fcol[at<Q>(0, i)];
+#pragma unroll
+    for (int k = 1; k < Q; ++k) {
+        const int p = px[1 + ex(k)] + py[1 + ey(k)] + pz[1 + ez(k)];
+        const S *src = fcol + (h.off[p >> 6] + (uint32_t)(p & 63)) + 64 * k;
+        if (complete)
+            v[k] = *src;
+        else
+            v[k] = ((h.mask[p >> 6] >> (p & 63)) & 1) ? *src : f[at<Q>(k, i)];
+    }
+}
+
+// one cell of the pass (i its slot): FP64, and form 1 of the reduced storages
+template <int Q, class S, int COLL>
+__device__ __forceinline__ void brick_cell(uint32_t i, int cls, bool complete, const BrickHood &h, uint32_t n,
+                                           int textbook, const S *__restrict__ fcol, S *__restrict__ f,
+                                           S *__restrict__ fnext, double tau, typename Store<S>::C *__restrict__ rho,
+                                           typename Store<S>::C *__restrict__ u, int macros, int fall,
+                                           long long *__restrict__ acc, const Shift &sh)
 {
     using T = Store<S>;
     using C = typename T::C;
+    if (!cls) return;
+    S v[Q];
+    brick_gather<Q, S>(i, textbook, complete, h, fcol, f, v);
     if (cls != 1 || fall) {
-        f[i] = v[0];
+        // a missing link's value is f's own: storing it again changes nothing
 #pragma unroll
-        for (int k = 1; k < Q; ++k)
-            if (present(k)) f[(uint32_t)k * n + i] = v[k];
+        for (int k = 0; k < Q; ++k) f[at<Q>(k, i)] = v[k];
     }
     if (cls == 2) {
 #pragma unroll
-        for (int k = 0; k < Q; ++k) fnext[(uint32_t)k * n + i] = v[k];
+        for (int k = 0; k < Q; ++k) fnext[at<Q>(k, i)] = v[k];
         return;
     }
+    C d[Q];
     if (cls == 4) {
         // direct-forcing band: collided after the forcing; with acc the
         // band's rho, unforced velocity and cleared accumulator are
         // written here (what k_band_macros computes from the stored f)
         if constexpr (COLL == MT_COLL_LBGK) {
             if (acc) {
-                C d[Q];
+                C r, x, y, z;
 #pragma unroll
                 for (int k = 0; k < Q; ++k) d[k] = full_sh<S>(sh, T::cv(v[k]), k);
-                C r, x, y, z;
                 macros_g<Q, C>(d, r, x, y, z);
                 rho[i] = r;
                 u[i] = x;
@@ -783,11 +800,10 @@ __device__ __forceinline__ void brick_finish(uint32_t i, int cls, const S *v, P 
         }
         return;
     }
-    C d[Q];
 #pragma unroll
-    for (int k = 0; k < Q; ++k) d[k] = full_sh<S>(sh, T::cv(v[k]), k);
+    for (int k = 0; k < Q; ++k) d[k] = T::cv(v[k]);
     C r, x, y, z;
-    macros_collide_store<Q, S, COLL>(d, r, x, y, z, tau, fnext, n, i, sh);
+    macros_collide_store<Q, S, COLL>(d, r, x, y, z, tau, fnext, i, sh);
     if (macros) {
         rho[i] = r;
         u[i] = x;
@@ -796,312 +812,317 @@ __device__ __forceinline__ void brick_finish(uint32_t i, int cls, const S *v, P 
     }
 }
 
-// one cell (local Morton index m) of brick b in the fused brick pass
-template <int Q, class S, int COLL>
-__device__ __forceinline__ void brick_cell(int64_t b, int m, const int32_t *s_idx, const uint8_t *__restrict__ bcls,
-                                           uint32_t n, int textbook, bool full, const S *__restrict__ fcol,
-                                           S *__restrict__ f, S *__restrict__ fnext, double tau,
-                                           typename Store<S>::C *__restrict__ rho,
-                                           typename Store<S>::C *__restrict__ u, int macros, int fall,
-                                           long long *__restrict__ acc, const Shift &sh)
-{
-    const int lx = (m & 1) | ((m >> 2) & 2), ly = ((m >> 1) & 1) | ((m >> 3) & 2),
-              lz = ((m >> 2) & 1) | ((m >> 4) & 2);
-    const int base = (lx + 1) + 6 * (ly + 1) + 36 * (lz + 1);
-    const int32_t ii = s_idx[base];
-    if (ii < 0) return;
-    const int cls = __ldg(bcls + 64 * b + m);
-    if (!cls) return;
-    const uint32_t i = (uint32_t)ii;
-    int32_t src[Q];
-#pragma unroll
-    for (int k = 1; k < Q; ++k) {
-        const int off = ex(k) + 6 * ey(k) + 36 * ez(k);
-        src[k] = s_idx[base + (textbook ? -off : off)];
+// Two x-adjacent cells of the reduced storages as one word: slots 2p and
+// 2p + 1 differ in x bit 0 only, so a direction's values of both are an
+// aligned 32-bit (FP16, BF16) or 64-bit (FP32) word.
+template <class S> struct CellPair {
+    using W = uint32_t;
+    using V = typename std::conditional<std::is_same<S, __half>::value, __half2, __nv_bfloat162>::type;
+    static __device__ __forceinline__ W ld(const S *p) { return __ldg((const unsigned int *)p); }
+    static __device__ __forceinline__ void st(S *p, W w) { *(unsigned int *)p = w; }
+    // (second of a, first of b)
+    static __device__ __forceinline__ W straddle(W a, W b) { return __byte_perm(a, b, 0x5432); }
+    static __device__ __forceinline__ float2 f2(W w)
+    {
+        V v;
+        memcpy(&v, &w, 4);
+        if constexpr (std::is_same<S, __half>::value)
+            return __half22float2(v);
+        else
+            return __bfloat1622float2(v);
     }
-    S v[Q];
-    v[0] = fcol[i];
-    if (full) {
-#pragma unroll
-        for (int k = 1; k < Q; ++k) v[k] = fcol[(uint32_t)k * n + (uint32_t)src[k]];
-    } else {
-#pragma unroll
-        for (int k = 1; k < Q; ++k)
-            v[k] = src[k] >= 0 ? fcol[(uint32_t)k * n + (uint32_t)src[k]] : f[(uint32_t)k * n + i];
+    static __device__ __forceinline__ W word(float2 x)
+    {
+        V v;
+        if constexpr (std::is_same<S, __half>::value)
+            v = __float22half2_rn(x);
+        else
+            v = __float22bfloat162_rn(x);
+        W w;
+        memcpy(&w, &v, 4);
+        return w;
     }
-    brick_finish<Q, S, COLL>(i, cls, v, [&](int k) { return full || src[k] >= 0; }, n, f, fnext, tau, rho, u,
-                             macros, fall, acc, sh);
-}
+    static __device__ __forceinline__ void st_one(S *p, W w, int h)
+    {
+        ((unsigned short *)p)[h] = (unsigned short)(h ? w >> 16 : w);
+    }
+    static __device__ __forceinline__ void put(W &w, int h, const S *p)
+    {
+        const unsigned int v = ((const unsigned short *)p)[h];
+        w = h ? (w & 0xffffu) | (v << 16) : (w & 0xffff0000u) | v;
+    }
+};
+template <> struct CellPair<float> {
+    using W = float2;
+    static __device__ __forceinline__ W ld(const float *p) { return __ldg((const float2 *)p); }
+    static __device__ __forceinline__ void st(float *p, W w) { *(float2 *)p = w; }
+    static __device__ __forceinline__ W straddle(W a, W b) { return make_float2(a.y, b.x); }
+    static __device__ __forceinline__ float2 f2(W w) { return w; }
+    static __device__ __forceinline__ W word(float2 x) { return x; }
+    static __device__ __forceinline__ void st_one(float *p, W w, int h) { p[h] = h ? w.y : w.x; }
+    static __device__ __forceinline__ void put(W &w, int h, const float *p)
+    {
+        if (h)
+            w.y = p[1];
+        else
+            w.x = p[0];
+    }
+};
 
-// one warp's brick b (see above); s_idx is the warp's 216-entry shared table;
-// UNROLL (form 3): the lane's two cells in one unrolled sequence
-template <int Q, class S, int COLL, bool UNROLL = false>
-__device__ __forceinline__ void brick_warp(int64_t b, int lane, int32_t *s_idx, const int32_t *__restrict__ halo,
-                                           const uint8_t *__restrict__ bcls, uint32_t n, int textbook,
-                                           const S *__restrict__ fcol, S *__restrict__ f, S *__restrict__ fnext,
-                                           double tau, typename Store<S>::C *__restrict__ rho,
-                                           typename Store<S>::C *__restrict__ u, int macros, int fall,
-                                           long long *__restrict__ acc, const Shift &sh)
+// The gather of a pair, lane = its y, z, x coordinates' bits (y0 z0 x1 y1 z1).
+// For each (y, z) offset the sources are the pair at the same x and, for
+// e_x = +-1, also the next pair on that side, whose near cell completes the
+// word.  All 9 + 2 x 18 loads are issued before the first is used.
+template <int Q, class S, bool TB>
+__device__ __forceinline__ void pair_gather(int lane, const BrickHood &h, const S *__restrict__ fcol,
+                                            typename CellPair<S>::W *v)
 {
-    using T = Store<S>;
-    using C = typename T::C;
-    const int32_t *hb = halo + 216 * b;
-    bool ok = true;
-    for (int h = lane; h < 216; h += 32) {
-        const int32_t e = __ldg(hb + h);
-        s_idx[h] = e;
-        ok &= e >= 0;
-    }
-    // every position of the neighbourhood holds a cell: no missing-link test per gather
-    const bool full = __all_sync(0xffffffffu, ok);
-    __syncwarp();
-    if constexpr (UNROLL) {
-        // both cells in one sequence: the second cell's gathers can be issued
-        // before the first cell's collision
+    using CP = CellPair<S>;
+    constexpr int sg = TB ? -1 : 1;
+    const int x1 = (lane >> 2) & 1;
+    const int y = (lane & 1) | ((lane >> 2) & 2), z = ((lane >> 1) & 1) | ((lane >> 3) & 2);
+    const int xm = 64 + 8 * x1, xl = x1 ? 64 : 8, xr = x1 ? 128 : 72;
+    typename CP::W e[Q];
 #pragma unroll
-        for (int part = 0; part < 2; ++part)
-            brick_cell<Q, S, COLL>(b, lane + 32 * part, s_idx, bcls, n, textbook, full, fcol, f, fnext, tau, rho, u,
-                                   macros, fall, acc, sh);
-    } else {
-#pragma unroll 1
-        for (int part = 0; part < 2; ++part)
-            brick_cell<Q, S, COLL>(b, lane + 32 * part, s_idx, bcls, n, textbook, full, fcol, f, fnext, tau, rho, u,
-                                   macros, fall, acc, sh);
-    }
-}
-
-// The reduced-precision form of brick_warp: both cells of a lane are
-// gathered first, then collided together with packed FP32 pairs (mt_pack2.cuh).
-// Cells that stream without colliding (class 2), band cells (class 4) and
-// absent cells take their own scalar paths; when only one cell of the pair
-// collides, the other lane of the pair repeats its values and is not stored.
-template <int Q, class S, int COLL>
-__device__ __forceinline__ void brick_warp_pair(int64_t b, int lane, int32_t *s_idx, const int32_t *__restrict__ halo,
-                                                const uint8_t *__restrict__ bcls, uint32_t n, int textbook,
-                                                const S *__restrict__ fcol, S *__restrict__ f, S *__restrict__ fnext,
-                                                double tau, float *__restrict__ rho, float *__restrict__ u, int macros,
-                                                int fall, long long *__restrict__ acc, const Shift &sh)
-{
-    using T = Store<S>;
-    const int32_t *hb = halo + 216 * b;
-    for (int h = lane; h < 216; h += 32) s_idx[h] = __ldg(hb + h);
-    __syncwarp();
-    int base[2], cls[2];
-    uint32_t idx[2];
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        const int m = lane + 32 * p;
-        const int lx = (m & 1) | ((m >> 2) & 2), ly = ((m >> 1) & 1) | ((m >> 3) & 2),
-                  lz = ((m >> 2) & 1) | ((m >> 4) & 2);
-        base[p] = (lx + 1) + 6 * (ly + 1) + 36 * (lz + 1);
-        const int32_t ii = s_idx[base[p]];
-        cls[p] = ii >= 0 ? (int)__ldg(bcls + 64 * b + m) : 0;
-        idx[p] = ii >= 0 ? (uint32_t)ii : 0u;
-    }
-    if (!cls[0] && !cls[1]) return;
-    bool coll[2];
-    float2 d[Q];
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        coll[p] = cls[p] == 1 || cls[p] == 3;
-        if (!cls[p]) continue;
-        const uint32_t i = idx[p];
-        const bool keep_f = cls[p] != 1 || fall;
-        // gather, store what this cell's class stores, keep the full FP32 value
+    for (int g = 0; g < 9; ++g) {
+        const int dy = g % 3 - 1, dz = g / 3 - 1;
+        const int pyz = axis_pos<1>(y + dy) + axis_pos<2>(z + dz);
+        const int pm = xm + pyz, pl = xl + pyz, pr = xr + pyz;
+        const S *sm = fcol + (h.off[pm >> 6] + (uint32_t)(pm & 63));
+        const S *sl = fcol + (h.off[pl >> 6] + (uint32_t)(pl & 63));
+        const S *sr = fcol + (h.off[pr >> 6] + (uint32_t)(pr & 63));
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
-            const int off = ex(k) + 6 * ey(k) + 36 * ez(k);
-            const int32_t src = k ? s_idx[base[p] + (textbook ? -off : off)] : (int32_t)i;
-            const S val = src >= 0 ? fcol[(uint32_t)k * n + (uint32_t)src] : f[(uint32_t)k * n + i];
-            if (keep_f && src >= 0) f[(uint32_t)k * n + i] = val;
-            if (cls[p] == 2) fnext[(uint32_t)k * n + i] = val;
-            const float fv = full_sh<S>(sh, T::cv(val), k);
-            if (p == 0)
-                d[k].x = fv;
-            else
-                d[k].y = fv;
+            if (ey(k) != sg * dy || ez(k) != sg * dz) continue;
+            v[k] = CP::ld(sm + 64 * k);
+            if (sg * ex(k) < 0) e[k] = CP::ld(sl + 64 * k);
+            if (sg * ex(k) > 0) e[k] = CP::ld(sr + 64 * k);
         }
-        if constexpr (COLL == MT_COLL_LBGK) {
-            if (cls[p] == 4 && acc) {
-                // direct-forcing band: macros of the streamed f, accumulator cleared
-                float dd[Q];
-#pragma unroll
-                for (int k = 0; k < Q; ++k) dd[k] = p == 0 ? d[k].x : d[k].y;
-                float r, x, y, z;
-                macros_g<Q, float>(dd, r, x, y, z);
-                rho[i] = r;
-                u[i] = x;
-                u[n + i] = y;
-                u[2 * n + i] = z;
-                acc[i] = 0;
-                acc[n + i] = 0;
-                acc[2 * n + i] = 0;
-            }
-        }
-    }
-    if (!coll[0] && !coll[1]) return;
-    // a pair with one colliding cell: the other lane repeats its values
-    if (!coll[1]) {
-#pragma unroll
-        for (int k = 0; k < Q; ++k) d[k].y = d[k].x;
-    } else if (!coll[0]) {
-#pragma unroll
-        for (int k = 0; k < Q; ++k) d[k].x = d[k].y;
-    }
-    float2 r, x, y, z;
-    p2::macros<Q>(d, r, x, y, z);
-    if (macros) {
-        if (coll[0]) {
-            rho[idx[0]] = r.x;
-            u[idx[0]] = x.x;
-            u[n + idx[0]] = y.x;
-            u[2 * n + idx[0]] = z.x;
-        }
-        if (coll[1]) {
-            rho[idx[1]] = r.y;
-            u[idx[1]] = x.y;
-            u[n + idx[1]] = y.y;
-            u[2 * n + idx[1]] = z.y;
-        }
-    }
-    float2 o[Q];
-    if constexpr (COLL == MT_COLL_LBGK) {
-        p2::lbgk<Q>(d, r, x, y, z, (float)(1.0 / tau), sh, o);  // stored deviations already
-    } else {
-        p2::cumulant(d, r, x, y, z, (float)(1.0 / tau), o);
-#pragma unroll
-        for (int k = 0; k < Q; ++k) o[k] = p2::sub(o[k], p2::bc(sh.v[k]));
     }
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
-        if (coll[0]) T::st(fnext, (uint32_t)k * n + idx[0], o[k].x);
-        if (coll[1]) T::st(fnext, (uint32_t)k * n + idx[1], o[k].y);
+        if (sg * ex(k) < 0) v[k] = CP::straddle(e[k], v[k]);
+        if (sg * ex(k) > 0) v[k] = CP::straddle(v[k], e[k]);
     }
 }
 
-// brick_warp for every storage: V = 1 the pair form (reduced storages), V = 0
-// the one-cell-at-a-time form
-template <int Q, class S, int COLL, int V>
-__device__ __forceinline__ void brick_warp_any(int64_t b, int lane, int32_t *s_idx, const int32_t *__restrict__ halo,
-                                               const uint8_t *__restrict__ bcls, uint32_t n, int textbook,
-                                               const S *__restrict__ fcol, S *__restrict__ f, S *__restrict__ fnext,
-                                               double tau, typename Store<S>::C *__restrict__ rho,
-                                               typename Store<S>::C *__restrict__ u, int macros, int fall,
-                                               long long *__restrict__ acc, const Shift &sh)
+// a missing link keeps f (bricks without BRICK_COMPLETE)
+template <int Q, class S>
+__device__ __forceinline__ void pair_missing(int lane, int textbook, const BrickHood &h, const S *own,
+                                             typename CellPair<S>::W *v)
 {
-    if constexpr (V == 1 && Store<S>::shifted && (COLL == MT_COLL_LBGK || Q == 27))
-        brick_warp_pair<Q, S, COLL>(b, lane, s_idx, halo, bcls, n, textbook, fcol, f, fnext, tau, rho, u, macros,
-                                    fall, acc, sh);
-    else
-        brick_warp<Q, S, COLL, V == 3>(b, lane, s_idx, halo, bcls, n, textbook, fcol, f, fnext, tau, rho, u, macros,
-                                       fall, acc, sh);
+    const int x1 = (lane >> 2) & 1;
+    const int y = (lane & 1) | ((lane >> 2) & 2), z = ((lane >> 1) & 1) | ((lane >> 3) & 2);
+    const int s = textbook ? -1 : 1;
+#pragma unroll
+    for (int k = 1; k < Q; ++k) {
+        const int pyz = axis_pos<1>(y + s * ey(k)) + axis_pos<2>(z + s * ez(k));
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int p = axis_pos<0>(2 * x1 + c + s * ex(k)) + pyz;
+            if (!((h.mask[p >> 6] >> (p & 63)) & 1)) CellPair<S>::put(v[k], c, own + 64 * k);
+        }
+    }
 }
 
-#ifndef MT_BRICK_MIN_BLOCKS
-#define MT_BRICK_MIN_BLOCKS 8  // resident 128-thread blocks per SM asked of the 16-bit one-cell passes (64 registers)
-#endif
-#ifndef MT_BRICK_MIN_BLOCKS_F32
-#define MT_BRICK_MIN_BLOCKS_F32 7  // resident blocks asked of the FP32 one-cell passes (72 registers)
-#endif
-#ifndef MT_BRICK_MIN_BLOCKS_Q19_LBGK
-#define MT_BRICK_MIN_BLOCKS_Q19_LBGK 10  // 16-bit D3Q19 LBGK one-cell passes: 48 registers, no spills
-#endif
-#ifndef MT_BRICK_PAIR_MIN_BLOCKS
-#define MT_BRICK_PAIR_MIN_BLOCKS 4  // the pair passes of every reduced storage (128 registers)
-#endif
-// resident blocks per SM asked of a brick pass (V: one cell or a pair per step)
-#ifndef MT_BRICK_WIDE_MIN_BLOCKS
-#define MT_BRICK_WIDE_MIN_BLOCKS 6  // the one-cell form with more registers (85), reduced storages
-#endif
-#ifndef MT_BRICK_UNROLL_MIN_BLOCKS
-#define MT_BRICK_UNROLL_MIN_BLOCKS 6  // the two cells of a lane in one unrolled sequence (form 3)
-#endif
+// One warp's brick for the reduced storages: a lane gathers, collides and
+// stores a pair of cells, the collision in packed FP32 (mt_pack2.cuh).
+// Against one cell per lane step (form 1) a pair has 45 loads of a word for
+// D3Q27 where the cells have 54 of a value, 27 addresses (the Q accesses of a
+// source pair are constant offsets) for 54, half the stores and conversions
+// and half the arithmetic's issue slots: 79 M instructions for the finest
+// level of the 4-level cumulant sphere where the cell-by-cell pass over a
+// [Q][n] array had 133 M, 128 us for 215 us (108 B of populations per cell:
+// 72 us at the measured copy rate), FP32 167 us for 310 us.  What bounds it
+// now: the FP32 pipe (65 % active) and the gathers' latency at 24 warps per SM
+// side by side, DRAM at 46 % of its peak.
+template <int Q, class S, int COLL>
+__device__ __forceinline__ void brick_warp_pair(int32_t b, int lane, BrickHood &h, const BrickTab &t, uint32_t n,
+                                                int textbook, const S *__restrict__ fcol, S *__restrict__ f,
+                                                S *__restrict__ fnext, double tau, float *__restrict__ rho,
+                                                float *__restrict__ u, int macros, int fall,
+                                                long long *__restrict__ acc, const Shift &sh)
+{
+    using CP = CellPair<S>;
+    const int flag = __ldg(t.flag + b);
+    const bool complete = flag & BRICK_COMPLETE, uniform = flag & BRICK_UNIFORM;
+    brick_hood<Q>(b, lane, t, complete, h);
+    const uint32_t i = 64u * (uint32_t)b + 2u * lane;
+    int c0 = 1, c1 = 1;
+    if (!uniform) {
+        const unsigned short cc = __ldg((const unsigned short *)(t.cls + i));
+        c0 = cc & 255;
+        c1 = cc >> 8;
+        if (!cc) return;
+    }
+    const uint32_t o = at<Q>(0, i);
+    typename CP::W v[Q];
+    if (textbook)
+        pair_gather<Q, S, true>(lane, h, fcol, v);
+    else
+        pair_gather<Q, S, false>(lane, h, fcol, v);
+    if (!complete) pair_missing<Q, S>(lane, textbook, h, f + o, v);
+    auto store = [&](S *p, bool s0, bool s1) {
+        if (s0 && s1) {
+#pragma unroll
+            for (int k = 0; k < Q; ++k) CP::st(p + 64 * k, v[k]);
+        } else if (s0 || s1) {
+            const int w = s1;
+#pragma unroll
+            for (int k = 0; k < Q; ++k) CP::st_one(p + 64 * k, v[k], w);
+        }
+    };
+    if (fall || !uniform) {
+        store(f + o, c0 && (c0 != 1 || fall), c1 && (c1 != 1 || fall));
+        store(fnext + o, c0 == 2, c1 == 2);
+    }
+    const bool k0 = c0 & 1, k1 = c1 & 1;  // classes 1 and 3
+    const bool b0 = c0 == 4 && acc, b1 = c1 == 4 && acc;
+    if (!(k0 || k1 || b0 || b1)) return;
+    float2 d[Q], r, x, y, z;
+    const float om = (float)(1.0 / tau);
+#pragma unroll
+    for (int k = 0; k < Q; ++k) d[k] = CP::f2(v[k]);
+    if constexpr (COLL == MT_COLL_LBGK)
+        p2::lbgk<Q, float2>(d, r, x, y, z, om, sh);
+    else
+        p2::cumulant<float2, false>(d, r, x, y, z, om, sh);
+#pragma unroll
+    for (int k = 0; k < Q; ++k) v[k] = CP::word(d[k]);
+    store(fnext + o, k0, k1);
+    const bool m0 = (macros && k0) || b0, m1 = (macros && k1) || b1;
+    if (m0 && m1) {
+        *(float2 *)(rho + i) = r;
+        *(float2 *)(u + i) = x;
+        *(float2 *)(u + n + i) = y;
+        *(float2 *)(u + 2 * n + i) = z;
+    } else if (m0 || m1) {
+        const uint32_t j = i + (m1 ? 1u : 0u);
+        rho[j] = m1 ? r.y : r.x;
+        u[j] = m1 ? x.y : x.x;
+        u[n + j] = m1 ? y.y : y.x;
+        u[2 * n + j] = m1 ? z.y : z.x;
+    }
+    if constexpr (COLL == MT_COLL_LBGK) {
+        // the band's accumulator restarts from zero
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            if (c ? b1 : b0) {
+                acc[i + c] = 0;
+                acc[n + i + c] = 0;
+                acc[2 * n + i + c] = 0;
+            }
+    }
+}
+
+// a brick in form V: the reduced storages' forms 0, 2, 3 are the pair form at
+// different numbers of resident blocks, 1 goes cell by cell; FP64 goes cell by
+// cell (3: the lane's two cells in one unrolled sequence)
+template <int Q, class S, int COLL, int V>
+__device__ __forceinline__ void brick_warp(int32_t b, int lane, BrickHood &h, const BrickTab &t, uint32_t n,
+                                           int textbook, const S *__restrict__ fcol, S *__restrict__ f,
+                                           S *__restrict__ fnext, double tau, typename Store<S>::C *__restrict__ rho,
+                                           typename Store<S>::C *__restrict__ u, int macros, int fall,
+                                           long long *__restrict__ acc, const Shift &sh)
+{
+    if constexpr (Store<S>::shifted && V != 1) {
+        brick_warp_pair<Q, S, COLL>(b, lane, h, t, n, textbook, fcol, f, fnext, tau, rho, u, macros, fall, acc, sh);
+    } else {
+        const bool complete = __ldg(t.flag + b) & BRICK_COMPLETE;
+        brick_hood<Q>(b, lane, t, complete, h);
+        const uint32_t i = 64u * (uint32_t)b + (uint32_t)lane;
+        const int c0 = __ldg(t.cls + i), c1 = __ldg(t.cls + i + 32);
+        if constexpr (V == 3) {
+            brick_cell<Q, S, COLL>(i, c0, complete, h, n, textbook, fcol, f, fnext, tau, rho, u, macros, fall, acc, sh);
+            brick_cell<Q, S, COLL>(i + 32, c1, complete, h, n, textbook, fcol, f, fnext, tau, rho, u, macros, fall, acc,
+                                   sh);
+        } else {
+#pragma unroll 1
+            for (int part = 0; part < 2; ++part)
+                brick_cell<Q, S, COLL>(i + 32 * part, part ? c1 : c0, complete, h, n, textbook, fcol, f, fnext, tau, rho,
+                                       u, macros, fall, acc, sh);
+        }
+    }
+}
+
+// Resident 128-thread blocks per SM asked of a brick pass.  Measured per launch
+// (finest level of the 4-level D3Q27 cumulant sphere, 4.28 M cells; direct-
+// forcing sphere R 8, D3Q19 LBGK, 8.9 M cells), pair form:
+//   D3Q27 FP16: 4 blocks 143.7 us, 5 136.2, 6 128.0, 7 124.6, 8 (spills) 144.4
+//   D3Q27 FP32: 4 blocks 191.5 us, 5 175.1, 6 (40 B of spills) 166.9, 7 183.3
+//   D3Q19 FP16: 5 blocks 216.1 us, 6 194.2, 7 183.3, 8 177.2, 9 175.1
+//   D3Q19 FP32: 5 blocks 283.0 us, 6 263.2, 7 250.9
 template <int Q, class S, int COLL, int V> constexpr int brick_min_blocks()
 {
-    if (V == 1 && Store<S>::shifted) return MT_BRICK_PAIR_MIN_BLOCKS;
-    if (V == 2 && Store<S>::shifted) return MT_BRICK_WIDE_MIN_BLOCKS;
-    if (V == 3) return Store<S>::shifted ? MT_BRICK_UNROLL_MIN_BLOCKS : 1;
-    if (Store<S>::bytes == 2) return (COLL == MT_COLL_LBGK && Q == 19) ? MT_BRICK_MIN_BLOCKS_Q19_LBGK : MT_BRICK_MIN_BLOCKS;
-    if (Store<S>::bytes == 4) return MT_BRICK_MIN_BLOCKS_F32;
-    return 1;
+    if (!Store<S>::shifted) return 1;
+    if (V == 1) return Store<S>::bytes == 2 ? ((COLL == MT_COLL_LBGK && Q == 19) ? 10 : 8) : 7;
+    if (Store<S>::bytes == 2) return Q == 19 ? (V == 0 ? 7 : (V == 2 ? 8 : 9)) : (V == 0 ? 6 : (V == 2 ? 7 : 8));
+    return V == 0 ? 6 : (V == 2 ? 5 : 7);
 }
-// the form a level runs until mt_case_tune_bricks times them: form 0 for
-// every storage (measured on the 4-level cumulant sphere and the
-// direct-forcing sphere: the pair form runs 2-4x longer per launch at half
-// the resident warps; FP32 form 0 at 7 resident blocks is as fast as or
-// faster than forms 2 and 3 at 6)
+// the form a level runs until mt_case_tune_bricks times them
 template <class S> constexpr int brick_default_variant() { return 0; }
 
 template <int Q, class S, int COLL, int V>
 __global__ void __launch_bounds__(128, brick_min_blocks<Q, S, COLL, V>()) k_brick_step(
-    int64_t nb, const int32_t *__restrict__ halo, const uint8_t *__restrict__ bcls, uint32_t n, int textbook,
-    const S *__restrict__ fcol, S *__restrict__ f, S *__restrict__ fnext, double tau,
-    typename Store<S>::C *__restrict__ rho, typename Store<S>::C *__restrict__ u, int macros, int fall,
-    long long *__restrict__ acc, const Shift sh)
+    int64_t nb, const BrickTab t, uint32_t n, int textbook, const S *__restrict__ fcol, S *__restrict__ f,
+    S *__restrict__ fnext, double tau, typename Store<S>::C *__restrict__ rho, typename Store<S>::C *__restrict__ u,
+    int macros, int fall, long long *__restrict__ acc, const Shift sh)
 {
-    __shared__ int32_t s_idx[4][216];
+    __shared__ BrickHood hood[4];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t b = 4 * (int64_t)blockIdx.x + w;
-    if (b >= nb) return;
-    brick_warp_any<Q, S, COLL, V>(b, lane, s_idx[w], halo, bcls, n, textbook, fcol, f, fnext, tau, rho, u, macros,
-                                  fall, acc, sh);
+    const int64_t j = 4 * (int64_t)blockIdx.x + w;
+    if (j >= nb) return;
+    brick_warp<Q, S, COLL, V>(__ldg(t.list + j), lane, hood[w], t, n, textbook, fcol, f, fnext, tau, rho, u, macros,
+                              fall, acc, sh);
 }
 
-// The same pass over the bricks of many cases (a batch): brick b of the work
+// The same pass over the bricks of many cases (a batch): brick j of the work
 // list belongs to the slot whose [off[s], off[s + 1]) range holds it; each
 // slot carries one case level's tables, buffers and relaxation time.
 template <int Q, class S, int COLL, int V>
 __global__ void __launch_bounds__(128, brick_min_blocks<Q, S, COLL, V>()) k_brick_step_batch(const BrickBatch *__restrict__ bb,
                                                                                              const Shift sh)
 {
-    __shared__ int32_t s_idx[4][216];
+    __shared__ BrickHood hood[4];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t b = 4 * (int64_t)blockIdx.x + w;
-    if (b >= bb->total) return;
+    const int64_t j = 4 * (int64_t)blockIdx.x + w;
+    if (j >= bb->total) return;
     int lo = 0, hi = bb->nslots;
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
-        if (bb->off[mid] <= b)
+        if (bb->off[mid] <= j)
             lo = mid;
         else
             hi = mid;
     }
     const BrickSlot &sl = bb->slot[lo];
     using C = typename Store<S>::C;
-    brick_warp_any<Q, S, COLL, V>(b - bb->off[lo], lane, s_idx[w], sl.halo, sl.cls, sl.n, sl.textbook,
-                               (const S *)sl.fcol, (S *)sl.f, (S *)sl.fnext, sl.tau, (C *)sl.rho, (C *)sl.u, sl.macros,
-                               sl.fall, sl.acc, sh);
+    const BrickTab t{sl.list, sl.nbr, sl.mask, sl.cls, sl.flag};
+    brick_warp<Q, S, COLL, V>(__ldg(t.list + (j - bb->off[lo])), lane, hood[w], t, sl.n, sl.textbook,
+                              (const S *)sl.fcol, (S *)sl.f, (S *)sl.fnext, sl.tau, (C *)sl.rho, (C *)sl.u, sl.macros,
+                              sl.fall, sl.acc, sh);
 }
 
 // The streamed f of the class-1 cells, from the buffer the last fused pass
 // read (the values that pass would have stored).
 template <int Q, class S>
-__global__ void __launch_bounds__(128) k_brick_pull(int64_t nb, const int32_t *__restrict__ halo,
-                                                    const uint8_t *__restrict__ bcls, uint32_t n, int textbook,
+__global__ void __launch_bounds__(128) k_brick_pull(int64_t nb, const BrickTab t, int textbook,
                                                     const S *__restrict__ fcol, S *__restrict__ f)
 {
-    __shared__ int32_t s_idx[4][216];
+    __shared__ BrickHood hood[4];
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t b = 4 * (int64_t)blockIdx.x + w;
-    if (b >= nb) return;
-    const int32_t *hb = halo + 216 * b;
-    for (int h = lane; h < 216; h += 32) s_idx[w][h] = __ldg(hb + h);
-    __syncwarp();
+    const int64_t j = 4 * (int64_t)blockIdx.x + w;
+    if (j >= nb) return;
+    const int32_t b = __ldg(t.list + j);
+    const bool complete = __ldg(t.flag + b) & BRICK_COMPLETE;
+    brick_hood<Q>(b, lane, t, complete, hood[w]);
     for (int part = 0; part < 2; ++part) {
-        const int m = lane + 32 * part;
-        const int lx = (m & 1) | ((m >> 2) & 2), ly = ((m >> 1) & 1) | ((m >> 3) & 2),
-                  lz = ((m >> 2) & 1) | ((m >> 4) & 2);
-        const int base = (lx + 1) + 6 * (ly + 1) + 36 * (lz + 1);
-        const int32_t ii = s_idx[w][base];
-        if (ii < 0 || __ldg(bcls + 64 * b + m) != 1) continue;
-        int32_t src[Q];
-#pragma unroll
-        for (int k = 1; k < Q; ++k) {
-            const int off = ex(k) + 6 * ey(k) + 36 * ez(k);
-            src[k] = s_idx[w][base + (textbook ? -off : off)];
-        }
+        const uint32_t i = 64u * (uint32_t)b + (uint32_t)lane + 32u * part;
+        if (__ldg(t.cls + i) != 1) continue;
         S v[Q];
-        pull_src32<Q, S>((uint32_t)ii, n, src, fcol, f, v);
+        brick_gather<Q, S>(i, textbook, complete, hood[w], fcol, f, v);
+#pragma unroll
+        for (int k = 0; k < Q; ++k) f[at<Q>(k, i)] = v[k];
     }
 }
 
@@ -1122,7 +1143,7 @@ __global__ void k_ib_collide(const int32_t *list, int64_t nl, int64_t n, const i
     C g[Q], fx, fy, fz;
     {
 #pragma unroll
-        for (int k = 0; k < Q; ++k) g[k] = full_sh<S>(sh, T::ld(f, k * n + i), k);
+        for (int k = 0; k < Q; ++k) g[k] = full_sh<S>(sh, T::ld(f, at<Q>(k, i)), k);
         C r, x, y, z;
         macros_g<Q, C>(g, r, x, y, z);
         ib_cell<Q, FH, S>(i, n, dr, nbr, fcol, r, g, fx, fy, fz, sh);
@@ -1130,17 +1151,17 @@ __global__ void k_ib_collide(const int32_t *list, int64_t nl, int64_t n, const i
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
         const C st = stored_sh<S>(sh, g[k], k);
-        T::st(f, k * n + i, st);
+        T::st(f, at<Q>(k, i), st);
         // the next collision reads the stored value
         S sv;
         T::st(&sv, 0, st);
-        g[k] = full_sh<S>(sh, T::cv(sv), k);
+        g[k] = T::cv(sv);
     }
     force[j] = (double)fx;
     force[nl + j] = (double)fy;
     force[2 * nl + j] = (double)fz;
     C r, x, y, z;
-    macros_collide_store<Q, S, COLL>(g, r, x, y, z, tau, fnext, n, i, sh);
+    macros_collide_store<Q, S, COLL>(g, r, x, y, z, tau, fnext, i, sh);
     if (macros) {
         rho[i] = r;
         u[i] = x;
@@ -1182,7 +1203,7 @@ __global__ void k_band_macros(const int32_t *band, int64_t nb, int64_t n, const 
     const int64_t i = band[j];
     C d[Q];
 #pragma unroll
-    for (int k = 0; k < Q; ++k) d[k] = full_sh<S>(sh, T::ld(f, k * n + i), k);
+    for (int k = 0; k < Q; ++k) d[k] = full_sh<S>(sh, T::ld(f, at<Q>(k, i)), k);
     C r, x, y, z;
     macros_g<Q, C>(d, r, x, y, z);
     rho[i] = r;
@@ -1197,13 +1218,13 @@ __global__ void k_band_macros(const int32_t *band, int64_t nb, int64_t n, const 
 // one marker: interpolate rho and u at X(t), force F = 2 rho (U - u), spread
 // F dv phi into the band cells; fk receives -F dv (the force on the body)
 // grid[(x - lo) + dx ((y - lo) + dy (z - lo))] = index of band cell (x, y, z) or -1
-static __global__ void k_band_grid(const int32_t *band, int64_t nb, const uint64_t *key, int64_t lx, int64_t ly,
+static __global__ void k_band_grid(const int32_t *band, int64_t nb, const LevelMap map, int64_t lx, int64_t ly,
                             int64_t lz, int64_t dx, int64_t dy, int64_t dz, int32_t *grid)
 {
     const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nb) return;
     const int32_t i = band[j];
-    const uint64_t k = key[i];
+    const uint64_t k = map.key(i);
     const int64_t x = (int64_t)compact3(k) - lx, y = (int64_t)compact3(k >> 1) - ly, z = (int64_t)compact3(k >> 2) - lz;
     if (x < 0 || y < 0 || z < 0 || x >= dx || y >= dy || z >= dz) return;
     grid[x + dx * (y + dy * z)] = i;
@@ -1330,7 +1351,7 @@ __global__ void k_band_collide(const int32_t *band, int64_t nb, int64_t n, doubl
         float rd = 0.f, jx = 0.f, jy = 0.f, jz = 0.f;
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
-            sd[k] = T::ld(f, k * n + i);
+            sd[k] = T::ld(f, at<Q>(k, i));
             rd += sd[k];
             jx += sd[k] * ex(k);
             jy += sd[k] * ey(k);
@@ -1356,7 +1377,7 @@ __global__ void k_band_collide(const int32_t *band, int64_t nb, int64_t n, doubl
             const float wk = (float)w<Q>(k);
             const float dfeq = wk * ((r - 1.f) + r * (3.f * eu + 4.5f * eu * eu - uu)) - sh.dw[k];
             const float ge = 3.f * (eg - ug) + 9.f * eu * eg;
-            T::st(fcol, k * n + i, fmaf(om, dfeq - sd[k], sd[k]) + fpre * wk * ge);
+            T::st(fcol, at<Q>(k, i), fmaf(om, dfeq - sd[k], sd[k]) + fpre * wk * ge);
         }
         return;
     }
@@ -1364,7 +1385,7 @@ __global__ void k_band_collide(const int32_t *band, int64_t nb, int64_t n, doubl
     C r = 0, jx = 0, jy = 0, jz = 0;
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
-        d[k] = full_sh<S>(sh, T::ld(f, k * n + i), k);
+        d[k] = full_sh<S>(sh, T::ld(f, at<Q>(k, i)), k);
         r += d[k];
         jx += d[k] * ex(k);
         jy += d[k] * ey(k);
@@ -1385,7 +1406,7 @@ __global__ void k_band_collide(const int32_t *band, int64_t nb, int64_t n, doubl
         const C ge = (C(3) * (ex(k) - x) + C(9) * eu * ex(k)) * gx + (C(3) * (ey(k) - y) + C(9) * eu * ey(k)) * gy +
                      (C(3) * (ez(k) - z) + C(9) * eu * ez(k)) * gz;
         const C out = d[k] - (d[k] - feq) * om + fpre * (C)w<Q>(k) * ge;
-        T::st(fcol, k * n + i, stored_sh<S>(sh, out, k));
+        T::st(fcol, at<Q>(k, i), stored_sh<S>(sh, out, k));
     }
 }
 
@@ -1430,31 +1451,41 @@ static __global__ void k_force_reduce(const double *force, int64_t nl, double *a
 
 static __global__ void k_force_tick(double *acc) { acc[3] += 1.0; }
 
+// Host arrays hold a level's stored cells in key order ([Q][nc], [nc]); slot[r]
+// is the slot of cell r.
 template <int Q, class S>
-__global__ void k_to_f64(const S *src, double *dst, int64_t n, const Shift sh)
+__global__ void k_to_f64(const S *src, double *dst, const int32_t *__restrict__ slot, int64_t nc, const Shift sh)
 {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= nc) return;
+    const int64_t i = slot[r];
 #pragma unroll
-    for (int k = 0; k < Q; ++k) dst[k * n + i] = (double)full_sh<S>(sh, Store<S>::ld(src, k * n + i), k);
+    for (int k = 0; k < Q; ++k) dst[k * nc + r] = (double)full_sh<S>(sh, Store<S>::ld(src, at<Q>(k, i)), k);
 }
 template <int Q, class S>
-__global__ void k_from_f64(const double *src, S *dst, int64_t n, const Shift sh)
+__global__ void k_from_f64(const double *src, S *dst, const int32_t *__restrict__ slot, int64_t nc, const Shift sh)
 {
-    using C = typename Store<S>::C;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= nc) return;
+    const int64_t i = slot[r];
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
-        const double v = src[k * n + i];
-        Store<S>::st(dst, k * n + i, stored_f64<S>(sh, v, k));
+        const double v = src[k * nc + r];
+        Store<S>::st(dst, at<Q>(k, i), stored_f64<S>(sh, v, k));
     }
 }
+// rho [nc] and u [3][nc] of the stored cells as FP64
 template <class C>
-__global__ void k_macro_to_f64(const C *src, double *dst, int64_t m)
+__global__ void k_macro_to_f64(const C *rho, const C *u, int64_t n, const int32_t *__restrict__ slot, int64_t nc,
+                               double *drho, double *du)
 {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i < m) dst[i] = (double)src[i];
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= nc) return;
+    const int64_t i = slot[r];
+    drho[r] = (double)rho[i];
+    du[r] = (double)u[i];
+    du[nc + r] = (double)u[n + i];
+    du[2 * nc + r] = (double)u[2 * n + i];
 }
 template <class S>
 __global__ void k_guard(const S *f, const S *fcol, int64_t total, int *err)
@@ -1596,22 +1627,24 @@ int band_collide(Ctx &ctx, Case &c, int l, void *out)
     return MT_OK;
 }
 
-// One fused brick pass of level l in the form `variant` (0 one cell per lane
-// step; 3 the lane's two cells in one unrolled sequence; for the reduced
-// storages also 1, a packed pair, and 2, one cell with more registers per
-// thread) on stream s, writing the next collision into fnext.
+// One fused brick pass of level l in the form `variant` (brick_warp) on stream
+// s, writing the next collision into fnext.
+inline BrickTab brick_tab(const Level &lv)
+{
+    return BrickTab{lv.blist, lv.bnbr, (const unsigned long long *)lv.bmask, lv.bcls, lv.bflag};
+}
 template <int Q, class S>
 void brick_launch(Case &c, int l, int variant, cudaStream_t s, S *fnext, int mac, int fall, long long *bacc)
 {
     using A = AmrTyped<S>;
     Level &lv = c.lv[l];
-    const unsigned g = grid_for(lv.nbrick, 4);
+    const unsigned g = grid_for(lv.nblist, 4);
+    if (!g) return;
     const uint32_t n32 = (uint32_t)lv.n;
     const int tb = c.d.stream_convention;
     auto go = [&](auto coll, auto v) {
         constexpr int COLL = decltype(coll)::value, V = decltype(v)::value;
-        k_brick_step<Q, S, COLL, V><<<g, 128, 0, s>>>(lv.nbrick, lv.bhalo, lv.bcls, n32, tb, A::fcol(lv), A::f(lv),
-                                                      fnext, c.d.tau[l], A::rho(lv), A::u(lv), mac, fall,
+        k_brick_step<Q, S, COLL, V><<<g, 128, 0, s>>>(lv.nblist, brick_tab(lv), n32, tb, A::fcol(lv), A::f(lv), fnext, c.d.tau[l], A::rho(lv), A::u(lv), mac, fall,
                                                       COLL == MT_COLL_LBGK ? bacc : nullptr, c.shift[l]);
     };
     using LB = std::integral_constant<int, MT_COLL_LBGK>;
@@ -1866,15 +1899,15 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
     }
     case PH_BAND_GRID:
         if (lv.nband && c.mgrid) {
-            k_band_grid<<<grid_for(lv.nband, 256), 256, 0, s>>>(lv.band, lv.nband, lv.key, c.mlo[0], c.mlo[1], c.mlo[2],
+            k_band_grid<<<grid_for(lv.nband, 256), 256, 0, s>>>(lv.band, lv.nband, lv.map(), c.mlo[0], c.mlo[1], c.mlo[2],
                                                                 c.mdim[0], c.mdim[1], c.mdim[2], c.mgrid);
             MT_LAUNCHED(ctx);
         }
         return MT_OK;
     case PH_SYNC_F:
-        if (lv.bricks) {
-            k_brick_pull<Q, S><<<grid_for(lv.nbrick, 4), 128, 0, s>>>(lv.nbrick, lv.bhalo, lv.bcls, (uint32_t)n,
-                                                                       c.d.stream_convention, A::fcol(lv), A::f(lv));
+        if (lv.bricks && lv.nblist) {
+            k_brick_pull<Q, S><<<grid_for(lv.nblist, 4), 128, 0, s>>>(lv.nblist, brick_tab(lv), c.d.stream_convention,
+                                                                       A::fcol(lv), A::f(lv));
             MT_LAUNCHED(ctx);
         }
         return MT_OK;
@@ -2056,9 +2089,9 @@ int AmrOps<S>::get(Ctx &ctx, Case &c, int l, int which, double *d_out)
     const S *src = (const S *)(which == 0 ? lv.f : lv.fcol);
     if (!lv.n) return MT_OK;
     if (c.d.q == 19)
-        k_to_f64<19, S><<<grid_for(lv.n, 256), 256, 0, ctx.stream>>>(src, d_out, lv.n, c.shift[l]);
+        k_to_f64<19, S><<<grid_for(lv.ncell, 256), 256, 0, ctx.stream>>>(src, d_out, lv.slot, lv.ncell, c.shift[l]);
     else
-        k_to_f64<27, S><<<grid_for(lv.n, 256), 256, 0, ctx.stream>>>(src, d_out, lv.n, c.shift[l]);
+        k_to_f64<27, S><<<grid_for(lv.ncell, 256), 256, 0, ctx.stream>>>(src, d_out, lv.slot, lv.ncell, c.shift[l]);
     MT_LAUNCHED(ctx);
     return MT_OK;
 }
@@ -2070,9 +2103,9 @@ int AmrOps<S>::set(Ctx &ctx, Case &c, int l, int which, const double *d_in)
     S *dst = (S *)(which == 0 ? lv.f : lv.fcol);
     if (!lv.n) return MT_OK;
     if (c.d.q == 19)
-        k_from_f64<19, S><<<grid_for(lv.n, 256), 256, 0, ctx.stream>>>(d_in, dst, lv.n, c.shift[l]);
+        k_from_f64<19, S><<<grid_for(lv.ncell, 256), 256, 0, ctx.stream>>>(d_in, dst, lv.slot, lv.ncell, c.shift[l]);
     else
-        k_from_f64<27, S><<<grid_for(lv.n, 256), 256, 0, ctx.stream>>>(d_in, dst, lv.n, c.shift[l]);
+        k_from_f64<27, S><<<grid_for(lv.ncell, 256), 256, 0, ctx.stream>>>(d_in, dst, lv.slot, lv.ncell, c.shift[l]);
     MT_LAUNCHED(ctx);
     return MT_OK;
 }
@@ -2083,9 +2116,8 @@ int AmrOps<S>::macros_out(Ctx &ctx, Case &c, int l, double *d_rho, double *d_u)
     using C = typename Store<S>::C;
     Level &lv = c.lv[l];
     if (!lv.n) return MT_OK;
-    k_macro_to_f64<C><<<grid_for(lv.n, 256), 256, 0, ctx.stream>>>((const C *)lv.rho, d_rho, lv.n);
-    MT_LAUNCHED(ctx);
-    k_macro_to_f64<C><<<grid_for(3 * lv.n, 256), 256, 0, ctx.stream>>>((const C *)lv.u, d_u, 3 * lv.n);
+    k_macro_to_f64<C><<<grid_for(lv.ncell, 256), 256, 0, ctx.stream>>>((const C *)lv.rho, (const C *)lv.u, lv.n,
+                                                                        lv.slot, lv.ncell, d_rho, d_u);
     MT_LAUNCHED(ctx);
     return MT_OK;
 }
@@ -2107,11 +2139,8 @@ int AmrOps<S>::batch_pass(Ctx &ctx, int q, int coll, const BrickBatch *d_desc, i
 }
 
 // ---- the brick pass autotuner (mt_case_tune_bricks) ----------------------
-// Each brick level's fused pass is timed in each of its forms (0 one cell per
-// lane step at 8 resident blocks per SM; 1 two cells with packed FP32 pairs;
-// 2 one cell at 6 blocks with more registers; 3 the lane's two cells in one
-// unrolled sequence at 6 blocks; FP64 has forms 0 and 3) on the case's own
-// bricks: one warm-up and three timed launches per form, CUDA
+// Each brick level's fused pass is timed in each of its forms (brick_warp; FP64
+// has forms 0 and 3) on the case's own bricks: one warm-up and three timed launches per form, CUDA
 // events on the case's stream.  The passes read the current post-collision
 // buffer and write the next collision into a scratch buffer; the f they
 // store is what the last real pass stored, and no macros are written, so the
@@ -2136,7 +2165,7 @@ int AmrOps<S>::tune_bricks(Ctx &ctx, Case &c, int32_t *variant, float *ms)
     int rc = MT_OK;
     for (int l = 0; l <= c.d.max_level && !rc; ++l) {
         Level &lv = c.lv[l];
-        if (!lv.bricks || !lv.nbrick) continue;
+        if (!lv.bricks || !lv.nblist) continue;
         float best = 0.f;
         int pick = lv.brick_variant;
         for (int v = 0; v < MT_BRICK_FORMS && !rc; ++v) {
@@ -2194,7 +2223,7 @@ __global__ void k_level_reduce(const S *f, int64_t n, const int32_t *list, int64
         double r = 0, jx = 0, jy = 0, jz = 0;
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
-            double v = (double)Store<S>::ld(f, (int64_t)k * n + i);
+            double v = (double)Store<S>::ld(f, at<Q>(k, i));
             if (Store<S>::shifted) v += sh.d[k];
             r += v;
             jx += v * ex(k);
@@ -2459,7 +2488,7 @@ __host__ __device__ __forceinline__ uint64_t cell_key_at(int L, int l, int64_t x
 
 template <class S> struct RemapLevels {
     struct Src {
-        const uint64_t *key = nullptr;
+        LevelMap map;
         const uint32_t *tag = nullptr;
         int64_t n = 0;
         const S *f = nullptr, *fcol = nullptr;
@@ -2478,22 +2507,23 @@ template <class S> struct RemapLevels {
 // (rho0, u0).  Solid cells hold zeros (the build's convention); a fluid cell
 // that is solid in the source takes the equilibrium at rest.  kind[i]: 0..3.
 template <int Q, class S>
-__global__ void k_remap(const uint64_t *dkey, const uint32_t *dtag, int64_t nd, int L, int l, RemapLevels<S> src,
+__global__ void k_remap(const LevelMap dmap, const int32_t *__restrict__ dslot, int64_t ncell, const uint32_t *dtag, int L, int l, RemapLevels<S> src,
                         double rho0, double ux0, double uy0, double uz0, S *fo, S *co, uint8_t *kind, const Shift dsh,
                         int same_shift)
 {
     using T = Store<S>;
     using C = typename T::C;
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= nd) return;
-    const uint64_t k = dkey[i];
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r >= ncell) return;
+    const int64_t i = dslot[r];
+    const uint64_t k = dmap.key(i);
     double a[Q], b[Q];
     auto put = [&](const double *pf, const double *pc, int kd) {
         for (int q = 0; q < Q; ++q) {
-            T::st(fo, q * nd + i, stored_sh<S>(dsh, (C)pf[q], q));
-            T::st(co, q * nd + i, stored_sh<S>(dsh, (C)pc[q], q));
+            T::st(fo, at<Q>(q, i), stored_sh<S>(dsh, (C)pf[q], q));
+            T::st(co, at<Q>(q, i), stored_sh<S>(dsh, (C)pc[q], q));
         }
-        kind[i] = (uint8_t)kd;
+        kind[r] = (uint8_t)kd;
     };
     if (dtag[i] & TAG_SF) {
         for (int q = 0; q < Q; ++q) a[q] = 0.0;
@@ -2501,7 +2531,7 @@ __global__ void k_remap(const uint64_t *dkey, const uint32_t *dtag, int64_t nd, 
         return;
     }
     const auto &same = src.lv[l];
-    int64_t j = same.n ? find_key(same.key, same.n, k) : -1;
+    int64_t j = same.n ? same.map.find(k) : -1;
     bool uncovered = false;
     if (j >= 0 && (same.tag[j] & TAG_SF)) {
         uncovered = true;
@@ -2510,16 +2540,16 @@ __global__ void k_remap(const uint64_t *dkey, const uint32_t *dtag, int64_t nd, 
     if (j >= 0) {
         if (same_shift) {
             for (int q = 0; q < Q; ++q) {
-                fo[q * nd + i] = same.f[q * same.n + j];
-                co[q * nd + i] = same.fcol[q * same.n + j];
+                fo[at<Q>(q, i)] = same.f[at<Q>(q, j)];
+                co[at<Q>(q, i)] = same.fcol[at<Q>(q, j)];
             }
         } else {
             for (int q = 0; q < Q; ++q) {
-                T::st(fo, q * nd + i, stored_sh<S>(dsh, full_v<S>(same.shift, T::ld(same.f, q * same.n + j), q), q));
-                T::st(co, q * nd + i, stored_sh<S>(dsh, full_v<S>(same.shift, T::ld(same.fcol, q * same.n + j), q), q));
+                T::st(fo, at<Q>(q, i), stored_sh<S>(dsh, full_v<S>(same.shift, T::ld(same.f, at<Q>(q, j)), q), q));
+                T::st(co, at<Q>(q, i), stored_sh<S>(dsh, full_v<S>(same.shift, T::ld(same.fcol, at<Q>(q, j)), q), q));
             }
         }
-        kind[i] = 0;
+        kind[r] = 0;
         return;
     }
     const int sh = L - l;
@@ -2529,11 +2559,11 @@ __global__ void k_remap(const uint64_t *dkey, const uint32_t *dtag, int64_t nd, 
         const auto &cs = src.lv[m];
         if (!cs.n) continue;
         const int up = l - m;
-        const int64_t jm = find_key(cs.key, cs.n, cell_key_at(L, m, x >> up, y >> up, z >> up));
+        const int64_t jm = cs.map.find(cell_key_at(L, m, x >> up, y >> up, z >> up));
         if (jm < 0) continue;
         for (int q = 0; q < Q; ++q) {
-            a[q] = (double)full_v<S>(cs.shift, T::ld(cs.f, q * cs.n + jm), q);
-            b[q] = (double)full_v<S>(cs.shift, T::ld(cs.fcol, q * cs.n + jm), q);
+            a[q] = (double)full_v<S>(cs.shift, T::ld(cs.f, at<Q>(q, jm)), q);
+            b[q] = (double)full_v<S>(cs.shift, T::ld(cs.fcol, at<Q>(q, jm)), q);
         }
         remap_rescale<Q>(a, src.up_f[m]);
         remap_rescale<Q>(b, src.up_c[m]);
@@ -2548,11 +2578,11 @@ __global__ void k_remap(const uint64_t *dkey, const uint32_t *dtag, int64_t nd, 
         for (int q = 0; q < Q; ++q) a[q] = b[q] = 0.0;
         for (int c = 0; c < side * side * side; ++c) {
             const int64_t cx = (x << d) + c % side, cy = (y << d) + (c / side) % side, cz = (z << d) + c / (side * side);
-            const int64_t jc = find_key(fine.key, fine.n, cell_key_at(L, l + d, cx, cy, cz));
+            const int64_t jc = fine.map.find(cell_key_at(L, l + d, cx, cy, cz));
             if (jc < 0 || (fine.tag[jc] & TAG_SF)) continue;
             for (int q = 0; q < Q; ++q) {
-                a[q] += (double)full_v<S>(fine.shift, T::ld(fine.f, q * fine.n + jc), q);
-                b[q] += (double)full_v<S>(fine.shift, T::ld(fine.fcol, q * fine.n + jc), q);
+                a[q] += (double)full_v<S>(fine.shift, T::ld(fine.f, at<Q>(q, jc)), q);
+                b[q] += (double)full_v<S>(fine.shift, T::ld(fine.fcol, at<Q>(q, jc)), q);
             }
             ++nch;
         }
@@ -2582,7 +2612,7 @@ int AmrOps<S>::remap(Ctx &ctx, Case &dst, Case &src, int64_t *counts)
     RemapLevels<S> rl;
     for (int m = 0; m <= L && m <= src.d.max_level; ++m) {
         if (!src.lv[m].n) continue;
-        rl.lv[m].key = src.lv[m].key;
+        rl.lv[m].map = src.lv[m].map();
         rl.lv[m].tag = src.lv[m].tag;
         rl.lv[m].n = src.lv[m].n;
         rl.lv[m].f = (const S *)src.lv[m].f;
@@ -2599,7 +2629,7 @@ int AmrOps<S>::remap(Ctx &ctx, Case &dst, Case &src, int64_t *counts)
     };
     uint8_t *kind = nullptr;
     int64_t maxn = 0;
-    for (int l = 0; l <= L; ++l) maxn = std::max(maxn, dst.lv[l].n);
+    for (int l = 0; l <= L; ++l) maxn = std::max(maxn, dst.lv[l].ncell);
     MT_CUDA(ctx, cudaMallocAsync(&kind, std::max<int64_t>(maxn, 1), ctx.stream));
     int rc = MT_OK;
     for (int l = 0; l <= L && !rc; ++l) {
@@ -2623,11 +2653,11 @@ int AmrOps<S>::remap(Ctx &ctx, Case &dst, Case &src, int64_t *counts)
         int same_shift = l <= src.d.max_level;
         for (int k = 0; k < 27; ++k) same_shift &= dst.shift[l].d[k] == src.shift[l].d[k];
         if (Q == 19)
-            k_remap<19, S><<<grid_for(lv.n, 128), 128, 0, ctx.stream>>>(lv.key, lv.tag, lv.n, L, l, rl, r0, u0, u1, u2,
+            k_remap<19, S><<<grid_for(lv.ncell, 128), 128, 0, ctx.stream>>>(lv.map(), lv.slot, lv.ncell, lv.tag, L, l, rl, r0, u0, u1, u2,
                                                                        (S *)lv.f, (S *)lv.fcol, kind, dst.shift[l],
                                                                        same_shift);
         else
-            k_remap<27, S><<<grid_for(lv.n, 128), 128, 0, ctx.stream>>>(lv.key, lv.tag, lv.n, L, l, rl, r0, u0, u1, u2,
+            k_remap<27, S><<<grid_for(lv.ncell, 128), 128, 0, ctx.stream>>>(lv.map(), lv.slot, lv.ncell, lv.tag, L, l, rl, r0, u0, u1, u2,
                                                                        (S *)lv.f, (S *)lv.fcol, kind, dst.shift[l],
                                                                        same_shift);
         cudaError_t e = cudaGetLastError();
@@ -2637,8 +2667,8 @@ int AmrOps<S>::remap(Ctx &ctx, Case &dst, Case &src, int64_t *counts)
         }
         ctx.launches++;
         if (counts) {
-            std::vector<uint8_t> hk((size_t)lv.n);
-            e = cudaMemcpyAsync(hk.data(), kind, lv.n, cudaMemcpyDeviceToHost, ctx.stream);
+            std::vector<uint8_t> hk((size_t)lv.ncell);
+            e = cudaMemcpyAsync(hk.data(), kind, lv.ncell, cudaMemcpyDeviceToHost, ctx.stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(ctx.stream);
             if (e != cudaSuccess) {
                 rc = set_err(ctx, MT_ERR_CUDA, std::string("remap counts: ") + cudaGetErrorString(e));

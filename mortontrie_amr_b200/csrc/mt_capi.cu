@@ -535,7 +535,7 @@ int mt_case_level_size(mt_ctx *h, int32_t id, int32_t level, int64_t *n)
     int rc = get_case(h, id, &c);
     if (rc) return rc;
     if (!n || level < 0 || level > c->d.max_level) return set_err(h->c, MT_ERR_ARG, "bad level");
-    *n = c->dense ? c->N : c->lv[level].n;
+    *n = c->dense ? c->N : c->lv[level].ncell;
     return MT_OK;
 }
 
@@ -555,12 +555,7 @@ int mt_case_get_keys(mt_ctx *h, int32_t id, int32_t level, uint64_t *keys, uint3
     }
     if (!c->built) return set_err(ctx, MT_ERR_STATE, "case not built");
     if (level < 0 || level > c->d.max_level) return set_err(ctx, MT_ERR_ARG, "bad level");
-    Level &lv = c->lv[level];
-    if (lv.n == 0) return MT_OK;
-    if (keys) MT_CUDA(ctx, cudaMemcpyAsync(keys, lv.key, 8 * lv.n, cudaMemcpyDeviceToHost, ctx.stream));
-    if (tags) MT_CUDA(ctx, cudaMemcpyAsync(tags, lv.tag, 4 * lv.n, cudaMemcpyDeviceToHost, ctx.stream));
-    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
-    return MT_OK;
+    return amr_get_keys(ctx, *c, level, keys, tags);
 }
 
 int mt_case_get_neighbors(mt_ctx *h, int32_t id, int32_t level, int32_t *nbr)
@@ -571,11 +566,7 @@ int mt_case_get_neighbors(mt_ctx *h, int32_t id, int32_t level, int32_t *nbr)
     Ctx &ctx = h->c;
     if (c->dense || !c->built) return set_err(ctx, MT_ERR_STATE, "neighbour tables exist for built multi-level cases");
     if (level < 0 || level > c->d.max_level || !nbr) return set_err(ctx, MT_ERR_ARG, "bad level");
-    Level &lv = c->lv[level];
-    if (lv.n == 0) return MT_OK;
-    MT_CUDA(ctx, cudaMemcpyAsync(nbr, lv.nbr, 4 * lv.n * (c->d.q - 1), cudaMemcpyDeviceToHost, ctx.stream));
-    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
-    return MT_OK;
+    return amr_get_neighbors(ctx, *c, level, nbr);
 }
 
 int mt_find(mt_ctx *h, int32_t id, int32_t level, const uint64_t *keys, int64_t n, int64_t *idx)
@@ -882,10 +873,7 @@ int mt_case_get_df_force_field(mt_ctx *h, int32_t id, int64_t *out)
     if (rc) return rc;
     Ctx &ctx = h->c;
     if (!out) return set_err(ctx, MT_ERR_ARG, "null output");
-    const size_t nb = sizeof(long long) * 3 * (size_t)c->lv[c->d.max_level].n;
-    MT_CUDA(ctx, cudaMemcpyAsync(out, c->acc, nb, cudaMemcpyDeviceToHost, ctx.stream));
-    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
-    return MT_OK;
+    return amr_df_force_field(ctx, *c, out, true);
 }
 
 int mt_case_set_df_force_field(mt_ctx *h, int32_t id, const int64_t *in)
@@ -895,9 +883,7 @@ int mt_case_set_df_force_field(mt_ctx *h, int32_t id, const int64_t *in)
     if (rc) return rc;
     Ctx &ctx = h->c;
     if (!in) return set_err(ctx, MT_ERR_ARG, "null input");
-    const size_t nb = sizeof(long long) * 3 * (size_t)c->lv[c->d.max_level].n;
-    MT_CUDA(ctx, cudaMemcpyAsync(c->acc, in, nb, cudaMemcpyHostToDevice, ctx.stream));
-    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
+    if ((rc = amr_df_force_field(ctx, *c, const_cast<int64_t *>(in), false))) return rc;
     c->primed = false;  // the band's next collision takes this force
     return MT_OK;
 }

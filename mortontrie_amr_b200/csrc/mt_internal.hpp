@@ -45,34 +45,49 @@ enum : int {
     DEVERR_NONFINITE = 8,         // NaN/Inf population found by the guard
 };
 
+// bflag bits
+enum : uint8_t {
+    BRICK_WORK = 1,      // some cell has work
+    BRICK_COMPLETE = 2,  // every source of every cell with work is stored
+    BRICK_UNIFORM = 4,   // all 64 cells are class 1
+};
+
 struct Level {
-    int64_t n = 0;
-    uint64_t *key = nullptr;   // sorted unique Morton keys
+    // slots: 64 per 4x4x4 Morton brick that holds a cell, bricks in key order;
+    // a slot without a cell has tag 0 and is in no list.  ncell cells are
+    // stored; in key order, cell r is slot[r], and a slot's rank is
+    // bstart[brick] + popcount(bmask[brick] below its local index).
+    int64_t n = 0, ncell = 0, nbrick = 0;
+    int low = 0;               // key bits below this level's cells
+    uint64_t *bkey = nullptr;
+    uint64_t *bmask = nullptr;
+    int32_t *bstart = nullptr;
+    int32_t *slot = nullptr;
+    // bnbr[27 * b + s] is the brick at offset (s % 3 - 1, s / 3 % 3 - 1, s / 9 - 1)
+    // or -1; exact (equal to the reference's find on every cell) when every
+    // periodic axis spans a multiple of 4 cells, else null
+    int32_t *bnbr = nullptr;
     uint32_t *tag = nullptr;
     int8_t *bcidx = nullptr;   // lat_bc index or -1
     int32_t *disrow = nullptr; // row in the dis table or -1
-    int32_t *nbr = nullptr;    // [(Q-1) * n]: index of the cell at key + e_k (k >= 1) or -1
-    void *f = nullptr, *fcol = nullptr;  // [Q * n] populations in the case's storage type
+    int32_t *nbr = nullptr;    // [(Q-1) * n]: slot of the cell at key + e_k (k >= 1) or -1
+    void *f = nullptr, *fcol = nullptr;  // populations in the case's storage type, at<Q>(k, slot)
     // fused schedule: the second post-collision buffer (the next substep's fcol,
     // swapped with fcol at each substep) and the lat_f cells it collides (IB
     // cells of the finest level excluded, they have their own kernel)
     void *fcol_alt = nullptr;
     int32_t *fused_list = nullptr; int64_t nfused = 0;
-    // 4x4x4 Morton bricks of the level's key set (fused schedule): a brick's
-    // cells are contiguous in key order, so a cell at local Morton index m is
-    // stored iff bit m of the brick's mask is set, at index
-    // start + popcount(mask & (2^m - 1)).  bnbr[27 * b + s] is the brick at
-    // offset (s % 3 - 1, s / 3 % 3 - 1, s / 9 - 1) or -1; bhalo resolves them per
-    // position of the 6x6x6 neighbourhood; bcls[64 * b + m] is
-    // the cell's work in the fused pass (0 none, 1 stream + collide, 2 stream + copy).
+    // the fused pass over bricks: bcls[slot] is the cell's work (0 none, 1
+    // stream + collide, 2 stream + copy, 3 as 1 with f stored, 4 a
+    // direct-forcing band cell), bflag[b] what the brick's cells share
+    // (BRICK_*), blist the bricks with any work
     bool bricks = false;
-    int brick_variant = 0;  // fused brick pass: 0 one cell per lane step, 1 two cells with packed FP32 pairs, 2 one cell with more registers, 3 both cells unrolled
-    int64_t nbrick = 0;
-    int32_t *bstart = nullptr;
-    uint64_t *bmask = nullptr;
-    int32_t *bnbr = nullptr;
+    int brick_variant = 0;  // form of the pass (mt_case_tune_bricks)
     uint8_t *bcls = nullptr;
-    int32_t *bhalo = nullptr;  // [216 * b]: cell index at each position of the brick's 6x6x6 neighbourhood, or -1
+    uint8_t *bflag = nullptr;
+    int32_t *blist = nullptr;
+    int64_t nblist = 0;
+    LevelMap map() const { return LevelMap{bkey, (const unsigned long long *)bmask, nbrick, low}; }
     void *rho = nullptr, *u = nullptr;   // [n], [3 * n] macroscopic fields (double, or float for reduced storage)
     int32_t *list[kNumSets] = {};
     int64_t nlist[kNumSets] = {};
@@ -101,8 +116,9 @@ struct Level {
 
 // one case level in a batched brick pass
 struct BrickSlot {
-    const int32_t *halo = nullptr;
-    const uint8_t *cls = nullptr;
+    const int32_t *list = nullptr, *nbr = nullptr;  // blist, bnbr
+    const unsigned long long *mask = nullptr;
+    const uint8_t *cls = nullptr, *flag = nullptr;
     const void *fcol = nullptr;  // current post-collision buffer
     void *f = nullptr, *fnext = nullptr, *rho = nullptr, *u = nullptr;
     long long *acc = nullptr;  // direct-forcing accumulator: band macros in the pass (finest level), else null
@@ -242,6 +258,11 @@ int amr_lbm_kernel(Ctx &ctx, Case &c, int level);
 int amr_step(Ctx &ctx, Case &c, int n);
 int amr_phase(Ctx &ctx, Case &c, int phase, int level);
 int amr_find(Ctx &ctx, Case &c, int level, const uint64_t *h_keys, int64_t n, int64_t *h_idx);
+// a level's cells in key order: keys and tags, the neighbour table by position,
+// the direct-forcing accumulator [3][ncell] (in either direction)
+int amr_get_keys(Ctx &ctx, Case &c, int level, uint64_t *h_keys, uint32_t *h_tags);
+int amr_get_neighbors(Ctx &ctx, Case &c, int level, int32_t *h_nbr);
+int amr_df_force_field(Ctx &ctx, Case &c, int64_t *h, bool get);
 int amr_guard(Ctx &ctx, Case &c, int *flags);
 int amr_get(Ctx &ctx, Case &c, int level, double *h_f, double *h_fcol);
 int amr_set(Ctx &ctx, Case &c, int level, const double *h_f, const double *h_fcol);

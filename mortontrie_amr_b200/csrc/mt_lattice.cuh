@@ -55,6 +55,9 @@ struct Shift {
     float dw[27];
     float u[3];
     double d[27];
+    // D3Q27: sums of s over the nine x lines (line = y + 3 z position) -- all
+    // three, the ends' difference, the ends' sum -- rounded to FP32
+    float k0[9], d1[9], s1[9];
 };
 inline Shift make_shift(int q, const double *us)
 {
@@ -69,6 +72,13 @@ inline Shift make_shift(int q, const double *us)
         s.dw[k] = (float)dw;
     }
     for (int a = 0; a < 3; ++a) s.u[a] = (float)us[a];
+    double line[9][3] = {};
+    for (int k = 0; k < q; ++k) line[(ey(k) + 1) + 3 * (ez(k) + 1)][ex(k) + 1] = s.d[k];
+    for (int j = 0; j < 9; ++j) {
+        s.k0[j] = (float)(line[j][0] + line[j][1] + line[j][2]);
+        s.d1[j] = (float)(line[j][2] - line[j][0]);
+        s.s1[j] = (float)(line[j][2] + line[j][0]);
+    }
     return s;
 }
 
@@ -166,6 +176,36 @@ MT_HD int64_t find_key(const uint64_t *k, int64_t n, uint64_t key)
     int64_t i = lower_bound_u64(k, n, key);
     return (i < n && k[i] == key) ? i : -1;
 }
+
+
+// Position of population k of slot i in a level's arrays.  A level is stored in
+// bricks of 4x4x4 cells, 64 slots each in Morton order whether or not every
+// cell exists, and a brick's Q x 64 populations are contiguous ([brick][Q][64]):
+// one brick's values of a direction fill whole 128-byte lines (one line at 16
+// bits), an x-adjacent pair of cells is an aligned word, and the Q accesses of
+// a cell differ by constant offsets.
+template <int Q> MT_HD constexpr int64_t at(int k, int64_t i) { return ((i >> 6) * Q + k) * 64 + (i & 63); }
+template <int Q> MT_HD constexpr int64_t at(int k, int32_t i) { return at<Q>(k, (int64_t)i); }
+template <int Q> MT_HD constexpr uint32_t at(int k, uint32_t i) { return ((i >> 6) * Q + k) * 64 + (i & 63); }
+
+// The stored cells of one level: brick keys in ascending order and each
+// brick's occupancy mask.  A cell's slot is 64 * brick + its local Morton index.
+struct LevelMap {
+    const uint64_t *bkey = nullptr;
+    const unsigned long long *bmask = nullptr;
+    int64_t nb = 0;
+    int low = 0;  // key bits below this level's cells
+    MT_HD uint64_t key(int64_t i) const { return (bkey[i >> 6] << (low + 6)) | ((uint64_t)(i & 63) << low); }
+    // the slot of a key, -1 where the level stores no such cell
+    MT_HD int64_t find(uint64_t k) const
+    {
+        if (k & (((uint64_t)1 << low) - 1)) return -1;
+        const int64_t b = find_key(bkey, nb, k >> (low + 6));
+        if (b < 0) return -1;
+        const int m = (int)((k >> low) & 63);
+        return ((bmask[b] >> m) & 1) ? 64 * b + m : -1;
+    }
+};
 
 // ---------------------------------------------------------------------------
 // FP64 physics in the reference's operation order

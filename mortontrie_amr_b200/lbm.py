@@ -503,9 +503,10 @@ class LBM_Manager:
         return out
 
     def tune_bricks(self):
-        """Time every form of every brick level's fused pass (0 one cell per
-        lane step, 1 a packed pair, 2 one cell with more registers, 3 the
-        lane's two cells unrolled together) and keep the fastest per level; returns (form per level, -1
+        """Time every form of every brick level's fused pass (reduced storages:
+        0, 2, 3 pairs of cells at different numbers of resident blocks, 1 one
+        cell per lane step; FP64: 0 one cell per lane step, 3 two unrolled)
+        and keep the fastest per level; returns (form per level, -1
         without bricks; ms per launch [level][form], -1 where not timed)."""
         v = np.zeros(self.L + 1, np.int32)
         ms = np.zeros((self.L + 1, BRICK_FORMS), np.float32)

@@ -210,6 +210,42 @@ def estimate_cells(spec: MeshSpec) -> list:
     return out
 
 
+def estimate_slots(spec: MeshSpec) -> list:
+    """Upper bound of the device slots per level: a level is stored in aligned
+    4x4x4 bricks of 64 slots, so its box with the ghost layer is rounded out
+    to whole bricks and only the bricks wholly under the next refinement box's
+    interior are left out; for an octree, the bricks each level's domain and
+    its one-cell layer touch."""
+    def bricks(lo, hi):
+        return int(np.prod([max(0, h - l) for l, h in zip(lo, hi)]))
+    if spec.octree is not None:
+        regions = octree_regions(spec)
+        out = [64 * bricks((0, 0, 0), tuple(-(-n // 4) for n in spec.coarse))]
+        for l in range(1, spec.max_level + 1):
+            d = regions[l].children().dilate(1)
+            c = (np.argwhere(d.mask) + d.lo) >> 2
+            c -= c.min(axis=0)
+            shape = c.max(axis=0) + 1
+            out.append(64 * int(np.unique(np.ravel_multi_index(c.T, shape)).size))
+        return out
+    out = []
+    lo, hi = (0, 0, 0), tuple(spec.coarse)
+    for l in range(spec.max_level + 1):
+        if bricks(lo, hi) == 0:
+            out.append(0)
+            continue
+        g = 1 if l > 0 else 0
+        n = bricks([(v - g) // 4 for v in lo], [-(-(v + g) // 4) for v in hi])
+        box = spec.refine[l] if l < spec.max_level else None
+        if box is not None:
+            n -= bricks([-(-(v + 1) // 4) for v in box[0]], [(v - 1) // 4 for v in box[1]])
+            lo, hi = tuple(2 * v for v in box[0]), tuple(2 * v for v in box[1])
+        else:
+            lo, hi = (0, 0, 0), (0, 0, 0)
+        out.append(64 * n)
+    return out
+
+
 class Region:
     """A set of cells of one level as a dense mask over its bounding box:
     cell (x, y, z) is in the set iff mask[x - lo[0], y - lo[1], z - lo[2]]."""

@@ -31,7 +31,7 @@ from typing import Optional
 import numpy as np
 
 from .case import CaseParams, df_sphere_case
-from .mesh import Markers, SpecMesh, Sphere, estimate_cells
+from .mesh import Markers, SpecMesh, Sphere, estimate_slots
 
 PERIOD = 2000          # finest steps of one oscillation
 AMPLITUDE = 0.5        # oscillation amplitude in sphere radii
@@ -166,15 +166,18 @@ def request_case(req: Request, mesh):
 
 def footprint_bytes(case, storage: str) -> int:
     """Device memory of a resident case: three population buffers, the
-    neighbour table, macros, tags and lists, bricks and halo tables."""
+    neighbour table, macros, tags and lists, brick tables (per slot: a level
+    is stored in whole 4x4x4 bricks)."""
     sb = {"f64": 8, "f32": 4, "f16": 2, "bf16": 2}[storage]
     q = case.params.q
     total = 0
     if isinstance(case.mesh, SpecMesh):
-        cells = estimate_cells(case.mesh.spec)
+        slots = estimate_slots(case.mesh.spec)
     else:
-        cells = [sum(int(v.size) for v in lv.values()) for lv in case.mesh.levels]
-    for n in cells:
+        top = case.mesh.spec.max_level
+        slots = [64 * int(np.unique(case.mesh.all_keys(l) >> np.uint64(3 * (top - l) + 6)).size)
+                 for l in range(top + 1)]
+    for n in slots:
         total += n * (3 * q * sb + 4 * (q - 1) + 4 * 4 + 8 + 4 + 16 + 8 + 20)
     total += int(case.mesh.markers.dv.size) * 80 if case.mesh.markers is not None else 0
     return total + (8 << 20)
