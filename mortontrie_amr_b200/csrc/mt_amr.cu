@@ -473,9 +473,12 @@ int amr_build(Ctx &ctx, Case &c)
         MT_LAUNCHED(ctx);
         int rc = select_indices(ctx, fl.n, IbLatf{fl.tag}, &fl.iblist, &fl.nib);
         if (rc) return rc;
-        // per-cell forces (3 * nib) and the 256-cell partial sums (3 * ceil(nib / 256))
-        if (fl.nib)
-            MT_CUDA(ctx, cudaMallocAsync(&c.ib_force, 8 * 3 * (fl.nib + grid_for(fl.nib, 256)), ctx.stream));
+        // the force partials of 32-cell blocks and the finished-block counter
+        if (fl.nib) {
+            const size_t bytes = 8 * (3 * (size_t)grid_for(fl.nib, 32) + 1);
+            MT_CUDA(ctx, cudaMallocAsync(&c.ib_force, bytes, ctx.stream));
+            MT_CUDA(ctx, cudaMemsetAsync(c.ib_force, 0, bytes, ctx.stream));
+        }
     }
     {
         int64_t maxn = 0;

@@ -497,51 +497,84 @@ __global__ void k_bc_set_eq(const int32_t *list, int64_t nl, int64_t n, double r
 // multi-direct-forcing sweeps (each cell only touches its own populations:
 // the sweeps run in registers).  g receives the new f, (fx, fy, fz) the
 // cell's momentum-exchange force.
+// The cell count is small (a sphere's skin), so the time is one thread's
+// chain of dependent loads: the wall distances of every link, then every
+// link's source slot, then every population are each read in one go, with
+// addresses selected instead of branches taken (a link without a source
+// reads the cell's own opposite population, which is its value), three
+// memory latencies in all; the walls are kept as a bit mask for the sweeps.
+// One launch, caches cold, D3Q19 FP16 / D3Q27 FP16 / D3Q27 FP64: 35 / 50 / 49 us
+// with the links' loads behind branches, 16 / 28 / 23 us so; two launches of
+// 4 us each that summed the force are gone (ib_force_sum).
+// FP32 multiplications and additions are paired into FMAs as written here
+// (pm_*), whatever surrounds them; in FP64 pm_fma is a multiplication and an
+// addition.
+__device__ __forceinline__ float pm_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float pm_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float pm_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double pm_mul(double a, double b) { return a * b; }
+__device__ __forceinline__ double pm_add(double a, double b) { return a + b; }
+__device__ __forceinline__ double pm_fma(double a, double b, double c) { return a * b + c; }
 template <int Q, int FH, class S>
-__device__ __forceinline__ void ib_cell(int64_t i, int64_t n, const double *dr, const int32_t *nbr, const S *fcol,
+__device__ __forceinline__ void ib_cell(int64_t i, int64_t n, const double *__restrict__ dr,
+                                        const int32_t *__restrict__ nbr, const S *__restrict__ fcol,
                                         typename Store<S>::C rho_b, typename Store<S>::C *g,
                                         typename Store<S>::C &fx, typename Store<S>::C &fy,
                                         typename Store<S>::C &fz, const Shift &sh)
 {
     using T = Store<S>;
     using C = typename T::C;
-    auto FC = [&](int k, int64_t idx) { return full_sh<S>(sh, T::ld(fcol, at<Q>(k, idx)), k); };
-    g[0] = FC(0, i);
+    C dd[Q], own[Q], src[Q];
+    uint32_t wall = 0;  // bit k: link k meets the wall
+#pragma unroll
+    for (int k = 1; k < Q; ++k) {
+        const double v = __ldg(dr + inv(k) - 1);
+        dd[k] = (C)v;
+        wall |= v != -1. ? 1u << k : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < Q; ++k) own[k] = T::ld(fcol, at<Q>(k, i));
+    int32_t si[Q];
+#pragma unroll
+    for (int k = 1; k < Q; ++k)
+        si[k] = __ldg(nbr + (int64_t)(((wall >> k) & 1 ? inv(k) : k) - 1) * n + i);
+#pragma unroll
+    for (int k = 1; k < Q; ++k) src[k] = T::ld(fcol, si[k] >= 0 ? at<Q>(k, si[k]) : at<Q>(inv(k), i));
+    g[0] = full_sh<S>(sh, own[0], 0);
     fx = 0;
     fy = 0;
     fz = 0;
 #pragma unroll
     for (int k = 1; k < Q; ++k) {
-        const C dd = (C)dr[inv(k) - 1];
-        if (dr[inv(k) - 1] != -1.) {
-            const C finc = FC(inv(k), i);
-            const int32_t si = nbr[(int64_t)(inv(k) - 1) * n + i];
-            const C fstr = si >= 0 ? FC(k, si) : finc;
+        // the value of a missing source is the cell's own opposite one
+        const C from = si[k] >= 0 ? full_sh<S>(sh, src[k], k) : full_sh<S>(sh, src[k], inv(k));
+        g[k] = from;
+        if ((wall >> k) & 1) {
+            const C finc = full_sh<S>(sh, own[inv(k)], inv(k));
+            const C fstr = from;
             C fnew;
             if (FH) {
-                if (dd < (C)0.5) {
-                    fnew = ((C)1.0 - (C)2.0 * dd) * finc + (C)2.0 * dd * fstr;
+                if (dd[k] < (C)0.5) {
+                    const C d2 = (C)2.0 * dd[k];
+                    fnew = pm_fma((C)1.0 - d2, finc, pm_mul(d2, fstr));
                 } else {
-                    const C feqw = (C)w19z(inv(k)) * rho_b;
-                    const C inv2d = (C)1.0 / ((C)2.0 * dd);
-                    fnew = inv2d * fstr + ((C)1.0 - inv2d) * feqw;
+                    const C feqw = pm_mul((C)w19z(inv(k)), rho_b);
+                    const C inv2d = (C)1.0 / ((C)2.0 * dd[k]);
+                    fnew = pm_fma(inv2d, fstr, pm_mul((C)1.0 - inv2d, feqw));
                 }
             } else {
-                fnew = ((C)1.0 - dd) * finc + dd * fstr;
+                fnew = pm_fma((C)1.0 - dd[k], finc, pm_mul(dd[k], fstr));
             }
             g[k] = fnew;
-            const C mt = finc + fnew;
-            fx += -mt * ex(k);
-            fy += -mt * ey(k);
-            fz += -mt * ez(k);
-        } else {
-            const int32_t si = nbr[(int64_t)(k - 1) * n + i];
-            g[k] = si < 0 ? FC(inv(k), i) : FC(k, si);
+            const C mt = pm_add(finc, fnew);
+            fx = pm_add(fx, -mt * ex(k));
+            fy = pm_add(fy, -mt * ey(k));
+            fz = pm_add(fz, -mt * ez(k));
         }
     }
     C ra = 0;
 #pragma unroll
-    for (int k = 0; k < Q; ++k) ra += g[k];
+    for (int k = 0; k < Q; ++k) ra = pm_add(ra, g[k]);
     if (ra < (C)0.3)
         g[0] += (C)1.0 * ((C)0.3 - ra);
     else if (ra < (C)0.5)
@@ -550,14 +583,15 @@ __device__ __forceinline__ void ib_cell(int64_t i, int64_t n, const double *dr, 
         g[0] += (C)1.0 * ((C)3.0 - ra);
     else if (ra > (C)2.0)
         g[0] += (C)0.5 * ((C)2.0 - ra);
+#pragma unroll 1
     for (int it = 0; it < 8; ++it) {
         C r = 0, ux = 0, uy = 0, uz = 0;
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
-            r += g[k];
-            ux += g[k] * ex(k);
-            uy += g[k] * ey(k);
-            uz += g[k] * ez(k);
+            r = pm_add(r, g[k]);
+            if (ex(k)) ux = pm_add(ux, ex(k) > 0 ? g[k] : -g[k]);
+            if (ey(k)) uy = pm_add(uy, ey(k) > 0 ? g[k] : -g[k]);
+            if (ez(k)) uz = pm_add(uz, ez(k) > 0 ? g[k] : -g[k]);
         }
         if (r <= (C)0.) continue;
         ux = ux / r;
@@ -565,36 +599,99 @@ __device__ __forceinline__ void ib_cell(int64_t i, int64_t n, const double *dr, 
         uz = uz / r;
         const C um = sqrt(ux * ux + uy * uy + uz * uz);
         if (um < (C)1e-10) continue;
-        const C mx = (C)-0.5 * r * ux, my = (C)-0.5 * r * uy, mz = (C)-0.5 * r * uz;
+        const C hr = pm_mul((C)-0.5, r);
+        const C mx = pm_mul(hr, ux), my = pm_mul(hr, uy), mz = pm_mul(hr, uz);
         C adj = 0;
 #pragma unroll
         for (int k = 1; k < Q; ++k) {
-            if (dr[inv(k) - 1] == -1.) continue;
-            const C df = (C)w19z(k) * (C)3.0 * (ex(k) * mx + ey(k) * my + ez(k) * mz);
-            g[k] += df;
-            adj -= df;
+            if (!((wall >> k) & 1)) continue;
+            C m = 0;
+            bool any = false;
+            auto part = [&](int e, C v) {
+                if (!e) return;
+                const C t = e > 0 ? v : -v;
+                m = any ? pm_add(m, t) : t;
+                any = true;
+            };
+            part(ex(k), mx);
+            part(ey(k), my);
+            part(ez(k), mz);
+            const C w3 = (C)w19z(k) * (C)3.0;
+            g[k] = pm_fma(w3, m, g[k]);
+            adj = pm_fma(-w3, m, adj);
         }
-        g[0] += adj;
+        g[0] = pm_add(g[0], adj);
+    }
+}
+
+// The force of one treat() call (LBM_Manager::accumIBForce) into the
+// accumulator, by the kernel that computed it: one warp per block adds its 32
+// cells in a fixed tree, and the last block to finish adds the blocks'
+// partials in block order (strided over the warp, then the same tree).
+// part: [3 * gridDim.x] partials, then the finished-block counter.
+constexpr int kIbBlock = 32;
+__device__ __forceinline__ void ib_force_sum(double fx, double fy, double fz, double *part, double *acc)
+{
+    const unsigned all = 0xffffffffu;
+    const int lane = threadIdx.x;
+    unsigned *done = (unsigned *)(part + 3 * (int64_t)gridDim.x);
+    auto tree = [&](double &x, double &y, double &z) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            x += __shfl_down_sync(all, x, o);
+            y += __shfl_down_sync(all, y, o);
+            z += __shfl_down_sync(all, z, o);
+        }
+    };
+    tree(fx, fy, fz);
+    unsigned last = 0;
+    if (lane == 0) {
+        double *p = part + 3 * (int64_t)blockIdx.x;
+        p[0] = fx;
+        p[1] = fy;
+        p[2] = fz;
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    }
+    if (!__shfl_sync(all, last, 0)) return;
+    __threadfence();
+    double x = 0., y = 0., z = 0.;
+    for (int64_t b = lane; b < gridDim.x; b += 32) {
+        x += __ldcg(part + 3 * b);
+        y += __ldcg(part + 3 * b + 1);
+        z += __ldcg(part + 3 * b + 2);
+    }
+    tree(x, y, z);
+    if (lane == 0) {
+        acc[0] += x;
+        acc[1] += y;
+        acc[2] += z;
+        acc[3] += 1.0;
+        *done = 0u;
     }
 }
 
 template <int Q, int FH, class S>
-__global__ void k_ib_treat(const int32_t *list, int64_t nl, int64_t n, const int32_t *disrow, const double *dis,
-                           const int32_t *nbr, const S *fcol, const typename Store<S>::C *rho, S *f, double *force, const Shift sh)
+__global__ void __launch_bounds__(kIbBlock) k_ib_treat(const int32_t *__restrict__ list, int64_t nl, int64_t n,
+                                                       const int32_t *__restrict__ disrow,
+                                                       const double *__restrict__ dis, const int32_t *__restrict__ nbr,
+                                                       const S *__restrict__ fcol,
+                                                       const typename Store<S>::C *__restrict__ rho, S *__restrict__ f,
+                                                       double *part, double *force, const Shift sh)
 {
     using T = Store<S>;
     using C = typename T::C;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= nl) return;
-    const int64_t i = list[j];
-    const double *dr = dis + (int64_t)disrow[i] * (Q - 1);
-    C g[Q], fx, fy, fz;
-    ib_cell<Q, FH, S>(i, n, dr, nbr, fcol, rho[i], g, fx, fy, fz, sh);
+    const int64_t j = blockIdx.x * (int64_t)kIbBlock + threadIdx.x;
+    C fx = 0, fy = 0, fz = 0;
+    if (j < nl) {
+        const int64_t i = list[j];
+        const double *dr = dis + (int64_t)disrow[i] * (Q - 1);
+        C g[Q];
+        ib_cell<Q, FH, S>(i, n, dr, nbr, fcol, rho[i], g, fx, fy, fz, sh);
 #pragma unroll
-    for (int k = 0; k < Q; ++k) T::st(f, at<Q>(k, i), stored_sh<S>(sh, g[k], k));
-    force[j] = (double)fx;
-    force[nl + j] = (double)fy;
-    force[2 * nl + j] = (double)fz;
+        for (int k = 0; k < Q; ++k) T::st(f, at<Q>(k, i), stored_sh<S>(sh, g[k], k));
+    }
+    ib_force_sum((double)fx, (double)fy, (double)fz, part, force);
 }
 
 // ---- fused schedule ---------------------------------------------------------
@@ -1130,44 +1227,43 @@ __global__ void __launch_bounds__(128) k_brick_pull(int64_t nb, const BrickTab t
 // rho_b is the density calculateMacros(level) gives at the start of the
 // substep: the macros of the cell's f before this treat.
 template <int Q, int FH, class S, int COLL>
-__global__ void k_ib_collide(const int32_t *list, int64_t nl, int64_t n, const int32_t *disrow, const double *dis,
-                             const int32_t *nbr, const S *fcol, S *f, S *fnext, double tau, double *force,
-                             typename Store<S>::C *rho, typename Store<S>::C *u, int macros, const Shift sh)
+__global__ void __launch_bounds__(kIbBlock) k_ib_collide(
+    const int32_t *__restrict__ list, int64_t nl, int64_t n, const int32_t *__restrict__ disrow,
+    const double *__restrict__ dis, const int32_t *__restrict__ nbr, const S *__restrict__ fcol, S *__restrict__ f,
+    S *__restrict__ fnext, double tau, double *part, double *force, typename Store<S>::C *__restrict__ rho,
+    typename Store<S>::C *__restrict__ u, int macros, const Shift sh)
 {
     using T = Store<S>;
     using C = typename T::C;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= nl) return;
-    const int64_t i = list[j];
-    const double *dr = dis + (int64_t)disrow[i] * (Q - 1);
-    C g[Q], fx, fy, fz;
-    {
-#pragma unroll
-        for (int k = 0; k < Q; ++k) g[k] = full_sh<S>(sh, T::ld(f, at<Q>(k, i)), k);
+    const int64_t j = blockIdx.x * (int64_t)kIbBlock + threadIdx.x;
+    C fx = 0, fy = 0, fz = 0;
+    if (j < nl) {
+        const int64_t i = list[j];
+        const double *dr = dis + (int64_t)disrow[i] * (Q - 1);
+        C g[Q];
         C r, x, y, z;
+#pragma unroll
+        for (int k = 0; k < Q; ++k) g[k] = full_sh<S>(sh, T::cv(f[at<Q>(k, i)]), k);
         macros_g<Q, C>(g, r, x, y, z);
         ib_cell<Q, FH, S>(i, n, dr, nbr, fcol, r, g, fx, fy, fz, sh);
-    }
 #pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        const C st = stored_sh<S>(sh, g[k], k);
-        T::st(f, at<Q>(k, i), st);
-        // the next collision reads the stored value
-        S sv;
-        T::st(&sv, 0, st);
-        g[k] = T::cv(sv);
+        for (int k = 0; k < Q; ++k) {
+            const C st = stored_sh<S>(sh, g[k], k);
+            T::st(f, at<Q>(k, i), st);
+            // the next collision reads the stored value
+            S sv;
+            T::st(&sv, 0, st);
+            g[k] = T::cv(sv);
+        }
+        macros_collide_store<Q, S, COLL>(g, r, x, y, z, tau, fnext, i, sh);
+        if (macros) {
+            rho[i] = r;
+            u[i] = x;
+            u[n + i] = y;
+            u[2 * n + i] = z;
+        }
     }
-    force[j] = (double)fx;
-    force[nl + j] = (double)fy;
-    force[2 * nl + j] = (double)fz;
-    C r, x, y, z;
-    macros_collide_store<Q, S, COLL>(g, r, x, y, z, tau, fnext, i, sh);
-    if (macros) {
-        rho[i] = r;
-        u[i] = x;
-        u[n + i] = y;
-        u[2 * n + i] = z;
-    }
+    ib_force_sum((double)fx, (double)fy, (double)fz, part, force);
 }
 
 // ---- direct-forcing immersed boundary (Lagrangian markers) --------------------
@@ -1407,45 +1503,6 @@ __global__ void k_band_collide(const int32_t *band, int64_t nb, int64_t n, doubl
                      (C(3) * (ez(k) - z) + C(9) * eu * ez(k)) * gz;
         const C out = d[k] - (d[k] - feq) * om + fpre * (C)w<Q>(k) * ge;
         T::st(fcol, at<Q>(k, i), stored_sh<S>(sh, out, k));
-    }
-}
-
-// fixed-order reduction of the per-cell IB force into the accumulator
-// (LBM_Manager::accumIBForce, one call per treat): stage 1 sums 256-cell
-// chunks into partials, stage 2 sums the partials in order
-static __global__ void k_force_partial(const double *force, int64_t nl, double *partial)
-{
-    __shared__ double s[3][256];
-    const int t = threadIdx.x;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + t;
-    for (int c = 0; c < 3; ++c) s[c][t] = j < nl ? force[c * nl + j] : 0.0;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (t < w)
-            for (int c = 0; c < 3; ++c) s[c][t] += s[c][t + w];
-        __syncthreads();
-    }
-    if (t == 0)
-        for (int c = 0; c < 3; ++c) partial[c * gridDim.x + blockIdx.x] = s[c][0];
-}
-
-static __global__ void k_force_reduce(const double *force, int64_t nl, double *acc)
-{
-    __shared__ double s[3][256];
-    const int t = threadIdx.x;
-    double a[3] = {0., 0., 0.};
-    for (int64_t j = t; j < nl; j += blockDim.x)
-        for (int c = 0; c < 3; ++c) a[c] += force[c * nl + j];
-    for (int c = 0; c < 3; ++c) s[c][t] = a[c];
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (t < w)
-            for (int c = 0; c < 3; ++c) s[c][t] += s[c][t + w];
-        __syncthreads();
-    }
-    if (t == 0) {
-        for (int c = 0; c < 3; ++c) acc[c] += s[c][0];
-        acc[3] += 1.0;
     }
 }
 
@@ -1830,19 +1887,16 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
             MT_LAUNCHED(ctx);
             return MT_OK;
         }
-        if (c.d.ib_method == MT_IB_FH)
-            k_ib_treat<Q, 1, S><<<grid_for(fl.nib, 64), 64, 0, s>>>(fl.iblist, fl.nib, fl.n, fl.disrow, c.dis, fl.nbr,
-                                                                     A::fcol(fl), A::rho(fl), A::f(fl), c.ib_force, c.shift[c.d.max_level]);
-        else
-            k_ib_treat<Q, 0, S><<<grid_for(fl.nib, 64), 64, 0, s>>>(fl.iblist, fl.nib, fl.n, fl.disrow, c.dis, fl.nbr,
-                                                                     A::fcol(fl), A::rho(fl), A::f(fl), c.ib_force, c.shift[c.d.max_level]);
-        MT_LAUNCHED(ctx);
-        // ib_force holds 3 * nib per-cell values followed by room for the partials
-        const unsigned nb = grid_for(fl.nib, 256);
-        double *partial = c.ib_force + 3 * fl.nib;
-        k_force_partial<<<nb, 256, 0, s>>>(c.ib_force, fl.nib, partial);
-        MT_LAUNCHED(ctx);
-        k_force_reduce<<<1, 256, 0, s>>>(partial, nb, c.force_acc);
+        {
+            const unsigned gi = grid_for(fl.nib, kIbBlock);
+            const Shift &fsh = c.shift[c.d.max_level];
+            if (c.d.ib_method == MT_IB_FH)
+                k_ib_treat<Q, 1, S><<<gi, kIbBlock, 0, s>>>(fl.iblist, fl.nib, fl.n, fl.disrow, c.dis, fl.nbr, A::fcol(fl),
+                                                            A::rho(fl), A::f(fl), c.ib_force, c.force_acc, fsh);
+            else
+                k_ib_treat<Q, 0, S><<<gi, kIbBlock, 0, s>>>(fl.iblist, fl.nib, fl.n, fl.disrow, c.dis, fl.nbr, A::fcol(fl),
+                                                            A::rho(fl), A::f(fl), c.ib_force, c.force_acc, fsh);
+        }
         MT_LAUNCHED(ctx);
         return MT_OK;
     }
@@ -1964,9 +2018,9 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
                 const double tau = c.d.tau[l];
                 auto ib = [&](auto fh, auto coll) {
                     constexpr int FH = decltype(fh)::value, COLL = decltype(coll)::value;
-                    k_ib_collide<Q, FH, S, COLL><<<grid_for(lv.nib, 64), 64, 0, is>>>(
+                    k_ib_collide<Q, FH, S, COLL><<<grid_for(lv.nib, kIbBlock), kIbBlock, 0, is>>>(
                         lv.iblist, lv.nib, n, lv.disrow, c.dis, lv.nbr, A::fcol(lv), A::f(lv), (S *)lv.fcol_alt, tau,
-                        c.ib_force, A::rho(lv), A::u(lv), mac, c.shift[l]);
+                        c.ib_force, c.force_acc, A::rho(lv), A::u(lv), mac, c.shift[l]);
                 };
                 using I0 = std::integral_constant<int, 0>;
                 using I1 = std::integral_constant<int, 1>;
@@ -1979,12 +2033,6 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
                         if (c.d.ib_method == MT_IB_FH) ib(I1{}, CU{}); else ib(I0{}, CU{});
                     }
                 }
-                MT_LAUNCHED(ctx);
-                const unsigned nb = grid_for(lv.nib, 256);
-                double *partial = c.ib_force + 3 * lv.nib;
-                k_force_partial<<<nb, 256, 0, is>>>(c.ib_force, lv.nib, partial);
-                MT_LAUNCHED(ctx);
-                k_force_reduce<<<1, 256, 0, is>>>(partial, nb, c.force_acc);
                 MT_LAUNCHED(ctx);
             }
         }

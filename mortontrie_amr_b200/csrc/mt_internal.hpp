@@ -156,7 +156,7 @@ struct Case {
     std::vector<uint8_t> h_reg[MT_MAX_LEVELS + 1];
     int64_t reg_lo[MT_MAX_LEVELS + 1][3] = {};
     int64_t reg_n[MT_MAX_LEVELS + 1][3] = {};
-    double *ib_force = nullptr;  // [3 * nib] per-cell force of the last treat()
+    double *ib_force = nullptr;  // force partials of treat() (ib_force_sum)
     double *force_acc = nullptr; // [4] fx, fy, fz, treat count
     double *h_force = nullptr;   // [6] page-locked: force_acc copy [4], then the guard flags (int) (mt_case_force_async)
     int *dev_err = nullptr;
