@@ -137,32 +137,40 @@ MT_HD void children(const MortonGeom &g, uint64_t code, int fine, uint64_t *ch)
 // explosion children (AMR_transDDF_explosion, LBM_Manager.cpp:1072-1128):
 // F2C sources need every child stored and skip children listed in dis;
 // ghost sources write only children in ghost_overlap_C2F and not in dis.
+// child[j]: the slot of the first child (the eight are consecutive), mask[j]
+// the slots to write.
 __global__ void k_expl_children(MortonGeom g, int fine, const int32_t *src, int64_t nsrc, int64_t nf2c,
-                                const LevelMap cmap, const LevelMap fmap, const uint32_t *ftag, const uint64_t *dkey, int64_t nd,
-                                int32_t *child, int *err)
+                                const LevelMap cmap, const LevelMap fmap, const uint32_t *ftag, const uint64_t *dkey,
+                                int64_t nd, int32_t *child, uint8_t *mask, int *err)
 {
     int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nsrc) return;
     uint64_t ch[8];
     children(g, cmap.key(src[j]), fine, ch);
+    const int64_t b = find_key(fmap.bkey, fmap.nb, ch[0] >> (fmap.low + 6));
+    const int m0 = (int)((ch[0] >> fmap.low) & 63);
+    const unsigned there = b >= 0 ? (unsigned)(fmap.bmask[b] >> m0) & 255u : 0u;
+    unsigned out = 0;
     for (int m = 0; m < 8; ++m) {
-        int32_t out = -1;
-        const bool in_dis = find_key(dkey, nd, ch[m]) >= 0;
-        const int64_t fi = fmap.find(ch[m]);
-        if (!in_dis) {
-            if (j < nf2c) {
-                if (fi < 0)
-                    atomicOr(err, DEVERR_MISSING_CHILD);
-                else
-                    out = (int32_t)fi;
-            } else if (fi >= 0 && (ftag[fi] & TAG_GC2F)) {
-                out = (int32_t)fi;
-            }
+        if (find_key(dkey, nd, ch[m]) >= 0) continue;
+        const bool stored = (there >> m) & 1u;
+        if (j < nf2c) {
+            if (!stored)
+                atomicOr(err, DEVERR_MISSING_CHILD);
+            else
+                out |= 1u << m;
+        } else if (stored && (ftag[64 * b + m0 + m] & TAG_GC2F)) {
+            out |= 1u << m;
         }
-        child[(int64_t)m * nsrc + j] = out;
     }
+    // slots without a cell may be written too: most sources (a ghost source has
+    // only its children next to the interface) then take whole-vector stores
+    if (out) out |= ~there & 255u;
+    child[j] = b >= 0 ? (int32_t)(64 * b + m0) : 0;
+    mask[j] = (uint8_t)out;
 }
 
+// child[j]: the slot of the first child; all eight are stored (else an error)
 __global__ void k_coal_children(MortonGeom g, int fine, const int32_t *src, int64_t nsrc, const LevelMap cmap,
                                 const LevelMap fmap, int32_t *child, int *err)
 {
@@ -170,11 +178,10 @@ __global__ void k_coal_children(MortonGeom g, int fine, const int32_t *src, int6
     if (j >= nsrc) return;
     uint64_t ch[8];
     children(g, cmap.key(src[j]), fine, ch);
-    for (int m = 0; m < 8; ++m) {
-        const int64_t fi = fmap.find(ch[m]);
-        if (fi < 0) atomicOr(err, DEVERR_MISSING_CHILD);
-        child[(int64_t)m * nsrc + j] = (int32_t)fi;
-    }
+    const int64_t b = find_key(fmap.bkey, fmap.nb, ch[0] >> (fmap.low + 6));
+    const int m0 = (int)((ch[0] >> fmap.low) & 63);
+    if (b < 0 || ((fmap.bmask[b] >> m0) & 255u) != 255u) atomicOr(err, DEVERR_MISSING_CHILD);
+    child[j] = b >= 0 ? (int32_t)(64 * b + m0) : 0;
 }
 
 // ---- the fused pass's tables over a level's bricks -----------------------------
@@ -200,9 +207,9 @@ __global__ void k_brick_cls(const uint32_t *tag, int64_t n, int ib_level, uint8_
 __global__ void k_brick_mark(const int32_t *child, int64_t count, uint8_t *bcls)
 {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (t >= count) return;
-    const int32_t ci = child[t];
-    if (ci >= 0 && bcls[ci] == 1) bcls[ci] = 3;
+    if (t >= 8 * count) return;
+    const int64_t ci = (int64_t)child[t >> 3] + (t & 7);
+    if (bcls[ci] == 1) bcls[ci] = 3;
 }
 
 // one warp per brick, two cells per lane
@@ -531,14 +538,15 @@ int amr_build(Ctx &ctx, Case &c)
         if (rc) return rc;
         fl.nexpl_f2c = cl.nlist[1];
         if (fl.nexpl) {
-            MT_CUDA(ctx, cudaMallocAsync(&fl.expl_child, 4 * 8 * fl.nexpl, ctx.stream));
+            MT_CUDA(ctx, cudaMallocAsync(&fl.expl_child, 4 * fl.nexpl, ctx.stream));
+            MT_CUDA(ctx, cudaMallocAsync(&fl.expl_mask, fl.nexpl, ctx.stream));
             k_expl_children<<<grid_for(fl.nexpl, 128), 128, 0, ctx.stream>>>(
                 c.geom, l, fl.expl_src, fl.nexpl, fl.nexpl_f2c, cl.map(), fl.map(), fl.tag, c.dis_key, c.ndis,
-                fl.expl_child, c.dev_err);
+                fl.expl_child, fl.expl_mask, c.dev_err);
             MT_LAUNCHED(ctx);
         }
         if (cl.nlist[1]) {
-            MT_CUDA(ctx, cudaMallocAsync(&cl.coal_child, 4 * 8 * cl.nlist[1], ctx.stream));
+            MT_CUDA(ctx, cudaMallocAsync(&cl.coal_child, 4 * cl.nlist[1], ctx.stream));
             k_coal_children<<<grid_for(cl.nlist[1], 128), 128, 0, ctx.stream>>>(
                 c.geom, l, cl.list[1], cl.nlist[1], cl.map(), fl.map(), cl.coal_child, c.dev_err);
             MT_LAUNCHED(ctx);
@@ -586,7 +594,7 @@ void amr_free(Case &c)
     for (int l = 0; l < kMaxLevels; ++l) {
         Level &lv = c.lv[l];
         void *ptrs[] = {lv.slot, lv.bkey, lv.tag, lv.bcidx, lv.disrow, lv.nbr, lv.f, lv.fcol, lv.rho, lv.u,
-                        lv.collide_list, lv.stream_list, lv.iblist, lv.expl_src, lv.expl_child, lv.coal_child,
+                        lv.collide_list, lv.stream_list, lv.iblist, lv.expl_src, lv.expl_child, lv.expl_mask, lv.coal_child,
                         lv.fcol_alt, lv.fused_list, lv.bstart, lv.bmask, lv.bnbr, lv.bcls, lv.bflag, lv.blist,
                         lv.band, lv.collide_nb, lv.draw_keys, lv.draw_set, lv.expl_prev, lv.info_prev};
         for (void *p : ptrs)
@@ -790,8 +798,8 @@ static int build_bricks(Ctx &ctx, Case &c, int l)
     k_brick_cls<<<grid_for(n, 256), 256, 0, ctx.stream>>>(lv.tag, n, ib_level, lv.bcls);
     MT_LAUNCHED(ctx);
     if (l > 0 && c.lv[l - 1].coal_child && c.lv[l - 1].nlist[1]) {
-        const int64_t cnt = 8 * c.lv[l - 1].nlist[1];
-        k_brick_mark<<<grid_for(cnt, 256), 256, 0, ctx.stream>>>(c.lv[l - 1].coal_child, cnt, lv.bcls);
+        const int64_t cnt = c.lv[l - 1].nlist[1];
+        k_brick_mark<<<grid_for(8 * cnt, 256), 256, 0, ctx.stream>>>(c.lv[l - 1].coal_child, cnt, lv.bcls);
         MT_LAUNCHED(ctx);
     }
     if (c.d.q == 19)

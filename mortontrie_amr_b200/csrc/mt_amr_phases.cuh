@@ -133,36 +133,53 @@ __global__ void k_collide(const int32_t *list, int64_t nl, int64_t n, double tau
 
 // fcol = f on overlap_C2F (Collision_Manager.cpp:45-52)
 template <int Q, class S>
-__global__ void k_copy_fcol(const int32_t *list, int64_t nl, int64_t n, const S *f, S *fcol)
+__global__ void k_copy_fcol(const int32_t *__restrict__ list, int64_t nl, const S *__restrict__ f,
+                            S *__restrict__ fcol)
 {
     const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nl) return;
     const int64_t i = list[j];
+    S v[Q];  // every load before the first store
 #pragma unroll
-    for (int k = 0; k < Q; ++k) fcol[at<Q>(k, i)] = f[at<Q>(k, i)];
+    for (int k = 0; k < Q; ++k) v[k] = f[at<Q>(k, i)];
+#pragma unroll
+    for (int k = 0; k < Q; ++k) fcol[at<Q>(k, i)] = v[k];
 }
 
-// ABPatternPull::stream (Stream_Manager.cpp:43-76): a missing neighbour keeps f
-template <int Q, class S>
-__global__ void k_stream(const int32_t *list, int64_t nl, int64_t n, int textbook, const int32_t *nbr, const S *fcol,
-                         S *f)
+// The eight children of a coarse cell are eight consecutive slots (base a
+// multiple of 8): per direction 16 bytes at 16-bit storage, 32 at FP32, 64 at
+// FP64, aligned.
+template <class S> __device__ __forceinline__ void store8(S *p, typename Store<S>::C v)
 {
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= nl) return;
-    const int64_t i = list[j];
-    f[at<Q>(0, i)] = fcol[at<Q>(0, i)];
+    constexpr int W = 16 / sizeof(S);  // values per 16-byte store
+    alignas(16) S w[W];
 #pragma unroll
-    for (int k = 1; k < Q; ++k) {
-        const int kk = textbook ? inv(k) : k;
-        const int32_t s = nbr[(int64_t)(kk - 1) * n + i];
-        if (s >= 0) f[at<Q>(k, i)] = fcol[at<Q>(k, s)];
+    for (int h = 0; h < W; ++h) Store<S>::st(w, h, v);
+#pragma unroll
+    for (int h = 0; h < 8 / W; ++h) ((uint4 *)p)[h] = *(const uint4 *)w;
+}
+template <class S> struct Eight {
+    static constexpr int W = 16 / sizeof(S);
+    uint4 w[8 / W];
+    __device__ __forceinline__ void load(const S *p)
+    {
+#pragma unroll
+        for (int h = 0; h < 8 / W; ++h) w[h] = __ldg((const uint4 *)p + h);
     }
-}
+    __device__ __forceinline__ typename Store<S>::C get(int m) const
+    {
+        return Store<S>::cv(((const S *)w)[m]);
+    }
+};
 
-// AMR_transDDF_explosion (LBM_Manager.cpp:1059-1129), eight threads per
-// coarse source cell, one per child: each computes the (identical) rescaled
-// populations and writes its own child, so the eight children of a source
-// (consecutive in key order) take one contiguous store per direction.
+// AMR_transDDF_explosion (LBM_Manager.cpp:1059-1129), one thread per coarse
+// source cell: the rescaled populations are the same for its children, written
+// by one vector store per direction (where a child is left out, by one store
+// per child).  child[j] the first child's slot, mask[j] the children written.
+// 4-level D3Q27 FP16 sphere, per launch up to 40 us with a thread per child,
+// which loaded and rescaled the same source eight times, 25 us so; the
+// coalescence, whose eight 2-byte loads per direction are one of 16 bytes,
+// 20 -> 13 us.
 // With a second post-collision buffer (fused schedule) the children of ghost
 // F2C cells (sources from nf2c on) are written to both: nothing else writes
 // them, and the reference keeps them over the second substep.
@@ -170,20 +187,19 @@ __global__ void k_stream(const int32_t *list, int64_t nl, int64_t n, int textboo
 // parent's previous step, [Q][ns]; the explosion then starts from
 // 1.5 fcol - 0.5 prev, the parent state extrapolated to the half step.
 template <int Q, class S>
-__global__ void k_explosion(const int32_t *__restrict__ src, const int32_t *__restrict__ child, int64_t ns,
-                            int64_t nc, const S *__restrict__ cfcol, int64_t nf, S *__restrict__ ffcol, double scale,
-                            S *__restrict__ ffcol2, int64_t nf2c, const Shift csh, const Shift fsh,
-                            const S *__restrict__ cprev = nullptr)
+__global__ void __launch_bounds__(64, 8) k_explosion(const int32_t *__restrict__ src, const int32_t *__restrict__ child,
+                                                  const uint8_t *__restrict__ mask, int64_t ns,
+                                                  const S *__restrict__ cfcol, S *__restrict__ ffcol, double scale,
+                                                  S *__restrict__ ffcol2, int64_t nf2c, const Shift csh,
+                                                  const Shift fsh, const S *__restrict__ cprev = nullptr)
 {
     using T = Store<S>;
     using C = typename T::C;
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t j = t >> 3;
-    const int m = (int)(t & 7);
+    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= ns) return;
-    const int32_t ch = child[(int64_t)m * ns + j];
-    if (ch < 0) return;
-    const int64_t i = src[j];
+    const unsigned mk = mask[j];
+    if (!mk) return;
+    const int64_t i = src[j], ch = child[j];
     C d[Q];
 #pragma unroll
     for (int k = 0; k < Q; ++k) d[k] = full_sh<S>(csh, T::ld(cfcol, at<Q>(k, i)), k);
@@ -193,13 +209,26 @@ __global__ void k_explosion(const int32_t *__restrict__ src, const int32_t *__re
     }
     C r, x, y, z;
     macros_g<Q, C>(d, r, x, y, z);
-    const bool both = ffcol2 && j >= nf2c;
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
         const C fe = feq_heluo_g<Q, C>(k, r, x, y, z);
-        const C v = stored_sh<S>(fsh, fe + (C)scale * (d[k] - fe), k);
-        T::st(ffcol, at<Q>(k, ch), v);
-        if (both) T::st(ffcol2, at<Q>(k, ch), v);
+        d[k] = stored_sh<S>(fsh, fe + (C)scale * (d[k] - fe), k);
+    }
+    const int nw = ffcol2 && j >= nf2c ? 2 : 1;
+#pragma unroll 1
+    for (int w = 0; w < nw; ++w) {
+        S *out = w ? ffcol2 : ffcol;
+        if (mk == 255u) {
+#pragma unroll
+            for (int k = 0; k < Q; ++k) store8<S>(out + at<Q>(k, ch), d[k]);
+        } else {
+#pragma unroll 1
+            for (int m = 0; m < 8; ++m)
+                if ((mk >> m) & 1u) {
+#pragma unroll
+                    for (int k = 0; k < Q; ++k) T::st(out, at<Q>(k, ch + m), d[k]);
+                }
+        }
     }
 }
 
@@ -215,27 +244,46 @@ __global__ void k_expl_save(const int32_t *__restrict__ src, int64_t ns, const S
     for (int k = 0; k < Q; ++k) prev[k * ns + j] = cfcol[at<Q>(k, i)];
 }
 
+// the mean of a coarse cell's eight children (first child's slot ch), summed in
+// the reference's child order
+template <int Q, class S>
+__device__ __forceinline__ void children_mean(const S *__restrict__ ff, int64_t ch, const Shift &fsh,
+                                              typename Store<S>::C *a)
+{
+    using C = typename Store<S>::C;
+    // as many directions' loads in flight as about 128 registers hold
+    constexpr int G = sizeof(S) == 2 ? Q : (sizeof(S) == 4 ? 14 : 7);
+#pragma unroll
+    for (int k0 = 0; k0 < Q; k0 += G) {
+        Eight<S> e[G];
+#pragma unroll
+        for (int h = 0; h < G; ++h)
+            if (k0 + h < Q) e[h].load(ff + at<Q>(k0 + h, ch));
+#pragma unroll
+        for (int h = 0; h < G; ++h) {
+            if (k0 + h >= Q) continue;
+            C s = 0;
+#pragma unroll
+            for (int m = 0; m < 8; ++m) s += full_sh<S>(fsh, e[h].get(m), k0 + h);
+            a[k0 + h] = s / (C)8.0;
+        }
+    }
+}
+
 // AMR_transDDF_coalescence (LBM_Manager.cpp:1131-1169)
 template <int Q, class S>
-__global__ void k_coalescence(const int32_t *list, const int32_t *child, int64_t nl, int64_t nc, S *cf, const S *ff,
-                              int64_t nf, double scale, const Shift csh, const Shift fsh)
+__global__ void __launch_bounds__(64) k_coalescence(const int32_t *__restrict__ list,
+                                                    const int32_t *__restrict__ child, int64_t nl, S *__restrict__ cf,
+                                                    const S *__restrict__ ff, double scale, const Shift csh,
+                                                    const Shift fsh)
 {
     using T = Store<S>;
     using C = typename T::C;
     const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nl) return;
     const int64_t i = list[j];
-    int32_t ch[8];
-#pragma unroll
-    for (int m = 0; m < 8; ++m) ch[m] = child[(int64_t)m * nl + j];
     C a[Q];
-#pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        C s = 0;
-#pragma unroll
-        for (int m = 0; m < 8; ++m) s += full_sh<S>(fsh, T::ld(ff, at<Q>(k, ch[m])), k);
-        a[k] = s / (C)8.0;
-    }
+    children_mean<Q, S>(ff, child[j], fsh, a);
     C r, x, y, z;
     macros_g<Q, C>(a, r, x, y, z);
 #pragma unroll
@@ -251,8 +299,8 @@ __global__ void k_coalescence(const int32_t *list, const int32_t *child, int64_t
 // macros of that f are written when `macros` is set (the level's last
 // substep of the coarse step: calculateMacros of every level follows).
 template <int Q, class S, int COLL>
-__global__ void k_coal_collide(const int32_t *__restrict__ list, const int32_t *__restrict__ child, int64_t nl,
-                               int64_t nc, S *__restrict__ cf, const S *__restrict__ ff, int64_t nf, double scale,
+__global__ void __launch_bounds__(64) k_coal_collide(const int32_t *__restrict__ list, const int32_t *__restrict__ child, int64_t nl,
+                               int64_t nc, S *__restrict__ cf, const S *__restrict__ ff, double scale,
                                double tau, S *__restrict__ cfnext, typename Store<S>::C *__restrict__ rho,
                                typename Store<S>::C *__restrict__ u, int macros, const Shift csh,
                                const Shift fsh)
@@ -262,17 +310,8 @@ __global__ void k_coal_collide(const int32_t *__restrict__ list, const int32_t *
     const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nl) return;
     const int64_t i = list[j];
-    int32_t ch[8];
-#pragma unroll
-    for (int m = 0; m < 8; ++m) ch[m] = child[(int64_t)m * nl + j];
     C a[Q];
-#pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        C s = 0;
-#pragma unroll
-        for (int m = 0; m < 8; ++m) s += full_sh<S>(fsh, T::ld(ff, at<Q>(k, ch[m])), k);
-        a[k] = s / (C)8.0;
-    }
+    children_mean<Q, S>(ff, child[j], fsh, a);
     C r, x, y, z;
     macros_g<Q, C>(a, r, x, y, z);
 #pragma unroll
@@ -369,30 +408,35 @@ __global__ void k_bc_neq_all(const int32_t *list, const int8_t *setb, int64_t nl
 // equilibrium at the boundary cell's own, never-updated density), East wall
 // cells copy the inner cell's fcol (BC/Outflow.cpp:39-52).
 template <int Q, class S>
-__global__ void k_bc_inout(const int32_t *list, int64_t nl, int east, int64_t n, const int32_t *nbr, double rho0,
-                           S *f, S *fcol, double ubx, double uby, double ubz, int *err, const Shift sh)
+__global__ void __launch_bounds__(64) k_bc_inout(const int32_t *__restrict__ west, int64_t nw,
+                                                 const int32_t *__restrict__ east, int64_t ne, int64_t n,
+                                                 const int32_t *__restrict__ nbr, double rho0, S *__restrict__ f,
+                                                 S *__restrict__ fcol, double ubx, double uby, double ubz, int *err,
+                                                 const Shift sh)
 {
     using T = Store<S>;
     using C = typename T::C;
     const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= nl) return;
-    const int64_t i = list[j];
-    const int32_t nb = nbr[(int64_t)((east ? 2 : 1) - 1) * n + i];
+    if (j >= nw + ne) return;
+    const bool out = j >= nw;
+    const int64_t i = out ? east[j - nw] : west[j];
+    const int32_t nb = nbr[(int64_t)((out ? 2 : 1) - 1) * n + i];
     if (nb < 0) {
         atomicOr(err, DEVERR_MISSING_BC_NBR);
         return;
     }
+    S v[Q];
+    if (out) {
+#pragma unroll
+        for (int k = 0; k < Q; ++k) v[k] = fcol[at<Q>(k, nb)];
+    } else {
+#pragma unroll
+        for (int k = 0; k < Q; ++k) T::st(v, k, stored_sh<S>(sh, feq_g<Q, C>(k, (C)rho0, (C)ubx, (C)uby, (C)ubz), k));
+    }
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
-        if (east) {
-            const S v = fcol[at<Q>(k, nb)];
-            fcol[at<Q>(k, i)] = v;
-            f[at<Q>(k, i)] = v;
-        } else {
-            const C v = stored_sh<S>(sh, feq_g<Q, C>(k, (C)rho0, (C)ubx, (C)uby, (C)ubz), k);
-            T::st(fcol, at<Q>(k, i), v);
-            T::st(f, at<Q>(k, i), v);
-        }
+        fcol[at<Q>(k, i)] = v[k];
+        f[at<Q>(k, i)] = v[k];
     }
 }
 
@@ -728,6 +772,17 @@ __device__ __forceinline__ void pull_cell(int64_t i, int64_t n, int textbook, co
 #pragma unroll
     for (int k = 1; k < Q; ++k) src[k] = __ldg(nbr + (int64_t)((textbook ? inv(k) : k) - 1) * n + i);
     pull_src<Q, S>(i, n, src, fcol, f, v);
+}
+
+// ABPatternPull::stream (Stream_Manager.cpp:43-76): a missing neighbour keeps f
+template <int Q, class S>
+__global__ void k_stream(const int32_t *__restrict__ list, int64_t nl, int64_t n, int textbook,
+                         const int32_t *__restrict__ nbr, const S *__restrict__ fcol, S *__restrict__ f)
+{
+    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (j >= nl) return;
+    S v[Q];
+    pull_cell<Q, S>(list[j], n, textbook, nbr, fcol, f, v);
 }
 
 // ABPatternPull::stream then the next collide, on lat_f cells that are not IB
@@ -1544,13 +1599,15 @@ __global__ void k_macro_to_f64(const C *rho, const C *u, int64_t n, const int32_
     du[nc + r] = (double)u[n + i];
     du[2 * nc + r] = (double)u[2 * n + i];
 }
+// (slots without a cell hold anything)
 template <class S>
-__global__ void k_guard(const S *f, const S *fcol, int64_t total, int *err)
+__global__ void k_guard(const S *f, const S *fcol, const uint32_t *__restrict__ tag, int q, int64_t total, int *err)
 {
     int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     bool bad = false;
     for (; j < total; j += (int64_t)gridDim.x * blockDim.x)
-        bad |= !isfinite((double)Store<S>::ld(f, j)) || !isfinite((double)Store<S>::ld(fcol, j));
+        if (tag[(j / (64 * q)) * 64 + (j & 63)])
+            bad |= !isfinite((double)Store<S>::ld(f, j)) || !isfinite((double)Store<S>::ld(fcol, j));
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(err, DEVERR_NONFINITE);
 }
 
@@ -1754,7 +1811,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         }
         if (int rc = band_collide<S, Q>(ctx, c, l, A::fcol(lv))) return rc;
         if (lv.nlist[2]) {
-            k_copy_fcol<Q, S><<<grid_for(lv.nlist[2], B), B, 0, s>>>(lv.list[2], lv.nlist[2], n, A::f(lv),
+            k_copy_fcol<Q, S><<<grid_for(lv.nlist[2], B), B, 0, s>>>(lv.list[2], lv.nlist[2], A::f(lv),
                                                                       A::fcol(lv));
             MT_LAUNCHED(ctx);
         }
@@ -1777,8 +1834,8 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         const double scale = c2f_scale(c, l);
         const bool ex = phase == PH_EXPLOSION_B && c.itime == MT_ITIME_EXTRAP;
         if (ex && !lv.expl_prev) return set_err(ctx, MT_ERR_STATE, "extrapolated explosion without saved sources");
-        k_explosion<Q, S><<<grid_for(8 * lv.nexpl, B), B, 0, s>>>(lv.expl_src, lv.expl_child, lv.nexpl, cl.n, A::fcol(cl),
-                                                               n, A::fcol(lv), scale, (S *)lv.fcol_alt,
+        k_explosion<Q, S><<<grid_for(lv.nexpl, 64), 64, 0, s>>>(lv.expl_src, lv.expl_child, lv.expl_mask, lv.nexpl,
+                                                               A::fcol(cl), A::fcol(lv), scale, (S *)lv.fcol_alt,
                                                                lv.nexpl_f2c, c.shift[l - 1], c.shift[l],
                                                                ex ? (const S *)lv.expl_prev : nullptr);
         MT_LAUNCHED(ctx);
@@ -1802,8 +1859,8 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         if (l >= c.d.max_level || !lv.nlist[1]) return MT_OK;
         Level &fl = c.lv[l + 1];
         const double scale = f2c_scale(c, l);
-        k_coalescence<Q, S><<<grid_for(lv.nlist[1], B), B, 0, s>>>(lv.list[1], lv.coal_child, lv.nlist[1], n,
-                                                                    A::f(lv), A::f(fl), fl.n, scale, c.shift[l], c.shift[l + 1]);
+        k_coalescence<Q, S><<<grid_for(lv.nlist[1], 64), 64, 0, s>>>(lv.list[1], lv.coal_child, lv.nlist[1], A::f(lv),
+                                                                      A::f(fl), scale, c.shift[l], c.shift[l + 1]);
         MT_LAUNCHED(ctx);
         return MT_OK;
     }
@@ -1870,11 +1927,15 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
     }
     case PH_BC_INOUT: {
         Level &l0 = c.lv[0];
-        for (int face = 0; face < 2; ++face) {
-            if (!l0.nbc[face]) continue;
-            k_bc_inout<Q, S><<<grid_for(l0.nbc[face], B), B, 0, s>>>(l0.bclist[face], l0.nbc[face], face, l0.n, l0.nbr,
-                                                                      c.d.rho0, A::f(l0), A::fcol(l0), c.face_u[0][0],
-                                                                      c.face_u[0][1], c.face_u[0][2], c.dev_err, c.shift[0]);
+        // one launch for both faces, unless East's inner neighbours are West cells
+        const int64_t nw = l0.nbc[0], ne = l0.nbc[1];
+        const bool one = c.d.extent0[0] > 2;
+        for (int part = 0; part < (one ? 1 : 2); ++part) {
+            const int64_t mw = one || part == 0 ? nw : 0, me = one || part == 1 ? ne : 0;
+            if (mw + me == 0) continue;
+            k_bc_inout<Q, S><<<grid_for(mw + me, 64), 64, 0, s>>>(
+                l0.bclist[0], mw, l0.bclist[1], me, l0.n, l0.nbr, c.d.rho0, A::f(l0), A::fcol(l0), c.face_u[0][0],
+                c.face_u[0][1], c.face_u[0][2], c.dev_err, c.shift[0]);
             MT_LAUNCHED(ctx);
         }
         return MT_OK;
@@ -1920,12 +1981,12 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         const double scale = f2c_scale(c, l);
         if (c.d.collision == MT_COLL_LBGK) {
             k_coal_collide<Q, S, MT_COLL_LBGK><<<grid_for(lv.nlist[1], 64), 64, 0, s>>>(
-                lv.list[1], lv.coal_child, lv.nlist[1], n, A::f(lv), A::f(fl), fl.n, scale, c.d.tau[l],
+                lv.list[1], lv.coal_child, lv.nlist[1], n, A::f(lv), A::f(fl), scale, c.d.tau[l],
                 (S *)lv.fcol_alt, A::rho(lv), A::u(lv), c.macros_now, c.shift[l], c.shift[l + 1]);
         } else {
             if constexpr (Q == 27)
                 k_coal_collide<Q, S, MT_COLL_CUMULANT><<<grid_for(lv.nlist[1], 64), 64, 0, s>>>(
-                    lv.list[1], lv.coal_child, lv.nlist[1], n, A::f(lv), A::f(fl), fl.n, scale, c.d.tau[l],
+                    lv.list[1], lv.coal_child, lv.nlist[1], n, A::f(lv), A::f(fl), scale, c.d.tau[l],
                     (S *)lv.fcol_alt, A::rho(lv), A::u(lv), c.macros_now, c.shift[l], c.shift[l + 1]);
         }
         MT_LAUNCHED(ctx);
@@ -1988,7 +2049,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
             if (int rc = band_collide<S, Q>(ctx, c, l, lv.fcol_alt)) return rc;
         }
         if (lv.nlist[2]) {
-            k_copy_fcol<Q, S><<<grid_for(lv.nlist[2], B), B, 0, s>>>(lv.list[2], lv.nlist[2], n, A::f(lv),
+            k_copy_fcol<Q, S><<<grid_for(lv.nlist[2], B), B, 0, s>>>(lv.list[2], lv.nlist[2], A::f(lv),
                                                                       (S *)lv.fcol_alt);
             MT_LAUNCHED(ctx);
         }
@@ -2500,7 +2561,7 @@ int AmrOps<S>::guard(Ctx &ctx, Case &c, bool current_only)
         if (!lv.n) continue;
         const int64_t total = lv.n * c.d.q;
         k_guard<S><<<(unsigned)std::min<int64_t>(grid_for(total, 256), 148 * 16), 256, 0, ctx.stream>>>(
-            (const S *)(current_only ? lv.fcol : lv.f), (const S *)lv.fcol, total, c.dev_err);
+            (const S *)(current_only ? lv.fcol : lv.f), (const S *)lv.fcol, lv.tag, c.d.q, total, c.dev_err);
         MT_LAUNCHED(ctx);
     }
     return MT_OK;

@@ -99,11 +99,12 @@ struct Level {
     int32_t *band = nullptr; int64_t nband = 0;             // direct-forcing band (finest level)
     int32_t *collide_nb = nullptr; int64_t ncollide_nb = 0; // lat_f (not band) then F2C
     // explosion sources on the parent level (F2C then ghost F2C) and their children on this level
-    int32_t *expl_src = nullptr; int32_t *expl_child = nullptr; int64_t nexpl = 0, nexpl_f2c = 0;
+    // (eight consecutive slots: the first child's, and which of them are written)
+    int32_t *expl_src = nullptr; int32_t *expl_child = nullptr; uint8_t *expl_mask = nullptr; int64_t nexpl = 0, nexpl_f2c = 0;
     void *expl_prev = nullptr;  // MT_ITIME_EXTRAP: [Q * nexpl] the sources' parent values at the parent's previous step
     double *info_prev = nullptr;  // mt_case_info: [3][nlist[0]] the lat_f velocities the last call saw
     bool info_have = false;
-    // coalescence: F2C cells of this level and their children on the next level
+    // coalescence: the first child's slot on the next level of each F2C cell of this one
     int32_t *coal_child = nullptr;
     // raw uploads, consumed by the build
     std::vector<uint64_t> raw_keys;
