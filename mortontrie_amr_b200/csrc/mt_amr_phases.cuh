@@ -964,63 +964,6 @@ __device__ __forceinline__ void brick_cell(uint32_t i, int cls, bool complete, c
     }
 }
 
-// Two x-adjacent cells of the reduced storages as one word: slots 2p and
-// 2p + 1 differ in x bit 0 only, so a direction's values of both are an
-// aligned 32-bit (FP16, BF16) or 64-bit (FP32) word.
-template <class S> struct CellPair {
-    using W = uint32_t;
-    using V = typename std::conditional<std::is_same<S, __half>::value, __half2, __nv_bfloat162>::type;
-    static __device__ __forceinline__ W ld(const S *p) { return __ldg((const unsigned int *)p); }
-    static __device__ __forceinline__ void st(S *p, W w) { *(unsigned int *)p = w; }
-    // (second of a, first of b)
-    static __device__ __forceinline__ W straddle(W a, W b) { return __byte_perm(a, b, 0x5432); }
-    static __device__ __forceinline__ float2 f2(W w)
-    {
-        V v;
-        memcpy(&v, &w, 4);
-        if constexpr (std::is_same<S, __half>::value)
-            return __half22float2(v);
-        else
-            return __bfloat1622float2(v);
-    }
-    static __device__ __forceinline__ W word(float2 x)
-    {
-        V v;
-        if constexpr (std::is_same<S, __half>::value)
-            v = __float22half2_rn(x);
-        else
-            v = __float22bfloat162_rn(x);
-        W w;
-        memcpy(&w, &v, 4);
-        return w;
-    }
-    static __device__ __forceinline__ void st_one(S *p, W w, int h)
-    {
-        ((unsigned short *)p)[h] = (unsigned short)(h ? w >> 16 : w);
-    }
-    static __device__ __forceinline__ void put(W &w, int h, const S *p)
-    {
-        const unsigned int v = ((const unsigned short *)p)[h];
-        w = h ? (w & 0xffffu) | (v << 16) : (w & 0xffff0000u) | v;
-    }
-};
-template <> struct CellPair<float> {
-    using W = float2;
-    static __device__ __forceinline__ W ld(const float *p) { return __ldg((const float2 *)p); }
-    static __device__ __forceinline__ void st(float *p, W w) { *(float2 *)p = w; }
-    static __device__ __forceinline__ W straddle(W a, W b) { return make_float2(a.y, b.x); }
-    static __device__ __forceinline__ float2 f2(W w) { return w; }
-    static __device__ __forceinline__ W word(float2 x) { return x; }
-    static __device__ __forceinline__ void st_one(float *p, W w, int h) { p[h] = h ? w.y : w.x; }
-    static __device__ __forceinline__ void put(W &w, int h, const float *p)
-    {
-        if (h)
-            w.y = p[1];
-        else
-            w.x = p[0];
-    }
-};
-
 // The gather of a pair, lane = its y, z, x coordinates' bits (y0 z0 x1 y1 z1).
 // For each (y, z) offset the sources are the pair at the same x and, for
 // e_x = +-1, also the next pair on that side, whose near cell completes the

@@ -20,46 +20,13 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
+
 #include "mt_internal.hpp"
+#include "mt_pack2.cuh"
+#include "mt_store.cuh"
 
 namespace mt {
-
-// index type I: uint32_t while the array fits 2^32 elements (one wide
-// multiply-add per address), int64_t beyond
-template <class S> struct Store;
-template <> struct Store<double> {
-    using C = double;
-    static constexpr bool shifted = false;
-    template <class I> __device__ static __forceinline__ double ld(const double *p, I i) { return __ldg(p + i); }
-    template <class I> __device__ static __forceinline__ void st(double *p, I i, double v) { p[i] = v; }
-};
-template <> struct Store<float> {
-    using C = float;
-    static constexpr bool shifted = true;
-    template <class I> __device__ static __forceinline__ float ld(const float *p, I i) { return __ldg(p + i); }
-    template <class I> __device__ static __forceinline__ void st(float *p, I i, float v) { p[i] = v; }
-};
-template <> struct Store<__half> {
-    using C = float;
-    static constexpr bool shifted = true;
-    template <class I> __device__ static __forceinline__ float ld(const __half *p, I i)
-    {
-        return __half2float(__ldg(p + i));
-    }
-    template <class I> __device__ static __forceinline__ void st(__half *p, I i, float v) { p[i] = __float2half_rn(v); }
-};
-template <> struct Store<__nv_bfloat16> {
-    using C = float;
-    static constexpr bool shifted = true;
-    template <class I> __device__ static __forceinline__ float ld(const __nv_bfloat16 *p, I i)
-    {
-        return __bfloat162float(__ldg(p + i));
-    }
-    template <class I> __device__ static __forceinline__ void st(__nv_bfloat16 *p, I i, float v)
-    {
-        p[i] = __float2bfloat16_rn(v);
-    }
-};
 
 struct DenseGeom {
     uint32_t m[3];  // per-axis bit masks within the 3b index bits
@@ -82,78 +49,13 @@ __device__ __forceinline__ uint32_t dense_nbr(const DenseGeom &g, uint32_t i, in
 
 enum { DM_FUSED = 0, DM_COLLIDE = 1, DM_PULL = 2 };
 
-// FP32 LBGK on deviations s_k = f_k - w_k: fcol - w = s + omega (feq - f)
-template <int Q>
-__device__ __forceinline__ void lbgk_dev(float *s, float omega)
-{
-    float dr = 0.f, jx = 0.f, jy = 0.f, jz = 0.f;
-#pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        dr += s[k];
-        if (ex(k)) jx += ex(k) * s[k];
-        if (ey(k)) jy += ey(k) * s[k];
-        if (ez(k)) jz += ez(k) * s[k];
-    }
-    const float rho = 1.f + dr;
-    const float ir = 1.f / rho;
-    const float ux = jx * ir, uy = jy * ir, uz = jz * ir;
-    const float uu = 1.5f * (ux * ux + uy * uy + uz * uz);
-#pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        const float eu = ex(k) * ux + ey(k) * uy + ez(k) * uz;
-        const float wk = (float)w<Q>(k);
-        // feq - w = w (drho + rho (3 eu + 4.5 eu^2 - 1.5 u^2))
-        const float dfeq = wk * (dr + rho * (3.f * eu + 4.5f * eu * eu - uu));
-        s[k] = fmaf(omega, dfeq - s[k], s[k]);
-    }
-}
-
-// FP32 LBGK on deviations, opposite directions paired: for q and inv(q) the
-// equilibrium shares its even part w (drho + rho (4.5 eu^2 - 1.5 u^2)) and
-// flips the sign of its odd part 3 w rho eu (D3Q19/27 list q, q+1 as a pair
-// for every odd q).
-template <int Q>
-__device__ __forceinline__ void lbgk_dev_pairs(float *s, float omega)
-{
-    float dr = 0.f, jx = 0.f, jy = 0.f, jz = 0.f;
-#pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        dr += s[k];
-        if (ex(k)) jx += ex(k) > 0 ? s[k] : -s[k];
-        if (ey(k)) jy += ey(k) > 0 ? s[k] : -s[k];
-        if (ez(k)) jz += ez(k) > 0 ? s[k] : -s[k];
-    }
-    const float rho = 1.f + dr;
-    const float ir = __frcp_rn(rho);
-    const float ux = jx * ir, uy = jy * ir, uz = jz * ir;
-    const float uu = 1.5f * (ux * ux + uy * uy + uz * uz);
-    {
-        const float d0 = (float)w<Q>(0) * (dr - rho * uu);
-        s[0] = fmaf(omega, d0 - s[0], s[0]);
-    }
-#pragma unroll
-    for (int k = 1; k < Q; k += 2) {
-        float eu = 0.f;
-        if (ex(k)) eu += ex(k) > 0 ? ux : -ux;
-        if (ey(k)) eu += ey(k) > 0 ? uy : -uy;
-        if (ez(k)) eu += ez(k) > 0 ? uz : -uz;
-        const float wk = (float)w<Q>(k);
-        const float wr = wk * rho;
-        const float even = fmaf(wr, fmaf(4.5f * eu, eu, -uu), wk * dr);
-        const float odd = 3.f * wr * eu;
-        const float dp = even + odd, dm = even - odd;
-        s[k] = fmaf(omega, dp - s[k], s[k]);
-        s[k + 1] = fmaf(omega, dm - s[k + 1], s[k + 1]);
-    }
-}
-
 // One cell per thread.  The three dilated coordinate parts of each axis at
 // offsets -1, 0, +1 are formed once; the pull source of direction k is then
 // px | py | pz of the right offsets (CONV 0: from x + e_k as the reference
 // streams, 1: from x - e_k).  IDX is the offset type: 32-bit while Q*N fits.
 template <int Q, class S, int COLL, int MODE, int CONV, class IDX>
 __global__ void __launch_bounds__(1024) k_dense(const S *__restrict__ A, S *__restrict__ B, IDX N, DenseGeom g,
-                                              double tau)
+                                              double tau, const Shift sh)
 {
     using T = Store<S>;
     using C = typename T::C;
@@ -190,56 +92,33 @@ __global__ void __launch_bounds__(1024) k_dense(const S *__restrict__ A, S *__re
                 for (int k = 0; k < 27; ++k) f[k] = o[k];
             }
         } else {
-            if constexpr (COLL == MT_COLL_LBGK) {
-                lbgk_dev_pairs<Q>(f, (float)(1.0 / tau));
-            } else {
-                float full[27], o[27];
-                float dr = 0.f, jx = 0.f, jy = 0.f, jz = 0.f;
-#pragma unroll
-                for (int k = 0; k < 27; ++k) {
-                    full[k] = (float)w<27>(k) + f[k];
-                    dr += f[k];
-                    jx += ex(k) * f[k];
-                    jy += ey(k) * f[k];
-                    jz += ez(k) * f[k];
-                }
-                const float rho = 1.f + dr;
-                const float ir = 1.f / rho;
-                cumulant_collide<float>(full, rho, jx * ir, jy * ir, jz * ir, (float)(1.0 / tau), o);
-#pragma unroll
-                for (int k = 0; k < 27; ++k) f[k] = o[k] - (float)w<27>(k);
-            }
+            [[maybe_unused]] float r, x, y, z;
+            if constexpr (COLL == MT_COLL_LBGK)
+                p2::lbgk_dev<Q, float>(f, (float)(1.0 / tau));
+            else
+                p2::cumulant<float, true>(f, r, x, y, z, (float)(1.0 / tau), sh);
         }
     }
 #pragma unroll
     for (int k = 0; k < Q; ++k) T::st(B, (IDX)k * N + (IDX)i, f[k]);
 }
 
-// Two x-adjacent cells per thread for 16-bit storage.  Cells i0 = 2p and
-// i0 + 1 differ only in x bit 0, which is index bit 0, so their populations
-// of one direction form an aligned 32-bit pair.  For e_x = 0 the two pull
-// sources are again an aligned pair (one load); for e_x = +-1 they straddle
-// two pairs (x0 + 1, x0 + 2 or x0 - 1, x0): two aligned loads and a byte
-// permute.  Stores and conversions are per pair.
-template <class S> struct Pair16;
-template <> struct Pair16<__half> {
-    using P = __half2;
-    __device__ static __forceinline__ float2 to_f2(P v) { return __half22float2(v); }
-    __device__ static __forceinline__ P from_f2(float2 v) { return __float22half2_rn(v); }
-};
-template <> struct Pair16<__nv_bfloat16> {
-    using P = __nv_bfloat162;
-    __device__ static __forceinline__ float2 to_f2(P v) { return __bfloat1622float2(v); }
-    __device__ static __forceinline__ P from_f2(float2 v) { return __float22bfloat162_rn(v); }
-};
-
-__device__ __forceinline__ uint32_t hi_lo(uint32_t a, uint32_t b) { return __byte_perm(a, b, 0x5432); }
-
-template <int Q, class S, int CONV>
-__global__ void __launch_bounds__(256) k_dense_pair(const S *__restrict__ A, S *__restrict__ B, uint32_t N,
-                                                   DenseGeom g, double tau)
+// Two x-adjacent cells per thread (reduced storages).  Cells i0 = 2p and i0 + 1
+// differ only in x bit 0, which is index bit 0, so their populations of one
+// direction form an aligned word.  For e_x = 0 the two pull sources are again
+// an aligned pair (one load); for e_x = +-1 they straddle two pairs (x0 + 1,
+// x0 + 2 or x0 - 1, x0): two aligned loads.  Stores and conversions are per
+// pair.  LBGK collides the two cells one after the other at 64 registers (the
+// packed form holds both cells' FP32 values: 80 or more); the cumulant, whose
+// arithmetic bounds the one-cell form, collides both in packed FP32 at 80
+// registers, 6 blocks of 128 threads.  128^3 per step: FP16 88.7 us cell by cell,
+// 66.4 us so (256^3: 550 -> 409 us, 4.4 TB/s); FP32 79.7 -> 79.5 us (5.7 TB/s),
+// 64^3 13.7 -> 11.9 us.  What bounds the FP16 cumulant is the FP32 pipe.
+template <int Q, class S, int COLL, int CONV>
+__global__ void __launch_bounds__(COLL == MT_COLL_LBGK ? 256 : 128, COLL == MT_COLL_LBGK ? (Q == 19 ? 4 : 3) : 6)
+    k_dense_pair(const S *__restrict__ A, S *__restrict__ B, uint32_t N, DenseGeom g, double tau, const Shift sh)
 {
-    using P = typename Pair16<S>::P;
+    using CP = CellPair<S>;
     const uint32_t pidx = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t i0 = pidx << 1;
     if (i0 >= N) return;
@@ -261,41 +140,37 @@ __global__ void __launch_bounds__(256) k_dense_pair(const S *__restrict__ A, S *
         pz[0] = (cz - lz) & mz;
     }
     constexpr int sg = CONV ? -1 : 1;
-    float fa[Q], fb[Q];
+    typename CP::W w[Q];
 #pragma unroll
     for (int k = 0; k < Q; ++k) {
         const int dx = sg * ex(k), dy = sg * ey(k), dz = sg * ez(k);
         const uint32_t yz = py[1 + dy] | pz[1 + dz];
         const S *base = A + (size_t)k * N;
-        uint32_t v;
-        if (dx == 0) {
-            v = __ldg((const unsigned int *)(base + (px[1] | yz)));
-        } else if (dx > 0) {
-            // (x0 + 1, x0 + 2): high half of pair x0, low half of pair x0 + 2
-            const uint32_t a = __ldg((const unsigned int *)(base + (px[1] | yz)));
-            const uint32_t b = __ldg((const unsigned int *)(base + (px[2] | yz)));
-            v = hi_lo(a, b);
-        } else {
-            // (x0 - 1, x0): high half of pair x0 - 2, low half of pair x0
-            const uint32_t a = __ldg((const unsigned int *)(base + (px[0] | yz)));
-            const uint32_t b = __ldg((const unsigned int *)(base + (px[1] | yz)));
-            v = hi_lo(a, b);
-        }
-        P pv;
-        memcpy(&pv, &v, 4);
-        const float2 f2 = Pair16<S>::to_f2(pv);
-        fa[k] = f2.x;
-        fb[k] = f2.y;
+        typename CP::W v = CP::ld(base + (px[1] | yz));
+        if (dx > 0) v = CP::straddle(v, CP::ld(base + (px[2] | yz)));
+        if (dx < 0) v = CP::straddle(CP::ld(base + (px[0] | yz)), v);
+        w[k] = v;
     }
     const float om = (float)(1.0 / tau);
-    lbgk_dev_pairs<Q>(fa, om);
-    lbgk_dev_pairs<Q>(fb, om);
+    if constexpr (COLL == MT_COLL_LBGK) {
+        float fa[Q], fb[Q];
 #pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        const P pv = Pair16<S>::from_f2(make_float2(fa[k], fb[k]));
-        uint32_t v;
-        memcpy(&v, &pv, 4);
-        *(unsigned int *)(B + (size_t)k * N + i0) = v;
+        for (int k = 0; k < Q; ++k) {
+            const float2 f2 = CP::f2(w[k]);
+            fa[k] = f2.x;
+            fb[k] = f2.y;
+        }
+        p2::lbgk_dev<Q, float>(fa, om);
+        p2::lbgk_dev<Q, float>(fb, om);
+#pragma unroll
+        for (int k = 0; k < Q; ++k) CP::st(B + (size_t)k * N + i0, CP::word(make_float2(fa[k], fb[k])));
+    } else {
+        float2 f[Q], r, x, y, z;
+#pragma unroll
+        for (int k = 0; k < Q; ++k) f[k] = CP::f2(w[k]);
+        p2::cumulant<float2, true>(f, r, x, y, z, om, sh);
+#pragma unroll
+        for (int k = 0; k < Q; ++k) CP::st(B + (size_t)k * N + i0, CP::word(f[k]));
     }
 }
 
@@ -431,6 +306,23 @@ static __global__ void k_sum_partials(const double *partial, int64_t nb, double 
     }
 }
 
+// the dense path stores f - w_q
+inline Shift dense_shift(int q)
+{
+    const double zero[3] = {0., 0., 0.};
+    return make_shift(q, zero);
+}
+
+// whether the fused pass works on pairs of cells: 16-bit storage always (its
+// one-cell form loads 2 bytes at a time), FP32 for the cumulant, whose
+// arithmetic bounds the one-cell form; FP32 LBGK runs one cell per thread at
+// the memory's rate.  32-bit element offsets.
+template <class S> inline bool dense_pairs(const Case &c)
+{
+    if (!Store<S>::shifted || c.N < 2 || (uint64_t)c.d.q * (uint64_t)c.N >= (1ull << 32)) return false;
+    return sizeof(S) == 2 || c.d.collision != MT_COLL_LBGK;
+}
+
 inline DenseGeom dense_geom(int bits)
 {
     DenseGeom g;
@@ -453,21 +345,30 @@ int DenseOps<S>::step(Ctx &ctx, Case &c, int mode)
     S *Bp = (S *)c.B;
     const int tb = c.d.stream_convention;
     const double tau = c.d.tau[0];
-    if constexpr (std::is_same<S, __half>::value || std::is_same<S, __nv_bfloat16>::value) {
-        // 16-bit storage, LBGK: two cells per thread with paired accesses
-        if (mode == DM_FUSED && c.d.collision == MT_COLL_LBGK && (uint64_t)c.d.q * c.N < (1ull << 32)) {
-            const unsigned pgrid = grid_for(c.N / 2, B);
+    const Shift sh = dense_shift(c.d.q);
+    if constexpr (Store<S>::shifted) {
+        if (mode == DM_FUSED && dense_pairs<S>(c)) {
+            const int PB = std::min(B, c.d.collision == MT_COLL_LBGK ? 256 : 128);
+            const unsigned pgrid = grid_for(c.N / 2, PB);
             const uint32_t n32 = (uint32_t)c.N;
-            if (c.d.q == 19) {
+            auto go = [&](auto q, auto coll) {
+                constexpr int QQ = decltype(q)::value, CC = decltype(coll)::value;
                 if (tb)
-                    k_dense_pair<19, S, 1><<<pgrid, B, 0, ctx.stream>>>(A, Bp, n32, g, tau);
+                    k_dense_pair<QQ, S, CC, 1><<<pgrid, PB, 0, ctx.stream>>>(A, Bp, n32, g, tau, sh);
                 else
-                    k_dense_pair<19, S, 0><<<pgrid, B, 0, ctx.stream>>>(A, Bp, n32, g, tau);
-            } else {
-                if (tb)
-                    k_dense_pair<27, S, 1><<<pgrid, B, 0, ctx.stream>>>(A, Bp, n32, g, tau);
+                    k_dense_pair<QQ, S, CC, 0><<<pgrid, PB, 0, ctx.stream>>>(A, Bp, n32, g, tau, sh);
+            };
+            using Q19 = std::integral_constant<int, 19>;
+            using Q27 = std::integral_constant<int, 27>;
+            using LB = std::integral_constant<int, MT_COLL_LBGK>;
+            using CU = std::integral_constant<int, MT_COLL_CUMULANT>;
+            if (c.d.collision != MT_COLL_LBGK)
+                go(Q27{}, CU{});
+            else if constexpr (sizeof(S) == 2) {
+                if (c.d.q == 19)
+                    go(Q19{}, LB{});
                 else
-                    k_dense_pair<27, S, 0><<<pgrid, B, 0, ctx.stream>>>(A, Bp, n32, g, tau);
+                    go(Q27{}, LB{});
             }
             MT_LAUNCHED(ctx);
             std::swap(c.A, c.B);
@@ -479,11 +380,11 @@ int DenseOps<S>::step(Ctx &ctx, Case &c, int mode)
     do {                                                                                                   \
         const IDX n = (IDX)c.N;                                                                            \
         if (mode == DM_COLLIDE)                                                                            \
-            k_dense<QQ, S, CC, DM_COLLIDE, 0, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau);          \
+            k_dense<QQ, S, CC, DM_COLLIDE, 0, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau, sh);          \
         else if (tb)                                                                                       \
-            k_dense<QQ, S, CC, DM_FUSED, 1, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau);            \
+            k_dense<QQ, S, CC, DM_FUSED, 1, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau, sh);            \
         else                                                                                               \
-            k_dense<QQ, S, CC, DM_FUSED, 0, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau);            \
+            k_dense<QQ, S, CC, DM_FUSED, 0, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau, sh);            \
     } while (0)
 #define MT_DENSE_LAUNCH(QQ, CC)                      \
     do {                                             \
@@ -604,10 +505,8 @@ template <class S>
 int DenseOps<S>::tune(Ctx &ctx, Case &c, float *ms_out, int *blocks_out, int *n_out)
 {
     static const int cand[] = {128, 256, 512, 1024};
-    // the paired 16-bit kernel is built for at most 256 threads per block
-    const bool pair16 = (std::is_same<S, __half>::value || std::is_same<S, __nv_bfloat16>::value) &&
-                        c.d.collision == MT_COLL_LBGK;
-    const int nc = pair16 ? 2 : (int)(sizeof(cand) / sizeof(cand[0]));
+    // the pair kernels are built for at most 256 (LBGK) or 128 (cumulant) threads per block
+    const int nc = !dense_pairs<S>(c) ? (int)(sizeof(cand) / sizeof(cand[0])) : (c.d.collision == MT_COLL_LBGK ? 2 : 1);
     cudaEvent_t e0, e1;
     MT_CUDA(ctx, cudaEventCreate(&e0));
     MT_CUDA(ctx, cudaEventCreate(&e1));
