@@ -23,6 +23,7 @@ COMMON = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", 
                  "--expt-relaxed-constexpr"]
 SOURCES = {
     "mt_capi.cu": [],
+    "mt_copy.cu": [],
     "mt_amr.cu": [],
     "mt_amr_f64.cu": ["--fmad=false"],
     "mt_amr_lp.cu": [],

@@ -1309,8 +1309,7 @@ int amr_get(Ctx &ctx, Case &c, int level, double *h_f, double *h_fcol)
             using S = std::remove_pointer_t<decltype(tag)>;
             return AmrOps<S>::get(ctx, c, level, which, d);
         });
-        if (!rc) MT_CUDA(ctx, cudaMemcpyAsync(dst, d, nb, cudaMemcpyDeviceToHost, ctx.stream));
-        MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
+        if (!rc) rc = copy_out(ctx, dst, d, nb);
     }
     cudaFreeAsync(d, ctx.stream);
     return rc;
@@ -1350,11 +1349,8 @@ int amr_macros(Ctx &ctx, Case &c, int level, double *h_rho, double *h_u)
         using S = std::remove_pointer_t<decltype(tag)>;
         return AmrOps<S>::macros_out(ctx, c, level, d, d + lv.ncell);
     });
-    if (!rc) {
-        if (h_rho) MT_CUDA(ctx, cudaMemcpyAsync(h_rho, d, sizeof(double) * lv.ncell, cudaMemcpyDeviceToHost, ctx.stream));
-        if (h_u) MT_CUDA(ctx, cudaMemcpyAsync(h_u, d + lv.ncell, sizeof(double) * 3 * lv.ncell, cudaMemcpyDeviceToHost, ctx.stream));
-    }
-    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
+    if (!rc && h_rho) rc = copy_out(ctx, h_rho, d, sizeof(double) * lv.ncell);
+    if (!rc && h_u) rc = copy_out(ctx, h_u, d + lv.ncell, sizeof(double) * 3 * lv.ncell);
     cudaFreeAsync(d, ctx.stream);
     return rc;
 }

@@ -155,6 +155,7 @@ int mt_destroy(mt_ctx *h)
         }
     for (cudaEvent_t e : h->c.markers)
         if (e) cudaEventDestroy(e);
+    copy_free(h->c);
     if (h->c.own_stream) cudaStreamDestroy(h->c.stream);
     delete h;
     return MT_OK;
@@ -678,8 +679,8 @@ int mt_case_get_populations(mt_ctx *h, int32_t id, int32_t level, double *f, dou
                 using S = std::remove_pointer_t<decltype(tag)>;
                 return DenseOps<S>::get(ctx, *c, d, pull);
             });
+            if (!rc) rc = copy_out(ctx, dst, d, nb);
             if (rc) break;
-            MT_CUDA(ctx, cudaMemcpyAsync(dst, d, nb, cudaMemcpyDeviceToHost, ctx.stream));
         }
         MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
         cudaFreeAsync(d, ctx.stream);
@@ -704,8 +705,8 @@ int mt_case_get_macros(mt_ctx *h, int32_t id, int32_t level, double *rho, double
             return DenseOps<S>::macros(ctx, *c, d, d + c->N);
         });
         if (!rc) {
-            if (rho) MT_CUDA(ctx, cudaMemcpyAsync(rho, d, sizeof(double) * c->N, cudaMemcpyDeviceToHost, ctx.stream));
-            if (u) MT_CUDA(ctx, cudaMemcpyAsync(u, d + c->N, sizeof(double) * 3 * c->N, cudaMemcpyDeviceToHost, ctx.stream));
+            if (rho) rc = copy_out(ctx, rho, d, sizeof(double) * c->N);
+            if (u && !rc) rc = copy_out(ctx, u, d + c->N, sizeof(double) * 3 * c->N);
         }
         MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
         cudaFreeAsync(d, ctx.stream);

@@ -5,7 +5,9 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <mutex>
 #include <type_traits>
 #include <string>
 #include <vector>
@@ -234,6 +236,7 @@ struct Batch {
     cudaStream_t free_stream = nullptr;  // the stream the batch last ran on
 };
 
+struct HostStage;
 struct Ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -245,6 +248,9 @@ struct Ctx {
     // stream markers (mt_marker_record): a ring of events, slot = ticket % size
     std::vector<cudaEvent_t> markers;
     int64_t next_marker = 0;
+    // page-locked staging of large results (mt_copy.cu), made when first needed
+    HostStage *stage = nullptr;
+    std::mutex stage_mutex;
 };
 constexpr int kMarkerRing = 64;
 
@@ -278,6 +284,10 @@ int amr_prime(Ctx &ctx, Case &c);
 int batch_step(Ctx &ctx, Batch &b, const std::vector<Case *> &cases, int n);
 void batch_drop(Batch &b);
 void batch_free(Batch &b);
+
+// `bytes` of device memory into host memory; synchronises the stream
+int copy_out(Ctx &ctx, void *host, const void *dev, size_t bytes);
+void copy_free(Ctx &ctx);
 
 // multi-level phases, one explicit instantiation per storage type
 // (mt_amr_f64.cu builds the FP64 one without FMA contraction)

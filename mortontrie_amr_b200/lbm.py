@@ -432,16 +432,16 @@ class LBM_Manager:
 
     def populations(self, level):
         n = self.size(level)
-        f = np.zeros((self.q, n))
-        fc = np.zeros((self.q, n))
+        f = np.empty((self.q, n))  # written whole
+        fc = np.empty((self.q, n))
         self.ctx.check(lib().mt_case_get_populations(self.ctx.h, self.id, level, _ptr(f, C.c_double),
                                                      _ptr(fc, C.c_double)), "get_populations")
         return f, fc
 
     def macros(self, level):
         n = self.size(level)
-        rho = np.zeros(n)
-        u = np.zeros((3, n))
+        rho = np.empty(n)  # written whole
+        u = np.empty((3, n))
         self.ctx.check(lib().mt_case_get_macros(self.ctx.h, self.id, level, _ptr(rho, C.c_double),
                                                 _ptr(u, C.c_double)), "get_macros")
         return rho, u
@@ -725,15 +725,15 @@ class DenseCase:
                        "set_populations")
 
     def populations(self):
-        f = np.zeros((self.q, self.n))
-        fc = np.zeros((self.q, self.n))
+        f = np.empty((self.q, self.n))  # written whole
+        fc = np.empty((self.q, self.n))
         self.ctx.check(lib().mt_case_get_populations(self.ctx.h, self.id, 0, _ptr(f, C.c_double),
                                                      _ptr(fc, C.c_double)), "get_populations")
         return f, fc
 
     def macros(self):
-        rho = np.zeros(self.n)
-        u = np.zeros((3, self.n))
+        rho = np.empty(self.n)  # written whole
+        u = np.empty((3, self.n))
         self.ctx.check(lib().mt_case_get_macros(self.ctx.h, self.id, 0, _ptr(rho, C.c_double), _ptr(u, C.c_double)),
                        "get_macros")
         return rho, u
