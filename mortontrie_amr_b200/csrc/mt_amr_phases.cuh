@@ -79,12 +79,12 @@ __global__ void k_macros(const int32_t *list, int64_t nl, int64_t n, const S *f,
 template <int Q, class S, int COLL, class I>
 __device__ __forceinline__ void macros_collide_store(typename Store<S>::C *d, typename Store<S>::C &r,
                                                      typename Store<S>::C &x, typename Store<S>::C &y,
-                                                     typename Store<S>::C &z, double tau, S *out, I i,
+                                                     typename Store<S>::C &z, const Relax tau, S *out, I i,
                                                      const Shift &sh)
 {
     using T = Store<S>;
     if constexpr (T::shifted) {
-        const float om = (float)(1.0 / tau);
+        const float om = tau.om;
         if constexpr (COLL == MT_COLL_LBGK) {
             p2::lbgk<Q, float>(d, r, x, y, z, om, sh);
         } else {
@@ -95,14 +95,12 @@ __device__ __forceinline__ void macros_collide_store(typename Store<S>::C *d, ty
     } else {
         macros_g<Q, double>(d, r, x, y, z);
         if constexpr (COLL == MT_COLL_LBGK) {
+            lbgk_ref<Q>(d, r, x, y, z, tau.tau, tau.inv);
 #pragma unroll
-            for (int k = 0; k < Q; ++k) {
-                const double fk = d[k];
-                out[at<Q>(k, i)] = fk - (fk - feq_ref<Q>(k, r, x, y, z)) / tau;
-            }
+            for (int k = 0; k < Q; ++k) out[at<Q>(k, i)] = d[k];
         } else if constexpr (Q == 27) {
             double o[27];
-            cumulant_collide<double>(d, r, x, y, z, 1. / tau, o);
+            cumulant_collide(d, r, x, y, z, tau.inv, o);
 #pragma unroll
             for (int k = 0; k < 27; ++k) out[at<Q>(k, i)] = o[k];
         }
@@ -112,7 +110,7 @@ __device__ __forceinline__ void macros_collide_store(typename Store<S>::C *d, ty
 // calculateMacros(level) + Collision_LBGK::collide / Collision_Cumulant::collide
 // on lat_f then overlap_F2C (Collision_Manager.cpp:13-53, Collision_Cumulant.cpp:22-159)
 template <int Q, class S, int COLL>
-__global__ void k_collide(const int32_t *list, int64_t nl, int64_t n, double tau, const S *f,
+__global__ void k_collide(const int32_t *list, int64_t nl, int64_t n, const Relax tau, const S *f,
                           typename Store<S>::C *rho, typename Store<S>::C *u, S *fcol, const Shift sh)
 {
     using T = Store<S>;
@@ -301,7 +299,7 @@ __global__ void __launch_bounds__(64) k_coalescence(const int32_t *__restrict__ 
 template <int Q, class S, int COLL>
 __global__ void __launch_bounds__(64) k_coal_collide(const int32_t *__restrict__ list, const int32_t *__restrict__ child, int64_t nl,
                                int64_t nc, S *__restrict__ cf, const S *__restrict__ ff, double scale,
-                               double tau, S *__restrict__ cfnext, typename Store<S>::C *__restrict__ rho,
+                               const Relax tau, S *__restrict__ cfnext, typename Store<S>::C *__restrict__ rho,
                                typename Store<S>::C *__restrict__ u, int macros, const Shift csh,
                                const Shift fsh)
 {
@@ -506,7 +504,7 @@ __global__ void k_bc_hh(const int32_t *list, int64_t nl, int east, int64_t n, in
 }
 
 template <class S>
-__global__ void k_bc_wall_collide(const int32_t *list, int64_t nl, int64_t n, double tau, const S *__restrict__ f,
+__global__ void k_bc_wall_collide(const int32_t *list, int64_t nl, int64_t n, const Relax tau, const S *__restrict__ f,
                                   S *__restrict__ fcol, const Shift sh)
 {
     using T = Store<S>;
@@ -796,7 +794,7 @@ __global__ void k_stream(const int32_t *__restrict__ list, int64_t nl, int64_t n
 template <int Q, class S, int COLL>
 __global__ void k_pull_collide(const int32_t *__restrict__ list, int64_t nl, int64_t n, int textbook,
                                const int32_t *__restrict__ nbr, const S *__restrict__ fcol, S *__restrict__ f,
-                               S *__restrict__ fnext, double tau, typename Store<S>::C *__restrict__ rho,
+                               S *__restrict__ fnext, const Relax tau, typename Store<S>::C *__restrict__ rho,
                                typename Store<S>::C *__restrict__ u, int macros, const Shift sh)
 {
     using T = Store<S>;
@@ -917,7 +915,7 @@ __device__ __forceinline__ void brick_gather(uint32_t i, int textbook, bool comp
 template <int Q, class S, int COLL>
 __device__ __forceinline__ void brick_cell(uint32_t i, int cls, bool complete, const BrickHood &h, uint32_t n,
                                            int textbook, const S *__restrict__ fcol, S *__restrict__ f,
-                                           S *__restrict__ fnext, double tau, typename Store<S>::C *__restrict__ rho,
+                                           S *__restrict__ fnext, const Relax tau, typename Store<S>::C *__restrict__ rho,
                                            typename Store<S>::C *__restrict__ u, int macros, int fall,
                                            long long *__restrict__ acc, const Shift &sh)
 {
@@ -1040,7 +1038,7 @@ __device__ __forceinline__ void pair_missing(int lane, int textbook, const Brick
 template <int Q, class S, int COLL>
 __device__ __forceinline__ void brick_warp_pair(int32_t b, int lane, BrickHood &h, const BrickTab &t, uint32_t n,
                                                 int textbook, const S *__restrict__ fcol, S *__restrict__ f,
-                                                S *__restrict__ fnext, double tau, float *__restrict__ rho,
+                                                S *__restrict__ fnext, const Relax tau, float *__restrict__ rho,
                                                 float *__restrict__ u, int macros, int fall,
                                                 long long *__restrict__ acc, const Shift &sh)
 {
@@ -1081,7 +1079,7 @@ __device__ __forceinline__ void brick_warp_pair(int32_t b, int lane, BrickHood &
     const bool b0 = c0 == 4 && acc, b1 = c1 == 4 && acc;
     if (!(k0 || k1 || b0 || b1)) return;
     float2 d[Q], r, x, y, z;
-    const float om = (float)(1.0 / tau);
+    const float om = tau.om;
 #pragma unroll
     for (int k = 0; k < Q; ++k) d[k] = CP::f2(v[k]);
     if constexpr (COLL == MT_COLL_LBGK)
@@ -1122,7 +1120,7 @@ __device__ __forceinline__ void brick_warp_pair(int32_t b, int lane, BrickHood &
 template <int Q, class S, int COLL, int V>
 __device__ __forceinline__ void brick_warp(int32_t b, int lane, BrickHood &h, const BrickTab &t, uint32_t n,
                                            int textbook, const S *__restrict__ fcol, S *__restrict__ f,
-                                           S *__restrict__ fnext, double tau, typename Store<S>::C *__restrict__ rho,
+                                           S *__restrict__ fnext, const Relax tau, typename Store<S>::C *__restrict__ rho,
                                            typename Store<S>::C *__restrict__ u, int macros, int fall,
                                            long long *__restrict__ acc, const Shift &sh)
 {
@@ -1166,7 +1164,7 @@ template <class S> constexpr int brick_default_variant() { return 0; }
 template <int Q, class S, int COLL, int V>
 __global__ void __launch_bounds__(128, brick_min_blocks<Q, S, COLL, V>()) k_brick_step(
     int64_t nb, const BrickTab t, uint32_t n, int textbook, const S *__restrict__ fcol, S *__restrict__ f,
-    S *__restrict__ fnext, double tau, typename Store<S>::C *__restrict__ rho, typename Store<S>::C *__restrict__ u,
+    S *__restrict__ fnext, const Relax tau, typename Store<S>::C *__restrict__ rho, typename Store<S>::C *__restrict__ u,
     int macros, int fall, long long *__restrict__ acc, const Shift sh)
 {
     __shared__ BrickHood hood[4];
@@ -1234,7 +1232,7 @@ template <int Q, int FH, class S, int COLL>
 __global__ void __launch_bounds__(kIbBlock) k_ib_collide(
     const int32_t *__restrict__ list, int64_t nl, int64_t n, const int32_t *__restrict__ disrow,
     const double *__restrict__ dis, const int32_t *__restrict__ nbr, const S *__restrict__ fcol, S *__restrict__ f,
-    S *__restrict__ fnext, double tau, double *part, double *force, typename Store<S>::C *__restrict__ rho,
+    S *__restrict__ fnext, const Relax tau, double *part, double *force, typename Store<S>::C *__restrict__ rho,
     typename Store<S>::C *__restrict__ u, int macros, const Shift sh)
 {
     using T = Store<S>;
@@ -1454,7 +1452,7 @@ static __global__ void __launch_bounds__(256) k_df_sum(const double *fk, int64_t
 // fcol = f - (f - feq(rho, u)) / tau + (1 - 1 / (2 tau)) w [3 (e - u) + 9 (e.u) e].g
 // (the band's rho and unforced velocity are written by k_band_macros)
 template <int Q, class S>
-__global__ void k_band_collide(const int32_t *band, int64_t nb, int64_t n, double tau, const S *f,
+__global__ void k_band_collide(const int32_t *band, int64_t nb, int64_t n, const Relax tau, const S *f,
                                const long long *acc, S *fcol, const Shift sh)
 {
     using T = Store<S>;
@@ -1485,7 +1483,7 @@ __global__ void k_band_collide(const int32_t *band, int64_t nb, int64_t n, doubl
         const float rs = (r > -1e-6f && r < 1e-6f) ? ((r < 0.f) ? -1e-6f : 1e-6f) : r;
         const float ir = 1.f / rs;
         const float x = (jx + 0.5f * gx) * ir, y = (jy + 0.5f * gy) * ir, z = (jz + 0.5f * gz) * ir;
-        const float om = (float)(1.0 / tau);
+        const float om = tau.om;
         const float fpre = 1.f - 0.5f * om;
         const float uu = 1.5f * (x * x + y * y + z * z);
         const float ug = x * gx + y * gy + z * gz;
@@ -1515,7 +1513,7 @@ __global__ void k_band_collide(const int32_t *band, int64_t nb, int64_t n, doubl
             gz = (C)((double)acc[2 * n + i] * kForceInv);
     const C rs = (r > C(-1e-6) && r < C(1e-6)) ? ((r < C(0)) ? C(-1e-6) : C(1e-6)) : r;
     const C x = (jx + gx * C(0.5)) / rs, y = (jy + gy * C(0.5)) / rs, z = (jz + gz * C(0.5)) / rs;
-    const C om = C(1) / C(tau);
+    const C om = (C)tau.inv;
     const C fpre = C(1) - C(0.5) * om;
     const C uu = x * x + y * y + z * z;
 #pragma unroll

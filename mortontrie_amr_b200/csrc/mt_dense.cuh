@@ -53,9 +53,14 @@ enum { DM_FUSED = 0, DM_COLLIDE = 1, DM_PULL = 2 };
 // offsets -1, 0, +1 are formed once; the pull source of direction k is then
 // px | py | pz of the right offsets (CONV 0: from x + e_k as the reference
 // streams, 1: from x - e_k).  IDX is the offset type: 32-bit while Q*N fits.
+// FP64: 128 registers (256 threads, 2 blocks per SM).  Bounded to 1024 threads it
+// had 64 and spilled (D3Q19 80 B, the cumulant 2.3 KB a thread); per step, with
+// the quotients of mt_lattice.cuh: 128^3 D3Q19 123 -> 103 us, 256^3 916 -> 779 us
+// (6.5 TB/s, the measured copy rate), D3Q27 LBGK 128^3 225 -> 150 us, cumulant 924
+// -> 236 us (at 80 registers 512 us, at 96 356 us).
 template <int Q, class S, int COLL, int MODE, int CONV, class IDX>
-__global__ void __launch_bounds__(1024) k_dense(const S *__restrict__ A, S *__restrict__ B, IDX N, DenseGeom g,
-                                              double tau, const Shift sh)
+__global__ void __launch_bounds__(sizeof(S) == 8 ? 256 : 1024, sizeof(S) == 8 ? 2 : 1) k_dense(const S *__restrict__ A, S *__restrict__ B, IDX N, DenseGeom g,
+                                              const Relax tau, const Shift sh)
 {
     using T = Store<S>;
     using C = typename T::C;
@@ -83,20 +88,19 @@ __global__ void __launch_bounds__(1024) k_dense(const S *__restrict__ A, S *__re
             double r, x, y, z;
             macros_ref<Q>(f, r, x, y, z);
             if constexpr (COLL == MT_COLL_LBGK) {
-#pragma unroll
-                for (int k = 0; k < Q; ++k) f[k] = f[k] - (f[k] - feq_ref<Q>(k, r, x, y, z)) / tau;
+                lbgk_ref<Q>(f, r, x, y, z, tau.tau, tau.inv);
             } else {
                 double o[27];
-                cumulant_collide<double>(f, r, x, y, z, 1. / tau, o);
+                cumulant_collide(f, r, x, y, z, tau.inv, o);
 #pragma unroll
                 for (int k = 0; k < 27; ++k) f[k] = o[k];
             }
         } else {
             [[maybe_unused]] float r, x, y, z;
             if constexpr (COLL == MT_COLL_LBGK)
-                p2::lbgk_dev<Q, float>(f, (float)(1.0 / tau));
+                p2::lbgk_dev<Q, float>(f, tau.om);
             else
-                p2::cumulant<float, true>(f, r, x, y, z, (float)(1.0 / tau), sh);
+                p2::cumulant<float, true>(f, r, x, y, z, tau.om, sh);
         }
     }
 #pragma unroll
@@ -116,7 +120,7 @@ __global__ void __launch_bounds__(1024) k_dense(const S *__restrict__ A, S *__re
 // 64^3 13.7 -> 11.9 us.  What bounds the FP16 cumulant is the FP32 pipe.
 template <int Q, class S, int COLL, int CONV>
 __global__ void __launch_bounds__(COLL == MT_COLL_LBGK ? 256 : 128, COLL == MT_COLL_LBGK ? (Q == 19 ? 4 : 3) : 6)
-    k_dense_pair(const S *__restrict__ A, S *__restrict__ B, uint32_t N, DenseGeom g, double tau, const Shift sh)
+    k_dense_pair(const S *__restrict__ A, S *__restrict__ B, uint32_t N, DenseGeom g, const Relax tau, const Shift sh)
 {
     using CP = CellPair<S>;
     const uint32_t pidx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -151,7 +155,7 @@ __global__ void __launch_bounds__(COLL == MT_COLL_LBGK ? 256 : 128, COLL == MT_C
         if (dx < 0) v = CP::straddle(CP::ld(base + (px[0] | yz)), v);
         w[k] = v;
     }
-    const float om = (float)(1.0 / tau);
+    const float om = tau.om;
     if constexpr (COLL == MT_COLL_LBGK) {
         float fa[Q], fb[Q];
 #pragma unroll
@@ -505,8 +509,10 @@ template <class S>
 int DenseOps<S>::tune(Ctx &ctx, Case &c, float *ms_out, int *blocks_out, int *n_out)
 {
     static const int cand[] = {128, 256, 512, 1024};
-    // the pair kernels are built for at most 256 (LBGK) or 128 (cumulant) threads per block
-    const int nc = !dense_pairs<S>(c) ? (int)(sizeof(cand) / sizeof(cand[0])) : (c.d.collision == MT_COLL_LBGK ? 2 : 1);
+    // the pair kernels are built for at most 256 (LBGK) or 128 (cumulant) threads per block, FP64 for 256
+    const int nc = sizeof(S) == 8 ? 2
+                   : !dense_pairs<S>(c) ? (int)(sizeof(cand) / sizeof(cand[0]))
+                                        : (c.d.collision == MT_COLL_LBGK ? 2 : 1);
     cudaEvent_t e0, e1;
     MT_CUDA(ctx, cudaEventCreate(&e0));
     MT_CUDA(ctx, cudaEventCreate(&e1));

@@ -9,7 +9,9 @@
 // within stated tolerances.
 #pragma once
 
+#include <cmath>
 #include <cstdint>
+#include <cstring>
 #include <type_traits>
 
 #ifndef MT_HD
@@ -81,6 +83,16 @@ inline Shift make_shift(int q, const double *us)
     }
     return s;
 }
+
+// A level's relaxation as kernels take it: the time, its reciprocal and the
+// FP32 rate, formed once on the host (an FP64 division costs a thread as much
+// as ten moments).
+struct Relax {
+    double tau = 1.0, inv = 1.0;
+    float om = 1.f;
+    Relax() = default;
+    Relax(double t) : tau(t), inv(1.0 / t), om((float)(1.0 / t)) {}
+};
 
 // D3Q19 weights used by the solid-boundary treatment for every Q; entries
 // 19..26 are zero (ComplexBoundary_Manager.cpp:102-107,184-189).
@@ -210,6 +222,27 @@ struct LevelMap {
 // ---------------------------------------------------------------------------
 // FP64 physics in the reference's operation order
 // ---------------------------------------------------------------------------
+// In the FP64 forms a direction's zero components are left out (x + 0 y is x:
+// the compiler has to keep such terms, a fifth of the operations), and
+// quotients by a divisor that several values share come from its reciprocal:
+// with rb = RN(1 / b), q = RN(x rb), r = x - q b (exact, one FMA), RN(q + r rb) is
+// RN(x / b) (Markstein, IBM J. Res. Dev. 34, 1990; Brisebarre, Muller & Raina,
+// IEEE Trans. Comput. 53, 2004), three operations where a division takes
+// about ten.  That holds while nothing over- or underflows: b within
+// 2^+-100, |x| below 2^900 and zero or above 2^-960 (differences and sums of
+// populations are); other cells divide.
+MT_HD double quot(double x, double b, double rb)
+{
+    const double q = x * rb;
+    return fma(fma(-q, b, x), rb, q);
+}
+// |x| < 2^e (false for infinities and NaN)
+template <int E> MT_HD bool below(double x)
+{
+    uint64_t bits;
+    memcpy(&bits, &x, 8);
+    return (uint32_t)((bits >> 32) & 0x7fffffffu) < (uint32_t)(E + 1023) << 20;
+}
 // LBM_Manager::calculateMacros(ddf, rho, v) (LBM_Manager.cpp:983-1001)
 template <int Q> MT_HD void macros_ref(const double *d, double &rho, double &ux, double &uy, double &uz)
 {
@@ -217,28 +250,63 @@ template <int Q> MT_HD void macros_ref(const double *d, double &rho, double &ux,
 #pragma unroll
     for (int i = 1; i < Q; ++i) {
         r += d[i];
-        vx += d[i] * ex(i);
-        vy += d[i] * ey(i);
-        vz += d[i] * ez(i);
+        if (ex(i)) vx += d[i] * ex(i);
+        if (ey(i)) vy += d[i] * ey(i);
+        if (ez(i)) vz += d[i] * ez(i);
     }
     const double s = (r > -1e-6 && r < 1e-6) ? ((r < 0.0) ? -1e-6 : 1e-6) : r;
     rho = r;
-    ux = vx / s;
-    uy = vy / s;
-    uz = vz / s;
+    if (below<100>(s) && below<900>(vx) && below<900>(vy) && below<900>(vz)) {
+        const double rs = 1.0 / s;
+        ux = quot(vx, s, rs);
+        uy = quot(vy, s, rs);
+        uz = quot(vz, s, rs);
+    } else {
+        ux = vx / s;
+        uy = vy / s;
+        uz = vz / s;
+    }
+}
+// e_i . u, zero components left out
+MT_HD double edot_ref(int i, double ux, double uy, double uz)
+{
+    if (ex(i) && ey(i) && ez(i)) return ex(i) * ux + ey(i) * uy + ez(i) * uz;
+    if (ex(i) && ey(i)) return ex(i) * ux + ey(i) * uy;
+    if (ex(i) && ez(i)) return ex(i) * ux + ez(i) * uz;
+    if (ey(i) && ez(i)) return ey(i) * uy + ez(i) * uz;
+    return ex(i) ? ex(i) * ux : (ey(i) ? ey(i) * uy : (ez(i) ? ez(i) * uz : 0.));
 }
 // LBM_Manager::calculateFeq (BGK), one direction (LBM_Manager.cpp:205-233)
 template <int Q> MT_HD double feq_ref(int i, double rho, double ux, double uy, double uz)
 {
     const double uu = ux * ux + uy * uy + uz * uz;
-    const double euv = ex(i) * ux + ey(i) * uy + ez(i) * uz;
+    const double euv = edot_ref(i, ux, uy, uz);
     return rho * w<Q>(i) * (1. + 3. * euv + 4.5 * euv * euv - 1.5 * uu);
+}
+// Collision_LBGK::collide on one cell in place (Collision_Manager.cpp:13-53):
+// f - (f - feq) / tau, rtau = RN(1 / tau)
+template <int Q>
+MT_HD void lbgk_ref(double *f, double rho, double ux, double uy, double uz, double tau, double rtau)
+{
+    if (below<500>(rho) && below<200>(ux) && below<200>(uy) && below<200>(uz) && below<100>(tau) && below<100>(rtau)) {
+#pragma unroll
+        for (int k = 0; k < Q; ++k) f[k] = f[k] - quot(f[k] - feq_ref<Q>(k, rho, ux, uy, uz), tau, rtau);
+    } else {
+        // (a copy the compiler cannot see through: it would otherwise form the
+        // equilibria both branches need ahead of them and hold all Q)
+        double r = rho;
+#ifdef __CUDA_ARCH__
+        asm volatile("" : "+d"(r));
+#endif
+#pragma unroll
+        for (int k = 0; k < Q; ++k) f[k] = f[k] - (f[k] - feq_ref<Q>(k, r, ux, uy, uz)) / tau;
+    }
 }
 // LBM_Manager::calculateFeq_HeLuo, one direction (LBM_Manager.cpp:235-263)
 template <int Q> MT_HD double feq_heluo_ref(int i, double rho, double ux, double uy, double uz)
 {
     const double uu = ux * ux + uy * uy + uz * uz;
-    const double euv = ex(i) * ux + ey(i) * uy + ez(i) * uz;
+    const double euv = edot_ref(i, ux, uy, uz);
     return w<Q>(i) * (rho + 1.0 * (3. * euv + 4.5 * euv * euv - 1.5 * uu));
 }
 
@@ -249,6 +317,10 @@ MT_HD double safe_irho_ref(double r) { return 1.0 / ((r > -1e-6 && r < 1e-6) ? (
 // path's arithmetic.
 template <int Q, class R> MT_HD void macros_g(const R *d, R &rho, R &ux, R &uy, R &uz)
 {
+    if constexpr (std::is_same<R, double>::value) {
+        macros_ref<Q>(d, rho, ux, uy, uz);
+        return;
+    }
     R r = d[0], vx = 0, vy = 0, vz = 0;
 #pragma unroll
     for (int i = 1; i < Q; ++i) {
@@ -259,47 +331,42 @@ template <int Q, class R> MT_HD void macros_g(const R *d, R &rho, R &ux, R &uy, 
     }
     const R s = (r > R(-1e-6) && r < R(1e-6)) ? ((r < R(0)) ? R(-1e-6) : R(1e-6)) : r;
     rho = r;
-    if constexpr (std::is_same<R, double>::value) {
-        ux = vx / s;
-        uy = vy / s;
-        uz = vz / s;
-    } else {
-        const R is = R(1) / s;
-        ux = vx * is;
-        uy = vy * is;
-        uz = vz * is;
-    }
+    const R is = R(1) / s;
+    ux = vx * is;
+    uy = vy * is;
+    uz = vz * is;
 }
 template <int Q, class R> MT_HD R feq_g(int i, R rho, R ux, R uy, R uz)
 {
+    if constexpr (std::is_same<R, double>::value) return feq_ref<Q>(i, rho, ux, uy, uz);
     const R uu = ux * ux + uy * uy + uz * uz;
     const R euv = ex(i) * ux + ey(i) * uy + ez(i) * uz;
     return rho * (R)w<Q>(i) * (R(1) + R(3) * euv + R(4.5) * euv * euv - R(1.5) * uu);
 }
 template <int Q, class R> MT_HD R feq_heluo_g(int i, R rho, R ux, R uy, R uz)
 {
+    if constexpr (std::is_same<R, double>::value) return feq_heluo_ref<Q>(i, rho, ux, uy, uz);
     const R uu = ux * ux + uy * uy + uz * uz;
     const R euv = ex(i) * ux + ey(i) * uy + ez(i) * uz;
     return (R)w<Q>(i) * (rho + R(1) * (R(3) * euv + R(4.5) * euv * euv - R(1.5) * uu));
 }
 
-template <class R>
-MT_HD void chim_back(R a0, R a1, R a2, R v, R v2, R &pn, R &pz, R &pp)
+// backward chimera step of one line (Collision_Cumulant.cpp:486-651); Z0, Z1, Z2
+// mark moments the relaxation set to zero, whose terms are left out
+template <bool Z0 = false, bool Z1 = false, bool Z2 = false>
+MT_HD void chim_back(double a0, double a1, double a2, double v, double v2, double &pn, double &pz, double &pp)
 {
-    if constexpr (std::is_same<R, double>::value) {
-        // the reference's expression order (Collision_Cumulant.cpp:486-651)
-        pz = a0 * (1 - v2) - a1 * 2 * v - a2;
-        pn = (a0 * (v2 - v) + a1 * (2 * v - 1) + a2) * R(0.5);
-        pp = (a0 * (v2 + v) + a1 * (2 * v + 1) + a2) * R(0.5);
-    } else {
-        // the same polynomials with shared terms: t = a0 v^2 + 2 v a1 + a2,
-        // h = (a0 v + a1) / 2; pz = a0 - t, pp = t / 2 + h, pn = t / 2 - h
-        const R t = a0 * v2 + (2 * v * a1 + a2);
-        const R h = R(0.5) * (a0 * v + a1);
-        pz = a0 - t;
-        pp = R(0.5) * t + h;
-        pn = R(0.5) * t - h;
+    const double t = Z1 ? 0. : a1 * 2 * v, n1 = Z1 ? 0. : a1 * (2 * v - 1), p1 = Z1 ? 0. : a1 * (2 * v + 1);
+    pz = Z0 ? -t : (Z1 ? a0 * (1 - v2) : a0 * (1 - v2) - t);
+    pn = Z0 ? n1 : (Z1 ? a0 * (v2 - v) : a0 * (v2 - v) + n1);
+    pp = Z0 ? p1 : (Z1 ? a0 * (v2 + v) : a0 * (v2 + v) + p1);
+    if (!Z2) {
+        pz = pz - a2;
+        pn = pn + a2;
+        pp = pp + a2;
     }
+    pn = pn * 0.5;
+    pp = pp * 0.5;
 }
 
 // D3Q27 cumulant collision (Collision_Cumulant.cpp:320-652): central moments
@@ -307,128 +374,18 @@ MT_HD void chim_back(R a0, R a1, R a2, R v, R v2, R &pn, R &pz, R &pp)
 // all cumulants of order >= 3 reset to zero, backward cumulant and chimera
 // transforms.  Slot (a,b,c) of the moment arrays is a + 3b + 9c.  The
 // (2,1,0), (1,0,2) and (0,2,1) moments keep their forward values in the
-// backward pass, as in the reference (Collision_Cumulant.cpp:451-454).
-// R = double reproduces the reference bit-for-bit without FMA contraction;
-// R = float is the reduced-precision variant.
-// The part of cumulant_collide after the forward central moments: cumulant
-// relaxation and the backward transforms (Collision_Cumulant.cpp:374-652);
-// m holds the 27 central moments about u, slot (a,b,c) = a + 3b + 9c, and is
-// overwritten.
-template <class R>
-MT_HD void cumulant_from_moments(R *m, R rho, R ux, R uy, R uz, R omega1, R *out)
+// backward pass, as in the reference (Collision_Cumulant.cpp:451-454).  FP64 in
+// the reference's expression order: bit-for-bit without FMA contraction
+// (terms with a moment that was set to zero left out).
+MT_HD void cumulant_collide(const double *f, double rho, double ux, double uy, double uz, double omega1, double *out)
 {
+    double m[27];
 #define MM(a, b, c) m[(a) + 3 * (b) + 9 * (c)]
-    R c200 = MM(2, 0, 0), c020 = MM(0, 2, 0), c002 = MM(0, 0, 2);
-    R c110 = MM(1, 1, 0), c101 = MM(1, 0, 1), c011 = MM(0, 1, 1);
-    const R k000 = MM(0, 0, 0);
-    const R om1 = omega1, om2 = 1;
-    const R ir = R(1) / ((rho > R(-1e-6) && rho < R(1e-6)) ? ((rho < R(0)) ? R(-1e-6) : R(1e-6)) : rho);
-    const R dxu = -(om1 * (2 * c200 - c020 - c002) + om2 * (c200 + c020 + c002 - k000)) * ir * R(0.5);
-    const R dyv = dxu + 3 * om1 * (c200 - c020) * R(0.5) * ir;
-    const R dzw = dxu + 3 * om1 * (c200 - c002) * R(0.5) * ir;
-    c110 *= (1 - om1);
-    c101 *= (1 - om1);
-    c011 *= (1 - om1);
-    const R ux2 = ux * ux, uy2 = uy * uy, uz2 = uz * uz;
-    const R x1 = (1 - om1) * (c200 - c020) - 3 * rho * (1 - om1 * R(0.5)) * (ux2 * dxu - uy2 * dyv);
-    const R x2 = (1 - om1) * (c200 - c002) - 3 * rho * (1 - om1 * R(0.5)) * (ux2 * dxu - uz2 * dzw);
-    const R x3 = k000 * om2 + (1 - om2) * (c200 + c020 + c002) -
-                 3 * rho * (1 - om2 * R(0.5)) * (ux2 * dxu + uy2 * dyv + uz2 * dzw);
-    if constexpr (std::is_same<R, double>::value)
-        c200 = (x1 + x2 + x3) / 3;  // the reference's expression
-    else
-        c200 = (x1 + x2 + x3) * R(1.0 / 3.0);
-    c020 = c200 - x1;
-    c002 = c200 - x2;
-
-    MM(1, 1, 0) = c110; MM(0, 1, 1) = c011; MM(1, 0, 1) = c101;
-    MM(2, 0, 0) = c200; MM(0, 2, 0) = c020; MM(0, 0, 2) = c002;
-    MM(1, 2, 0) = 0; MM(0, 1, 2) = 0; MM(2, 0, 1) = 0;
-    MM(1, 1, 1) = 0;
-    MM(2, 1, 1) = 0 + (MM(2, 0, 0) * MM(0, 1, 1) + 2 * MM(1, 1, 0) * MM(1, 0, 1)) * ir;
-    MM(1, 2, 1) = 0 + (MM(0, 2, 0) * MM(1, 0, 1) + 2 * MM(0, 1, 1) * MM(1, 1, 0)) * ir;
-    MM(1, 1, 2) = 0 + (MM(0, 0, 2) * MM(1, 1, 0) + 2 * MM(1, 0, 1) * MM(0, 1, 1)) * ir;
-    MM(2, 2, 0) = 0 + (MM(2, 0, 0) * MM(0, 2, 0) + 2 * MM(1, 1, 0) * MM(1, 1, 0)) * ir;
-    MM(0, 2, 2) = 0 + (MM(0, 2, 0) * MM(0, 0, 2) + 2 * MM(0, 1, 1) * MM(0, 1, 1)) * ir;
-    MM(2, 0, 2) = 0 + (MM(0, 0, 2) * MM(2, 0, 0) + 2 * MM(1, 0, 1) * MM(1, 0, 1)) * ir;
-    MM(1, 2, 2) = 0 + (MM(0, 0, 2) * MM(1, 2, 0) + MM(0, 2, 0) * MM(1, 0, 2) + 4 * MM(0, 1, 1) * MM(1, 1, 1) +
-                       2 * (MM(1, 0, 1) * MM(0, 2, 1) + MM(1, 1, 0) * MM(0, 1, 2))) * ir;
-    MM(2, 1, 2) = 0 + (MM(2, 0, 0) * MM(0, 1, 2) + MM(0, 0, 2) * MM(2, 1, 0) + 4 * MM(1, 0, 1) * MM(1, 1, 1) +
-                       2 * (MM(1, 1, 0) * MM(1, 0, 2) + MM(0, 1, 1) * MM(2, 0, 1))) * ir;
-    MM(2, 2, 1) = 0 + (MM(0, 2, 0) * MM(2, 0, 1) + MM(2, 0, 0) * MM(0, 2, 1) + 4 * MM(1, 1, 0) * MM(1, 1, 1) +
-                       2 * (MM(0, 1, 1) * MM(2, 1, 0) + MM(1, 0, 1) * MM(1, 2, 0))) * ir;
-    {
-        const R a = (4 * MM(1, 1, 1) * MM(1, 1, 1) + MM(2, 0, 0) * MM(0, 2, 2) + MM(0, 2, 0) * MM(2, 0, 2) +
-                     MM(0, 0, 2) * MM(2, 2, 0) +
-                     4 * (MM(0, 1, 1) * MM(2, 1, 1) + MM(1, 0, 1) * MM(1, 2, 1) + MM(1, 1, 0) * MM(1, 1, 2)) +
-                     2 * (MM(1, 2, 0) * MM(1, 0, 2) + MM(2, 1, 0) * MM(0, 1, 2) + MM(2, 0, 1) * MM(0, 2, 1))) * ir;
-        const R b = (16 * MM(1, 1, 0) * MM(1, 0, 1) * MM(0, 1, 1) +
-                     4 * (MM(1, 0, 1) * MM(1, 0, 1) * MM(0, 2, 0) + MM(0, 1, 1) * MM(0, 1, 1) * MM(2, 0, 0) +
-                          MM(1, 1, 0) * MM(1, 1, 0) * MM(0, 0, 2)) +
-                     2 * MM(2, 0, 0) * MM(0, 2, 0) * MM(0, 0, 2)) * ir * ir;
-        MM(2, 2, 2) = 0 + a - b;
-    }
-    R p1[27], p2[27];
-    const R vx2 = ux * ux, vy2 = uy * uy, vz2 = uz * uz;
-#pragma unroll
-    for (int cc = 0; cc < 3; ++cc)
-#pragma unroll
-        for (int b = 0; b < 3; ++b)
-            chim_back<R>(MM(0, b, cc), MM(1, b, cc), MM(2, b, cc), ux, vx2, p1[0 + 3 * b + 9 * cc],
-                         p1[1 + 3 * b + 9 * cc], p1[2 + 3 * b + 9 * cc]);
-#pragma unroll
-    for (int ix = 0; ix < 3; ++ix)
-#pragma unroll
-        for (int cc = 0; cc < 3; ++cc)
-            chim_back<R>(p1[ix + 0 + 9 * cc], p1[ix + 3 + 9 * cc], p1[ix + 6 + 9 * cc], uy, vy2, p2[ix + 0 + 9 * cc],
-                         p2[ix + 3 + 9 * cc], p2[ix + 6 + 9 * cc]);
-#pragma unroll
-    for (int ix = 0; ix < 3; ++ix)
-#pragma unroll
-        for (int iy = 0; iy < 3; ++iy)
-            chim_back<R>(p2[ix + 3 * iy + 0], p2[ix + 3 * iy + 9], p2[ix + 3 * iy + 18], uz, vz2, m[ix + 3 * iy + 0],
-                         m[ix + 3 * iy + 9], m[ix + 3 * iy + 18]);
-#pragma unroll
-    for (int i = 0; i < 27; ++i) out[i] = m[(ex(i) + 1) + 3 * (ey(i) + 1) + 9 * (ez(i) + 1)];
-#undef MM
-}
-
-template <class R>
-MT_HD void cumulant_collide(const R *f, R rho, R ux, R uy, R uz, R omega1, R *out)
-{
-    R m[27];
-#define MM(a, b, c) m[(a) + 3 * (b) + 9 * (c)]
-    if constexpr (!std::is_same<R, double>::value) {
-        // reduced precision: the same central moments by three chimera passes
-        // (x, then y, then z lines of three), a quarter of the operations
-        R g[27];
-#pragma unroll
-        for (int i = 0; i < 27; ++i) g[(ex(i) + 1) + 3 * (ey(i) + 1) + 9 * (ez(i) + 1)] = f[i];
-        const R v[3] = {ux, uy, uz};
-#pragma unroll
-        for (int ax = 0; ax < 3; ++ax) {
-            const int st = ax == 0 ? 1 : (ax == 1 ? 3 : 9);
-            const R u = v[ax], u2 = u * u;
-#pragma unroll
-            for (int line = 0; line < 9; ++line) {
-                // base index of the line: the two other axes' positions
-                const int o1 = line % 3, o2 = line / 3;
-                const int bidx = ax == 0 ? 3 * o1 + 9 * o2 : (ax == 1 ? o1 + 9 * o2 : o1 + 3 * o2);
-                const R fm = g[bidx], f0 = g[bidx + st], fp = g[bidx + 2 * st];
-                const R k0 = fm + f0 + fp, d1 = fp - fm, s1 = fp + fm;
-                g[bidx] = k0;
-                g[bidx + st] = d1 - u * k0;
-                g[bidx + 2 * st] = s1 - 2 * u * d1 + u2 * k0;
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 27; ++i) m[i] = g[i];
-    } else {
 #pragma unroll
     for (int i = 0; i < 27; ++i) m[i] = 0;
 #pragma unroll
     for (int i = 0; i < 27; ++i) {
-        const R cx = ex(i) - ux, cy = ey(i) - uy, cz = ez(i) - uz, fi = f[i];
+        const double cx = ex(i) - ux, cy = ey(i) - uy, cz = ez(i) - uz, fi = f[i];
         MM(0, 0, 0) += fi;
         MM(1, 0, 0) += cx * fi;
         MM(0, 1, 0) += cy * fi;
@@ -440,25 +397,78 @@ MT_HD void cumulant_collide(const R *f, R rho, R ux, R uy, R uz, R omega1, R *ou
         MM(1, 0, 1) += cx * cz * fi;
         MM(0, 1, 1) += cy * cz * fi;
         MM(2, 1, 0) += cx * cx * cy * fi;
-        MM(2, 0, 1) += cx * cx * cz * fi;
         MM(0, 2, 1) += cy * cy * cz * fi;
-        MM(1, 2, 0) += cx * cy * cy * fi;
         MM(1, 0, 2) += cx * cz * cz * fi;
-        MM(0, 1, 2) += cy * cz * cz * fi;
-        MM(1, 1, 1) += cx * cy * cz * fi;
-        MM(2, 2, 0) += cx * cx * cy * cy * fi;
-        MM(2, 0, 2) += cx * cx * cz * cz * fi;
-        MM(0, 2, 2) += cy * cy * cz * cz * fi;
-        MM(2, 1, 1) += cx * cx * cy * cz * fi;
-        MM(1, 2, 1) += cx * cy * cy * cz * fi;
-        MM(1, 1, 2) += cx * cy * cz * cz * fi;
-        MM(2, 2, 1) += cx * cx * cy * cy * cz * fi;
-        MM(2, 1, 2) += cx * cx * cy * cz * cz * fi;
-        MM(1, 2, 2) += cx * cy * cy * cz * cz * fi;
-        MM(2, 2, 2) += cx * cx * cy * cy * cz * cz * fi;
     }
+    double c200 = MM(2, 0, 0), c020 = MM(0, 2, 0), c002 = MM(0, 0, 2);
+    double c110 = MM(1, 1, 0), c101 = MM(1, 0, 1), c011 = MM(0, 1, 1);
+    const double k000 = MM(0, 0, 0);
+    const double om1 = omega1;
+    const double ir = 1. / ((rho > -1e-6 && rho < 1e-6) ? ((rho < 0.) ? -1e-6 : 1e-6) : rho);
+    // bulk rate 1: om2 = 1, and the terms with 1 - om2 vanish
+    const double dxu = -(om1 * (2 * c200 - c020 - c002) + (c200 + c020 + c002 - k000)) * ir * 0.5;
+    const double dyv = dxu + 3 * om1 * (c200 - c020) * 0.5 * ir;
+    const double dzw = dxu + 3 * om1 * (c200 - c002) * 0.5 * ir;
+    c110 *= (1 - om1);
+    c101 *= (1 - om1);
+    c011 *= (1 - om1);
+    const double ux2 = ux * ux, uy2 = uy * uy, uz2 = uz * uz;
+    const double x1 = (1 - om1) * (c200 - c020) - 3 * rho * (1 - om1 * 0.5) * (ux2 * dxu - uy2 * dyv);
+    const double x2 = (1 - om1) * (c200 - c002) - 3 * rho * (1 - om1 * 0.5) * (ux2 * dxu - uz2 * dzw);
+    const double x3 = k000 - 3 * rho * (1 - 0.5) * (ux2 * dxu + uy2 * dyv + uz2 * dzw);
+    c200 = (x1 + x2 + x3) / 3;
+    c020 = c200 - x1;
+    c002 = c200 - x2;
+
+    MM(1, 1, 0) = c110; MM(0, 1, 1) = c011; MM(1, 0, 1) = c101;
+    MM(2, 0, 0) = c200; MM(0, 2, 0) = c020; MM(0, 0, 2) = c002;
+    // (1,2,0), (0,1,2), (2,0,1) and (1,1,1) are zero
+    MM(2, 1, 1) = (MM(2, 0, 0) * MM(0, 1, 1) + 2 * MM(1, 1, 0) * MM(1, 0, 1)) * ir;
+    MM(1, 2, 1) = (MM(0, 2, 0) * MM(1, 0, 1) + 2 * MM(0, 1, 1) * MM(1, 1, 0)) * ir;
+    MM(1, 1, 2) = (MM(0, 0, 2) * MM(1, 1, 0) + 2 * MM(1, 0, 1) * MM(0, 1, 1)) * ir;
+    MM(2, 2, 0) = (MM(2, 0, 0) * MM(0, 2, 0) + 2 * MM(1, 1, 0) * MM(1, 1, 0)) * ir;
+    MM(0, 2, 2) = (MM(0, 2, 0) * MM(0, 0, 2) + 2 * MM(0, 1, 1) * MM(0, 1, 1)) * ir;
+    MM(2, 0, 2) = (MM(0, 0, 2) * MM(2, 0, 0) + 2 * MM(1, 0, 1) * MM(1, 0, 1)) * ir;
+    MM(1, 2, 2) = (MM(0, 2, 0) * MM(1, 0, 2) + 2 * (MM(1, 0, 1) * MM(0, 2, 1))) * ir;
+    MM(2, 1, 2) = (MM(0, 0, 2) * MM(2, 1, 0) + 2 * (MM(1, 1, 0) * MM(1, 0, 2))) * ir;
+    MM(2, 2, 1) = (MM(2, 0, 0) * MM(0, 2, 1) + 2 * (MM(0, 1, 1) * MM(2, 1, 0))) * ir;
+    {
+        const double a = (MM(2, 0, 0) * MM(0, 2, 2) + MM(0, 2, 0) * MM(2, 0, 2) + MM(0, 0, 2) * MM(2, 2, 0) +
+                          4 * (MM(0, 1, 1) * MM(2, 1, 1) + MM(1, 0, 1) * MM(1, 2, 1) + MM(1, 1, 0) * MM(1, 1, 2))) * ir;
+        const double b = (16 * MM(1, 1, 0) * MM(1, 0, 1) * MM(0, 1, 1) +
+                          4 * (MM(1, 0, 1) * MM(1, 0, 1) * MM(0, 2, 0) + MM(0, 1, 1) * MM(0, 1, 1) * MM(2, 0, 0) +
+                               MM(1, 1, 0) * MM(1, 1, 0) * MM(0, 0, 2)) +
+                          2 * MM(2, 0, 0) * MM(0, 2, 0) * MM(0, 0, 2)) * ir * ir;
+        MM(2, 2, 2) = a - b;
     }
-    cumulant_from_moments<R>(m, rho, ux, uy, uz, omega1, out);
+    double p1[27], p2[27];
+    const double vx2 = ux * ux, vy2 = uy * uy, vz2 = uz * uz;
+#define XLINE(b, c) MM(0, b, c), MM(1, b, c), MM(2, b, c), ux, vx2, p1[3 * (b) + 9 * (c)], p1[1 + 3 * (b) + 9 * (c)], \
+                    p1[2 + 3 * (b) + 9 * (c)]
+    chim_back<>(XLINE(0, 0));
+    chim_back<>(XLINE(1, 0));
+    chim_back<false, true, false>(XLINE(2, 0));  // (1,2,0) = 0
+    chim_back<false, false, true>(XLINE(0, 1));  // (2,0,1) = 0
+    chim_back<false, true, false>(XLINE(1, 1));  // (1,1,1) = 0
+    chim_back<>(XLINE(2, 1));
+    chim_back<>(XLINE(0, 2));
+    chim_back<true, false, false>(XLINE(1, 2));  // (0,1,2) = 0
+    chim_back<>(XLINE(2, 2));
+#undef XLINE
+#pragma unroll
+    for (int ix = 0; ix < 3; ++ix)
+#pragma unroll
+        for (int cc = 0; cc < 3; ++cc)
+            chim_back<>(p1[ix + 0 + 9 * cc], p1[ix + 3 + 9 * cc], p1[ix + 6 + 9 * cc], uy, vy2, p2[ix + 0 + 9 * cc],
+                        p2[ix + 3 + 9 * cc], p2[ix + 6 + 9 * cc]);
+#pragma unroll
+    for (int ix = 0; ix < 3; ++ix)
+#pragma unroll
+        for (int iy = 0; iy < 3; ++iy)
+            chim_back<>(p2[ix + 3 * iy + 0], p2[ix + 3 * iy + 9], p2[ix + 3 * iy + 18], uz, vz2, m[ix + 3 * iy + 0],
+                        m[ix + 3 * iy + 9], m[ix + 3 * iy + 18]);
+#pragma unroll
+    for (int i = 0; i < 27; ++i) out[i] = m[(ex(i) + 1) + 3 * (ey(i) + 1) + 9 * (ez(i) + 1)];
 #undef MM
 }
 
