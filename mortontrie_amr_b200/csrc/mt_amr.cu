@@ -291,6 +291,46 @@ struct IbLatf {
     }
 };
 
+// indices satisfying pred, ascending; their number is known
+template <class Pred>
+static int select_known(Ctx &ctx, int64_t n, Pred pred, int64_t count, int32_t **out, int64_t *nout)
+{
+    *out = nullptr;
+    *nout = count;
+    if (!count) return MT_OK;
+    cub::CountingInputIterator<int32_t> it(0);
+    size_t tmp = 0;
+    MT_CUDA(ctx, cub::DeviceSelect::If(nullptr, tmp, it, (int32_t *)nullptr, (int *)nullptr, (int)n, pred, ctx.stream));
+    // one allocation for the selected count and the scratch
+    char *buf = nullptr;
+    MT_CUDA(ctx, cudaMallocAsync(out, sizeof(int32_t) * count, ctx.stream));
+    MT_CUDA(ctx, cudaMallocAsync(&buf, tmp + 256, ctx.stream));
+    MT_CUDA(ctx, cub::DeviceSelect::If(buf + 256, tmp, it, *out, (int *)buf, (int)n, pred, ctx.stream));
+    cudaFreeAsync(buf, ctx.stream);
+    return MT_OK;
+}
+
+// how many slots carry each tag bit (0..8) and each boundary set (9..34): the
+// sizes of a level's lists, read back once
+constexpr int kTagBits = 9;
+__global__ void k_count_sets(const uint32_t *__restrict__ tag, const int8_t *__restrict__ bc, int64_t n,
+                             unsigned *__restrict__ count)
+{
+    __shared__ unsigned s[kTagBits + 26];
+    for (int k = threadIdx.x; k < kTagBits + 26; k += blockDim.x) s[k] = 0;
+    __syncthreads();
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const uint32_t t = i < n ? tag[i] : 0u;
+    for (int k = 0; k < kTagBits; ++k) {
+        const unsigned m = __ballot_sync(0xffffffffu, (t >> k) & 1u);
+        if (m && (threadIdx.x & 31) == 0) atomicAdd(s + k, __popc(m));
+    }
+    if (t & TAG_BC) atomicAdd(s + kTagBits + bc[i], 1u);
+    __syncthreads();
+    for (int k = threadIdx.x; k < kTagBits + 26; k += blockDim.x)
+        if (s[k]) atomicAdd(count + k, s[k]);
+}
+
 template <class Pred>
 static int select_indices(Ctx &ctx, int64_t n, Pred pred, int32_t **out, int64_t *nout)
 {
@@ -426,14 +466,24 @@ static int build_level(Ctx &ctx, Case &c, int l)
         });
         if (rc) return rc;
     }
+    unsigned *d_count = nullptr, count[kTagBits + 26];
+    MT_CUDA(ctx, cudaMallocAsync(&d_count, sizeof(count), ctx.stream));
+    MT_CUDA(ctx, cudaMemsetAsync(d_count, 0, sizeof(count), ctx.stream));
+    k_count_sets<<<grid_for(n, 256), 256, 0, ctx.stream>>>(lv.tag, lv.bcidx, n, d_count);
+    MT_LAUNCHED(ctx);
+    MT_CUDA(ctx, cudaMemcpyAsync(count, d_count, sizeof(count), cudaMemcpyDeviceToHost, ctx.stream));
+    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
+    cudaFreeAsync(d_count, ctx.stream);
     const uint32_t bits[kNumSets] = {TAG_LATF, TAG_F2C, TAG_C2F, TAG_GC2F, TAG_GF2C, TAG_SF};
     for (int s = 0; s < kNumSets; ++s) {
-        int rc = select_indices(ctx, n, TagHas{lv.tag, bits[s]}, &lv.list[s], &lv.nlist[s]);
+        int at = 0;
+        while ((bits[s] >> at) != 1u) ++at;
+        int rc = select_known(ctx, n, TagHas{lv.tag, bits[s]}, count[at], &lv.list[s], &lv.nlist[s]);
         if (rc) return rc;
     }
     if (l == 0)
         for (int b = 0; b < 26; ++b) {
-            int rc = select_indices(ctx, n, BcIs{lv.bcidx, (int8_t)b}, &lv.bclist[b], &lv.nbc[b]);
+            int rc = select_known(ctx, n, BcIs{lv.bcidx, (int8_t)b}, count[kTagBits + b], &lv.bclist[b], &lv.nbc[b]);
             if (rc) return rc;
         }
     int rc = concat_lists(ctx, lv.list[0], lv.nlist[0], lv.list[1], lv.nlist[1], &lv.collide_list, &lv.ncollide);

@@ -1202,6 +1202,35 @@ __global__ void __launch_bounds__(128, brick_min_blocks<Q, S, COLL, V>()) k_bric
                               sl.fall, sl.acc, sh);
 }
 
+// ABPatternPull::stream (Stream_Manager.cpp:43-76) over bricks: the lat_f and
+// overlap_C2F cells pull from sources found as in the fused pass, without the
+// neighbour table's 4 (Q - 1) B per cell (D3Q19 FP64: 304 B of populations).
+template <int Q, class S>
+__global__ void __launch_bounds__(128) k_stream_bricks(int64_t nb, const int32_t *__restrict__ nbr,
+                                                       const unsigned long long *__restrict__ mask,
+                                                       const uint32_t *__restrict__ tag, int textbook,
+                                                       const S *__restrict__ fcol, S *__restrict__ f)
+{
+    __shared__ BrickHood hood[4];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t b = 4 * (int64_t)blockIdx.x + w;
+    if (b >= nb) return;
+    const uint32_t i0 = 64u * (uint32_t)b + (uint32_t)lane;
+    const uint32_t t0 = __ldg(tag + i0), t1 = __ldg(tag + i0 + 32);
+    if (!__any_sync(0xffffffffu, ((t0 | t1) & (TAG_LATF | TAG_C2F)) != 0)) return;
+    brick_hood<Q>((int32_t)b, lane, BrickTab{nullptr, nbr, mask, nullptr, nullptr}, false, hood[w]);
+#pragma unroll 1
+    for (int part = 0; part < 2; ++part) {
+        if (!((part ? t1 : t0) & (TAG_LATF | TAG_C2F))) continue;
+        const uint32_t i = i0 + 32u * part;
+        S v[Q];
+        brick_gather<Q, S>(i, textbook, false, hood[w], fcol, f, v);
+        // a missing link's value is f's own: storing it again changes nothing
+#pragma unroll
+        for (int k = 0; k < Q; ++k) f[at<Q>(k, i)] = v[k];
+    }
+}
+
 // The streamed f of the class-1 cells, from the buffer the last fused pass
 // read (the values that pass would have stored).
 template <int Q, class S>
@@ -1784,7 +1813,12 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         return MT_OK;
     }
     case PH_STREAM:
-        if (lv.nstream) {
+        if (lv.nstream && lv.bnbr && n * Q < ((int64_t)1 << 32)) {
+            k_stream_bricks<Q, S><<<grid_for(lv.nbrick, 4), 128, 0, s>>>(lv.nbrick, lv.bnbr,
+                                                                        (const unsigned long long *)lv.bmask, lv.tag,
+                                                                        c.d.stream_convention, A::fcol(lv), A::f(lv));
+            MT_LAUNCHED(ctx);
+        } else if (lv.nstream) {
             k_stream<Q, S><<<grid_for(lv.nstream, B), B, 0, s>>>(lv.stream_list, lv.nstream, n, c.d.stream_convention,
                                                                   lv.nbr, A::fcol(lv), A::f(lv));
             MT_LAUNCHED(ctx);
