@@ -212,6 +212,18 @@ __global__ void k_brick_mark(const int32_t *child, int64_t count, uint8_t *bcls)
     if (bcls[ci] == 1) bcls[ci] = 3;
 }
 
+// MT_ITIME_HOLD: the C2F cells the explosion writes (class 6).  Its sources do not
+// change between a fine level's two substeps, so the first substep's explosion
+// writes both post-collision buffers, the second one is left out, and the
+// pass leaves these cells' next collision alone.
+__global__ void k_brick_exploded(const int32_t *child, const uint8_t *mask, int64_t count, uint8_t *bcls)
+{
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= 8 * count || !((mask[t >> 3] >> (t & 7)) & 1)) return;
+    const int64_t ci = (int64_t)child[t >> 3] + (t & 7);
+    if (bcls[ci] == 2) bcls[ci] = 6;
+}
+
 // one warp per brick, two cells per lane
 template <int Q>
 __global__ void k_brick_flag(int64_t nb, const uint8_t *__restrict__ bcls, const int32_t *__restrict__ nbr,
@@ -827,7 +839,9 @@ static int fused_lbm_kernel(Ctx &ctx, Case &c, int l, bool last_parent)
 
 static int record_fused_step(Ctx &ctx, Case &c)
 {
+    c.fused_now = true;
     int rc = fused_lbm_kernel(ctx, c, 0, true);
+    c.fused_now = false;
     if (rc) return rc;
     if (c.d.bc_mode == MT_BC_NEQ)
         if ((rc = amr_phase(ctx, c, PH_MACROS, 0))) return rc;
@@ -850,6 +864,11 @@ static int build_bricks(Ctx &ctx, Case &c, int l)
     if (l > 0 && c.lv[l - 1].coal_child && c.lv[l - 1].nlist[1]) {
         const int64_t cnt = c.lv[l - 1].nlist[1];
         k_brick_mark<<<grid_for(8 * cnt, 256), 256, 0, ctx.stream>>>(c.lv[l - 1].coal_child, cnt, lv.bcls);
+        MT_LAUNCHED(ctx);
+    }
+    if (l > 0 && lv.nexpl && c.itime == MT_ITIME_HOLD) {
+        k_brick_exploded<<<grid_for(8 * lv.nexpl, 256), 256, 0, ctx.stream>>>(lv.expl_child, lv.expl_mask, lv.nexpl,
+                                                                             lv.bcls);
         MT_LAUNCHED(ctx);
     }
     if (c.d.q == 19)
@@ -1242,7 +1261,7 @@ int batch_step(Ctx &ctx, Batch &B, const std::vector<Case *> &cases, int n)
                 (int64_t)((cases.size() + kMaxBatchSlots - 1) / kMaxBatchSlots);
         MT_CUDA(ctx, cudaMallocAsync(&B.ddesc[g], sizeof(BrickBatch) * R.cap, ctx.stream));
         R.dbase = B.ddesc[g];
-        for (Case *c : cases) c->no_side = true;
+        for (Case *c : cases) c->no_side = c->fused_now = true;
         const int64_t before = ctx.launches;
         cudaGraph_t captured = nullptr;
         cudaError_t e = cudaStreamBeginCapture(ctx.stream, cudaStreamCaptureModeThreadLocal);
@@ -1250,7 +1269,7 @@ int batch_step(Ctx &ctx, Batch &B, const std::vector<Case *> &cases, int n)
         int r = MT_OK;
         for (int k = 0; k < steps && !r; ++k) r = record_batch_step(ctx, R, cases);
         e = cudaStreamEndCapture(ctx.stream, &captured);
-        for (Case *c : cases) c->no_side = false;
+        for (Case *c : cases) c->no_side = c->fused_now = false;
         if (r || e != cudaSuccess) {
             if (captured) cudaGraphDestroy(captured);
             batch_drop(B);

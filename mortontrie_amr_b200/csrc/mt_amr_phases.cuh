@@ -178,9 +178,10 @@ template <class S> struct Eight {
 // which loaded and rescaled the same source eight times, 25 us so; the
 // coalescence, whose eight 2-byte loads per direction are one of 16 bytes,
 // 20 -> 13 us.
-// With a second post-collision buffer (fused schedule) the children of ghost
-// F2C cells (sources from nf2c on) are written to both: nothing else writes
-// them, and the reference keeps them over the second substep.
+// With a second post-collision buffer (fused schedule) the children of sources
+// from nf2c on are written to both: those of ghost F2C cells, since nothing
+// else writes them and the reference keeps them over the second substep, and
+// all of them where one explosion serves both substeps (k_brick_exploded).
 // cprev (MT_ITIME_EXTRAP, second substep): the sources' parent values at the
 // parent's previous step, [Q][ns]; the explosion then starts from
 // 1.5 fcol - 0.5 prev, the parent state extrapolated to the half step.
@@ -844,7 +845,8 @@ __global__ void k_pull_copy(const int32_t *__restrict__ list, int64_t nl, int64_
 // reference's find() returns.
 // Classes (bcls): 1 stream + collide, 3 the same with the streamed f stored, 2
 // stream (f stored) + copy, 4 a direct-forcing band cell (stream; collided
-// after the forcing).  The streamed f of class-1 cells is read by nothing in
+// after the forcing), 6 stream (f stored; the explosion wrote the next
+// collision).  The streamed f of class-1 cells is read by nothing in
 // the coarse step (their next collision is computed here, a missing link's
 // f never changes), so it is stored only when `fall` is set or when the
 // state leaves the fused schedule (k_brick_pull).
@@ -934,6 +936,7 @@ __device__ __forceinline__ void brick_cell(uint32_t i, int cls, bool complete, c
         for (int k = 0; k < Q; ++k) fnext[at<Q>(k, i)] = v[k];
         return;
     }
+    if (cls == 6) return;
     C d[Q];
     if (cls == 4) {
         // direct-forcing band: collided after the forcing; with acc the
@@ -1833,10 +1836,13 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         Level &cl = c.lv[l - 1];
         const double scale = c2f_scale(c, l);
         const bool ex = phase == PH_EXPLOSION_B && c.itime == MT_ITIME_EXTRAP;
+        // held parent state over bricks: once, into both buffers (k_brick_exploded)
+        const bool once = c.fused_now && lv.bricks && c.itime == MT_ITIME_HOLD;
+        if (once && phase == PH_EXPLOSION_B) return MT_OK;
         if (ex && !lv.expl_prev) return set_err(ctx, MT_ERR_STATE, "extrapolated explosion without saved sources");
         k_explosion<Q, S><<<grid_for(lv.nexpl, 64), 64, 0, s>>>(lv.expl_src, lv.expl_child, lv.expl_mask, lv.nexpl,
                                                                A::fcol(cl), A::fcol(lv), scale, (S *)lv.fcol_alt,
-                                                               lv.nexpl_f2c, c.shift[l - 1], c.shift[l],
+                                                               once ? 0 : lv.nexpl_f2c, c.shift[l - 1], c.shift[l],
                                                                ex ? (const S *)lv.expl_prev : nullptr);
         MT_LAUNCHED(ctx);
         if (ex) {

@@ -969,6 +969,16 @@ int mt_case_set_interface_time(mt_ctx *h, int32_t id, int32_t mode)
         return set_err(ctx, MT_ERR_ARG, "mode must be MT_ITIME_REFERENCE, MT_ITIME_HOLD or MT_ITIME_EXTRAP");
     c->prev_stale = true;
     if (mode != c->itime) {
+        if (c->built) {
+            // the brick classes depend on the mode
+            if ((rc = amr_sync_f(ctx, *c))) return rc;
+            c->primed = false;
+            amr_drop_fused(*c);
+            for (Batch *b : ctx.batches)
+                if (b)
+                    for (int32_t x : b->ids)
+                        if (x == id) batch_drop(*b);
+        }
         // the captured steps bake the explosion launches in
         if (c->graph) cudaGraphExecDestroy(c->graph);
         c->graph = nullptr;

@@ -81,7 +81,8 @@ struct Level {
     int32_t *fused_list = nullptr; int64_t nfused = 0;
     // the fused pass over bricks: bcls[slot] is the cell's work (0 none, 1
     // stream + collide, 2 stream + copy, 3 as 1 with f stored, 4 a
-    // direct-forcing band cell), bflag[b] what the brick's cells share
+    // direct-forcing band cell, 6 stream only: the explosion wrote the next
+    // collision), bflag[b] what the brick's cells share
     // (BRICK_*), blist the bricks with any work
     bool bricks = false;
     int brick_variant = 0;  // form of the pass (mt_case_tune_bricks)
@@ -203,6 +204,7 @@ struct Case {
     int64_t mlo[3] = {0, 0, 0}, mdim[3] = {0, 0, 0};
     bool use_bricks = true;  // fused pass over 4x4x4 bricks where a level allows it (else cell lists)
     bool primed = false;
+    bool fused_now = false;  // set while a fused step is recorded
     int par0 = 0;
     cudaGraphExec_t fgraph[2] = {nullptr, nullptr};
     int64_t fgraph_launches[2] = {0, 0};
