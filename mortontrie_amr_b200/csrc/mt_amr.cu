@@ -547,6 +547,11 @@ int amr_build(Ctx &ctx, Case &c)
             const size_t bytes = 8 * (3 * (size_t)grid_for(fl.nib, 32) + 1);
             MT_CUDA(ctx, cudaMallocAsync(&c.ib_force, bytes, ctx.stream));
             MT_CUDA(ctx, cudaMemsetAsync(c.ib_force, 0, bytes, ctx.stream));
+            if ((rc = amr_dispatch(c, [&](auto *tag) {
+                     using S = std::remove_pointer_t<decltype(tag)>;
+                     return AmrOps<S>::ib_tables(ctx, c);
+                 })))
+                return rc;
         }
     }
     {
@@ -669,7 +674,7 @@ void amr_free(Case &c)
     }
     if (c.h_force) cudaFreeHost(c.h_force);
     c.h_force = nullptr;
-    void *ptrs[] = {c.dis_key, c.dis, c.ib_force, c.force_acc, c.dev_err, c.bc_tmp, c.bc_all, c.bc_setb, c.bc_tmp_all,
+    void *ptrs[] = {c.dis_key, c.dis, c.ib_wall, c.ib_src, c.ib_dist, c.ib_force, c.force_acc, c.dev_err, c.bc_tmp, c.bc_all, c.bc_setb, c.bc_tmp_all,
                     c.mref, c.mdv, c.path, c.mforce, c.tstep, c.acc, c.mgrid};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -680,6 +685,9 @@ void amr_free(Case &c)
     c.nbc_all = 0;
     c.dis_key = nullptr;
     c.dis = nullptr;
+    c.ib_wall = nullptr;
+    c.ib_src = nullptr;
+    c.ib_dist = nullptr;
     c.ib_force = nullptr;
     c.force_acc = nullptr;
     c.dev_err = nullptr;

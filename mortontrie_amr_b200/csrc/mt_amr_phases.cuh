@@ -547,14 +547,42 @@ __global__ void k_bc_set_eq(const int32_t *list, int64_t nl, int64_t n, double r
 // the sweeps run in registers).  g receives the new f, (fx, fy, fz) the
 // cell's momentum-exchange force.
 // The cell count is small (a sphere's skin), so the time is one thread's
-// chain of dependent loads: the wall distances of every link, then every
-// link's source slot, then every population are each read in one go, with
-// addresses selected instead of branches taken (a link without a source
-// reads the cell's own opposite population, which is its value), three
-// memory latencies in all; the walls are kept as a bit mask for the sweeps.
+// chain of dependent loads.  What does not change is laid out once per case,
+// by cell of the IB list (IbTab, k_ib_tables): a mask of the wall links, each
+// link's wall distance and its source slot.  A cell then loads its tables in
+// one round and every population in a second, with addresses selected instead
+// of branches taken (a link without a source reads the cell's own opposite
+// population, which is its value).
 // One launch, caches cold, D3Q19 FP16 / D3Q27 FP16 / D3Q27 FP64: 35 / 50 / 49 us
-// with the links' loads behind branches, 16 / 28 / 23 us so; two launches of
-// 4 us each that summed the force are gone (ib_force_sum).
+// with the links' loads behind branches, 16 / 28 / 23 us from the neighbour
+// table and the distance rows in three rounds; two launches of 4 us each that
+// summed the force are gone (ib_force_sum).
+template <class C> struct IbTab {
+    const uint32_t *__restrict__ wall;  // [nib] bit k: link k meets the wall
+    const int32_t *__restrict__ src;    // [(Q - 1) nib] link k's source slot, -1 none
+    const C *__restrict__ dist;         // [(Q - 1) nib] link k's wall distance
+    int64_t nib;
+};
+template <int Q, class C>
+__global__ void k_ib_tables(const int32_t *__restrict__ list, int64_t nl, int64_t n, const int32_t *__restrict__ disrow,
+                            const double *__restrict__ dis, const int32_t *__restrict__ nbr, uint32_t *wall,
+                            int32_t *src, C *dist)
+{
+    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (j >= nl) return;
+    const int64_t i = list[j];
+    const double *dr = dis + (int64_t)disrow[i] * (Q - 1);
+    uint32_t m = 0;
+    for (int k = 1; k < Q; ++k) {
+        const double v = dr[inv(k) - 1];
+        const bool hit = v != -1.;
+        if (hit) m |= 1u << k;
+        // a wall link interpolates with the population arriving from the far side
+        src[(int64_t)(k - 1) * nl + j] = nbr[(int64_t)((hit ? inv(k) : k) - 1) * n + i];
+        dist[(int64_t)(k - 1) * nl + j] = (C)v;
+    }
+    wall[j] = m;
+}
 // FP32 multiplications and additions are paired into FMAs as written here
 // (pm_*), whatever surrounds them; in FP64 pm_fma is a multiplication and an
 // addition.
@@ -565,28 +593,22 @@ __device__ __forceinline__ double pm_mul(double a, double b) { return a * b; }
 __device__ __forceinline__ double pm_add(double a, double b) { return a + b; }
 __device__ __forceinline__ double pm_fma(double a, double b, double c) { return a * b + c; }
 template <int Q, int FH, class S>
-__device__ __forceinline__ void ib_cell(int64_t i, int64_t n, const double *__restrict__ dr,
-                                        const int32_t *__restrict__ nbr, const S *__restrict__ fcol,
-                                        typename Store<S>::C rho_b, typename Store<S>::C *g,
-                                        typename Store<S>::C &fx, typename Store<S>::C &fy,
+__device__ __forceinline__ void ib_cell(int64_t i, int64_t j, const IbTab<typename Store<S>::C> &t,
+                                        const S *__restrict__ fcol, typename Store<S>::C rho_b,
+                                        typename Store<S>::C *g, typename Store<S>::C &fx, typename Store<S>::C &fy,
                                         typename Store<S>::C &fz, const Shift &sh)
 {
     using T = Store<S>;
     using C = typename T::C;
+    const uint32_t wall = __ldg(t.wall + j);
     C dd[Q], own[Q], src[Q];
-    uint32_t wall = 0;  // bit k: link k meets the wall
-#pragma unroll
-    for (int k = 1; k < Q; ++k) {
-        const double v = __ldg(dr + inv(k) - 1);
-        dd[k] = (C)v;
-        wall |= v != -1. ? 1u << k : 0u;
-    }
-#pragma unroll
-    for (int k = 0; k < Q; ++k) own[k] = T::ld(fcol, at<Q>(k, i));
     int32_t si[Q];
 #pragma unroll
-    for (int k = 1; k < Q; ++k)
-        si[k] = __ldg(nbr + (int64_t)(((wall >> k) & 1 ? inv(k) : k) - 1) * n + i);
+    for (int k = 1; k < Q; ++k) si[k] = __ldg(t.src + (int64_t)(k - 1) * t.nib + j);
+#pragma unroll
+    for (int k = 1; k < Q; ++k) dd[k] = __ldg(t.dist + (int64_t)(k - 1) * t.nib + j);
+#pragma unroll
+    for (int k = 0; k < Q; ++k) own[k] = T::ld(fcol, at<Q>(k, i));
 #pragma unroll
     for (int k = 1; k < Q; ++k) src[k] = T::ld(fcol, si[k] >= 0 ? at<Q>(k, si[k]) : at<Q>(inv(k), i));
     g[0] = full_sh<S>(sh, own[0], 0);
@@ -721,9 +743,8 @@ __device__ __forceinline__ void ib_force_sum(double fx, double fy, double fz, do
 }
 
 template <int Q, int FH, class S>
-__global__ void __launch_bounds__(kIbBlock) k_ib_treat(const int32_t *__restrict__ list, int64_t nl, int64_t n,
-                                                       const int32_t *__restrict__ disrow,
-                                                       const double *__restrict__ dis, const int32_t *__restrict__ nbr,
+__global__ void __launch_bounds__(kIbBlock) k_ib_treat(const int32_t *__restrict__ list, int64_t nl,
+                                                       const IbTab<typename Store<S>::C> t,
                                                        const S *__restrict__ fcol,
                                                        const typename Store<S>::C *__restrict__ rho, S *__restrict__ f,
                                                        double *part, double *force, const Shift sh)
@@ -734,9 +755,8 @@ __global__ void __launch_bounds__(kIbBlock) k_ib_treat(const int32_t *__restrict
     C fx = 0, fy = 0, fz = 0;
     if (j < nl) {
         const int64_t i = list[j];
-        const double *dr = dis + (int64_t)disrow[i] * (Q - 1);
         C g[Q];
-        ib_cell<Q, FH, S>(i, n, dr, nbr, fcol, rho[i], g, fx, fy, fz, sh);
+        ib_cell<Q, FH, S>(i, j, t, fcol, rho[i], g, fx, fy, fz, sh);
 #pragma unroll
         for (int k = 0; k < Q; ++k) T::st(f, at<Q>(k, i), stored_sh<S>(sh, g[k], k));
     }
@@ -1262,8 +1282,8 @@ __global__ void __launch_bounds__(128) k_brick_pull(int64_t nb, const BrickTab t
 // substep: the macros of the cell's f before this treat.
 template <int Q, int FH, class S, int COLL>
 __global__ void __launch_bounds__(kIbBlock) k_ib_collide(
-    const int32_t *__restrict__ list, int64_t nl, int64_t n, const int32_t *__restrict__ disrow,
-    const double *__restrict__ dis, const int32_t *__restrict__ nbr, const S *__restrict__ fcol, S *__restrict__ f,
+    const int32_t *__restrict__ list, int64_t nl, int64_t n, const IbTab<typename Store<S>::C> t,
+    const S *__restrict__ fcol, S *__restrict__ f,
     S *__restrict__ fnext, const Relax tau, double *part, double *force, typename Store<S>::C *__restrict__ rho,
     typename Store<S>::C *__restrict__ u, int macros, const Shift sh)
 {
@@ -1273,13 +1293,12 @@ __global__ void __launch_bounds__(kIbBlock) k_ib_collide(
     C fx = 0, fy = 0, fz = 0;
     if (j < nl) {
         const int64_t i = list[j];
-        const double *dr = dis + (int64_t)disrow[i] * (Q - 1);
         C g[Q];
         C r, x, y, z;
 #pragma unroll
         for (int k = 0; k < Q; ++k) g[k] = full_sh<S>(sh, T::cv(f[at<Q>(k, i)]), k);
         macros_g<Q, C>(g, r, x, y, z);
-        ib_cell<Q, FH, S>(i, n, dr, nbr, fcol, r, g, fx, fy, fz, sh);
+        ib_cell<Q, FH, S>(i, j, t, fcol, r, g, fx, fy, fz, sh);
 #pragma unroll
         for (int k = 0; k < Q; ++k) {
             const C st = stored_sh<S>(sh, g[k], k);
@@ -1618,6 +1637,10 @@ template <class S> struct AmrTyped {
     static S *fcol(Level &lv) { return (S *)lv.fcol; }
     static C *rho(Level &lv) { return (C *)lv.rho; }
     static C *u(Level &lv) { return (C *)lv.u; }
+    static IbTab<C> ib(const Case &c)
+    {
+        return IbTab<C>{c.ib_wall, c.ib_src, (const C *)c.ib_dist, c.lv[c.d.max_level].nib};
+    }
 };
 
 inline int upload_bdry_tables(Ctx &ctx)
@@ -1958,11 +1981,11 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
             const unsigned gi = grid_for(fl.nib, kIbBlock);
             const Shift &fsh = c.shift[c.d.max_level];
             if (c.d.ib_method == MT_IB_FH)
-                k_ib_treat<Q, 1, S><<<gi, kIbBlock, 0, s>>>(fl.iblist, fl.nib, fl.n, fl.disrow, c.dis, fl.nbr, A::fcol(fl),
-                                                            A::rho(fl), A::f(fl), c.ib_force, c.force_acc, fsh);
+                k_ib_treat<Q, 1, S><<<gi, kIbBlock, 0, s>>>(fl.iblist, fl.nib, A::ib(c), A::fcol(fl), A::rho(fl),
+                                                            A::f(fl), c.ib_force, c.force_acc, fsh);
             else
-                k_ib_treat<Q, 0, S><<<gi, kIbBlock, 0, s>>>(fl.iblist, fl.nib, fl.n, fl.disrow, c.dis, fl.nbr, A::fcol(fl),
-                                                            A::rho(fl), A::f(fl), c.ib_force, c.force_acc, fsh);
+                k_ib_treat<Q, 0, S><<<gi, kIbBlock, 0, s>>>(fl.iblist, fl.nib, A::ib(c), A::fcol(fl), A::rho(fl),
+                                                            A::f(fl), c.ib_force, c.force_acc, fsh);
         }
         MT_LAUNCHED(ctx);
         return MT_OK;
@@ -2086,7 +2109,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
                 auto ib = [&](auto fh, auto coll) {
                     constexpr int FH = decltype(fh)::value, COLL = decltype(coll)::value;
                     k_ib_collide<Q, FH, S, COLL><<<grid_for(lv.nib, kIbBlock), kIbBlock, 0, is>>>(
-                        lv.iblist, lv.nib, n, lv.disrow, c.dis, lv.nbr, A::fcol(lv), A::f(lv), (S *)lv.fcol_alt, tau,
+                        lv.iblist, lv.nib, n, A::ib(c), A::fcol(lv), A::f(lv), (S *)lv.fcol_alt, tau,
                         c.ib_force, c.force_acc, A::rho(lv), A::u(lv), mac, c.shift[l]);
                 };
                 using I0 = std::integral_constant<int, 0>;
@@ -2149,6 +2172,25 @@ template <class S>
 int AmrOps<S>::phase(Ctx &ctx, Case &c, int phase, int level)
 {
     return c.d.q == 19 ? amr_phase_q<S, 19>(ctx, c, phase, level) : amr_phase_q<S, 27>(ctx, c, phase, level);
+}
+
+template <class S>
+int AmrOps<S>::ib_tables(Ctx &ctx, Case &c)
+{
+    using C = typename Store<S>::C;
+    Level &fl = c.lv[c.d.max_level];
+    const int64_t nib = fl.nib, links = c.d.q - 1;
+    MT_CUDA(ctx, cudaMallocAsync(&c.ib_wall, sizeof(uint32_t) * nib, ctx.stream));
+    MT_CUDA(ctx, cudaMallocAsync(&c.ib_src, sizeof(int32_t) * links * nib, ctx.stream));
+    MT_CUDA(ctx, cudaMallocAsync(&c.ib_dist, sizeof(C) * links * nib, ctx.stream));
+    if (c.d.q == 19)
+        k_ib_tables<19, C><<<grid_for(nib, 128), 128, 0, ctx.stream>>>(fl.iblist, nib, fl.n, fl.disrow, c.dis, fl.nbr,
+                                                                      c.ib_wall, c.ib_src, (C *)c.ib_dist);
+    else
+        k_ib_tables<27, C><<<grid_for(nib, 128), 128, 0, ctx.stream>>>(fl.iblist, nib, fl.n, fl.disrow, c.dis, fl.nbr,
+                                                                      c.ib_wall, c.ib_src, (C *)c.ib_dist);
+    MT_LAUNCHED(ctx);
+    return MT_OK;
 }
 
 template <class S>

@@ -160,6 +160,9 @@ struct Case {
     std::vector<uint8_t> h_reg[MT_MAX_LEVELS + 1];
     int64_t reg_lo[MT_MAX_LEVELS + 1][3] = {};
     int64_t reg_n[MT_MAX_LEVELS + 1][3] = {};
+    uint32_t *ib_wall = nullptr;  // treat()'s tables by IB cell (IbTab)
+    int32_t *ib_src = nullptr;
+    void *ib_dist = nullptr;
     double *ib_force = nullptr;  // force partials of treat() (ib_force_sum)
     double *force_acc = nullptr; // [4] fx, fy, fz, treat count
     double *h_force = nullptr;   // [6] page-locked: force_acc copy [4], then the guard flags (int) (mt_case_force_async)
@@ -296,6 +299,8 @@ void copy_free(Ctx &ctx);
 template <class S> struct AmrOps {
     static int phase(Ctx &ctx, Case &c, int phase, int level);
     static int upload_tables(Ctx &ctx);
+    // treat()'s per-cell tables on the finest level (IbTab)
+    static int ib_tables(Ctx &ctx, Case &c);
     static int alloc(Ctx &ctx, Case &c, int level);
     static int init_eq(Ctx &ctx, Case &c, double rho0, const double *u0);
     static int get(Ctx &ctx, Case &c, int level, int which, double *d_out);      // which: 0 f, 1 fcol
