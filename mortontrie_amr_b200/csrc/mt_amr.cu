@@ -323,13 +323,14 @@ static int select_known(Ctx &ctx, int64_t n, Pred pred, int64_t count, int32_t *
 }
 
 // how many slots carry each tag bit (0..8) and each boundary set (9..34): the
-// sizes of a level's lists, read back once
-constexpr int kTagBits = 9;
+// sizes of a level's lists, read back once; and how many cells are both
+// collided and copied (35)
+constexpr int kTagBits = 9, kCounts = kTagBits + 27;
 __global__ void k_count_sets(const uint32_t *__restrict__ tag, const int8_t *__restrict__ bc, int64_t n,
                              unsigned *__restrict__ count)
 {
-    __shared__ unsigned s[kTagBits + 26];
-    for (int k = threadIdx.x; k < kTagBits + 26; k += blockDim.x) s[k] = 0;
+    __shared__ unsigned s[kCounts];
+    for (int k = threadIdx.x; k < kCounts; k += blockDim.x) s[k] = 0;
     __syncthreads();
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     const uint32_t t = i < n ? tag[i] : 0u;
@@ -338,8 +339,9 @@ __global__ void k_count_sets(const uint32_t *__restrict__ tag, const int8_t *__r
         if (m && (threadIdx.x & 31) == 0) atomicAdd(s + k, __popc(m));
     }
     if (t & TAG_BC) atomicAdd(s + kTagBits + bc[i], 1u);
+    if ((t & TAG_C2F) && (t & (TAG_LATF | TAG_F2C))) atomicAdd(s + kCounts - 1, 1u);
     __syncthreads();
-    for (int k = threadIdx.x; k < kTagBits + 26; k += blockDim.x)
+    for (int k = threadIdx.x; k < kCounts; k += blockDim.x)
         if (s[k]) atomicAdd(count + k, s[k]);
 }
 
@@ -478,7 +480,7 @@ static int build_level(Ctx &ctx, Case &c, int l)
         });
         if (rc) return rc;
     }
-    unsigned *d_count = nullptr, count[kTagBits + 26];
+    unsigned *d_count = nullptr, count[kCounts];
     MT_CUDA(ctx, cudaMallocAsync(&d_count, sizeof(count), ctx.stream));
     MT_CUDA(ctx, cudaMemsetAsync(d_count, 0, sizeof(count), ctx.stream));
     k_count_sets<<<grid_for(n, 256), 256, 0, ctx.stream>>>(lv.tag, lv.bcidx, n, d_count);
@@ -486,6 +488,7 @@ static int build_level(Ctx &ctx, Case &c, int l)
     MT_CUDA(ctx, cudaMemcpyAsync(count, d_count, sizeof(count), cudaMemcpyDeviceToHost, ctx.stream));
     MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
     cudaFreeAsync(d_count, ctx.stream);
+    lv.mixed = count[kCounts - 1] != 0;
     const uint32_t bits[kNumSets] = {TAG_LATF, TAG_F2C, TAG_C2F, TAG_GC2F, TAG_GF2C, TAG_SF};
     for (int s = 0; s < kNumSets; ++s) {
         int at = 0;
@@ -737,6 +740,22 @@ int amr_init_equilibrium(Ctx &ctx, Case &c, double rho0, const double *u0)
 // computes the macros it needs from the same populations the reference's
 // calculateMacros(level) reads just before collide(level), so the separate
 // macros pass of each substep is folded into it.
+// the second stream of the IB cells' work
+static int make_side(Ctx &ctx, Case &c)
+{
+    if (c.side) return MT_OK;
+    MT_CUDA(ctx, cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking));
+    MT_CUDA(ctx, cudaEventCreateWithFlags(&c.ev_fork, cudaEventDisableTiming));
+    MT_CUDA(ctx, cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming));
+    return MT_OK;
+}
+// (the brick stream can leave cells out)
+static bool ib_beside_stream(const Case &c)
+{
+    const Level &lv = c.lv[c.d.max_level];
+    return c.d.ib_method != MT_IB_DF && lv.nib && lv.nstream && lv.bnbr && lv.n * c.d.q < ((int64_t)1 << 32);
+}
+
 int amr_lbm_kernel(Ctx &ctx, Case &c, int l)
 {
     const int L = c.d.max_level;
@@ -753,12 +772,32 @@ int amr_lbm_kernel(Ctx &ctx, Case &c, int l)
             if ((rc = amr_lbm_kernel(ctx, c, l + 1))) return rc;
         if (l > 0 && sub == 0) RUN(PH_EXPLOSION, l);
         if (l > 0 && sub == 1 && c.itime != MT_ITIME_REFERENCE) RUN(PH_EXPLOSION_B, l);
-        RUN(PH_STREAM, l);
-        if (l == 0) {
-            if (c.d.bc_mode == MT_BC_NEQ) RUN(PH_BC, 0);
-            if (c.d.bc_mode == MT_BC_ZOUHE_HH) RUN(PH_BC_HH, 0);
-        } else if (l == L) {
-            RUN(PH_IB, L);
+        if (l > 0 && l == L && ib_beside_stream(c)) {
+            // treat() reads fcol and writes every population of its cells, so
+            // their stream would be overwritten: left out, the two run side by
+            // side
+            if ((rc = make_side(ctx, c))) return rc;
+            cudaStream_t main = ctx.stream;
+            MT_CUDA(ctx, cudaEventRecord(c.ev_fork, main));
+            MT_CUDA(ctx, cudaStreamWaitEvent(c.side, c.ev_fork, 0));
+            ctx.stream = c.side;
+            rc = amr_phase(ctx, c, PH_IB, L);
+            ctx.stream = main;
+            c.skip_ib = true;
+            if (!rc) rc = amr_phase(ctx, c, PH_STREAM, l);
+            c.skip_ib = false;
+            // (joined on an error too: the streams may be capturing)
+            MT_CUDA(ctx, cudaEventRecord(c.ev_join, c.side));
+            MT_CUDA(ctx, cudaStreamWaitEvent(main, c.ev_join, 0));
+            if (rc) return rc;
+        } else {
+            RUN(PH_STREAM, l);
+            if (l == 0) {
+                if (c.d.bc_mode == MT_BC_NEQ) RUN(PH_BC, 0);
+                if (c.d.bc_mode == MT_BC_ZOUHE_HH) RUN(PH_BC_HH, 0);
+            } else if (l == L) {
+                RUN(PH_IB, L);
+            }
         }
         if (l < L) RUN(PH_COALESCENCE, l);
         if (l == 0) break;
@@ -771,9 +810,7 @@ static int record_step(Ctx &ctx, Case &c)
 {
     int rc = amr_lbm_kernel(ctx, c, 0);
     if (rc) return rc;
-    for (int l = 0; l <= c.d.max_level; ++l)
-        if ((rc = amr_phase(ctx, c, PH_MACROS, l))) return rc;
-    return MT_OK;
+    return amr_phase(ctx, c, PH_MACROS_ALL, 0);
 }
 
 static int capture(Ctx &ctx, Case &c, int (*record)(Ctx &, Case &), cudaGraphExec_t *out, int64_t *launches)
@@ -894,11 +931,8 @@ static int build_bricks(Ctx &ctx, Case &c, int l)
 static int prime_fused(Ctx &ctx, Case &c)
 {
     const int L = c.d.max_level;
-    if (!c.side && L > 0 && c.lv[L].nib) {
-        MT_CUDA(ctx, cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking));
-        MT_CUDA(ctx, cudaEventCreateWithFlags(&c.ev_fork, cudaEventDisableTiming));
-        MT_CUDA(ctx, cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming));
-    }
+    if (L > 0 && c.lv[L].nib)
+        if (int rc = make_side(ctx, c)) return rc;
     for (int l = 0; l <= L; ++l) {
         Level &lv = c.lv[l];
         if (!lv.n) continue;

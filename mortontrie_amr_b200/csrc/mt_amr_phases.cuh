@@ -69,6 +69,39 @@ __global__ void k_macros(const int32_t *list, int64_t nl, int64_t n, const S *f,
     u[2 * n + i] = z;
 }
 
+// the same for every level in one launch (the end of a coarse step): level l's
+// blocks are [block[l], block[l + 1])
+template <class S> struct MacroLevels {
+    int nlev = 0;
+    unsigned block[kMaxLevels + 1] = {};
+    const int32_t *list[kMaxLevels] = {};
+    int64_t nl[kMaxLevels] = {}, n[kMaxLevels] = {};
+    const S *f[kMaxLevels] = {};
+    typename Store<S>::C *rho[kMaxLevels] = {}, *u[kMaxLevels] = {};
+    float shift[kMaxLevels][27] = {};
+};
+template <int Q, class S>
+__global__ void k_macros_all(const __grid_constant__ MacroLevels<S> m)
+{
+    using T = Store<S>;
+    using C = typename T::C;
+    int l = 0;
+    while (l + 1 < m.nlev && blockIdx.x >= m.block[l + 1]) ++l;
+    const int64_t j = (blockIdx.x - m.block[l]) * (int64_t)blockDim.x + threadIdx.x;
+    if (j >= m.nl[l]) return;
+    const int64_t i = m.list[l][j], n = m.n[l];
+    const S *__restrict__ f = m.f[l];
+    C d[Q];
+#pragma unroll
+    for (int k = 0; k < Q; ++k) d[k] = full_v<S>(m.shift[l], T::ld(f, at<Q>(k, i)), k);
+    C r, x, y, z;
+    macros_g<Q, C>(d, r, x, y, z);
+    m.rho[l][i] = r;
+    m.u[l][i] = x;
+    m.u[l][n + i] = y;
+    m.u[l][2 * n + i] = z;
+}
+
 // The macros (rho, u into r, x, y, z) of one cell from its stored values d (in
 // the compute type; overwritten) and its post-collision populations into
 // out[at(k, i)]: LBM_Manager::calculateMacros with Collision_LBGK::collide
@@ -107,14 +140,34 @@ __device__ __forceinline__ void macros_collide_store(typename Store<S>::C *d, ty
     }
 }
 
+// fcol = f of one overlap_C2F cell (Collision_Manager.cpp:45-52)
+template <int Q, class S>
+__device__ __forceinline__ void copy_fcol(int64_t i, const S *__restrict__ f, S *__restrict__ fcol)
+{
+    S v[Q];  // every load before the first store
+#pragma unroll
+    for (int k = 0; k < Q; ++k) v[k] = f[at<Q>(k, i)];
+#pragma unroll
+    for (int k = 0; k < Q; ++k) fcol[at<Q>(k, i)] = v[k];
+}
+
 // calculateMacros(level) + Collision_LBGK::collide / Collision_Cumulant::collide
-// on lat_f then overlap_F2C (Collision_Manager.cpp:13-53, Collision_Cumulant.cpp:22-159)
+// on lat_f then overlap_F2C (Collision_Manager.cpp:13-53, Collision_Cumulant.cpp:22-159),
+// and the copy on overlap_C2F by the blocks behind them (other cells, nothing
+// shared: one launch less per substep, 3-5 us of a small level's 15)
 template <int Q, class S, int COLL>
-__global__ void k_collide(const int32_t *list, int64_t nl, int64_t n, const Relax tau, const S *f,
-                          typename Store<S>::C *rho, typename Store<S>::C *u, S *fcol, const Shift sh)
+__global__ void k_collide(const int32_t *__restrict__ list, int64_t nl, const int32_t *__restrict__ copy, int64_t ncopy,
+                          int64_t n, const Relax tau, const S *__restrict__ f, typename Store<S>::C *__restrict__ rho,
+                          typename Store<S>::C *__restrict__ u, S *__restrict__ fcol, const Shift sh)
 {
     using T = Store<S>;
     using C = typename T::C;
+    const int64_t nb = (nl + blockDim.x - 1) / blockDim.x;
+    if (blockIdx.x >= nb) {
+        const int64_t c = (blockIdx.x - nb) * (int64_t)blockDim.x + threadIdx.x;
+        if (c < ncopy) copy_fcol<Q, S>(copy[c], f, fcol);
+        return;
+    }
     const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nl) return;
     const int64_t i = list[j];
@@ -127,21 +180,6 @@ __global__ void k_collide(const int32_t *list, int64_t nl, int64_t n, const Rela
     u[i] = x;
     u[n + i] = y;
     u[2 * n + i] = z;
-}
-
-// fcol = f on overlap_C2F (Collision_Manager.cpp:45-52)
-template <int Q, class S>
-__global__ void k_copy_fcol(const int32_t *__restrict__ list, int64_t nl, const S *__restrict__ f,
-                            S *__restrict__ fcol)
-{
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= nl) return;
-    const int64_t i = list[j];
-    S v[Q];  // every load before the first store
-#pragma unroll
-    for (int k = 0; k < Q; ++k) v[k] = f[at<Q>(k, i)];
-#pragma unroll
-    for (int k = 0; k < Q; ++k) fcol[at<Q>(k, i)] = v[k];
 }
 
 // The eight children of a coarse cell are eight consecutive slots (base a
@@ -1228,23 +1266,27 @@ __global__ void __launch_bounds__(128, brick_min_blocks<Q, S, COLL, V>()) k_bric
 // ABPatternPull::stream (Stream_Manager.cpp:43-76) over bricks: the lat_f and
 // overlap_C2F cells pull from sources found as in the fused pass, without the
 // neighbour table's 4 (Q - 1) B per cell (D3Q19 FP64: 304 B of populations).
+// skip_ib: without the IB cells, which treat() writes whole (amr_lbm_kernel).
 template <int Q, class S>
 __global__ void __launch_bounds__(128) k_stream_bricks(int64_t nb, const int32_t *__restrict__ nbr,
                                                        const unsigned long long *__restrict__ mask,
-                                                       const uint32_t *__restrict__ tag, int textbook,
+                                                       const uint32_t *__restrict__ tag, int skip_ib, int textbook,
                                                        const S *__restrict__ fcol, S *__restrict__ f)
 {
     __shared__ BrickHood hood[4];
+    auto streamed = [skip_ib](uint32_t t) {
+        return (t & (TAG_LATF | TAG_C2F)) && !(skip_ib && (t & TAG_LATF) && (t & TAG_IB));
+    };
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t b = 4 * (int64_t)blockIdx.x + w;
     if (b >= nb) return;
     const uint32_t i0 = 64u * (uint32_t)b + (uint32_t)lane;
     const uint32_t t0 = __ldg(tag + i0), t1 = __ldg(tag + i0 + 32);
-    if (!__any_sync(0xffffffffu, ((t0 | t1) & (TAG_LATF | TAG_C2F)) != 0)) return;
+    if (!__any_sync(0xffffffffu, streamed(t0) || streamed(t1))) return;
     brick_hood<Q>((int32_t)b, lane, BrickTab{nullptr, nbr, mask, nullptr, nullptr}, false, hood[w]);
 #pragma unroll 1
     for (int part = 0; part < 2; ++part) {
-        if (!((part ? t1 : t0) & (TAG_LATF | TAG_C2F))) continue;
+        if (!streamed(part ? t1 : t0)) continue;
         const uint32_t i = i0 + 32u * part;
         S v[Q];
         brick_gather<Q, S>(i, textbook, false, hood[w], fcol, f, v);
@@ -1762,6 +1804,38 @@ int band_collide(Ctx &ctx, Case &c, int l, void *out)
     return MT_OK;
 }
 
+// collide(level): macros and collision of lat_f and overlap_F2C with the copy on
+// overlap_C2F, then the direct-forcing band with its force (band_collide)
+template <class S, int Q>
+int collide_level(Ctx &ctx, Case &c, int l, S *fcol)
+{
+    using A = AmrTyped<S>;
+    Level &lv = c.lv[l];
+    const int32_t *cl = lv.nband ? lv.collide_nb : lv.collide_list;
+    const int64_t ncl = lv.nband ? lv.ncollide_nb : lv.ncollide, ncopy = lv.nlist[2];
+    // one launch for both; where some cell is in both lists the copy comes last
+    auto launch = [&](int64_t n0, int64_t n1) {
+        if (n0 + n1 == 0) return MT_OK;
+        // the cumulant model exists for D3Q27 only (checked at case creation)
+        const int B = c.d.collision == MT_COLL_LBGK ? 128 : 64;
+        const unsigned g = grid_for(n0, B) + grid_for(n1, B);
+        if (c.d.collision == MT_COLL_LBGK) {
+            k_collide<Q, S, MT_COLL_LBGK><<<g, B, 0, ctx.stream>>>(cl, n0, lv.list[2], n1, lv.n, c.d.tau[l], A::f(lv),
+                                                                   A::rho(lv), A::u(lv), fcol, c.shift[l]);
+        } else {
+            if constexpr (Q == 27)
+                k_collide<Q, S, MT_COLL_CUMULANT><<<g, B, 0, ctx.stream>>>(cl, n0, lv.list[2], n1, lv.n, c.d.tau[l],
+                                                                           A::f(lv), A::rho(lv), A::u(lv), fcol,
+                                                                           c.shift[l]);
+        }
+        MT_LAUNCHED(ctx);
+        return MT_OK;
+    };
+    if (int rc = launch(ncl, lv.mixed ? 0 : ncopy)) return rc;
+    if (int rc = band_collide<S, Q>(ctx, c, l, fcol)) return rc;
+    return lv.mixed ? launch(0, ncopy) : MT_OK;
+}
+
 // One fused brick pass of level l in the form `variant` (brick_warp) on stream
 // s, writing the next collision into fnext.
 inline BrickTab brick_tab(const Level &lv)
@@ -1814,35 +1888,38 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
             MT_LAUNCHED(ctx);
         }
         return MT_OK;
-    case PH_COLLIDE: {
-        // the direct-forcing band collides with its force (band_collide)
-        const int32_t *cl = lv.nband ? lv.collide_nb : lv.collide_list;
-        const int64_t ncl = lv.nband ? lv.ncollide_nb : lv.ncollide;
-        if (ncl) {
-            if (c.d.collision == MT_COLL_LBGK) {
-                k_collide<Q, S, MT_COLL_LBGK><<<grid_for(ncl, B), B, 0, s>>>(cl, ncl, n, c.d.tau[l], A::f(lv),
-                                                                             A::rho(lv), A::u(lv), A::fcol(lv), c.shift[l]);
-            } else {
-                // the cumulant model exists for D3Q27 only (checked at case creation)
-                if constexpr (Q == 27)
-                    k_collide<Q, S, MT_COLL_CUMULANT><<<grid_for(ncl, 64), 64, 0, s>>>(
-                        cl, ncl, n, c.d.tau[l], A::f(lv), A::rho(lv), A::u(lv), A::fcol(lv), c.shift[l]);
-            }
-            MT_LAUNCHED(ctx);
+    case PH_MACROS_ALL: {
+        MacroLevels<S> m;
+        unsigned blocks = 0;
+        for (int k = 0; k <= c.d.max_level; ++k) {
+            Level &x = c.lv[k];
+            if (!x.ncollide) continue;
+            const int j = m.nlev++;
+            m.block[j] = blocks;
+            m.list[j] = x.collide_list;
+            m.nl[j] = x.ncollide;
+            m.n[j] = x.n;
+            m.f[j] = A::f(x);
+            m.rho[j] = A::rho(x);
+            m.u[j] = A::u(x);
+            for (int q = 0; q < 27; ++q) m.shift[j][q] = c.shift[k].v[q];
+            blocks += grid_for(x.ncollide, B);
         }
-        if (int rc = band_collide<S, Q>(ctx, c, l, A::fcol(lv))) return rc;
-        if (lv.nlist[2]) {
-            k_copy_fcol<Q, S><<<grid_for(lv.nlist[2], B), B, 0, s>>>(lv.list[2], lv.nlist[2], A::f(lv),
-                                                                      A::fcol(lv));
+        m.block[m.nlev] = blocks;
+        if (blocks) {
+            k_macros_all<Q, S><<<blocks, B, 0, s>>>(m);
             MT_LAUNCHED(ctx);
         }
         return MT_OK;
     }
+    case PH_COLLIDE:
+        return collide_level<S, Q>(ctx, c, l, A::fcol(lv));
     case PH_STREAM:
         if (lv.nstream && lv.bnbr && n * Q < ((int64_t)1 << 32)) {
             k_stream_bricks<Q, S><<<grid_for(lv.nbrick, 4), 128, 0, s>>>(lv.nbrick, lv.bnbr,
                                                                         (const unsigned long long *)lv.bmask, lv.tag,
-                                                                        c.d.stream_convention, A::fcol(lv), A::f(lv));
+                                                                        c.skip_ib ? 1 : 0, c.d.stream_convention,
+                                                                        A::fcol(lv), A::f(lv));
             MT_LAUNCHED(ctx);
         } else if (lv.nstream) {
             k_stream<Q, S><<<grid_for(lv.nstream, B), B, 0, s>>>(lv.stream_list, lv.nstream, n, c.d.stream_convention,
@@ -1995,11 +2072,13 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         if (lv.nlist[1]) {
             if (c.d.collision == MT_COLL_LBGK) {
                 k_collide<Q, S, MT_COLL_LBGK><<<grid_for(lv.nlist[1], B), B, 0, s>>>(
-                    lv.list[1], lv.nlist[1], n, c.d.tau[l], A::f(lv), A::rho(lv), A::u(lv), A::fcol(lv), c.shift[l]);
+                    lv.list[1], lv.nlist[1], nullptr, 0, n, c.d.tau[l], A::f(lv), A::rho(lv), A::u(lv), A::fcol(lv),
+                    c.shift[l]);
             } else {
                 if constexpr (Q == 27)
                     k_collide<Q, S, MT_COLL_CUMULANT><<<grid_for(lv.nlist[1], 64), 64, 0, s>>>(
-                        lv.list[1], lv.nlist[1], n, c.d.tau[l], A::f(lv), A::rho(lv), A::u(lv), A::fcol(lv), c.shift[l]);
+                        lv.list[1], lv.nlist[1], nullptr, 0, n, c.d.tau[l], A::f(lv), A::rho(lv), A::u(lv), A::fcol(lv),
+                    c.shift[l]);
             }
             MT_LAUNCHED(ctx);
         }
@@ -2061,28 +2140,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         // and the copy of C2F (the first collide(level) of the next substep)
         if (!n) return MT_OK;
         MT_CUDA(ctx, cudaMemcpyAsync(lv.fcol_alt, lv.fcol, sizeof(S) * Q * n, cudaMemcpyDeviceToDevice, s));
-        {
-            const int32_t *cl = lv.nband ? lv.collide_nb : lv.collide_list;
-            const int64_t ncl = lv.nband ? lv.ncollide_nb : lv.ncollide;
-            if (ncl) {
-                if (c.d.collision == MT_COLL_LBGK) {
-                    k_collide<Q, S, MT_COLL_LBGK><<<grid_for(ncl, B), B, 0, s>>>(
-                        cl, ncl, n, c.d.tau[l], A::f(lv), A::rho(lv), A::u(lv), (S *)lv.fcol_alt, c.shift[l]);
-                } else {
-                    if constexpr (Q == 27)
-                        k_collide<Q, S, MT_COLL_CUMULANT><<<grid_for(ncl, 64), 64, 0, s>>>(
-                            cl, ncl, n, c.d.tau[l], A::f(lv), A::rho(lv), A::u(lv), (S *)lv.fcol_alt, c.shift[l]);
-                }
-                MT_LAUNCHED(ctx);
-            }
-            if (int rc = band_collide<S, Q>(ctx, c, l, lv.fcol_alt)) return rc;
-        }
-        if (lv.nlist[2]) {
-            k_copy_fcol<Q, S><<<grid_for(lv.nlist[2], B), B, 0, s>>>(lv.list[2], lv.nlist[2], A::f(lv),
-                                                                      (S *)lv.fcol_alt);
-            MT_LAUNCHED(ctx);
-        }
-        return MT_OK;
+        return collide_level<S, Q>(ctx, c, l, (S *)lv.fcol_alt);
     case PH_PULL_COLLIDE: {
         // stream(level) of this substep fused with collide(level) of the next,
         // reading fcol and writing f and fcol_alt; treat() on the finest level

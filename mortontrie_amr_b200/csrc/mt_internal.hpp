@@ -24,7 +24,7 @@ constexpr int kNumSets = 6;  // lat_f, F2C, C2F, ghost C2F, ghost F2C, solid
 // then the fused schedule's own passes
 enum { PH_MACROS = 0, PH_COLLIDE, PH_STREAM, PH_EXPLOSION, PH_COALESCENCE, PH_BC, PH_IB, PH_BC_INOUT,
        PH_BC_FACE0 = 8, PH_F2C_COLLIDE = 16, PH_PULL_COLLIDE, PH_PRIME, PH_COAL_COLLIDE,
-       PH_SYNC_F, PH_DF, PH_BAND_GRID, PH_FACE_EQ0 = 24, PH_BC_HH = 32, PH_EXPLOSION_B, PH_EXPL_SAVE };
+       PH_SYNC_F, PH_DF, PH_BAND_GRID, PH_FACE_EQ0 = 24, PH_BC_HH = 32, PH_EXPLOSION_B, PH_EXPL_SAVE, PH_MACROS_ALL };
 
 // per-cell tag bits (which reference index sets the cell belongs to)
 enum : uint32_t {
@@ -94,6 +94,7 @@ struct Level {
     void *rho = nullptr, *u = nullptr;   // [n], [3 * n] macroscopic fields (double, or float for reduced storage)
     int32_t *list[kNumSets] = {};
     int64_t nlist[kNumSets] = {};
+    bool mixed = false;  // some C2F cell is lat_f or F2C too: its copy comes after its collision
     int32_t *collide_list = nullptr; int64_t ncollide = 0;  // lat_f then F2C
     int32_t *stream_list = nullptr;  int64_t nstream = 0;   // lat_f then C2F
     int32_t *bclist[26] = {};
@@ -215,6 +216,7 @@ struct Case {
     // overlaps the finest level's fused pass (disjoint cells)
     int macros_now = 0;  // set while recording a level's last substep of the coarse step
     int pull_mode = 0;   // PH_PULL_COLLIDE: 0 every cell, 1 the IB cells only (a batch runs the bricks)
+    bool skip_ib = false; // PH_STREAM leaves the IB cells to treat() (amr_lbm_kernel)
     bool no_side = false; // IB on the calling stream (batch recording)
     int in_batch = 0;     // batches holding the case
     bool f_stale = false; // fused passes left class-1 brick cells' streamed f unstored (amr_sync_f)
