@@ -208,14 +208,18 @@ template <class S> struct Eight {
     }
 };
 
-// AMR_transDDF_explosion (LBM_Manager.cpp:1059-1129), one thread per coarse
-// source cell: the rescaled populations are the same for its children, written
+// AMR_transDDF_explosion (LBM_Manager.cpp:1059-1129) per coarse source cell:
+// the rescaled populations are the same for its children, written
 // by one vector store per direction (where a child is left out, by one store
 // per child).  child[j] the first child's slot, mask[j] the children written.
 // 4-level D3Q27 FP16 sphere, per launch up to 40 us with a thread per child,
 // which loaded and rescaled the same source eight times, 25 us so; the
 // coalescence, whose eight 2-byte loads per direction are one of 16 bytes,
 // 20 -> 13 us.
+// Most levels have a few thousand sources, a fraction of what the GPU holds, and
+// one thread's instructions are the time: three warps share 32 sources, each
+// with all of the loads and the moments and a third of the directions'
+// equilibria and stores.
 // With a second post-collision buffer (fused schedule) the children of sources
 // from nf2c on are written to both: those of ghost F2C cells, since nothing
 // else writes them and the reference keeps them over the second substep, and
@@ -223,16 +227,17 @@ template <class S> struct Eight {
 // cprev (MT_ITIME_EXTRAP, second substep): the sources' parent values at the
 // parent's previous step, [Q][ns]; the explosion then starts from
 // 1.5 fcol - 0.5 prev, the parent state extrapolated to the half step.
+constexpr int kExplParts = 3;
 template <int Q, class S>
-__global__ void __launch_bounds__(64, 8) k_explosion(const int32_t *__restrict__ src, const int32_t *__restrict__ child,
-                                                  const uint8_t *__restrict__ mask, int64_t ns,
-                                                  const S *__restrict__ cfcol, S *__restrict__ ffcol, double scale,
-                                                  S *__restrict__ ffcol2, int64_t nf2c, const Shift csh,
-                                                  const Shift fsh, const S *__restrict__ cprev = nullptr)
+__global__ void __launch_bounds__(32 * kExplParts) k_explosion(
+    const int32_t *__restrict__ src, const int32_t *__restrict__ child, const uint8_t *__restrict__ mask, int64_t ns,
+    const S *__restrict__ cfcol, S *__restrict__ ffcol, double scale, S *__restrict__ ffcol2, int64_t nf2c,
+    const Shift csh, const Shift fsh, const S *__restrict__ cprev = nullptr)
 {
     using T = Store<S>;
     using C = typename T::C;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t j = blockIdx.x * (int64_t)32 + (threadIdx.x & 31);
+    const int part = threadIdx.x >> 5;
     if (j >= ns) return;
     const unsigned mk = mask[j];
     if (!mk) return;
@@ -246,27 +251,36 @@ __global__ void __launch_bounds__(64, 8) k_explosion(const int32_t *__restrict__
     }
     C r, x, y, z;
     macros_g<Q, C>(d, r, x, y, z);
-#pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        const C fe = feq_heluo_g<Q, C>(k, r, x, y, z);
-        d[k] = stored_sh<S>(fsh, fe + (C)scale * (d[k] - fe), k);
-    }
     const int nw = ffcol2 && j >= nf2c ? 2 : 1;
-#pragma unroll 1
-    for (int w = 0; w < nw; ++w) {
-        S *out = w ? ffcol2 : ffcol;
-        if (mk == 255u) {
+    auto write = [&](auto p) {
+        constexpr int K0 = decltype(p)::value * Q / kExplParts, K1 = (decltype(p)::value + 1) * Q / kExplParts;
 #pragma unroll
-            for (int k = 0; k < Q; ++k) store8<S>(out + at<Q>(k, ch), d[k]);
-        } else {
-#pragma unroll 1
-            for (int m = 0; m < 8; ++m)
-                if ((mk >> m) & 1u) {
-#pragma unroll
-                    for (int k = 0; k < Q; ++k) T::st(out, at<Q>(k, ch + m), d[k]);
-                }
+        for (int k = K0; k < K1; ++k) {
+            const C fe = feq_heluo_g<Q, C>(k, r, x, y, z);
+            d[k] = stored_sh<S>(fsh, fe + (C)scale * (d[k] - fe), k);
         }
-    }
+#pragma unroll 1
+        for (int w = 0; w < nw; ++w) {
+            S *out = w ? ffcol2 : ffcol;
+            if (mk == 255u) {
+#pragma unroll
+                for (int k = K0; k < K1; ++k) store8<S>(out + at<Q>(k, ch), d[k]);
+            } else {
+#pragma unroll 1
+                for (int m = 0; m < 8; ++m)
+                    if ((mk >> m) & 1u) {
+#pragma unroll
+                        for (int k = K0; k < K1; ++k) T::st(out, at<Q>(k, ch + m), d[k]);
+                    }
+            }
+        }
+    };
+    if (part == 0)
+        write(std::integral_constant<int, 0>{});
+    else if (part == 1)
+        write(std::integral_constant<int, 1>{});
+    else
+        write(std::integral_constant<int, 2>{});
 }
 
 // the explosion sources' parent values into prev [Q][ns] (MT_ITIME_EXTRAP)
@@ -1940,7 +1954,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         const bool once = c.fused_now && lv.bricks && c.itime == MT_ITIME_HOLD;
         if (once && phase == PH_EXPLOSION_B) return MT_OK;
         if (ex && !lv.expl_prev) return set_err(ctx, MT_ERR_STATE, "extrapolated explosion without saved sources");
-        k_explosion<Q, S><<<grid_for(lv.nexpl, 64), 64, 0, s>>>(lv.expl_src, lv.expl_child, lv.expl_mask, lv.nexpl,
+        k_explosion<Q, S><<<grid_for(lv.nexpl, 32), 32 * kExplParts, 0, s>>>(lv.expl_src, lv.expl_child, lv.expl_mask, lv.nexpl,
                                                                A::fcol(cl), A::fcol(lv), scale, (S *)lv.fcol_alt,
                                                                once ? 0 : lv.nexpl_f2c, c.shift[l - 1], c.shift[l],
                                                                ex ? (const S *)lv.expl_prev : nullptr);
