@@ -325,7 +325,7 @@ static int select_known(Ctx &ctx, int64_t n, Pred pred, int64_t count, int32_t *
 // how many slots carry each tag bit (0..8) and each boundary set (9..34): the
 // sizes of a level's lists, read back once; and how many cells are both
 // collided and copied (35)
-constexpr int kTagBits = 9, kCounts = kTagBits + 27;
+constexpr int kTagBits = 9, kCounts = kTagBits + 28;
 __global__ void k_count_sets(const uint32_t *__restrict__ tag, const int8_t *__restrict__ bc, int64_t n,
                              unsigned *__restrict__ count)
 {
@@ -339,7 +339,8 @@ __global__ void k_count_sets(const uint32_t *__restrict__ tag, const int8_t *__r
         if (m && (threadIdx.x & 31) == 0) atomicAdd(s + k, __popc(m));
     }
     if (t & TAG_BC) atomicAdd(s + kTagBits + bc[i], 1u);
-    if ((t & TAG_C2F) && (t & (TAG_LATF | TAG_F2C))) atomicAdd(s + kCounts - 1, 1u);
+    if ((t & TAG_C2F) && (t & (TAG_LATF | TAG_F2C))) atomicAdd(s + kCounts - 2, 1u);
+    if ((t & (TAG_C2F | TAG_GC2F)) && (t & (TAG_F2C | TAG_GF2C))) atomicAdd(s + kCounts - 1, 1u);
     __syncthreads();
     for (int k = threadIdx.x; k < kCounts; k += blockDim.x)
         if (s[k]) atomicAdd(count + k, s[k]);
@@ -488,7 +489,8 @@ static int build_level(Ctx &ctx, Case &c, int l)
     MT_CUDA(ctx, cudaMemcpyAsync(count, d_count, sizeof(count), cudaMemcpyDeviceToHost, ctx.stream));
     MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
     cudaFreeAsync(d_count, ctx.stream);
-    lv.mixed = count[kCounts - 1] != 0;
+    lv.mixed = count[kCounts - 2] != 0;
+    lv.chained = count[kCounts - 1] != 0;
     const uint32_t bits[kNumSets] = {TAG_LATF, TAG_F2C, TAG_C2F, TAG_GC2F, TAG_GF2C, TAG_SF};
     for (int s = 0; s < kNumSets; ++s) {
         int at = 0;
@@ -710,6 +712,12 @@ void amr_free(Case &c)
     if (c.ev_join) cudaEventDestroy(c.ev_join);
     c.side = nullptr;
     c.ev_fork = c.ev_join = nullptr;
+    for (Case::Branch &b : c.branch) {
+        if (b.s) cudaStreamDestroy(b.s);
+        if (b.fork) cudaEventDestroy(b.fork);
+        if (b.join) cudaEventDestroy(b.join);
+    }
+    c.branch.clear();
 }
 
 // ----------------------------------------------------------------------------
@@ -864,17 +872,42 @@ static int fused_lbm_kernel(Ctx &ctx, Case &c, int l, bool last_parent)
     } while (0)
     for (int sub = 0; sub < 2; ++sub) {
         const bool last = last_parent && (l == 0 || sub == 1);
+        const int mac = last && !(l == 0 && c.d.bc_mode == MT_BC_NEQ);
         swap_buffers(c, l);
         if (l == 0 && c.d.bc_mode == MT_BC_ZOUHE_OUTFLOW) RUN(PH_BC_INOUT, 0);
-        if (l < L)
-            if ((rc = fused_lbm_kernel(ctx, c, l + 1, last))) return rc;
-        if (l > 0 && sub == 0) RUN(PH_EXPLOSION, l);
-        if (l > 0 && sub == 1 && c.itime != MT_ITIME_REFERENCE) RUN(PH_EXPLOSION_B, l);
-        c.macros_now = last && !(l == 0 && c.d.bc_mode == MT_BC_NEQ);
-        RUN(PH_PULL_COLLIDE, l);
-        if (l == L && c.lv[l].nband) RUN(PH_DF, l);
-        if (l == 0 && c.d.bc_mode == MT_BC_NEQ) RUN(PH_BC, 0);
-        if (l < L) RUN(PH_COAL_COLLIDE, l);
+        auto own = [&]() -> int {
+            if (l > 0 && sub == 0) RUN(PH_EXPLOSION, l);
+            if (l > 0 && sub == 1 && c.itime != MT_ITIME_REFERENCE) RUN(PH_EXPLOSION_B, l);
+            c.macros_now = mac;
+            RUN(PH_PULL_COLLIDE, l);
+            if (l == L && c.lv[l].nband) RUN(PH_DF, l);
+            if (l == 0 && c.d.bc_mode == MT_BC_NEQ) RUN(PH_BC, 0);
+            return MT_OK;
+        };
+        if (l < L && l < (int)c.branch.size() && !c.lv[l].chained) {
+            // the finer levels read this level's fcol, which its own work leaves
+            // alone (its explosion writes none of their sources): side by side
+            Case::Branch &b = c.branch[l];
+            cudaStream_t main = ctx.stream;
+            MT_CUDA(ctx, cudaEventRecord(b.fork, main));
+            MT_CUDA(ctx, cudaStreamWaitEvent(b.s, b.fork, 0));
+            ctx.stream = b.s;
+            rc = own();
+            ctx.stream = main;
+            if (!rc) rc = fused_lbm_kernel(ctx, c, l + 1, last);
+            // (joined on an error too: the streams may be capturing)
+            MT_CUDA(ctx, cudaEventRecord(b.join, b.s));
+            MT_CUDA(ctx, cudaStreamWaitEvent(main, b.join, 0));
+            if (rc) return rc;
+        } else {
+            if (l < L)
+                if ((rc = fused_lbm_kernel(ctx, c, l + 1, last))) return rc;
+            if ((rc = own())) return rc;
+        }
+        if (l < L) {
+            c.macros_now = mac;
+            RUN(PH_COAL_COLLIDE, l);
+        }
         c.macros_now = 0;
         if (l == 0) break;
     }
@@ -911,7 +944,7 @@ static int build_bricks(Ctx &ctx, Case &c, int l)
         k_brick_mark<<<grid_for(8 * cnt, 256), 256, 0, ctx.stream>>>(c.lv[l - 1].coal_child, cnt, lv.bcls);
         MT_LAUNCHED(ctx);
     }
-    if (l > 0 && lv.nexpl && c.itime == MT_ITIME_HOLD) {
+    if (l > 0 && lv.nexpl && c.itime == MT_ITIME_HOLD && !lv.chained) {
         k_brick_exploded<<<grid_for(8 * lv.nexpl, 256), 256, 0, ctx.stream>>>(lv.expl_child, lv.expl_mask, lv.nexpl,
                                                                              lv.bcls);
         MT_LAUNCHED(ctx);
@@ -933,6 +966,13 @@ static int prime_fused(Ctx &ctx, Case &c)
     const int L = c.d.max_level;
     if (L > 0 && c.lv[L].nib)
         if (int rc = make_side(ctx, c)) return rc;
+    while ((int)c.branch.size() < L) {
+        c.branch.emplace_back();
+        Case::Branch &b = c.branch.back();
+        MT_CUDA(ctx, cudaStreamCreateWithFlags(&b.s, cudaStreamNonBlocking));
+        MT_CUDA(ctx, cudaEventCreateWithFlags(&b.fork, cudaEventDisableTiming));
+        MT_CUDA(ctx, cudaEventCreateWithFlags(&b.join, cudaEventDisableTiming));
+    }
     for (int l = 0; l <= L; ++l) {
         Level &lv = c.lv[l];
         if (!lv.n) continue;

@@ -1634,7 +1634,7 @@ __global__ void k_band_collide(const int32_t *band, int64_t nb, int64_t n, const
     }
 }
 
-static __global__ void k_force_tick(double *acc) { acc[3] += 1.0; }
+static __global__ void k_force_tick(double *acc, double steps) { acc[3] += steps; }
 
 // Host arrays hold a level's stored cells in key order ([Q][nc], [nc]); slot[r]
 // is the slot of cell r.
@@ -1790,7 +1790,7 @@ int df_force(Ctx &ctx, Case &c, int l, bool band_macros_done = false)
         MT_LAUNCHED(ctx);
     }
     if (!c.nm) {
-        k_force_tick<<<1, 1, 0, s>>>(c.force_acc);
+        k_force_tick<<<1, 1, 0, s>>>(c.force_acc, 1.0);
         MT_LAUNCHED(ctx);
         return MT_OK;
     }
@@ -1951,7 +1951,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         const double scale = c2f_scale(c, l);
         const bool ex = phase == PH_EXPLOSION_B && c.itime == MT_ITIME_EXTRAP;
         // held parent state over bricks: once, into both buffers (k_brick_exploded)
-        const bool once = c.fused_now && lv.bricks && c.itime == MT_ITIME_HOLD;
+        const bool once = c.fused_now && lv.bricks && c.itime == MT_ITIME_HOLD && !lv.chained;
         if (once && phase == PH_EXPLOSION_B) return MT_OK;
         if (ex && !lv.expl_prev) return set_err(ctx, MT_ERR_STATE, "extrapolated explosion without saved sources");
         k_explosion<Q, S><<<grid_for(lv.nexpl, 32), 32 * kExplParts, 0, s>>>(lv.expl_src, lv.expl_child, lv.expl_mask, lv.nexpl,
@@ -2064,7 +2064,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         if (c.d.ib_method == MT_IB_DF) return df_force<S, Q>(ctx, c, c.d.max_level);
         Level &fl = c.lv[c.d.max_level];
         if (!fl.nib) {
-            k_force_tick<<<1, 1, 0, s>>>(c.force_acc);
+            k_force_tick<<<1, 1, 0, s>>>(c.force_acc, 1.0);
             MT_LAUNCHED(ctx);
             return MT_OK;
         }
@@ -2174,8 +2174,11 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         }
         if (ib_level) {
             if (!lv.nib) {
-                k_force_tick<<<1, 1, 0, s>>>(c.force_acc);
-                MT_LAUNCHED(ctx);
+                // the coarse step's 2^L counts at its last substep (3 us a launch)
+                if (mac) {
+                    k_force_tick<<<1, 1, 0, s>>>(c.force_acc, (double)(1 << L));
+                    MT_LAUNCHED(ctx);
+                }
             } else {
                 const double tau = c.d.tau[l];
                 auto ib = [&](auto fh, auto coll) {

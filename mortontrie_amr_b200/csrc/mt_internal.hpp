@@ -94,7 +94,8 @@ struct Level {
     void *rho = nullptr, *u = nullptr;   // [n], [3 * n] macroscopic fields (double, or float for reduced storage)
     int32_t *list[kNumSets] = {};
     int64_t nlist[kNumSets] = {};
-    bool mixed = false;  // some C2F cell is lat_f or F2C too: its copy comes after its collision
+    bool mixed = false;    // some C2F cell is lat_f or F2C too: its copy comes after its collision
+    bool chained = false;  // some source of the finer level's explosion is written by this level's
     int32_t *collide_list = nullptr; int64_t ncollide = 0;  // lat_f then F2C
     int32_t *stream_list = nullptr;  int64_t nstream = 0;   // lat_f then C2F
     int32_t *bclist[26] = {};
@@ -222,6 +223,12 @@ struct Case {
     bool f_stale = false; // fused passes left class-1 brick cells' streamed f unstored (amr_sync_f)
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    // a coarse level's own work beside its finer levels' substeps, per level (fused_lbm_kernel)
+    struct Branch {
+        cudaStream_t s = nullptr;
+        cudaEvent_t fork = nullptr, join = nullptr;
+    };
+    std::vector<Branch> branch;
 };
 
 // Cases stepped together (mt_batch_*): one batched brick pass per level,

@@ -1,0 +1,68 @@
+"""A level's own work beside its finer levels' substeps, one explosion for
+both substeps, and the launches that the phase order merges, where the order
+matters: interface options changed on the way, and sets that overlap."""
+import numpy as np
+import pytest
+from helpers import TAG_BC
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    from mortontrie_amr_b200.lbm import Context
+    c = Context(0)
+    yield c
+    c.close()
+
+
+def _sphere(levels=2):
+    from mortontrie_amr_b200.case import sphere_case
+    return sphere_case(coarse=(36, 20, 24), max_level=levels, refine=[((7, 4, 5), (21, 17, 19)),
+                                                                      ((17, 12, 13), (39, 31, 35))][:levels],
+                       center=(14, 11, 12), radius=2.5, re=40.0)
+
+
+def _oracle_equal(mgr, oc, levels):
+    for l in levels:
+        f, fcol = mgr.populations(l)
+        g = oc.get(l)
+        keep = (g["tags"] & TAG_BC) == 0
+        assert np.array_equal(f[:, keep], g["f"][:, keep]), l
+        assert np.array_equal(fcol, g["fcol"]), l
+
+
+@pytest.mark.parametrize("schedule", ["phases", "fused"])
+@pytest.mark.parametrize("order", [("reference", "hold", "reference"), ("hold", "extrap", "hold")])
+def test_interface_option_changed_between_steps(ctx, schedule, order):
+    """FP64, bit for bit against the oracle taking the same options."""
+    import oracle as O
+    from mortontrie_amr_b200.lbm import LBM_Manager
+    case = _sphere()
+    mgr = LBM_Manager(ctx, case, schedule=schedule, interface_time=order[0])
+    oc = O.OracleCase(case)
+    for mode in order:
+        mgr.set_interface_time(mode)
+        oc.set_interface_time(mode)
+        mgr.fluidSimulate(2)
+        oc.step(2)
+    ctx.synchronize()
+    _oracle_equal(mgr, oc, range(case.max_level + 1))
+    mgr.close()
+
+
+def test_cells_in_both_overlaps(ctx):
+    """Cells that are overlap_F2C and overlap_C2F at once keep the reference's
+    order, collision first and copy last."""
+    import oracle as O
+    from mortontrie_amr_b200.lbm import LBM_Manager
+    case = _sphere()
+    d = case.mesh.levels[1]
+    d["overlap_C2F"] = np.sort(np.concatenate([d["overlap_C2F"], d["overlap_F2C"][::7]]))
+    mgr = LBM_Manager(ctx, case)
+    oc = O.OracleCase(case)
+    mgr.fluidSimulate(3)
+    oc.step(3)
+    ctx.synchronize()
+    _oracle_equal(mgr, oc, range(case.max_level + 1))
+    mgr.close()
