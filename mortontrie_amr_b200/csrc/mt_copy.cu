@@ -24,8 +24,8 @@ struct Job;
 // page-locked ring and copying threads of one context, made at its first large
 // copy, given back with it
 struct HostStage {
-    static constexpr size_t kChunk = 1u << 20;
-    static constexpr int kSlots = 24;  // 24 MiB
+    static constexpr size_t kChunk = 1u << 19;
+    static constexpr int kSlots = 16;  // 8 MiB, page-locked in about 2 ms
     char *buf = nullptr;
     cudaEvent_t ev[kSlots] = {};
     std::mutex busy;  // one copy at a time; another thread's takes the plain path
@@ -40,8 +40,14 @@ struct HostStage {
 
 namespace {
 
-// below this a plain copy is over before the threads are awake
-constexpr size_t kStagedFrom = 2u << 20;
+// Arrays of this size are fresh mappings (the C library maps every allocation
+// of 32 MiB and more, and reuses the pages of smaller ones): every page of the
+// copy is a fault.  262 MB of a 4-level sphere's fields, 16 cores: 67 ms by
+// plain copies, 52 with 2 threads, 46 with 4, 36 with 8.  Smaller arrays have
+// their pages already, and a caller's own threads that still spin keep the
+// copying threads from their cores: 34 MB of fields 5.9-7.5 ms plain, 7-27 ms
+// by threads.
+constexpr size_t kStagedFrom = 32u << 20;
 
 // chunk c of the copy: filled by the stream, emptied by one thread
 struct Job {
