@@ -964,7 +964,7 @@ static int build_bricks(Ctx &ctx, Case &c, int l)
 static int prime_fused(Ctx &ctx, Case &c)
 {
     const int L = c.d.max_level;
-    if (L > 0 && c.lv[L].nib)
+    if (L > 0 && (c.lv[L].nib || c.lv[L].nband))
         if (int rc = make_side(ctx, c)) return rc;
     while ((int)c.branch.size() < L) {
         c.branch.emplace_back();

@@ -66,3 +66,25 @@ def test_cells_in_both_overlaps(ctx):
     ctx.synchronize()
     _oracle_equal(mgr, oc, range(case.max_level + 1))
     mgr.close()
+
+
+@pytest.mark.parametrize("schedule", ["phases", "fused"])
+@pytest.mark.parametrize("markers", [1, 6, 199, 201])
+def test_marker_counts(ctx, schedule, markers):
+    """Direct forcing by few and odd numbers of markers (a warp each, four to a
+    block): FP64 bit for bit, the body force to the order of its sum."""
+    from helpers import run_oracle
+    from mortontrie_amr_b200.case import df_sphere_case
+    from mortontrie_amr_b200.lbm import LBM_Manager
+    case = df_sphere_case(radius=2, max_level=1, re=50.0, oscillating=True, period=60)
+    m = case.mesh.markers
+    m.ref, m.dv = np.ascontiguousarray(m.ref[:, :markers]), np.ascontiguousarray(m.dv[:markers])
+    mgr = LBM_Manager(ctx, case, schedule=schedule)
+    mgr.fluidSimulate(5)
+    ctx.synchronize()
+    oc = run_oracle(case, 5)
+    _oracle_equal(mgr, oc, range(case.max_level + 1))
+    fg, fo = mgr.force(), oc.force()
+    assert fg[3] == fo[3] == 10
+    assert np.abs(fg[:3] - fo[:3]).max() <= 1e-12 * np.abs(fo[:3]).max()
+    mgr.close()
