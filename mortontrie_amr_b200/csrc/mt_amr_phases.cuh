@@ -1226,12 +1226,15 @@ __device__ __forceinline__ void brick_warp(int32_t b, int lane, BrickHood &h, co
 //   D3Q27 FP32: 4 blocks 191.5 us, 5 175.1, 6 (40 B of spills) 166.9, 7 183.3
 //   D3Q19 FP16: 5 blocks 216.1 us, 6 194.2, 7 183.3, 8 177.2, 9 175.1
 //   D3Q19 FP32: 5 blocks 283.0 us, 6 263.2, 7 250.9
+// Form 0 is what a level runs untuned: the fastest number, but 7 for D3Q19 at 16
+// bits, where 9 (56 registers, 52 B of spills) lose on levels of less than a
+// wave (a 537,000-cell sphere's coarse step 141 us with 7, 146 with 9).
 template <int Q, class S, int COLL, int V> constexpr int brick_min_blocks()
 {
     if (!Store<S>::shifted) return 1;
     if (V == 1) return Store<S>::bytes == 2 ? ((COLL == MT_COLL_LBGK && Q == 19) ? 10 : 8) : 7;
-    if (Store<S>::bytes == 2) return Q == 19 ? (V == 0 ? 7 : (V == 2 ? 8 : 9)) : (V == 0 ? 6 : (V == 2 ? 7 : 8));
-    return V == 0 ? 6 : (V == 2 ? 5 : 7);
+    if (Store<S>::bytes == 2) return Q == 19 ? (V == 0 ? 7 : (V == 2 ? 8 : 9)) : (V == 0 ? 7 : (V == 2 ? 6 : 8));
+    return Q == 19 ? (V == 0 ? 7 : (V == 2 ? 6 : 5)) : (V == 0 ? 6 : (V == 2 ? 5 : 7));
 }
 // the form a level runs until mt_case_tune_bricks times them
 template <class S> constexpr int brick_default_variant() { return 0; }
