@@ -551,8 +551,8 @@ def batched_section(ctx, torch, steps=20, warmup=2, solve_steps=2000, n_cases=64
     """Batched uneven instances: 64 seeded cases (cavities and spheres, 4
     domain sizes, 1-3 refinement levels, Re 10-200, D3Q19 LBGK or D3Q27
     cumulant, stress-continuous interface factors).  All cases in one batch
-    (FP16 storage, fused schedule, one batched brick pass per level, substep
-    and model) against the same cases solved one at a time in the plain form
+    (FP16 storage, fused schedule, every case a branch of one captured
+    step) against the same cases solved one at a time in the plain form
     (FP64, phase order) and one at a time with FP16 storage.  Cases/h assume
     `solve_steps` coarse steps per case at the measured per-step times;
     accuracy compares the batched FP16 state with plain FP64 after the same

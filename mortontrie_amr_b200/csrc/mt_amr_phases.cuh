@@ -1253,33 +1253,6 @@ __global__ void __launch_bounds__(128, brick_min_blocks<Q, S, COLL, V>()) k_bric
                               fall, acc, sh);
 }
 
-// The same pass over the bricks of many cases (a batch): brick j of the work
-// list belongs to the slot whose [off[s], off[s + 1]) range holds it; each
-// slot carries one case level's tables, buffers and relaxation time.
-template <int Q, class S, int COLL, int V>
-__global__ void __launch_bounds__(128, brick_min_blocks<Q, S, COLL, V>()) k_brick_step_batch(const BrickBatch *__restrict__ bb,
-                                                                                             const Shift sh)
-{
-    __shared__ BrickHood hood[4];
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t j = 4 * (int64_t)blockIdx.x + w;
-    if (j >= bb->total) return;
-    int lo = 0, hi = bb->nslots;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (bb->off[mid] <= j)
-            lo = mid;
-        else
-            hi = mid;
-    }
-    const BrickSlot &sl = bb->slot[lo];
-    using C = typename Store<S>::C;
-    const BrickTab t{sl.list, sl.nbr, sl.mask, sl.cls, sl.flag};
-    brick_warp<Q, S, COLL, V>(__ldg(t.list + (j - bb->off[lo])), lane, hood[w], t, sl.n, sl.textbook,
-                              (const S *)sl.fcol, (S *)sl.f, (S *)sl.fnext, sl.tau, (C *)sl.rho, (C *)sl.u, sl.macros,
-                              sl.fall, sl.acc, sh);
-}
-
 // ABPatternPull::stream (Stream_Manager.cpp:43-76) over bricks: the lat_f and
 // overlap_C2F cells pull from sources found as in the fused pass, without the
 // neighbour table's 4 (Q - 1) B per cell (D3Q19 FP64: 304 B of populations).
@@ -2137,7 +2110,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         if (int rc = df_force<S, Q>(ctx, c, l, lv.bricks)) return rc;
         {
             // the body force beside the band's collision (6 us of a substep's chain)
-            const bool sum = lv.nband && c.nm, fork = sum && c.side && !c.no_side;
+            const bool sum = lv.nband && c.nm, fork = sum && c.side;
             if (fork) {
                 MT_CUDA(ctx, cudaEventRecord(c.ev_fork, s));
                 MT_CUDA(ctx, cudaStreamWaitEvent(c.side, c.ev_fork, 0));
@@ -2184,7 +2157,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         // level 0's boundary sweep reads the streamed f of inner cells
         const int fall = (l == 0 && c.d.bc_mode == MT_BC_NEQ) ? 1 : 0;
         cudaStream_t is = s;
-        if (ib_level && lv.nib && c.side && !c.no_side) {
+        if (ib_level && lv.nib && c.side) {
             MT_CUDA(ctx, cudaEventRecord(c.ev_fork, s));
             MT_CUDA(ctx, cudaStreamWaitEvent(c.side, c.ev_fork, 0));
             is = c.side;
@@ -2218,9 +2191,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
                 MT_LAUNCHED(ctx);
             }
         }
-        if (c.pull_mode == 1) {
-            // the batch runs this level's bricks
-        } else if (lv.bricks) {
+        if (lv.bricks) {
             // the band's macros come out of the pass (the direct-forcing step skips k_band_macros)
             long long *bacc = (l == L && lv.nband) ? c.acc : nullptr;
             brick_launch<Q, S>(c, l, lv.brick_variant, s, (S *)lv.fcol_alt, mac, fall, bacc);
@@ -2367,22 +2338,6 @@ int AmrOps<S>::macros_out(Ctx &ctx, Case &c, int l, double *d_rho, double *d_u)
     if (!lv.n) return MT_OK;
     k_macro_to_f64<C><<<grid_for(lv.ncell, 256), 256, 0, ctx.stream>>>((const C *)lv.rho, (const C *)lv.u, lv.n,
                                                                         lv.slot, lv.ncell, d_rho, d_u);
-    MT_LAUNCHED(ctx);
-    return MT_OK;
-}
-
-template <class S>
-int AmrOps<S>::batch_pass(Ctx &ctx, int q, int coll, const BrickBatch *d_desc, int64_t total, const Shift &sh)
-{
-    const unsigned g = grid_for(total, 4);
-    if (!g) return MT_OK;
-    constexpr int V = brick_default_variant<S>();
-    if (q == 19)
-        k_brick_step_batch<19, S, MT_COLL_LBGK, V><<<g, 128, 0, ctx.stream>>>(d_desc, sh);
-    else if (coll == MT_COLL_LBGK)
-        k_brick_step_batch<27, S, MT_COLL_LBGK, V><<<g, 128, 0, ctx.stream>>>(d_desc, sh);
-    else
-        k_brick_step_batch<27, S, MT_COLL_CUMULANT, V><<<g, 128, 0, ctx.stream>>>(d_desc, sh);
     MT_LAUNCHED(ctx);
     return MT_OK;
 }

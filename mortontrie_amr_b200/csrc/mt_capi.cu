@@ -1310,6 +1310,8 @@ int mt_case_set_brick_forms(mt_ctx *h, int32_t id, const int32_t *form)
         if (c->fgraph[p]) cudaGraphExecDestroy(c->fgraph[p]);
         c->fgraph[p] = nullptr;
     }
+    for (Batch *b : ctx.batches)
+        if (b && std::find(b->ids.begin(), b->ids.end(), id) != b->ids.end()) batch_drop(*b);
     return MT_OK;
 }
 

@@ -120,31 +120,6 @@ struct Level {
     int64_t ndraw = 0;
 };
 
-// one case level in a batched brick pass
-struct BrickSlot {
-    const int32_t *list = nullptr, *nbr = nullptr;  // blist, bnbr
-    const unsigned long long *mask = nullptr;
-    const uint8_t *cls = nullptr, *flag = nullptr;
-    const void *fcol = nullptr;  // current post-collision buffer
-    void *f = nullptr, *fnext = nullptr, *rho = nullptr, *u = nullptr;
-    long long *acc = nullptr;  // direct-forcing accumulator: band macros in the pass (finest level), else null
-    Relax tau;
-    uint32_t n = 0;
-    int32_t textbook = 0, fall = 0, macros = 0;
-};
-constexpr int kMaxBatchSlots = 128;
-// a member level with at least this many bricks fills the GPU by itself: it
-// runs its own brick pass (same kernel as alone) beside the batched one
-constexpr int64_t kBatchOwnBricks = 8192;
-// a batched brick pass: slots and the prefix offsets of their bricks
-struct BrickBatch {
-    int32_t nslots = 0;
-    int32_t pad = 0;
-    int64_t total = 0;
-    int64_t off[kMaxBatchSlots + 1] = {};
-    BrickSlot slot[kMaxBatchSlots];
-};
-
 struct Case {
     mt_case_desc d{};
     bool dense = false;
@@ -216,9 +191,7 @@ struct Case {
     // second stream of the fused schedule: the IB cells' treat + collision
     // overlaps the finest level's fused pass (disjoint cells)
     int macros_now = 0;  // set while recording a level's last substep of the coarse step
-    int pull_mode = 0;   // PH_PULL_COLLIDE: 0 every cell, 1 the IB cells only (a batch runs the bricks)
     bool skip_ib = false; // PH_STREAM leaves the IB cells to treat() (amr_lbm_kernel)
-    bool no_side = false; // IB on the calling stream (batch recording)
     int in_batch = 0;     // batches holding the case
     bool f_stale = false; // fused passes left class-1 brick cells' streamed f unstored (amr_sync_f)
     cudaStream_t side = nullptr;
@@ -231,23 +204,20 @@ struct Case {
     std::vector<Branch> branch;
 };
 
-// Cases stepped together (mt_batch_*): one batched brick pass per level,
-// substep and model family over all of them, their other phases on parallel
-// graph branches.  Level 0 of every member swaps buffers once per coarse
+// Cases stepped together (mt_batch_*): every member's step is a parallel branch
+// of one captured graph.  Level 0 of every member swaps buffers once per coarse
 // step, so two captured graphs alternate (par).
+constexpr size_t kBatchStreams = 32;  // members beyond share a branch
 struct Batch {
     std::vector<int32_t> ids;
     // [0], [1]: one coarse step from level-0 parity 0 / 1; [2]: two coarse
     // steps (back to the same parity, valid from either)
     cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
     int64_t graph_launches[3] = {0, 0, 0};
-    BrickBatch *ddesc[3] = {nullptr, nullptr, nullptr};
-    std::vector<BrickBatch> hdesc[3];  // host copies (kept alive for the asynchronous upload)
     int par = 0;
     std::vector<cudaStream_t> pool;
     std::vector<cudaEvent_t> ev_join;
     cudaEvent_t ev_fork = nullptr;
-    cudaStream_t free_stream = nullptr;  // the stream the batch last ran on
 };
 
 struct HostStage;
@@ -328,8 +298,6 @@ template <class S> struct AmrOps {
     // infoPrint's diagnostics per level into d_out [(max_level + 1) * 4]
     // (mt_case_info)
     static int info(Ctx &ctx, Case &c, double *d_out);
-    // batched brick pass (descriptor in device memory, total bricks known on the host)
-    static int batch_pass(Ctx &ctx, int q, int coll, const BrickBatch *d_desc, int64_t total, const Shift &sh);
     // src's state carried onto dst's lattice (same Q, levels, storage)
     static int remap(Ctx &ctx, Case &dst, Case &src, int64_t *counts);
 };

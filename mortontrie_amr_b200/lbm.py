@@ -656,9 +656,9 @@ class LBM_Manager:
 
 
 class Batch:
-    """Independent multi-level cases stepped together (mt_batch_*): one
-    batched brick pass per level, substep and model family; each member ends
-    a step exactly where it would stepped alone under the fused schedule."""
+    """Independent multi-level cases stepped together (mt_batch_*), each member
+    a parallel branch of one captured step; each member ends a step exactly
+    where it would stepped alone under the fused schedule."""
 
     def __init__(self, ctx: Context, managers=()):
         self.ctx = ctx
