@@ -547,7 +547,7 @@ int amr_build(Ctx &ctx, Case &c)
         MT_LAUNCHED(ctx);
         int rc = select_indices(ctx, fl.n, IbLatf{fl.tag}, &fl.iblist, &fl.nib);
         if (rc) return rc;
-        // the force partials of 32-cell blocks and the finished-block counter
+        // the force partials of 32-cell blocks and the number of calls
         if (fl.nib) {
             const size_t bytes = 8 * (3 * (size_t)grid_for(fl.nib, 32) + 1);
             MT_CUDA(ctx, cudaMallocAsync(&c.ib_force, bytes, ctx.stream));
@@ -679,7 +679,7 @@ void amr_free(Case &c)
     }
     if (c.h_force) cudaFreeHost(c.h_force);
     c.h_force = nullptr;
-    void *ptrs[] = {c.dis_key, c.dis, c.ib_wall, c.ib_src, c.ib_dist, c.ib_force, c.force_acc, c.dev_err, c.bc_tmp, c.bc_all, c.bc_setb, c.bc_tmp_all,
+    void *ptrs[] = {c.dis_key, c.dis, c.ib_wall, c.ib_src, c.ib_factor, c.ib_force, c.force_acc, c.dev_err, c.bc_tmp, c.bc_all, c.bc_setb, c.bc_tmp_all,
                     c.mref, c.mdv, c.path, c.mforce, c.tstep, c.acc, c.mgrid};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -692,7 +692,7 @@ void amr_free(Case &c)
     c.dis = nullptr;
     c.ib_wall = nullptr;
     c.ib_src = nullptr;
-    c.ib_dist = nullptr;
+    c.ib_factor = nullptr;
     c.ib_force = nullptr;
     c.force_acc = nullptr;
     c.dev_err = nullptr;
@@ -818,7 +818,20 @@ static int record_step(Ctx &ctx, Case &c)
 {
     int rc = amr_lbm_kernel(ctx, c, 0);
     if (rc) return rc;
-    return amr_phase(ctx, c, PH_MACROS_ALL, 0);
+    if (!c.side) {
+        if ((rc = amr_phase(ctx, c, PH_IB_SUM, 0))) return rc;
+        return amr_phase(ctx, c, PH_MACROS_ALL, 0);
+    }
+    cudaStream_t main = ctx.stream;
+    MT_CUDA(ctx, cudaEventRecord(c.ev_fork, main));
+    MT_CUDA(ctx, cudaStreamWaitEvent(c.side, c.ev_fork, 0));
+    ctx.stream = c.side;
+    rc = amr_phase(ctx, c, PH_IB_SUM, 0);
+    ctx.stream = main;
+    if (!rc) rc = amr_phase(ctx, c, PH_MACROS_ALL, 0);
+    MT_CUDA(ctx, cudaEventRecord(c.ev_join, c.side));
+    MT_CUDA(ctx, cudaStreamWaitEvent(main, c.ev_join, 0));
+    return rc;
 }
 
 static int capture(Ctx &ctx, Case &c, int (*record)(Ctx &, Case &), cudaGraphExec_t *out, int64_t *launches)
@@ -920,6 +933,11 @@ static int record_fused_step(Ctx &ctx, Case &c)
     c.fused_now = true;
     int rc = fused_lbm_kernel(ctx, c, 0, true);
     c.fused_now = false;
+    if (c.side_open) {
+        MT_CUDA(ctx, cudaEventRecord(c.ev_join, c.side));
+        MT_CUDA(ctx, cudaStreamWaitEvent(ctx.stream, c.ev_join, 0));
+        c.side_open = false;
+    }
     if (rc) return rc;
     if (c.d.bc_mode == MT_BC_NEQ)
         if ((rc = amr_phase(ctx, c, PH_MACROS, 0))) return rc;

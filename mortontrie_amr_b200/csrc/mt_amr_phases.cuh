@@ -601,37 +601,43 @@ __global__ void k_bc_set_eq(const int32_t *list, int64_t nl, int64_t n, double r
 // The cell count is small (a sphere's skin), so the time is one thread's
 // chain of dependent loads.  What does not change is laid out once per case,
 // by cell of the IB list (IbTab, k_ib_tables): a mask of the wall links, each
-// link's wall distance and its source slot.  A cell then loads its tables in
-// one round and every population in a second, with addresses selected instead
-// of branches taken (a link without a source reads the cell's own opposite
-// population, which is its value).
+// link's interpolation factor and its source slot.  A cell then loads its tables
+// in one round and every population in a second, with addresses and operands
+// selected instead of branches taken (a link without a source reads the cell's
+// own opposite population, which is its value).  One warp per SM has only its
+// own instructions to issue, 6 cycles each: a wall link costs no division, a
+// sweep one (quot) instead of three and a root.
 // One launch, caches cold, D3Q19 FP16 / D3Q27 FP16 / D3Q27 FP64: 35 / 50 / 49 us
 // with the links' loads behind branches, 16 / 28 / 23 us from the neighbour
 // table and the distance rows in three rounds; two launches of 4 us each that
-// summed the force are gone (ib_force_sum).
+// summed the force are gone (ib_force_add).
 template <class C> struct IbTab {
-    const uint32_t *__restrict__ wall;  // [nib] bit k: link k meets the wall
-    const int32_t *__restrict__ src;    // [(Q - 1) nib] link k's source slot, -1 none
-    const C *__restrict__ dist;         // [(Q - 1) nib] link k's wall distance
+    const uint2 *__restrict__ wall;  // [nib] x bit k: link k meets the wall, y bit k: closer than half a link
+    const int32_t *__restrict__ src; // [(Q - 1) nib] link k's source slot, -1 none
+    // [(Q - 1) nib] of wall links the distance d (distance-weighted); or 2 d where
+    // closer than half a link, else 1 / (2 d) (Filippova-Haenel)
+    const C *__restrict__ factor;
     int64_t nib;
 };
 template <int Q, class C>
 __global__ void k_ib_tables(const int32_t *__restrict__ list, int64_t nl, int64_t n, const int32_t *__restrict__ disrow,
-                            const double *__restrict__ dis, const int32_t *__restrict__ nbr, uint32_t *wall,
-                            int32_t *src, C *dist)
+                            const double *__restrict__ dis, const int32_t *__restrict__ nbr, int fh, uint2 *wall,
+                            int32_t *src, C *factor)
 {
     const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nl) return;
     const int64_t i = list[j];
     const double *dr = dis + (int64_t)disrow[i] * (Q - 1);
-    uint32_t m = 0;
+    uint2 m = make_uint2(0, 0);
     for (int k = 1; k < Q; ++k) {
         const double v = dr[inv(k) - 1];
         const bool hit = v != -1.;
-        if (hit) m |= 1u << k;
+        const C d = (C)v;
+        if (hit) m.x |= 1u << k;
+        if (hit && d < (C)0.5) m.y |= 1u << k;
         // a wall link interpolates with the population arriving from the far side
         src[(int64_t)(k - 1) * nl + j] = nbr[(int64_t)((hit ? inv(k) : k) - 1) * n + i];
-        dist[(int64_t)(k - 1) * nl + j] = (C)v;
+        factor[(int64_t)(k - 1) * nl + j] = !fh ? d : d < (C)0.5 ? (C)2.0 * d : (C)1.0 / ((C)2.0 * d);
     }
     wall[j] = m;
 }
@@ -644,6 +650,21 @@ __device__ __forceinline__ float pm_fma(float a, float b, float c) { return __fm
 __device__ __forceinline__ double pm_mul(double a, double b) { return a * b; }
 __device__ __forceinline__ double pm_add(double a, double b) { return a + b; }
 __device__ __forceinline__ double pm_fma(double a, double b, double c) { return a * b + c; }
+// x / b from rb = 1 / b: one correction gives the rounded quotient (FP64: mt_lattice's
+// quot; FP32: all 2^23 mantissas of b with 100 x each, no difference)
+__device__ __forceinline__ float pm_quot(float x, float b, float rb)
+{
+    const float q = __fmul_rn(x, rb);
+    return __fmaf_rn(__fmaf_rn(-q, b, x), rb, q);
+}
+__device__ __forceinline__ double pm_quot(double x, double b, double rb) { return quot(x, b, rb); }
+template <class C> __device__ constexpr C pm_tiny() { return sizeof(C) == 8 ? (C)0x1p-100 : (C)0x1p-40f; }
+template <class C> __device__ constexpr C pm_huge() { return sizeof(C) == 8 ? (C)0x1p100 : (C)0x1p40f; }
+// the smallest s with sqrt(s) >= 1e-10
+template <class C> __device__ constexpr C pm_still()
+{
+    return sizeof(C) == 8 ? (C)0x1.79ca10c924223p-67 : (C)0x1.79ca1p-67f;
+}
 template <int Q, int FH, class S>
 __device__ __forceinline__ void ib_cell(int64_t i, int64_t j, const IbTab<typename Store<S>::C> &t,
                                         const S *__restrict__ fcol, typename Store<S>::C rho_b,
@@ -652,13 +673,14 @@ __device__ __forceinline__ void ib_cell(int64_t i, int64_t j, const IbTab<typena
 {
     using T = Store<S>;
     using C = typename T::C;
-    const uint32_t wall = __ldg(t.wall + j);
-    C dd[Q], own[Q], src[Q];
+    const uint2 masks = __ldg(t.wall + j);
+    const uint32_t wall = masks.x;
+    C fac[Q], own[Q], src[Q];
     int32_t si[Q];
 #pragma unroll
     for (int k = 1; k < Q; ++k) si[k] = __ldg(t.src + (int64_t)(k - 1) * t.nib + j);
 #pragma unroll
-    for (int k = 1; k < Q; ++k) dd[k] = __ldg(t.dist + (int64_t)(k - 1) * t.nib + j);
+    for (int k = 1; k < Q; ++k) fac[k] = __ldg(t.factor + (int64_t)(k - 1) * t.nib + j);
 #pragma unroll
     for (int k = 0; k < Q; ++k) own[k] = T::ld(fcol, at<Q>(k, i));
 #pragma unroll
@@ -675,19 +697,11 @@ __device__ __forceinline__ void ib_cell(int64_t i, int64_t j, const IbTab<typena
         if ((wall >> k) & 1) {
             const C finc = full_sh<S>(sh, own[inv(k)], inv(k));
             const C fstr = from;
-            C fnew;
-            if (FH) {
-                if (dd[k] < (C)0.5) {
-                    const C d2 = (C)2.0 * dd[k];
-                    fnew = pm_fma((C)1.0 - d2, finc, pm_mul(d2, fstr));
-                } else {
-                    const C feqw = pm_mul((C)w19z(inv(k)), rho_b);
-                    const C inv2d = (C)1.0 / ((C)2.0 * dd[k]);
-                    fnew = pm_fma(inv2d, fstr, pm_mul((C)1.0 - inv2d, feqw));
-                }
-            } else {
-                fnew = pm_fma((C)1.0 - dd[k], finc, pm_mul(dd[k], fstr));
-            }
+            // FH: near (1 - 2 d) finc + 2 d fstr, else 1 / (2 d) fstr + (1 - 1 / (2 d)) feq
+            const C a = fac[k], b = (C)1.0 - a;
+            const bool near = !FH || ((masks.y >> k) & 1);
+            const C fnew = near ? pm_fma(b, finc, pm_mul(a, fstr))
+                                : pm_fma(a, fstr, pm_mul(b, pm_mul((C)w19z(inv(k)), rho_b)));
             g[k] = fnew;
             const C mt = pm_add(finc, fnew);
             fx = pm_add(fx, -mt * ex(k));
@@ -717,11 +731,18 @@ __device__ __forceinline__ void ib_cell(int64_t i, int64_t j, const IbTab<typena
             if (ez(k)) uz = pm_add(uz, ez(k) > 0 ? g[k] : -g[k]);
         }
         if (r <= (C)0.) continue;
-        ux = ux / r;
-        uy = uy / r;
-        uz = uz / r;
-        const C um = sqrt(ux * ux + uy * uy + uz * uz);
-        if (um < (C)1e-10) continue;
+        if (r > pm_tiny<C>() && r < pm_huge<C>()) {
+            const C rr = (C)1.0 / r;
+            ux = pm_quot(ux, r, rr);
+            uy = pm_quot(uy, r, rr);
+            uz = pm_quot(uz, r, rr);
+        } else {
+            ux = ux / r;
+            uy = uy / r;
+            uz = uz / r;
+        }
+        // |u| < 1e-10, the root taken on the bound
+        if (ux * ux + uy * uy + uz * uz < pm_still<C>()) continue;
         const C hr = pm_mul((C)-0.5, r);
         const C mx = pm_mul(hr, ux), my = pm_mul(hr, uy), mz = pm_mul(hr, uz);
         C adj = 0;
@@ -747,50 +768,49 @@ __device__ __forceinline__ void ib_cell(int64_t i, int64_t j, const IbTab<typena
     }
 }
 
-// The force of one treat() call (LBM_Manager::accumIBForce) into the
-// accumulator, by the kernel that computed it: one warp per block adds its 32
-// cells in a fixed tree, and the last block to finish adds the blocks'
-// partials in block order (strided over the warp, then the same tree).
-// part: [3 * gridDim.x] partials, then the finished-block counter.
+// The force of treat() (LBM_Manager::accumIBForce): the kernel that computed it
+// adds each 32-cell block's sum (a fixed tree) to the block's own partial, and
+// once per coarse step k_ib_force_sum adds the partials in block order
+// (strided over the warp, then the same tree) to the accumulator.  (Finished
+// in every launch by the last block, behind a fence and a counter, the sum
+// was 2 us at the end of the substep's longest kernel.)
+// part: [3 * blocks] partials, then the number of calls.
 constexpr int kIbBlock = 32;
-__device__ __forceinline__ void ib_force_sum(double fx, double fy, double fz, double *part, double *acc)
+__device__ __forceinline__ void ib_force_tree(double &x, double &y, double &z)
 {
-    const unsigned all = 0xffffffffu;
-    const int lane = threadIdx.x;
-    unsigned *done = (unsigned *)(part + 3 * (int64_t)gridDim.x);
-    auto tree = [&](double &x, double &y, double &z) {
 #pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            x += __shfl_down_sync(all, x, o);
-            y += __shfl_down_sync(all, y, o);
-            z += __shfl_down_sync(all, z, o);
-        }
-    };
-    tree(fx, fy, fz);
-    unsigned last = 0;
-    if (lane == 0) {
-        double *p = part + 3 * (int64_t)blockIdx.x;
-        p[0] = fx;
-        p[1] = fy;
-        p[2] = fz;
-        __threadfence();
-        last = atomicAdd(done, 1u) == gridDim.x - 1;
+    for (int o = 16; o; o >>= 1) {
+        x += __shfl_down_sync(0xffffffffu, x, o);
+        y += __shfl_down_sync(0xffffffffu, y, o);
+        z += __shfl_down_sync(0xffffffffu, z, o);
     }
-    if (!__shfl_sync(all, last, 0)) return;
-    __threadfence();
+}
+__device__ __forceinline__ void ib_force_add(double fx, double fy, double fz, double *part)
+{
+    ib_force_tree(fx, fy, fz);
+    if (threadIdx.x != 0) return;
+    double *p = part + 3 * (int64_t)blockIdx.x;
+    p[0] += fx;
+    p[1] += fy;
+    p[2] += fz;
+    if (blockIdx.x == 0) part[3 * (int64_t)gridDim.x] += 1.0;
+}
+static __global__ void __launch_bounds__(32) k_ib_force_sum(double *part, int64_t nb, double *acc)
+{
     double x = 0., y = 0., z = 0.;
-    for (int64_t b = lane; b < gridDim.x; b += 32) {
-        x += __ldcg(part + 3 * b);
-        y += __ldcg(part + 3 * b + 1);
-        z += __ldcg(part + 3 * b + 2);
+    for (int64_t b = threadIdx.x; b < nb; b += 32) {
+        x += part[3 * b];
+        y += part[3 * b + 1];
+        z += part[3 * b + 2];
+        part[3 * b] = part[3 * b + 1] = part[3 * b + 2] = 0.;
     }
-    tree(x, y, z);
-    if (lane == 0) {
+    ib_force_tree(x, y, z);
+    if (threadIdx.x == 0) {
         acc[0] += x;
         acc[1] += y;
         acc[2] += z;
-        acc[3] += 1.0;
-        *done = 0u;
+        acc[3] += part[3 * nb];
+        part[3 * nb] = 0.;
     }
 }
 
@@ -799,7 +819,7 @@ __global__ void __launch_bounds__(kIbBlock) k_ib_treat(const int32_t *__restrict
                                                        const IbTab<typename Store<S>::C> t,
                                                        const S *__restrict__ fcol,
                                                        const typename Store<S>::C *__restrict__ rho, S *__restrict__ f,
-                                                       double *part, double *force, const Shift sh)
+                                                       double *part, const Shift sh)
 {
     using T = Store<S>;
     using C = typename T::C;
@@ -812,7 +832,7 @@ __global__ void __launch_bounds__(kIbBlock) k_ib_treat(const int32_t *__restrict
 #pragma unroll
         for (int k = 0; k < Q; ++k) T::st(f, at<Q>(k, i), stored_sh<S>(sh, g[k], k));
     }
-    ib_force_sum((double)fx, (double)fy, (double)fz, part, force);
+    ib_force_add((double)fx, (double)fy, (double)fz, part);
 }
 
 // ---- fused schedule ---------------------------------------------------------
@@ -1316,7 +1336,7 @@ template <int Q, int FH, class S, int COLL>
 __global__ void __launch_bounds__(kIbBlock) k_ib_collide(
     const int32_t *__restrict__ list, int64_t nl, int64_t n, const IbTab<typename Store<S>::C> t,
     const S *__restrict__ fcol, S *__restrict__ f,
-    S *__restrict__ fnext, const Relax tau, double *part, double *force, typename Store<S>::C *__restrict__ rho,
+    S *__restrict__ fnext, const Relax tau, double *part, typename Store<S>::C *__restrict__ rho,
     typename Store<S>::C *__restrict__ u, int macros, const Shift sh)
 {
     using T = Store<S>;
@@ -1348,7 +1368,7 @@ __global__ void __launch_bounds__(kIbBlock) k_ib_collide(
             u[2 * n + i] = z;
         }
     }
-    ib_force_sum((double)fx, (double)fy, (double)fz, part, force);
+    ib_force_add((double)fx, (double)fy, (double)fz, part);
 }
 
 // ---- direct-forcing immersed boundary (Lagrangian markers) --------------------
@@ -1662,7 +1682,7 @@ template <class S> struct AmrTyped {
     static C *u(Level &lv) { return (C *)lv.u; }
     static IbTab<C> ib(const Case &c)
     {
-        return IbTab<C>{c.ib_wall, c.ib_src, (const C *)c.ib_dist, c.lv[c.d.max_level].nib};
+        return IbTab<C>{c.ib_wall, c.ib_src, (const C *)c.ib_factor, c.lv[c.d.max_level].nib};
     }
 };
 
@@ -1787,6 +1807,15 @@ int band_collide(Ctx &ctx, Case &c, int l, void *out)
     if (!lv.nband) return MT_OK;
     k_band_collide<Q, S><<<grid_for(lv.nband, 64), 64, 0, ctx.stream>>>(lv.band, lv.nband, lv.n, c.d.tau[l],
                                                                          A::f(lv), c.acc, (S *)out, c.shift[l]);
+    MT_LAUNCHED(ctx);
+    return MT_OK;
+}
+
+// treat()'s forces since the last call into the accumulator
+inline bool has_ib_cells(const Case &c) { return c.d.ib_method != MT_IB_DF && c.lv[c.d.max_level].nib; }
+inline int ib_force_sum(Ctx &ctx, Case &c, cudaStream_t s)
+{
+    k_ib_force_sum<<<1, 32, 0, s>>>(c.ib_force, grid_for(c.lv[c.d.max_level].nib, kIbBlock), c.force_acc);
     MT_LAUNCHED(ctx);
     return MT_OK;
 }
@@ -2049,10 +2078,10 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
             const Shift &fsh = c.shift[c.d.max_level];
             if (c.d.ib_method == MT_IB_FH)
                 k_ib_treat<Q, 1, S><<<gi, kIbBlock, 0, s>>>(fl.iblist, fl.nib, A::ib(c), A::fcol(fl), A::rho(fl),
-                                                            A::f(fl), c.ib_force, c.force_acc, fsh);
+                                                            A::f(fl), c.ib_force, fsh);
             else
                 k_ib_treat<Q, 0, S><<<gi, kIbBlock, 0, s>>>(fl.iblist, fl.nib, A::ib(c), A::fcol(fl), A::rho(fl),
-                                                            A::f(fl), c.ib_force, c.force_acc, fsh);
+                                                            A::f(fl), c.ib_force, fsh);
         }
         MT_LAUNCHED(ctx);
         return MT_OK;
@@ -2175,7 +2204,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
                     constexpr int FH = decltype(fh)::value, COLL = decltype(coll)::value;
                     k_ib_collide<Q, FH, S, COLL><<<grid_for(lv.nib, kIbBlock), kIbBlock, 0, is>>>(
                         lv.iblist, lv.nib, n, A::ib(c), A::fcol(lv), A::f(lv), (S *)lv.fcol_alt, tau,
-                        c.ib_force, c.force_acc, A::rho(lv), A::u(lv), mac, c.shift[l]);
+                        c.ib_force, A::rho(lv), A::u(lv), mac, c.shift[l]);
                 };
                 using I0 = std::integral_constant<int, 0>;
                 using I1 = std::integral_constant<int, 1>;
@@ -2225,8 +2254,16 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
             MT_CUDA(ctx, cudaEventRecord(c.ev_join, is));
             MT_CUDA(ctx, cudaStreamWaitEvent(s, c.ev_join, 0));
         }
+        // the coarse step's last: its force, beside the coarser levels' work
+        // (record_fused_step waits for it)
+        if (ib_level && lv.nib && mac) {
+            if (int rc = ib_force_sum(ctx, c, is)) return rc;
+            c.side_open = is != s;
+        }
         return MT_OK;
     }
+    case PH_IB_SUM:
+        return has_ib_cells(c) ? ib_force_sum(ctx, c, s) : MT_OK;
     }
     return set_err(ctx, MT_ERR_ARG, "unknown phase");
 }
@@ -2243,15 +2280,16 @@ int AmrOps<S>::ib_tables(Ctx &ctx, Case &c)
     using C = typename Store<S>::C;
     Level &fl = c.lv[c.d.max_level];
     const int64_t nib = fl.nib, links = c.d.q - 1;
-    MT_CUDA(ctx, cudaMallocAsync(&c.ib_wall, sizeof(uint32_t) * nib, ctx.stream));
+    const int fh = c.d.ib_method == MT_IB_FH;
+    MT_CUDA(ctx, cudaMallocAsync(&c.ib_wall, sizeof(uint2) * nib, ctx.stream));
     MT_CUDA(ctx, cudaMallocAsync(&c.ib_src, sizeof(int32_t) * links * nib, ctx.stream));
-    MT_CUDA(ctx, cudaMallocAsync(&c.ib_dist, sizeof(C) * links * nib, ctx.stream));
+    MT_CUDA(ctx, cudaMallocAsync(&c.ib_factor, sizeof(C) * links * nib, ctx.stream));
     if (c.d.q == 19)
         k_ib_tables<19, C><<<grid_for(nib, 128), 128, 0, ctx.stream>>>(fl.iblist, nib, fl.n, fl.disrow, c.dis, fl.nbr,
-                                                                      c.ib_wall, c.ib_src, (C *)c.ib_dist);
+                                                                      fh, c.ib_wall, c.ib_src, (C *)c.ib_factor);
     else
         k_ib_tables<27, C><<<grid_for(nib, 128), 128, 0, ctx.stream>>>(fl.iblist, nib, fl.n, fl.disrow, c.dis, fl.nbr,
-                                                                      c.ib_wall, c.ib_src, (C *)c.ib_dist);
+                                                                      fh, c.ib_wall, c.ib_src, (C *)c.ib_factor);
     MT_LAUNCHED(ctx);
     return MT_OK;
 }

@@ -801,7 +801,8 @@ int mt_ib_treat(mt_ctx *h, int32_t id)
     Case *c;
     int rc = get_case(h, id, &c);
     if (rc) return rc;
-    return phase_call(h, id, PH_IB, c->d.max_level);
+    if ((rc = phase_call(h, id, PH_IB, c->d.max_level))) return rc;
+    return amr_phase(h->c, *c, PH_IB_SUM, 0);
 }
 
 int mt_lbm_kernel(mt_ctx *h, int32_t id, int32_t level)
@@ -814,7 +815,8 @@ int mt_lbm_kernel(mt_ctx *h, int32_t id, int32_t level)
     if (level < 0 || level > c->d.max_level) return set_err(ctx, MT_ERR_ARG, "bad level");
     if ((rc = amr_sync_f(ctx, *c))) return rc;
     c->primed = false;
-    return amr_lbm_kernel(ctx, *c, level);
+    if ((rc = amr_lbm_kernel(ctx, *c, level))) return rc;
+    return amr_phase(ctx, *c, PH_IB_SUM, 0);
 }
 
 int mt_step(mt_ctx *h, int32_t id, int32_t n)

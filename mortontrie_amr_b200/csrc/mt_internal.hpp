@@ -24,7 +24,8 @@ constexpr int kNumSets = 6;  // lat_f, F2C, C2F, ghost C2F, ghost F2C, solid
 // then the fused schedule's own passes
 enum { PH_MACROS = 0, PH_COLLIDE, PH_STREAM, PH_EXPLOSION, PH_COALESCENCE, PH_BC, PH_IB, PH_BC_INOUT,
        PH_BC_FACE0 = 8, PH_F2C_COLLIDE = 16, PH_PULL_COLLIDE, PH_PRIME, PH_COAL_COLLIDE,
-       PH_SYNC_F, PH_DF, PH_BAND_GRID, PH_FACE_EQ0 = 24, PH_BC_HH = 32, PH_EXPLOSION_B, PH_EXPL_SAVE, PH_MACROS_ALL };
+       PH_SYNC_F, PH_DF, PH_BAND_GRID, PH_FACE_EQ0 = 24, PH_BC_HH = 32, PH_EXPLOSION_B, PH_EXPL_SAVE, PH_MACROS_ALL,
+       PH_IB_SUM };
 
 // per-cell tag bits (which reference index sets the cell belongs to)
 enum : uint32_t {
@@ -137,10 +138,10 @@ struct Case {
     std::vector<uint8_t> h_reg[MT_MAX_LEVELS + 1];
     int64_t reg_lo[MT_MAX_LEVELS + 1][3] = {};
     int64_t reg_n[MT_MAX_LEVELS + 1][3] = {};
-    uint32_t *ib_wall = nullptr;  // treat()'s tables by IB cell (IbTab)
+    uint2 *ib_wall = nullptr;  // treat()'s tables by IB cell (IbTab)
     int32_t *ib_src = nullptr;
-    void *ib_dist = nullptr;
-    double *ib_force = nullptr;  // force partials of treat() (ib_force_sum)
+    void *ib_factor = nullptr;
+    double *ib_force = nullptr;  // force partials of treat() (ib_force_add)
     double *force_acc = nullptr; // [4] fx, fy, fz, treat count
     double *h_force = nullptr;   // [6] page-locked: force_acc copy [4], then the guard flags (int) (mt_case_force_async)
     int *dev_err = nullptr;
@@ -191,6 +192,7 @@ struct Case {
     // second stream of the fused schedule: the IB cells' treat + collision
     // overlaps the finest level's fused pass (disjoint cells)
     int macros_now = 0;  // set while recording a level's last substep of the coarse step
+    bool side_open = false; // work on the side stream that the step's end has to wait for
     bool skip_ib = false; // PH_STREAM leaves the IB cells to treat() (amr_lbm_kernel)
     int in_batch = 0;     // batches holding the case
     bool f_stale = false; // fused passes left class-1 brick cells' streamed f unstored (amr_sync_f)
