@@ -707,17 +707,7 @@ void amr_free(Case &c)
         if (c.fgraph[p]) cudaGraphExecDestroy(c.fgraph[p]);
         c.fgraph[p] = nullptr;
     }
-    if (c.side) cudaStreamDestroy(c.side);
-    if (c.ev_fork) cudaEventDestroy(c.ev_fork);
-    if (c.ev_join) cudaEventDestroy(c.ev_join);
     c.side = nullptr;
-    c.ev_fork = c.ev_join = nullptr;
-    for (Case::Branch &b : c.branch) {
-        if (b.s) cudaStreamDestroy(b.s);
-        if (b.fork) cudaEventDestroy(b.fork);
-        if (b.join) cudaEventDestroy(b.join);
-    }
-    c.branch.clear();
 }
 
 // ----------------------------------------------------------------------------
@@ -748,13 +738,33 @@ int amr_init_equilibrium(Ctx &ctx, Case &c, double rho0, const double *u0)
 // computes the macros it needs from the same populations the reference's
 // calculateMacros(level) reads just before collide(level), so the separate
 // macros pass of each substep is folded into it.
-// the second stream of the IB cells' work
+int make_branch(Ctx &ctx, Branch &b)
+{
+    if (!b.s) MT_CUDA(ctx, cudaStreamCreateWithFlags(&b.s, cudaStreamNonBlocking));
+    if (!b.fork) MT_CUDA(ctx, cudaEventCreateWithFlags(&b.fork, cudaEventDisableTiming));
+    if (!b.join) MT_CUDA(ctx, cudaEventCreateWithFlags(&b.join, cudaEventDisableTiming));
+    return MT_OK;
+}
+void free_branch(Branch &b)
+{
+    if (b.s) cudaStreamDestroy(b.s);
+    if (b.fork) cudaEventDestroy(b.fork);
+    if (b.join) cudaEventDestroy(b.join);
+    b = Branch{};
+}
+void free_side(Side &side)
+{
+    for (Branch &b : side.level) free_branch(b);
+    side.level.clear();
+    free_branch(side);
+}
 static int make_side(Ctx &ctx, Case &c)
 {
-    if (c.side) return MT_OK;
-    MT_CUDA(ctx, cudaStreamCreateWithFlags(&c.side, cudaStreamNonBlocking));
-    MT_CUDA(ctx, cudaEventCreateWithFlags(&c.ev_fork, cudaEventDisableTiming));
-    MT_CUDA(ctx, cudaEventCreateWithFlags(&c.ev_join, cudaEventDisableTiming));
+    if (!c.side) c.side = &ctx.side;
+    if (int rc = make_branch(ctx, *c.side)) return rc;
+    if ((int)c.side->level.size() < c.d.max_level) c.side->level.resize(c.d.max_level);
+    for (int l = 0; l < c.d.max_level; ++l)
+        if (int rc = make_branch(ctx, c.side->level[l])) return rc;
     return MT_OK;
 }
 // (the brick stream can leave cells out)
@@ -786,17 +796,17 @@ int amr_lbm_kernel(Ctx &ctx, Case &c, int l)
             // side
             if ((rc = make_side(ctx, c))) return rc;
             cudaStream_t main = ctx.stream;
-            MT_CUDA(ctx, cudaEventRecord(c.ev_fork, main));
-            MT_CUDA(ctx, cudaStreamWaitEvent(c.side, c.ev_fork, 0));
-            ctx.stream = c.side;
+            MT_CUDA(ctx, cudaEventRecord(c.side->fork, main));
+            MT_CUDA(ctx, cudaStreamWaitEvent(c.side->s, c.side->fork, 0));
+            ctx.stream = c.side->s;
             rc = amr_phase(ctx, c, PH_IB, L);
             ctx.stream = main;
             c.skip_ib = true;
             if (!rc) rc = amr_phase(ctx, c, PH_STREAM, l);
             c.skip_ib = false;
             // (joined on an error too: the streams may be capturing)
-            MT_CUDA(ctx, cudaEventRecord(c.ev_join, c.side));
-            MT_CUDA(ctx, cudaStreamWaitEvent(main, c.ev_join, 0));
+            MT_CUDA(ctx, cudaEventRecord(c.side->join, c.side->s));
+            MT_CUDA(ctx, cudaStreamWaitEvent(main, c.side->join, 0));
             if (rc) return rc;
         } else {
             RUN(PH_STREAM, l);
@@ -823,14 +833,14 @@ static int record_step(Ctx &ctx, Case &c)
         return amr_phase(ctx, c, PH_MACROS_ALL, 0);
     }
     cudaStream_t main = ctx.stream;
-    MT_CUDA(ctx, cudaEventRecord(c.ev_fork, main));
-    MT_CUDA(ctx, cudaStreamWaitEvent(c.side, c.ev_fork, 0));
-    ctx.stream = c.side;
+    MT_CUDA(ctx, cudaEventRecord(c.side->fork, main));
+    MT_CUDA(ctx, cudaStreamWaitEvent(c.side->s, c.side->fork, 0));
+    ctx.stream = c.side->s;
     rc = amr_phase(ctx, c, PH_IB_SUM, 0);
     ctx.stream = main;
     if (!rc) rc = amr_phase(ctx, c, PH_MACROS_ALL, 0);
-    MT_CUDA(ctx, cudaEventRecord(c.ev_join, c.side));
-    MT_CUDA(ctx, cudaStreamWaitEvent(main, c.ev_join, 0));
+    MT_CUDA(ctx, cudaEventRecord(c.side->join, c.side->s));
+    MT_CUDA(ctx, cudaStreamWaitEvent(main, c.side->join, 0));
     return rc;
 }
 
@@ -897,10 +907,10 @@ static int fused_lbm_kernel(Ctx &ctx, Case &c, int l, bool last_parent)
             if (l == 0 && c.d.bc_mode == MT_BC_NEQ) RUN(PH_BC, 0);
             return MT_OK;
         };
-        if (l < L && l < (int)c.branch.size() && !c.lv[l].chained) {
+        if (l < L && !c.lv[l].chained) {
             // the finer levels read this level's fcol, which its own work leaves
             // alone (its explosion writes none of their sources): side by side
-            Case::Branch &b = c.branch[l];
+            Branch &b = c.side->level[l];
             cudaStream_t main = ctx.stream;
             MT_CUDA(ctx, cudaEventRecord(b.fork, main));
             MT_CUDA(ctx, cudaStreamWaitEvent(b.s, b.fork, 0));
@@ -934,8 +944,8 @@ static int record_fused_step(Ctx &ctx, Case &c)
     int rc = fused_lbm_kernel(ctx, c, 0, true);
     c.fused_now = false;
     if (c.side_open) {
-        MT_CUDA(ctx, cudaEventRecord(c.ev_join, c.side));
-        MT_CUDA(ctx, cudaStreamWaitEvent(ctx.stream, c.ev_join, 0));
+        MT_CUDA(ctx, cudaEventRecord(c.side->join, c.side->s));
+        MT_CUDA(ctx, cudaStreamWaitEvent(ctx.stream, c.side->join, 0));
         c.side_open = false;
     }
     if (rc) return rc;
@@ -982,15 +992,8 @@ static int build_bricks(Ctx &ctx, Case &c, int l)
 static int prime_fused(Ctx &ctx, Case &c)
 {
     const int L = c.d.max_level;
-    if (L > 0 && (c.lv[L].nib || c.lv[L].nband))
+    if (L > 0)
         if (int rc = make_side(ctx, c)) return rc;
-    while ((int)c.branch.size() < L) {
-        c.branch.emplace_back();
-        Case::Branch &b = c.branch.back();
-        MT_CUDA(ctx, cudaStreamCreateWithFlags(&b.s, cudaStreamNonBlocking));
-        MT_CUDA(ctx, cudaEventCreateWithFlags(&b.fork, cudaEventDisableTiming));
-        MT_CUDA(ctx, cudaEventCreateWithFlags(&b.join, cudaEventDisableTiming));
-    }
     for (int l = 0; l <= L; ++l) {
         Level &lv = c.lv[l];
         if (!lv.n) continue;
@@ -1126,16 +1129,21 @@ int record_batch_step(Ctx &ctx, Batch &B, const std::vector<Case *> &cases)
     cudaStream_t main = ctx.stream;
     const size_t P = std::min(B.pool.size(), cases.size());
     MT_CUDA(ctx, cudaEventRecord(B.ev_fork, main));
-    for (size_t p = 0; p < P; ++p) MT_CUDA(ctx, cudaStreamWaitEvent(B.pool[p], B.ev_fork, 0));
+    for (size_t p = 0; p < P; ++p) MT_CUDA(ctx, cudaStreamWaitEvent(B.pool[p].s, B.ev_fork, 0));
     int rc = MT_OK;
     for (size_t i = 0; i < cases.size() && !rc; ++i) {
-        ctx.stream = B.pool[i % P];
-        rc = record_fused_step(ctx, *cases[i]);
+        Case &c = *cases[i];
+        Side *own = c.side;
+        ctx.stream = B.pool[i % P].s;
+        c.side = B.side[i % P].get();
+        if (c.d.max_level > 0) rc = make_side(ctx, c);
+        if (!rc) rc = record_fused_step(ctx, c);
+        c.side = own;
     }
     ctx.stream = main;
     for (size_t p = 0; p < P; ++p) {
-        MT_CUDA(ctx, cudaEventRecord(B.ev_join[p], B.pool[p]));
-        MT_CUDA(ctx, cudaStreamWaitEvent(main, B.ev_join[p], 0));
+        MT_CUDA(ctx, cudaEventRecord(B.pool[p].join, B.pool[p].s));
+        MT_CUDA(ctx, cudaStreamWaitEvent(main, B.pool[p].join, 0));
     }
     return rc;
 }
@@ -1154,11 +1162,11 @@ void batch_drop(Batch &b)
 void batch_free(Batch &b)
 {
     batch_drop(b);
-    for (cudaStream_t s : b.pool) cudaStreamDestroy(s);
-    for (cudaEvent_t e : b.ev_join) cudaEventDestroy(e);
+    for (Branch &x : b.pool) free_branch(x);
+    for (auto &x : b.side) free_side(*x);
     if (b.ev_fork) cudaEventDestroy(b.ev_fork);
     b.pool.clear();
-    b.ev_join.clear();
+    b.side.clear();
     b.ev_fork = nullptr;
 }
 
@@ -1172,13 +1180,11 @@ int batch_step(Ctx &ctx, Batch &B, const std::vector<Case *> &cases, int n)
         if (!c->primed && (rc = prime_fused(ctx, *c))) return rc;
     }
     const size_t P = std::min<size_t>(kBatchStreams, cases.size());
-    while (B.ev_join.size() < P) {
-        cudaStream_t st;
-        cudaEvent_t e;
-        MT_CUDA(ctx, cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-        B.pool.push_back(st);
-        MT_CUDA(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-        B.ev_join.push_back(e);
+    while (B.pool.size() < P) {
+        Branch b;
+        if ((rc = make_branch(ctx, b))) return rc;
+        B.pool.push_back(b);
+        B.side.emplace_back(new Side);
     }
     if (!B.ev_fork) MT_CUDA(ctx, cudaEventCreateWithFlags(&B.ev_fork, cudaEventDisableTiming));
     // capture graph g (0/1: one step from that parity, 2: two steps)

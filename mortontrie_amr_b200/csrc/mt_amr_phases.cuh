@@ -2155,14 +2155,14 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
             // the body force beside the band's collision (6 us of a substep's chain)
             const bool sum = lv.nband && c.nm, fork = sum && c.side;
             if (fork) {
-                MT_CUDA(ctx, cudaEventRecord(c.ev_fork, s));
-                MT_CUDA(ctx, cudaStreamWaitEvent(c.side, c.ev_fork, 0));
+                MT_CUDA(ctx, cudaEventRecord(c.side->fork, s));
+                MT_CUDA(ctx, cudaStreamWaitEvent(c.side->s, c.side->fork, 0));
             }
-            int rc = sum ? df_sum(ctx, c, fork ? c.side : s) : MT_OK;
+            int rc = sum ? df_sum(ctx, c, fork ? c.side->s : s) : MT_OK;
             if (!rc) rc = band_collide<S, Q>(ctx, c, l, lv.fcol_alt);
             if (fork) {
-                MT_CUDA(ctx, cudaEventRecord(c.ev_join, c.side));
-                MT_CUDA(ctx, cudaStreamWaitEvent(s, c.ev_join, 0));
+                MT_CUDA(ctx, cudaEventRecord(c.side->join, c.side->s));
+                MT_CUDA(ctx, cudaStreamWaitEvent(s, c.side->join, 0));
             }
             return rc;
         }
@@ -2201,9 +2201,9 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         const int fall = (l == 0 && c.d.bc_mode == MT_BC_NEQ) ? 1 : 0;
         cudaStream_t is = s;
         if (ib_level && lv.nib && c.side) {
-            MT_CUDA(ctx, cudaEventRecord(c.ev_fork, s));
-            MT_CUDA(ctx, cudaStreamWaitEvent(c.side, c.ev_fork, 0));
-            is = c.side;
+            MT_CUDA(ctx, cudaEventRecord(c.side->fork, s));
+            MT_CUDA(ctx, cudaStreamWaitEvent(c.side->s, c.side->fork, 0));
+            is = c.side->s;
         }
         if (ib_level) {
             if (!lv.nib) {
@@ -2265,8 +2265,8 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
             }
         }
         if (is != s) {
-            MT_CUDA(ctx, cudaEventRecord(c.ev_join, is));
-            MT_CUDA(ctx, cudaStreamWaitEvent(s, c.ev_join, 0));
+            MT_CUDA(ctx, cudaEventRecord(c.side->join, is));
+            MT_CUDA(ctx, cudaStreamWaitEvent(s, c.side->join, 0));
         }
         // the coarse step's last: its force, beside the coarser levels' work
         // (record_fused_step waits for it)

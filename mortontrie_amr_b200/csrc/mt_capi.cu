@@ -156,6 +156,7 @@ int mt_destroy(mt_ctx *h)
     for (cudaEvent_t e : h->c.markers)
         if (e) cudaEventDestroy(e);
     copy_free(h->c);
+    free_side(h->c.side);
     if (h->c.own_stream) cudaStreamDestroy(h->c.stream);
     delete h;
     return MT_OK;
