@@ -109,7 +109,8 @@ __global__ void k_macros_all(const __grid_constant__ MacroLevels<S> m)
 // (Collision_Cumulant.cpp:22-159).  Shared by every kernel that collides one
 // cell; the reduced storages run the arithmetic of the packed pairs
 // (mt_pack2.cuh), so a cell's result does not depend on the kernel.
-template <int Q, class S, int COLL, class I>
+// (a kernel that shares a cell among several threads stores directions K0 to K1)
+template <int Q, class S, int COLL, int K0 = 0, int K1 = Q, class I>
 __device__ __forceinline__ void macros_collide_store(typename Store<S>::C *d, typename Store<S>::C &r,
                                                      typename Store<S>::C &x, typename Store<S>::C &y,
                                                      typename Store<S>::C &z, const Relax tau, S *out, I i,
@@ -124,18 +125,18 @@ __device__ __forceinline__ void macros_collide_store(typename Store<S>::C *d, ty
             p2::cumulant<float, false>(d, r, x, y, z, om, sh);
         }
 #pragma unroll
-        for (int k = 0; k < Q; ++k) T::st(out, at<Q>(k, i), d[k]);
+        for (int k = K0; k < K1; ++k) T::st(out, at<Q>(k, i), d[k]);
     } else {
         macros_g<Q, double>(d, r, x, y, z);
         if constexpr (COLL == MT_COLL_LBGK) {
             lbgk_ref<Q>(d, r, x, y, z, tau.tau, tau.inv);
 #pragma unroll
-            for (int k = 0; k < Q; ++k) out[at<Q>(k, i)] = d[k];
+            for (int k = K0; k < K1; ++k) out[at<Q>(k, i)] = d[k];
         } else if constexpr (Q == 27) {
             double o[27];
             cumulant_collide(d, r, x, y, z, tau.inv, o);
 #pragma unroll
-            for (int k = 0; k < 27; ++k) out[at<Q>(k, i)] = o[k];
+            for (int k = K0; k < K1; ++k) out[at<Q>(k, i)] = o[k];
         }
     }
 }
@@ -241,9 +242,25 @@ template <class S> struct Eight {
 // cprev (MT_ITIME_EXTRAP, second substep): the sources' parent values at the
 // parent's previous step, [Q][ns]; the explosion then starts from
 // 1.5 fcol - 0.5 prev, the parent state extrapolated to the half step.
-constexpr int kExplParts = 3;
+// (4 blocks per SM: left to itself the compiler takes 48 registers and has a
+// few of the loads in flight.)
+constexpr int kParts = 3;
+// f(0), f(1) or f(2), the argument a constant
+template <class F> __device__ __forceinline__ void by_part(int part, F &&f)
+{
+    if (part == 0)
+        f(std::integral_constant<int, 0>{});
+    else if (part == 1)
+        f(std::integral_constant<int, 1>{});
+    else
+        f(std::integral_constant<int, 2>{});
+}
+// the directions of part P of kParts
+template <int Q, int P> struct PartOf {
+    static constexpr int K0 = P * Q / kParts, K1 = (P + 1) * Q / kParts;
+};
 template <int Q, class S>
-__global__ void __launch_bounds__(32 * kExplParts) k_explosion(
+__global__ void __launch_bounds__(32 * kParts, 4) k_explosion(
     const int32_t *__restrict__ src, const int32_t *__restrict__ child, const uint8_t *__restrict__ mask, int64_t ns,
     const S *__restrict__ cfcol, S *__restrict__ ffcol, double scale, S *__restrict__ ffcol2, int64_t nf2c,
     const Shift csh, const Shift fsh, const S *__restrict__ cprev = nullptr)
@@ -266,8 +283,8 @@ __global__ void __launch_bounds__(32 * kExplParts) k_explosion(
     C r, x, y, z;
     macros_g<Q, C>(d, r, x, y, z);
     const int nw = ffcol2 && j >= nf2c ? 2 : 1;
-    auto write = [&](auto p) {
-        constexpr int K0 = decltype(p)::value * Q / kExplParts, K1 = (decltype(p)::value + 1) * Q / kExplParts;
+    by_part(part, [&](auto p) {
+        constexpr int K0 = PartOf<Q, decltype(p)::value>::K0, K1 = PartOf<Q, decltype(p)::value>::K1;
 #pragma unroll
         for (int k = K0; k < K1; ++k) {
             const C fe = feq_heluo_g<Q, C>(k, r, x, y, z);
@@ -288,13 +305,7 @@ __global__ void __launch_bounds__(32 * kExplParts) k_explosion(
                     }
             }
         }
-    };
-    if (part == 0)
-        write(std::integral_constant<int, 0>{});
-    else if (part == 1)
-        write(std::integral_constant<int, 1>{});
-    else
-        write(std::integral_constant<int, 2>{});
+    });
 }
 
 // the explosion sources' parent values into prev [Q][ns] (MT_ITIME_EXTRAP)
@@ -309,53 +320,79 @@ __global__ void k_expl_save(const int32_t *__restrict__ src, int64_t ns, const S
     for (int k = 0; k < Q; ++k) prev[k * ns + j] = cfcol[at<Q>(k, i)];
 }
 
-// the mean of a coarse cell's eight children (first child's slot ch), summed in
-// the reference's child order
-template <int Q, class S>
+// The mean of a coarse cell's eight children at directions K0 to K1
+// (LBM_Manager.cpp:1141-1152).
+template <int Q, int K0, int K1, class S>
 __device__ __forceinline__ void children_mean(const S *__restrict__ ff, int64_t ch, const Shift &fsh,
                                               typename Store<S>::C *a)
 {
     using C = typename Store<S>::C;
-    // as many directions' loads in flight as about 128 registers hold
-    constexpr int G = sizeof(S) == 2 ? Q : (sizeof(S) == 4 ? 14 : 7);
+    Eight<S> e[K1 - K0];
 #pragma unroll
-    for (int k0 = 0; k0 < Q; k0 += G) {
-        Eight<S> e[G];
+    for (int k = K0; k < K1; ++k) e[k - K0].load(ff + at<Q>(k, ch));
 #pragma unroll
-        for (int h = 0; h < G; ++h)
-            if (k0 + h < Q) e[h].load(ff + at<Q>(k0 + h, ch));
+    for (int k = K0; k < K1; ++k) {
+        C s = 0;
 #pragma unroll
-        for (int h = 0; h < G; ++h) {
-            if (k0 + h >= Q) continue;
-            C s = 0;
-#pragma unroll
-            for (int m = 0; m < 8; ++m) s += full_sh<S>(fsh, e[h].get(m), k0 + h);
-            a[k0 + h] = s / (C)8.0;
-        }
+        for (int m = 0; m < 8; ++m) s += full_sh<S>(fsh, e[k - K0].get(m), k);
+        a[k] = s / (C)8.0;
     }
 }
 
-// AMR_transDDF_coalescence (LBM_Manager.cpp:1131-1169)
+// AMR_transDDF_coalescence (LBM_Manager.cpp:1131-1169) of 32 cells by kParts
+// warps: each takes the means of a third of the directions, all need the
+// moments of the whole, so the means go through shared memory, and each stores
+// its third of the rescaled populations (val: as stored, for a collision).
+// A level's few thousand cells leave most of the GPU idle and one thread's
+// instructions are the time, as in the explosion.  Per coarse step, against a
+// thread with all of a cell: 4-level D3Q27 FP32 sphere 425 -> 393 us, FP32 cavity
+// over three levels 116 -> 107 us, 3-level D3Q27 FP64 sphere 153 -> 144 us.
 template <int Q, class S>
-__global__ void __launch_bounds__(64) k_coalescence(const int32_t *__restrict__ list,
-                                                    const int32_t *__restrict__ child, int64_t nl, S *__restrict__ cf,
-                                                    const S *__restrict__ ff, double scale, const Shift csh,
-                                                    const Shift fsh)
+__device__ __forceinline__ void coalesce(typename Store<S>::C (*mean)[32], typename Store<S>::C (*val)[32], int part,
+                                         int lane, bool on, int64_t i, int64_t ch, S *__restrict__ cf,
+                                         const S *__restrict__ ff, double scale, const Shift &csh, const Shift &fsh)
 {
     using T = Store<S>;
     using C = typename T::C;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= nl) return;
-    const int64_t i = list[j];
+    by_part(part, [&](auto p) {
+        constexpr int K0 = PartOf<Q, decltype(p)::value>::K0, K1 = PartOf<Q, decltype(p)::value>::K1;
+        C a[Q];
+        children_mean<Q, K0, K1>(ff, ch, fsh, a);
+#pragma unroll
+        for (int k = K0; k < K1; ++k) mean[k][lane] = a[k];
+    });
+    __syncthreads();
     C a[Q];
-    children_mean<Q, S>(ff, child[j], fsh, a);
+#pragma unroll
+    for (int k = 0; k < Q; ++k) a[k] = mean[k][lane];
     C r, x, y, z;
     macros_g<Q, C>(a, r, x, y, z);
+    by_part(part, [&](auto p) {
+        constexpr int K0 = PartOf<Q, decltype(p)::value>::K0, K1 = PartOf<Q, decltype(p)::value>::K1;
 #pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        const C fe = feq_heluo_g<Q, C>(k, r, x, y, z);
-        T::st(cf, at<Q>(k, i), stored_sh<S>(csh, fe + (C)scale * (a[k] - fe), k));
-    }
+        for (int k = K0; k < K1; ++k) {
+            const C fe = feq_heluo_g<Q, C>(k, r, x, y, z);
+            const C st = stored_sh<S>(csh, fe + (C)scale * (a[k] - fe), k);
+            if (on) T::st(cf, at<Q>(k, i), st);
+            if (val) {
+                S sv;
+                T::st(&sv, 0, st);
+                val[k][lane] = T::cv(sv);
+            }
+        }
+    });
+}
+template <int Q, class S>
+__global__ void __launch_bounds__(32 * kParts, 4) k_coalescence(const int32_t *__restrict__ list,
+                                                             const int32_t *__restrict__ child, int64_t nl,
+                                                             S *__restrict__ cf, const S *__restrict__ ff, double scale,
+                                                             const Shift csh, const Shift fsh)
+{
+    using C = typename Store<S>::C;
+    __shared__ C mean[Q][32];
+    const int lane = threadIdx.x & 31;
+    const int64_t j0 = blockIdx.x * (int64_t)32 + lane, j = j0 < nl ? j0 : nl - 1;
+    coalesce<Q, S>(mean, nullptr, threadIdx.x >> 5, lane, j0 < nl, list[j], child[j], cf, ff, scale, csh, fsh);
 }
 
 // Fused schedule: coalescence onto the F2C cells, then (the cells' f being
@@ -364,36 +401,42 @@ __global__ void __launch_bounds__(64) k_coalescence(const int32_t *__restrict__ 
 // macros of that f are written when `macros` is set (the level's last
 // substep of the coarse step: calculateMacros of every level follows).
 template <int Q, class S, int COLL>
-__global__ void __launch_bounds__(64) k_coal_collide(const int32_t *__restrict__ list, const int32_t *__restrict__ child, int64_t nl,
-                               int64_t nc, S *__restrict__ cf, const S *__restrict__ ff, double scale,
-                               const Relax tau, S *__restrict__ cfnext, typename Store<S>::C *__restrict__ rho,
-                               typename Store<S>::C *__restrict__ u, int macros, const Shift csh,
-                               const Shift fsh)
+__global__ void __launch_bounds__(32 * kParts, 4) k_coal_collide(
+    const int32_t *__restrict__ list, const int32_t *__restrict__ child, int64_t nl, int64_t nc, S *__restrict__ cf,
+    const S *__restrict__ ff, double scale, const Relax tau, S *__restrict__ cfnext,
+    typename Store<S>::C *__restrict__ rho, typename Store<S>::C *__restrict__ u, int macros, const Shift csh,
+    const Shift fsh)
 {
-    using T = Store<S>;
-    using C = typename T::C;
-    const int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= nl) return;
+    using C = typename Store<S>::C;
+    __shared__ C mean[Q][32], val[Q][32];
+    const int lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const int64_t j0 = blockIdx.x * (int64_t)32 + lane, j = j0 < nl ? j0 : nl - 1;
+    const bool on = j0 < nl;
     const int64_t i = list[j];
-    C a[Q];
-    children_mean<Q, S>(ff, child[j], fsh, a);
-    C r, x, y, z;
-    macros_g<Q, C>(a, r, x, y, z);
+    coalesce<Q, S>(mean, val, part, lane, on, i, child[j], cf, ff, scale, csh, fsh);
+    __syncthreads();
+    if (!on) return;
+    auto collide = [&](auto k0, auto k1) {
+        C a[Q], r, x, y, z;
 #pragma unroll
-    for (int k = 0; k < Q; ++k) {
-        const C fe = feq_heluo_g<Q, C>(k, r, x, y, z);
-        const C st = stored_sh<S>(csh, fe + (C)scale * (a[k] - fe), k);
-        T::st(cf, at<Q>(k, i), st);
-        S sv;
-        T::st(&sv, 0, st);
-        a[k] = T::cv(sv);
-    }
-    macros_collide_store<Q, S, COLL>(a, r, x, y, z, tau, cfnext, i, csh);
-    if (macros) {
-        rho[i] = r;
-        u[i] = x;
-        u[nc + i] = y;
-        u[2 * nc + i] = z;
+        for (int k = 0; k < Q; ++k) a[k] = val[k][lane];
+        macros_collide_store<Q, S, COLL, decltype(k0)::value, decltype(k1)::value>(a, r, x, y, z, tau, cfnext, i, csh);
+        if (macros && part == 0) {
+            rho[i] = r;
+            u[i] = x;
+            u[nc + i] = y;
+            u[2 * nc + i] = z;
+        }
+    };
+    if constexpr (COLL == MT_COLL_LBGK) {
+        by_part(part, [&](auto p) {
+            using D = PartOf<Q, decltype(p)::value>;
+            collide(std::integral_constant<int, D::K0>{}, std::integral_constant<int, D::K1>{});
+        });
+    } else if (part == 0) {
+        // a third of its outputs costs as much as all of them (done by each part,
+        // the FP64 sphere's step was 160 us)
+        collide(std::integral_constant<int, 0>{}, std::integral_constant<int, Q>{});
     }
 }
 
@@ -1970,7 +2013,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         const bool once = c.fused_now && lv.bricks && c.itime == MT_ITIME_HOLD && !lv.chained;
         if (once && phase == PH_EXPLOSION_B) return MT_OK;
         if (ex && !lv.expl_prev) return set_err(ctx, MT_ERR_STATE, "extrapolated explosion without saved sources");
-        k_explosion<Q, S><<<grid_for(lv.nexpl, 32), 32 * kExplParts, 0, s>>>(lv.expl_src, lv.expl_child, lv.expl_mask, lv.nexpl,
+        k_explosion<Q, S><<<grid_for(lv.nexpl, 32), 32 * kParts, 0, s>>>(lv.expl_src, lv.expl_child, lv.expl_mask, lv.nexpl,
                                                                A::fcol(cl), A::fcol(lv), scale, (S *)lv.fcol_alt,
                                                                once ? 0 : lv.nexpl_f2c, c.shift[l - 1], c.shift[l],
                                                                ex ? (const S *)lv.expl_prev : nullptr);
@@ -1995,7 +2038,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         if (l >= c.d.max_level || !lv.nlist[1]) return MT_OK;
         Level &fl = c.lv[l + 1];
         const double scale = f2c_scale(c, l);
-        k_coalescence<Q, S><<<grid_for(lv.nlist[1], 64), 64, 0, s>>>(lv.list[1], lv.coal_child, lv.nlist[1], A::f(lv),
+        k_coalescence<Q, S><<<grid_for(lv.nlist[1], 32), 32 * kParts, 0, s>>>(lv.list[1], lv.coal_child, lv.nlist[1], A::f(lv),
                                                                       A::f(fl), scale, c.shift[l], c.shift[l + 1]);
         MT_LAUNCHED(ctx);
         return MT_OK;
@@ -2121,12 +2164,12 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         Level &fl = c.lv[l + 1];
         const double scale = f2c_scale(c, l);
         if (c.d.collision == MT_COLL_LBGK) {
-            k_coal_collide<Q, S, MT_COLL_LBGK><<<grid_for(lv.nlist[1], 64), 64, 0, s>>>(
+            k_coal_collide<Q, S, MT_COLL_LBGK><<<grid_for(lv.nlist[1], 32), 32 * kParts, 0, s>>>(
                 lv.list[1], lv.coal_child, lv.nlist[1], n, A::f(lv), A::f(fl), scale, c.d.tau[l],
                 (S *)lv.fcol_alt, A::rho(lv), A::u(lv), c.macros_now, c.shift[l], c.shift[l + 1]);
         } else {
             if constexpr (Q == 27)
-                k_coal_collide<Q, S, MT_COLL_CUMULANT><<<grid_for(lv.nlist[1], 64), 64, 0, s>>>(
+                k_coal_collide<Q, S, MT_COLL_CUMULANT><<<grid_for(lv.nlist[1], 32), 32 * kParts, 0, s>>>(
                     lv.list[1], lv.coal_child, lv.nlist[1], n, A::f(lv), A::f(fl), scale, c.d.tau[l],
                     (S *)lv.fcol_alt, A::rho(lv), A::u(lv), c.macros_now, c.shift[l], c.shift[l + 1]);
         }

@@ -194,14 +194,14 @@ cudaError_t staged(Ctx &ctx, HostStage &st, char *dst, const char *src, size_t b
 int copy_out(Ctx &ctx, void *host, const void *dev, size_t bytes)
 {
     if (!bytes) return MT_OK;
-    cudaPointerAttributes attr{};
-    bool pageable = true;
-    if (cudaPointerGetAttributes(&attr, host) == cudaSuccess)
-        pageable = attr.type == cudaMemoryTypeUnregistered;
-    else
+    auto pageable = [&] {
+        cudaPointerAttributes attr{};
+        if (cudaPointerGetAttributes(&attr, host) == cudaSuccess) return attr.type == cudaMemoryTypeUnregistered;
         cudaGetLastError();
+        return true;
+    };
     const int nthreads = (int)std::min<unsigned>(8, std::thread::hardware_concurrency() / 2);
-    if (pageable && bytes >= kStagedFrom && nthreads >= 2) {
+    if (bytes >= kStagedFrom && nthreads >= 2 && pageable()) {
         HostStage *st = nullptr;
         {
             std::lock_guard<std::mutex> lk(ctx.stage_mutex);
