@@ -302,16 +302,16 @@ int mt_case_status(mt_ctx *ctx, int32_t case_id);
  * kernel at 128, 256, 512 and 1024 threads per block on the case's own state
  * (writing only the scratch array, so the state is unchanged) and keeps the
  * fastest; ms_per_candidate (nullable) receives the mean launch time of each
- * candidate the kernel is built for (the paired 16-bit LBGK kernel: 128 and
- * 256 only; the other slots are left unwritten). */
+ * candidate the kernel is built for (FP64 and the paired LBGK kernel: 128 and
+ * 256, the paired cumulant kernel: 128; the other slots are left unwritten). */
 int mt_case_tune(mt_ctx *ctx, int32_t case_id, int32_t *best_block, float *ms_per_candidate);
 /* Forms of the multi-level fused brick pass (no reference counterpart):
  * for FP32 / FP16 / BF16 storage
  * 0: a lane gathers, collides and stores two x-adjacent cells together (packed
- *    FP32 arithmetic) at 6 resident 128-thread blocks per SM (16-bit D3Q19: 7),
+ *    FP32 arithmetic) at 7 resident 128-thread blocks per SM (FP32 D3Q27: 6),
  *    the default;
- * 2, 3: form 0 at other numbers of resident blocks (16 bits 7 and 8, D3Q19 8
- *    and 9; FP32 5 and 7);
+ * 2, 3: form 0 at other numbers of resident blocks (16 bits 6 and 8, D3Q19 8
+ *    and 9; FP32 5 and 7, D3Q19 6 and 5);
  * 1: one cell per lane step;
  * for FP64
  * 0: one cell per lane step, the default;
