@@ -114,12 +114,13 @@ __global__ void __launch_bounds__(sizeof(S) == 8 ? 256 : 1024, sizeof(S) == 8 ? 
 // x0 + 2 or x0 - 1, x0): two aligned loads.  Stores and conversions are per
 // pair.  LBGK collides the two cells one after the other at 64 registers (the
 // packed form holds both cells' FP32 values: 80 or more); the cumulant, whose
-// arithmetic bounds the one-cell form, collides both in packed FP32 at 80
-// registers, 6 blocks of 128 threads.  128^3 per step: FP16 88.7 us cell by cell,
-// 66.4 us so (256^3: 550 -> 409 us, 4.4 TB/s); FP32 79.7 -> 79.5 us (5.7 TB/s),
-// 64^3 13.7 -> 11.9 us.  What bounds the FP16 cumulant is the FP32 pipe.
+// arithmetic bounds the one-cell form, collides both in packed FP32 in blocks of
+// 128 threads, 7 per SM at 16 bits (72 registers, 8 B of spills: 128^3 57.4 us
+// with 6, 55.6 with 7, 256^3 411 / 401 us), 6 at FP32 (76.6 / 77.9 us).  Cell by
+// cell: FP16 128^3 88.7 us, 256^3 550 us, FP32 79.7 us, 64^3 13.7 us.  What bounds
+// the FP16 cumulant is the FP32 pipe.
 template <int Q, class S, int COLL, int CONV>
-__global__ void __launch_bounds__(COLL == MT_COLL_LBGK ? 256 : 128, COLL == MT_COLL_LBGK ? (Q == 19 ? 4 : 3) : 6)
+__global__ void __launch_bounds__(COLL == MT_COLL_LBGK ? 256 : 128, COLL == MT_COLL_LBGK ? (Q == 19 ? 4 : 3) : (sizeof(S) == 2 ? 7 : 6))
     k_dense_pair(const S *__restrict__ A, S *__restrict__ B, uint32_t N, DenseGeom g, const Relax tau, const Shift sh)
 {
     using CP = CellPair<S>;
