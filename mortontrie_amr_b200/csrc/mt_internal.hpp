@@ -203,8 +203,6 @@ struct Case {
     int par0 = 0;
     cudaGraphExec_t fgraph[2] = {nullptr, nullptr};
     int64_t fgraph_launches[2] = {0, 0};
-    // second stream of the fused schedule: the IB cells' treat + collision
-    // overlaps the finest level's fused pass (disjoint cells)
     int macros_now = 0;  // set while recording a level's last substep of the coarse step
     bool side_open = false; // work on the side stream that the step's end has to wait for
     bool skip_ib = false; // PH_STREAM leaves the IB cells to treat() (amr_lbm_kernel)
