@@ -1305,6 +1305,7 @@ int amr_get(Ctx &ctx, Case &c, int level, double *h_f, double *h_fcol)
         if (!rc) rc = copy_out(ctx, dst, d, nb);
     }
     cudaFreeAsync(d, ctx.stream);
+    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
     return rc;
 }
 
@@ -1345,6 +1346,7 @@ int amr_macros(Ctx &ctx, Case &c, int level, double *h_rho, double *h_u)
     if (!rc && h_rho) rc = copy_out(ctx, h_rho, d, sizeof(double) * lv.ncell);
     if (!rc && h_u) rc = copy_out(ctx, h_u, d + lv.ncell, sizeof(double) * 3 * lv.ncell);
     cudaFreeAsync(d, ctx.stream);
+    MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
     return rc;
 }
 

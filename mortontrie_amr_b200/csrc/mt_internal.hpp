@@ -281,7 +281,7 @@ int batch_step(Ctx &ctx, Batch &b, const std::vector<Case *> &cases, int n);
 void batch_drop(Batch &b);
 void batch_free(Batch &b);
 
-// `bytes` of device memory into host memory; synchronises the stream
+// `bytes` of device memory into host memory, landed once the stream is synchronised
 int copy_out(Ctx &ctx, void *host, const void *dev, size_t bytes);
 void copy_free(Ctx &ctx);
 
