@@ -49,6 +49,47 @@ __device__ __forceinline__ uint32_t dense_nbr(const DenseGeom &g, uint32_t i, in
 
 enum { DM_FUSED = 0, DM_COLLIDE = 1, DM_PULL = 2 };
 
+// FP32 LBGK on deviations, opposite directions paired: for q and inv(q) the
+// equilibrium shares its even part w (drho + rho (4.5 eu^2 - 1.5 u^2)) and
+// flips the sign of its odd part 3 w rho eu (D3Q19/27 list q, q+1 as a pair
+// for every odd q).
+// The compiler pairs multiplications and additions into FMAs as it does for
+// these expressions; written otherwise they round otherwise.
+template <int Q>
+__device__ __forceinline__ void lbgk_dev_pairs(float *s, float omega)
+{
+    float dr = 0.f, jx = 0.f, jy = 0.f, jz = 0.f;
+#pragma unroll
+    for (int k = 0; k < Q; ++k) {
+        dr += s[k];
+        if (ex(k)) jx += ex(k) > 0 ? s[k] : -s[k];
+        if (ey(k)) jy += ey(k) > 0 ? s[k] : -s[k];
+        if (ez(k)) jz += ez(k) > 0 ? s[k] : -s[k];
+    }
+    const float rho = 1.f + dr;
+    const float ir = __frcp_rn(rho);
+    const float ux = jx * ir, uy = jy * ir, uz = jz * ir;
+    const float uu = 1.5f * (ux * ux + uy * uy + uz * uz);
+    {
+        const float d0 = (float)w<Q>(0) * (dr - rho * uu);
+        s[0] = fmaf(omega, d0 - s[0], s[0]);
+    }
+#pragma unroll
+    for (int k = 1; k < Q; k += 2) {
+        float eu = 0.f;
+        if (ex(k)) eu += ex(k) > 0 ? ux : -ux;
+        if (ey(k)) eu += ey(k) > 0 ? uy : -uy;
+        if (ez(k)) eu += ez(k) > 0 ? uz : -uz;
+        const float wk = (float)w<Q>(k);
+        const float wr = wk * rho;
+        const float even = fmaf(wr, fmaf(4.5f * eu, eu, -uu), wk * dr);
+        const float odd = 3.f * wr * eu;
+        const float dp = even + odd, dm = even - odd;
+        s[k] = fmaf(omega, dp - s[k], s[k]);
+        s[k + 1] = fmaf(omega, dm - s[k + 1], s[k + 1]);
+    }
+}
+
 // One cell per thread.  The three dilated coordinate parts of each axis at
 // offsets -1, 0, +1 are formed once; the pull source of direction k is then
 // px | py | pz of the right offsets (CONV 0: from x + e_k as the reference
@@ -98,7 +139,7 @@ __global__ void __launch_bounds__(sizeof(S) == 8 ? 256 : 1024, sizeof(S) == 8 ? 
         } else {
             [[maybe_unused]] float r, x, y, z;
             if constexpr (COLL == MT_COLL_LBGK)
-                p2::lbgk_dev<Q, float>(f, tau.om);
+                lbgk_dev_pairs<Q>(f, tau.om);
             else
                 p2::cumulant<float, true>(f, r, x, y, z, tau.om, sh);
         }
@@ -115,9 +156,9 @@ __global__ void __launch_bounds__(sizeof(S) == 8 ? 256 : 1024, sizeof(S) == 8 ? 
 // pair.  LBGK collides the two cells one after the other at 64 registers (the
 // packed form holds both cells' FP32 values: 80 or more); the cumulant, whose
 // arithmetic bounds the one-cell form, collides both in packed FP32 in blocks of
-// 128 threads, 7 per SM at 16 bits (72 registers, 8 B of spills: 128^3 57.4 us
-// with 6, 55.6 with 7, 256^3 411 / 401 us), 6 at FP32 (76.6 / 77.9 us).  Cell by
-// cell: FP16 128^3 88.7 us, 256^3 550 us, FP32 79.7 us, 64^3 13.7 us.  What bounds
+// 128 threads, 7 per SM at 16 bits (72 registers: 256^3 416 us), 6 at FP32 (128^3
+// 77.3 us, 64^3 11.5 us).  Cell by cell: FP16 256^3 550 us, FP32 128^3 79.7 us,
+// 64^3 13.7 us.  What bounds
 // the FP16 cumulant is the FP32 pipe.
 template <int Q, class S, int COLL, int CONV>
 __global__ void __launch_bounds__(COLL == MT_COLL_LBGK ? 256 : 128, COLL == MT_COLL_LBGK ? (Q == 19 ? 4 : 3) : (sizeof(S) == 2 ? 7 : 6))
@@ -165,8 +206,8 @@ __global__ void __launch_bounds__(COLL == MT_COLL_LBGK ? 256 : 128, COLL == MT_C
             fa[k] = f2.x;
             fb[k] = f2.y;
         }
-        p2::lbgk_dev<Q, float>(fa, om);
-        p2::lbgk_dev<Q, float>(fb, om);
+        lbgk_dev_pairs<Q>(fa, om);
+        lbgk_dev_pairs<Q>(fb, om);
 #pragma unroll
         for (int k = 0; k < Q; ++k) CP::st(B + (size_t)k * N + i0, CP::word(make_float2(fa[k], fb[k])));
     } else {

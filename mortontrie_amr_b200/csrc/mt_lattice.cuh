@@ -57,9 +57,6 @@ struct Shift {
     float dw[27];
     float u[3];
     double d[27];
-    // D3Q27: sums of s over the nine x lines (line = y + 3 z position) -- all
-    // three, the ends' difference, the ends' sum -- rounded to FP32
-    float k0[9], d1[9], s1[9];
 };
 inline Shift make_shift(int q, const double *us)
 {
@@ -74,13 +71,6 @@ inline Shift make_shift(int q, const double *us)
         s.dw[k] = (float)dw;
     }
     for (int a = 0; a < 3; ++a) s.u[a] = (float)us[a];
-    double line[9][3] = {};
-    for (int k = 0; k < q; ++k) line[(ey(k) + 1) + 3 * (ez(k) + 1)][ex(k) + 1] = s.d[k];
-    for (int j = 0; j < 9; ++j) {
-        s.k0[j] = (float)(line[j][0] + line[j][1] + line[j][2]);
-        s.d1[j] = (float)(line[j][2] - line[j][0]);
-        s.s1[j] = (float)(line[j][2] + line[j][0]);
-    }
     return s;
 }
 

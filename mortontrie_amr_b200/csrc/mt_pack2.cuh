@@ -67,6 +67,8 @@ __device__ __forceinline__ float safe_inv(float r)
 {
     return 1.f / ((r > -1e-6f && r < 1e-6f) ? ((r < 0.f) ? -1e-6f : 1e-6f) : r);
 }
+__device__ __forceinline__ float inv(float r) { return 1.f / r; }
+__device__ __forceinline__ float2 inv(float2 r) { return make_float2(1.f / r.x, 1.f / r.y); }
 __device__ __forceinline__ float2 safe_inv(float2 r) { return make_float2(safe_inv(r.x), safe_inv(r.y)); }
 
 // e_k . u with the lattice constants folded
@@ -131,44 +133,6 @@ __device__ __forceinline__ void lbgk(V *s, V &rho, V &ux, V &uy, V &uz, float om
     }
 }
 
-// The same about u_s = 0 from the deviations alone (shift_k = w_k): the weights
-// sum to 1 and their first moment is zero, so rho - 1 and the momentum are sums
-// of deviations, without cancellation, and the equilibrium's even part
-// w (rho - 1 + rho (4.5 (e.u)^2 - 1.5 u^2)) and odd part 3 w rho e.u serve
-// both directions of a pair.
-template <int Q, class V>
-__device__ __forceinline__ void lbgk_dev(V *s, float om)
-{
-    V rd = s[0], jx = bc<V>(0.f), jy = bc<V>(0.f), jz = bc<V>(0.f);
-#pragma unroll
-    for (int k = 1; k < Q; k += 2) {
-        const V df = sub(s[k], s[k + 1]);
-        rd = add(rd, add(s[k], s[k + 1]));
-        if (ex(k) > 0) jx = add(jx, df);
-        if (ex(k) < 0) jx = sub(jx, df);
-        if (ey(k) > 0) jy = add(jy, df);
-        if (ey(k) < 0) jy = sub(jy, df);
-        if (ez(k) > 0) jz = add(jz, df);
-        if (ez(k) < 0) jz = sub(jz, df);
-    }
-    const V rho = add(rd, bc<V>(1.f));
-    const V is = safe_inv(rho);
-    const V ux = mul(jx, is), uy = mul(jy, is), uz = mul(jz, is);
-    const V nuu = mul(bc<V>(-1.5f), fma(ux, ux, fma(uy, uy, mul(uz, uz))));
-    auto relax = [&](V &f, V feq) { f = fma(bc<V>(om), sub(feq, f), f); };
-    relax(s[0], mul(bc<V>((float)w<Q>(0)), fma(rho, nuu, rd)));
-#pragma unroll
-    for (int k = 1; k < Q; k += 2) {
-        const float wk = (float)w<Q>(k);
-        const V e = eu<Q, V>(k, ux, uy, uz);
-        const V wr = mul(bc<V>(wk), rho);
-        const V even = fma(wr, fma(mul(bc<V>(4.5f), e), e, nuu), mul(bc<V>(wk), rd));
-        const V odd = mul(mul(bc<V>(3.f), wr), e);
-        relax(s[k], add(even, odd));
-        relax(s[k + 1], sub(even, odd));
-    }
-}
-
 // backward chimera step of one line (chim_back's FP32 polynomials); Z0, Z1,
 // Z2 mark inputs known to be zero
 template <bool Z0, bool Z1, bool Z2, class V>
@@ -191,21 +155,37 @@ __device__ __forceinline__ void chim_back(V a0, V a1, V a2, V v, V tv, V v2, V &
 
 // Macros and D3Q27 cumulant collision in place on stored deviations s_k = f_k -
 // shift_k (Collision_Cumulant.cpp:320-652): forward central moments by x, y, z
-// chimera passes, rho and the momentum from the x pass's line sums,
-// second-order cumulants relaxed with omega1 and bulk rate 1, higher cumulants
+// chimera passes, second-order cumulants relaxed with omega1 and bulk rate 1, higher cumulants
 // zero, backward transform (the moments the relaxation zeroes left out).  The
 // (2,1,0), (1,0,2), (0,2,1) moments keep their forward values
 // (Collision_Cumulant.cpp:451-454).
-// DEV: the line sums are taken on the deviations, which give rho - 1 and the
-// momentum (less u_s) without cancellation, and the shift's own line sums are
-// added once; else on the full populations.
+// DEV (the dense cube, u_s = 0): rho - 1 and the momentum are sums of the
+// deviations in direction order, without cancellation; else they come from the
+// x pass's line sums of the full populations.  (Line sums of the deviations, the
+// shift's own added once, would serve both and spare 60 packed additions of
+// about 600 a pair, 256^3 FP16 416 -> 405 us, but round otherwise: results of
+// this path do not change with the kernel that computes them.)
 template <class V, bool DEV>
 __device__ __forceinline__ void cumulant(V *s, V &rho, V &ux, V &uy, V &uz, float om1, const Shift &sh)
 {
     V g[27];
+    if constexpr (DEV) {
+        V r = s[0], jx = bc<V>(0.f), jy = bc<V>(0.f), jz = bc<V>(0.f);
 #pragma unroll
-    for (int i = 0; i < 27; ++i)
-        g[(ex(i) + 1) + 3 * (ey(i) + 1) + 9 * (ez(i) + 1)] = DEV ? s[i] : addc(s[i], sh.v[i]);
+        for (int i = 1; i < 27; ++i) {
+            r = add(r, s[i]);
+            if (ex(i)) jx = ex(i) > 0 ? add(jx, s[i]) : sub(jx, s[i]);
+            if (ey(i)) jy = ey(i) > 0 ? add(jy, s[i]) : sub(jy, s[i]);
+            if (ez(i)) jz = ez(i) > 0 ? add(jz, s[i]) : sub(jz, s[i]);
+        }
+        rho = add(r, bc<V>(1.f));
+        const V is = inv(rho);
+        ux = mul(jx, is);
+        uy = mul(jy, is);
+        uz = mul(jz, is);
+    }
+#pragma unroll
+    for (int i = 0; i < 27; ++i) g[(ex(i) + 1) + 3 * (ey(i) + 1) + 9 * (ez(i) + 1)] = addc(s[i], sh.v[i]);
     {
         // x lines: slot 0 line total k0, slot 1 difference d1, slot 2 sum of the ends s1
         V r, jx, jy, jz;
@@ -213,10 +193,11 @@ __device__ __forceinline__ void cumulant(V *s, V &rho, V &ux, V &uy, V &uz, floa
         for (int line = 0; line < 9; ++line) {
             const int b = 3 * line, ly = line % 3, lz = line / 3;
             const V fm = g[b], f0 = g[b + 1], fp = g[b + 2];
-            const V s1 = add(fp, fm), d1 = sub(fp, fm), k0 = add(s1, f0);
-            g[b] = DEV ? addc(k0, sh.k0[line]) : k0;
-            g[b + 1] = DEV ? addc(d1, sh.d1[line]) : d1;
-            g[b + 2] = DEV ? addc(s1, sh.s1[line]) : s1;
+            const V s1 = add(fp, fm), d1 = sub(fp, fm), k0 = DEV ? add(add(fm, f0), fp) : add(s1, f0);
+            g[b] = k0;
+            g[b + 1] = d1;
+            g[b + 2] = s1;
+            if constexpr (DEV) continue;
             r = line ? add(r, k0) : k0;
             jx = line ? add(jx, d1) : d1;
             // (line 0 is the first of both, with the sign -1)
@@ -225,11 +206,13 @@ __device__ __forceinline__ void cumulant(V *s, V &rho, V &ux, V &uy, V &uz, floa
             if (lz == 2) jz = add(jz, k0);
             if (lz == 0) jz = line ? sub(jz, k0) : neg(k0);
         }
-        rho = DEV ? add(r, bc<V>(1.f)) : r;
-        const V is = safe_inv(rho);
-        ux = mul(DEV ? addc(jx, sh.u[0]) : jx, is);
-        uy = mul(DEV ? addc(jy, sh.u[1]) : jy, is);
-        uz = mul(DEV ? addc(jz, sh.u[2]) : jz, is);
+        if constexpr (!DEV) {
+            rho = r;
+            const V is = safe_inv(rho);
+            ux = mul(jx, is);
+            uy = mul(jy, is);
+            uz = mul(jz, is);
+        }
         const V u2 = mul(ux, ux), mu = neg(ux), m2u = mul(ux, bc<V>(-2.f));
 #pragma unroll
         for (int line = 0; line < 9; ++line) {
