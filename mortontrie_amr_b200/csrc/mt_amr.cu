@@ -758,15 +758,26 @@ void free_side(Side &side)
     side.level.clear();
     free_branch(side);
 }
+static int open_side(Ctx &ctx, Side &side, int levels)
+{
+    if (int rc = make_branch(ctx, side)) return rc;
+    if ((int)side.level.size() < levels) side.level.resize(levels);
+    for (int l = 0; l < levels; ++l)
+        if (int rc = make_branch(ctx, side.level[l])) return rc;
+    return MT_OK;
+}
 static int make_side(Ctx &ctx, Case &c)
 {
     if (!c.side) c.side = &ctx.side;
-    if (int rc = make_branch(ctx, *c.side)) return rc;
-    if ((int)c.side->level.size() < c.d.max_level) c.side->level.resize(c.d.max_level);
-    for (int l = 0; l < c.d.max_level; ++l)
-        if (int rc = make_branch(ctx, c.side->level[l])) return rc;
-    return MT_OK;
+    return open_side(ctx, *c.side, c.d.max_level);
 }
+// A case holds its side streams only while its work is issued: it may move to
+// another context between two calls (mt_case_transfer), and the one it leaves
+// may be destroyed.
+struct SideScope {
+    Case &c;
+    ~SideScope() { c.side = nullptr; }
+};
 // (the brick stream can leave cells out)
 static bool ib_beside_stream(const Case &c)
 {
@@ -774,7 +785,7 @@ static bool ib_beside_stream(const Case &c)
     return c.d.ib_method != MT_IB_DF && lv.nib && lv.nstream && lv.bnbr && lv.n * c.d.q < ((int64_t)1 << 32);
 }
 
-int amr_lbm_kernel(Ctx &ctx, Case &c, int l)
+static int phase_lbm_kernel(Ctx &ctx, Case &c, int l)
 {
     const int L = c.d.max_level;
     int rc;
@@ -787,7 +798,7 @@ int amr_lbm_kernel(Ctx &ctx, Case &c, int l)
         RUN(PH_COLLIDE, l);
         if (l == 0 && c.d.bc_mode == MT_BC_ZOUHE_OUTFLOW) RUN(PH_BC_INOUT, 0);
         if (l < L)
-            if ((rc = amr_lbm_kernel(ctx, c, l + 1))) return rc;
+            if ((rc = phase_lbm_kernel(ctx, c, l + 1))) return rc;
         if (l > 0 && sub == 0) RUN(PH_EXPLOSION, l);
         if (l > 0 && sub == 1 && c.itime != MT_ITIME_REFERENCE) RUN(PH_EXPLOSION_B, l);
         if (l > 0 && l == L && ib_beside_stream(c)) {
@@ -824,9 +835,15 @@ int amr_lbm_kernel(Ctx &ctx, Case &c, int l)
     return MT_OK;
 }
 
+int amr_lbm_kernel(Ctx &ctx, Case &c, int l)
+{
+    SideScope scope{c};
+    return phase_lbm_kernel(ctx, c, l);
+}
+
 static int record_step(Ctx &ctx, Case &c)
 {
-    int rc = amr_lbm_kernel(ctx, c, 0);
+    int rc = phase_lbm_kernel(ctx, c, 0);
     if (rc) return rc;
     if (!c.side) {
         if ((rc = amr_phase(ctx, c, PH_IB_SUM, 0))) return rc;
@@ -847,6 +864,7 @@ static int record_step(Ctx &ctx, Case &c)
 static int capture(Ctx &ctx, Case &c, int (*record)(Ctx &, Case &), cudaGraphExec_t *out, int64_t *launches)
 {
     const int64_t before = ctx.launches;
+    SideScope scope{c};
     MT_CUDA(ctx, cudaStreamBeginCapture(ctx.stream, cudaStreamCaptureModeThreadLocal));
     int rc = record(ctx, c);
     cudaGraph_t captured = nullptr;
@@ -940,6 +958,8 @@ static int fused_lbm_kernel(Ctx &ctx, Case &c, int l, bool last_parent)
 
 static int record_fused_step(Ctx &ctx, Case &c)
 {
+    if (c.d.max_level > 0)
+        if (int rc = make_side(ctx, c)) return rc;
     c.fused_now = true;
     int rc = fused_lbm_kernel(ctx, c, 0, true);
     c.fused_now = false;
@@ -992,8 +1012,8 @@ static int build_bricks(Ctx &ctx, Case &c, int l)
 static int prime_fused(Ctx &ctx, Case &c)
 {
     const int L = c.d.max_level;
-    if (L > 0)
-        if (int rc = make_side(ctx, c)) return rc;
+    if (L > 0)  // (made here, not while the step is captured)
+        if (int rc = open_side(ctx, ctx.side, L)) return rc;
     for (int l = 0; l <= L; ++l) {
         Level &lv = c.lv[l];
         if (!lv.n) continue;
@@ -1133,12 +1153,10 @@ int record_batch_step(Ctx &ctx, Batch &B, const std::vector<Case *> &cases)
     int rc = MT_OK;
     for (size_t i = 0; i < cases.size() && !rc; ++i) {
         Case &c = *cases[i];
-        Side *own = c.side;
+        SideScope scope{c};
         ctx.stream = B.pool[i % P].s;
         c.side = B.side[i % P].get();
-        if (c.d.max_level > 0) rc = make_side(ctx, c);
-        if (!rc) rc = record_fused_step(ctx, c);
-        c.side = own;
+        rc = record_fused_step(ctx, c);
     }
     ctx.stream = main;
     for (size_t p = 0; p < P; ++p) {

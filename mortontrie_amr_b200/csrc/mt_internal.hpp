@@ -208,7 +208,7 @@ struct Case {
     bool skip_ib = false; // PH_STREAM leaves the IB cells to treat() (amr_lbm_kernel)
     int in_batch = 0;     // batches holding the case
     bool f_stale = false; // fused passes left class-1 brick cells' streamed f unstored (amr_sync_f)
-    Side *side = nullptr;  // the context's, or a batch's while that records its step
+    Side *side = nullptr;  // while work is issued: the context's, or the batch's branch's (SideScope)
 };
 
 // Cases stepped together (mt_batch_*): every member's step is a parallel branch
