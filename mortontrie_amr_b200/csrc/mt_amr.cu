@@ -1156,7 +1156,9 @@ int record_batch_step(Ctx &ctx, Batch &B, const std::vector<Case *> &cases)
         SideScope scope{c};
         ctx.stream = B.pool[i % P].s;
         c.side = B.side[i % P].get();
-        rc = record_fused_step(ctx, c);
+        // (a single-level member too: its forcing forks)
+        rc = make_side(ctx, c);
+        if (!rc) rc = record_fused_step(ctx, c);
     }
     ctx.stream = main;
     for (size_t p = 0; p < P; ++p) {

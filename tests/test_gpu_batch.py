@@ -141,3 +141,47 @@ def test_large_member_runs_its_own_pass(ctx, storage):
     batch.close()
     for m in alone + members:
         m.close()
+
+
+@pytest.mark.parametrize("with_levels", [False, True])
+def test_single_level_direct_forcing_member(ctx, with_levels):
+    """A direct-forcing sphere without refinement steps in a batch, by itself
+    and after members with levels, as alone."""
+    from mortontrie_amr_b200.case import df_sphere_case
+    from mortontrie_amr_b200.lbm import Batch, LBM_Manager
+    cases = (_mix()[:2] if with_levels else []) + [
+        df_sphere_case(radius=3, max_level=0, re=40.0, oscillating=True, period=100)]
+    alone = [LBM_Manager(ctx, c, "f64", schedule="fused") for c in cases]
+    members = [LBM_Manager(ctx, c, "f64") for c in cases]
+    batch = Batch(ctx, members)
+    for m in alone:
+        m.fluidSimulate(3)
+    batch.step(3)
+    ctx.synchronize()
+    for a, m in zip(alone, members):
+        _assert_same(_state(a), _state(m))
+    batch.close()
+
+
+def test_members_sharing_branches(ctx):
+    """More members than branches, of 0 to 2 levels: those that share a branch
+    follow one another on its streams, each as it steps alone."""
+    from mortontrie_amr_b200.case import cavity_case, df_sphere_case
+    from mortontrie_amr_b200.lbm import Batch, LBM_Manager
+    kinds = [df_sphere_case(radius=3, max_level=0, re=40.0, oscillating=True, period=100),
+             cavity_case(q=19, coarse=(16, 16, 16), max_level=1, re=100.0),
+             cavity_case(q=27, collision="Cumulant", coarse=(24, 24, 24), max_level=2, re=60.0),
+             cavity_case(q=19, coarse=(16, 16, 20), max_level=1, re=80.0), _mix()[5]]
+    alone = [LBM_Manager(ctx, c, "f64", schedule="fused") for c in kinds]
+    for m in alone:
+        m.fluidSimulate(3)
+    want = [_state(m) for m in alone]
+    members = [LBM_Manager(ctx, kinds[(3 * i) % 5], "f64") for i in range(39)]
+    batch = Batch(ctx, members)
+    batch.step(3)
+    ctx.synchronize()
+    for i, m in enumerate(members):
+        _assert_same(want[(3 * i) % 5], _state(m))
+    batch.close()
+    for m in alone + members:
+        m.close()
