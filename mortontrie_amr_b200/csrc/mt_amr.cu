@@ -138,10 +138,10 @@ MT_HD void children(const MortonGeom &g, uint64_t code, int fine, uint64_t *ch)
 // F2C sources need every child stored and skip children listed in dis;
 // ghost sources write only children in ghost_overlap_C2F and not in dis.
 // child[j]: the slot of the first child (the eight are consecutive), mask[j]
-// the slots to write.
+// the slots to write.  found: EXPL_*, what some written child is besides.
 __global__ void k_expl_children(MortonGeom g, int fine, const int32_t *src, int64_t nsrc, int64_t nf2c,
                                 const LevelMap cmap, const LevelMap fmap, const uint32_t *ftag, const uint64_t *dkey,
-                                int64_t nd, int32_t *child, uint8_t *mask, int *err)
+                                int64_t nd, int32_t *child, uint8_t *mask, int *err, int *found)
 {
     int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (j >= nsrc) return;
@@ -163,6 +163,14 @@ __global__ void k_expl_children(MortonGeom g, int fine, const int32_t *src, int6
             out |= 1u << m;
         }
     }
+    int is = 0;
+    for (int m = 0; m < 8; ++m)
+        if ((out >> m) & 1u) {
+            const uint32_t t = ftag[64 * b + m0 + m];
+            if (t & (TAG_F2C | TAG_GF2C)) is |= EXPL_SOURCE;
+            if ((t & TAG_LATF) && !(t & TAG_C2F)) is |= EXPL_COLLIDED;
+        }
+    if (is) atomicOr(found, is);
     // slots without a cell may be written too: most sources (a ghost source has
     // only its children next to the interface) then take whole-vector stores
     if (out) out |= ~there & 255u;
@@ -325,7 +333,7 @@ static int select_known(Ctx &ctx, int64_t n, Pred pred, int64_t count, int32_t *
 // how many slots carry each tag bit (0..8) and each boundary set (9..34): the
 // sizes of a level's lists, read back once; and how many cells are both
 // collided and copied (35)
-constexpr int kTagBits = 9, kCounts = kTagBits + 28;
+constexpr int kTagBits = 9, kCounts = kTagBits + 27;
 __global__ void k_count_sets(const uint32_t *__restrict__ tag, const int8_t *__restrict__ bc, int64_t n,
                              unsigned *__restrict__ count)
 {
@@ -339,8 +347,7 @@ __global__ void k_count_sets(const uint32_t *__restrict__ tag, const int8_t *__r
         if (m && (threadIdx.x & 31) == 0) atomicAdd(s + k, __popc(m));
     }
     if (t & TAG_BC) atomicAdd(s + kTagBits + bc[i], 1u);
-    if ((t & TAG_C2F) && (t & (TAG_LATF | TAG_F2C))) atomicAdd(s + kCounts - 2, 1u);
-    if ((t & (TAG_C2F | TAG_GC2F)) && (t & (TAG_F2C | TAG_GF2C))) atomicAdd(s + kCounts - 1, 1u);
+    if ((t & TAG_C2F) && (t & (TAG_LATF | TAG_F2C))) atomicAdd(s + kCounts - 1, 1u);
     __syncthreads();
     for (int k = threadIdx.x; k < kCounts; k += blockDim.x)
         if (s[k]) atomicAdd(count + k, s[k]);
@@ -489,8 +496,7 @@ static int build_level(Ctx &ctx, Case &c, int l)
     MT_CUDA(ctx, cudaMemcpyAsync(count, d_count, sizeof(count), cudaMemcpyDeviceToHost, ctx.stream));
     MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
     cudaFreeAsync(d_count, ctx.stream);
-    lv.mixed = count[kCounts - 2] != 0;
-    lv.chained = count[kCounts - 1] != 0;
+    lv.mixed = count[kCounts - 1] != 0;
     const uint32_t bits[kNumSets] = {TAG_LATF, TAG_F2C, TAG_C2F, TAG_GC2F, TAG_GF2C, TAG_SF};
     for (int s = 0; s < kNumSets; ++s) {
         int at = 0;
@@ -518,8 +524,10 @@ int amr_build(Ctx &ctx, Case &c)
         c.geom.periodic[a] = c.d.periodic[a];
         c.geom.extent0[a] = c.d.extent0[a];
     }
-    MT_CUDA(ctx, cudaMallocAsync(&c.dev_err, sizeof(int), ctx.stream));
-    MT_CUDA(ctx, cudaMemsetAsync(c.dev_err, 0, sizeof(int), ctx.stream));
+    // the error flags, then the levels' EXPL_* flags, read back together below
+    int herr[1 + kMaxLevels];
+    MT_CUDA(ctx, cudaMallocAsync(&c.dev_err, sizeof(herr), ctx.stream));
+    MT_CUDA(ctx, cudaMemsetAsync(c.dev_err, 0, sizeof(herr), ctx.stream));
     MT_CUDA(ctx, cudaMallocAsync(&c.force_acc, 4 * sizeof(double), ctx.stream));
     MT_CUDA(ctx, cudaMemsetAsync(c.force_acc, 0, 4 * sizeof(double), ctx.stream));
     for (int l = 0; l <= L; ++l) {
@@ -614,7 +622,7 @@ int amr_build(Ctx &ctx, Case &c)
             MT_CUDA(ctx, cudaMallocAsync(&fl.expl_mask, fl.nexpl, ctx.stream));
             k_expl_children<<<grid_for(fl.nexpl, 128), 128, 0, ctx.stream>>>(
                 c.geom, l, fl.expl_src, fl.nexpl, fl.nexpl_f2c, cl.map(), fl.map(), fl.tag, c.dis_key, c.ndis,
-                fl.expl_child, fl.expl_mask, c.dev_err);
+                fl.expl_child, fl.expl_mask, c.dev_err, c.dev_err + 1 + l);
             MT_LAUNCHED(ctx);
         }
         if (cl.nlist[1]) {
@@ -624,13 +632,14 @@ int amr_build(Ctx &ctx, Case &c)
             MT_LAUNCHED(ctx);
         }
     }
-    int herr = 0;
-    MT_CUDA(ctx, cudaMemcpyAsync(&herr, c.dev_err, sizeof(int), cudaMemcpyDeviceToHost, ctx.stream));
+    MT_CUDA(ctx, cudaMemcpyAsync(herr, c.dev_err, sizeof(herr), cudaMemcpyDeviceToHost, ctx.stream));
     MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
-    if (herr & DEVERR_MISSING_CHILD)
+    if (herr[0] & DEVERR_MISSING_CHILD)
         return set_err(ctx, MT_ERR_MESH, "a child of an overlap_F2C cell is not stored on the finer level");
-    if (herr & DEVERR_DIS_NOT_FINEST) return set_err(ctx, MT_ERR_MESH, "a dis key is not a finest-level cell");
+    if (herr[0] & DEVERR_DIS_NOT_FINEST) return set_err(ctx, MT_ERR_MESH, "a dis key is not a finest-level cell");
     for (int l = 0; l <= L; ++l) {
+        c.lv[l].chained = herr[1 + l] & EXPL_SOURCE;
+        c.lv[l].hold_once = herr[1 + l] == 0;
         c.lv[l].raw_keys.clear();
         c.lv[l].raw_keys.shrink_to_fit();
         c.lv[l].raw_set.clear();
@@ -992,7 +1001,7 @@ static int build_bricks(Ctx &ctx, Case &c, int l)
         k_brick_mark<<<grid_for(8 * cnt, 256), 256, 0, ctx.stream>>>(c.lv[l - 1].coal_child, cnt, lv.bcls);
         MT_LAUNCHED(ctx);
     }
-    if (l > 0 && lv.nexpl && c.itime == MT_ITIME_HOLD && !lv.chained) {
+    if (l > 0 && lv.nexpl && c.itime == MT_ITIME_HOLD && lv.hold_once) {
         k_brick_exploded<<<grid_for(8 * lv.nexpl, 256), 256, 0, ctx.stream>>>(lv.expl_child, lv.expl_mask, lv.nexpl,
                                                                              lv.bcls);
         MT_LAUNCHED(ctx);

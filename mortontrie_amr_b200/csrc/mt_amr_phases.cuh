@@ -2012,7 +2012,7 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         const double scale = c2f_scale(c, l);
         const bool ex = phase == PH_EXPLOSION_B && c.itime == MT_ITIME_EXTRAP;
         // held parent state over bricks: once, into both buffers (k_brick_exploded)
-        const bool once = c.fused_now && lv.bricks && c.itime == MT_ITIME_HOLD && !lv.chained;
+        const bool once = c.fused_now && lv.bricks && c.itime == MT_ITIME_HOLD && lv.hold_once;
         if (once && phase == PH_EXPLOSION_B) return MT_OK;
         if (ex && !lv.expl_prev) return set_err(ctx, MT_ERR_STATE, "extrapolated explosion without saved sources");
         k_explosion<Q, S><<<grid_for(lv.nexpl, 32), 32 * kParts, 0, s>>>(lv.expl_src, lv.expl_child, lv.expl_mask, lv.nexpl,

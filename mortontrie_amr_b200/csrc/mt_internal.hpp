@@ -49,6 +49,12 @@ enum : int {
     DEVERR_NONFINITE = 8,         // NaN/Inf population found by the guard
 };
 
+// what a child that the explosion writes may be besides (k_expl_children)
+enum : int {
+    EXPL_SOURCE = 1,    // F2C or ghost F2C: a source of the next finer level's explosion
+    EXPL_COLLIDED = 2,  // lat_f and not C2F: a pass computes its next collision
+};
+
 // bflag bits
 enum : uint8_t {
     BRICK_WORK = 1,      // some cell has work
@@ -97,7 +103,11 @@ struct Level {
     int32_t *list[kNumSets] = {};
     int64_t nlist[kNumSets] = {};
     bool mixed = false;    // some C2F cell is lat_f or F2C too: its copy comes after its collision
-    bool chained = false;  // some source of the finer level's explosion is written by this level's
+    // what this level's explosion writes (the mesher's lattices: neither): a
+    // source of the finer level's explosion; and, held parent state, nothing
+    // but cells whose next collision is the copy alone, so that one explosion
+    // can serve both substeps
+    bool chained = false, hold_once = true;
     int32_t *collide_list = nullptr; int64_t ncollide = 0;  // lat_f then F2C
     int32_t *stream_list = nullptr;  int64_t nstream = 0;   // lat_f then C2F
     int32_t *bclist[26] = {};

@@ -88,3 +88,40 @@ def test_marker_counts(ctx, schedule, markers):
     assert fg[3] == fo[3] == 10
     assert np.abs(fg[:3] - fo[:3]).max() <= 1e-12 * np.abs(fo[:3]).max()
     mgr.close()
+
+
+def _sets_moved(what):
+    """The nested sphere with some written children of level 1 taken out of
+    overlap_C2F: collided like any cell (lat_f), or also sources of level 2's
+    explosion (overlap_F2C, their children copied on level 2)."""
+    case = _sphere()
+    one, two = case.mesh.levels[1], case.mesh.levels[2]
+    some = one["overlap_C2F"][::37]
+    one["overlap_C2F"] = np.setdiff1d(one["overlap_C2F"], some)
+    to = "lat_f" if what == "collided" else "overlap_F2C"
+    one[to] = np.sort(np.concatenate([one[to], some]))
+    if what == "sources":
+        children = (some[:, None] + np.arange(8, dtype=np.uint64)).ravel()
+        two["overlap_C2F"] = np.sort(np.concatenate([two["overlap_C2F"], children]))
+    return case
+
+
+@pytest.mark.parametrize("what", ["collided", "sources"])
+@pytest.mark.parametrize("itime", ["reference", "hold", "extrap"])
+@pytest.mark.parametrize("schedule", ["phases", "fused", "fused_lists"])
+def test_exploded_cells_outside_the_copied_overlap(ctx, what, itime, schedule):
+    """FP64, bit for bit against the oracle: children that the explosion writes
+    and that something else than the copy writes too keep the order of a level's
+    own work and both explosions of a held parent state."""
+    import oracle as O
+    from mortontrie_amr_b200.lbm import LBM_Manager
+    case = _sets_moved(what)
+    mgr = LBM_Manager(ctx, case, schedule=schedule, interface_time=itime)
+    oc = O.OracleCase(case)
+    oc.set_interface_time(itime)
+    for n in (1, 2):
+        mgr.fluidSimulate(n)
+        oc.step(n)
+        ctx.synchronize()
+        _oracle_equal(mgr, oc, range(case.max_level + 1))
+    mgr.close()
