@@ -40,6 +40,13 @@ int get_case(mt_ctx *h, int32_t id, Case **out)
     return MT_OK;
 }
 
+// captured steps of the batches that hold the case, dropped with what they bake in
+void drop_batches(Ctx &ctx, int32_t id)
+{
+    for (Batch *b : ctx.batches)
+        if (b && std::find(b->ids.begin(), b->ids.end(), id) != b->ids.end()) batch_drop(*b);
+}
+
 int check_desc(Ctx &ctx, const mt_case_desc *d)
 {
     if (!d) return set_err(ctx, MT_ERR_ARG, "null case description");
@@ -977,10 +984,7 @@ int mt_case_set_interface_time(mt_ctx *h, int32_t id, int32_t mode)
             if ((rc = amr_sync_f(ctx, *c))) return rc;
             c->primed = false;
             amr_drop_fused(*c);
-            for (Batch *b : ctx.batches)
-                if (b)
-                    for (int32_t x : b->ids)
-                        if (x == id) batch_drop(*b);
+            drop_batches(ctx, id);
         }
         // the captured steps bake the explosion launches in
         if (c->graph) cudaGraphExecDestroy(c->graph);
@@ -1072,10 +1076,7 @@ int mt_case_set_markers(mt_ctx *h, int32_t id, int64_t nm, const double *ref, co
         if (c->fgraph[p]) cudaGraphExecDestroy(c->fgraph[p]);
         c->fgraph[p] = nullptr;
     }
-    for (Batch *b : ctx.batches)
-        if (b)
-            for (int32_t x : b->ids)
-                if (x == id) batch_drop(*b);
+    drop_batches(ctx, id);
     MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
     return MT_OK;
 }
@@ -1288,6 +1289,7 @@ int mt_case_tune_bricks(mt_ctx *h, int32_t id, int32_t *variant, float *ms)
         if (c->fgraph[p]) cudaGraphExecDestroy(c->fgraph[p]);
         c->fgraph[p] = nullptr;
     }
+    drop_batches(ctx, id);
     if (prev != MT_SCHED_FUSED) return mt_case_set_schedule(h, id, prev);
     return MT_OK;
 }
@@ -1313,8 +1315,7 @@ int mt_case_set_brick_forms(mt_ctx *h, int32_t id, const int32_t *form)
         if (c->fgraph[p]) cudaGraphExecDestroy(c->fgraph[p]);
         c->fgraph[p] = nullptr;
     }
-    for (Batch *b : ctx.batches)
-        if (b && std::find(b->ids.begin(), b->ids.end(), id) != b->ids.end()) batch_drop(*b);
+    drop_batches(ctx, id);
     return MT_OK;
 }
 

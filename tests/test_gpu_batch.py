@@ -185,3 +185,34 @@ def test_members_sharing_branches(ctx):
     batch.close()
     for m in alone + members:
         m.close()
+
+
+def _pass_forms(batch):
+    """The forms of the brick passes that two steps of the batch (one graph) launch."""
+    import re
+    import torch
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as p:
+        batch.step(2)
+        batch.ctx.synchronize()
+    if not any("mt::k_" in e.name for e in p.events()):
+        pytest.skip("no kernel trace on this machine")
+    names = [e.name for e in p.events() if "k_brick_step" in e.name]
+    return {int(re.search(r"k_brick_step<\d+, \w+, \d+, (\d+)>", n).group(1)) for n in names}
+
+
+def test_tuned_member_steps_in_its_new_forms(ctx):
+    """The tuner's choice reaches a batch that has captured its step before."""
+    from mortontrie_amr_b200.case import sphere_case
+    from mortontrie_amr_b200.lbm import Batch, LBM_Manager
+    case = sphere_case(coarse=(128, 64, 64), refine=[((36, 24, 24), (60, 40, 40))], center=(48, 32, 32), radius=3.0,
+                       mesh="device")
+    m = LBM_Manager(ctx, case, "f16", schedule="fused")
+    m.set_brick_forms([1, 1])  # cell by cell, never the fastest on levels of this size
+    batch = Batch(ctx, [m])
+    batch.step(2)
+    assert _pass_forms(batch) == {1}
+    v, _ = m.tune_bricks()
+    assert _pass_forms(batch) == set(v[v >= 0].tolist())
+    batch.close()
+    m.close()
