@@ -649,7 +649,7 @@ int amr_build(Ctx &ctx, Case &c)
     return MT_OK;
 }
 
-void amr_drop_fused(Case &c)
+void amr_drop_fused(Ctx &ctx, Case &c)
 {
     for (int p = 0; p < 2; ++p) {
         if (c.fgraph[p]) cudaGraphExecDestroy(c.fgraph[p]);
@@ -659,7 +659,7 @@ void amr_drop_fused(Case &c)
         Level &lv = c.lv[l];
         void *ptrs[] = {lv.fused_list, lv.bcls, lv.bflag, lv.blist};
         for (void *p : ptrs)
-            if (p) cudaFree(p);
+            if (p) cudaFreeAsync(p, ctx.stream);
         lv.fused_list = nullptr;
         lv.nfused = 0;
         lv.bcls = nullptr;

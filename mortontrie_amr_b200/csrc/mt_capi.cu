@@ -939,7 +939,7 @@ int mt_case_set_schedule(mt_ctx *h, int32_t id, int32_t schedule)
     if (c->schedule == MT_SCHED_PHASES || bricks != c->use_bricks) {
         c->primed = false;
         // the fused graphs bake in the pass each level uses
-        amr_drop_fused(*c);
+        amr_drop_fused(ctx, *c);
     }
     c->use_bricks = bricks;
     c->schedule = MT_SCHED_FUSED;
@@ -983,7 +983,7 @@ int mt_case_set_interface_time(mt_ctx *h, int32_t id, int32_t mode)
             // the brick classes depend on the mode
             if ((rc = amr_sync_f(ctx, *c))) return rc;
             c->primed = false;
-            amr_drop_fused(*c);
+            amr_drop_fused(ctx, *c);
             drop_batches(ctx, id);
         }
         // the captured steps bake the explosion launches in

@@ -325,7 +325,7 @@ template <class S> struct AmrOps {
 };
 void amr_free(Case &c);
 // forget the fused schedule's graphs and brick tables (rebuilt at the next fused step)
-void amr_drop_fused(Case &c);
+void amr_drop_fused(Ctx &ctx, Case &c);
 
 // dense uniform path, one explicit instantiation per storage type
 // (mt_dense_f64.cu builds the FP64 one without FMA contraction)

@@ -125,3 +125,31 @@ def test_exploded_cells_outside_the_copied_overlap(ctx, what, itime, schedule):
         ctx.synchronize()
         _oracle_equal(mgr, oc, range(case.max_level + 1))
     mgr.close()
+
+
+def test_interface_option_changed_while_steps_run(ctx):
+    """The brick tables that an option drops stay with the steps still running:
+    memory that another context takes meanwhile is not theirs."""
+    from mortontrie_amr_b200.case import cavity_case
+    from mortontrie_amr_b200.lbm import Context, LBM_Manager
+    case = cavity_case(q=19, coarse=(32, 32, 32), max_level=2, re=100.0)
+    want = LBM_Manager(ctx, case, schedule="fused", scaling="standard", interface_time="hold")
+    got = LBM_Manager(ctx, case, schedule="fused", scaling="standard", interface_time="hold")
+    other = Context(0)
+    for mode in ("extrap", "hold"):
+        for m in (want, got):
+            m.fluidSimulate(30)
+            if m is want:
+                ctx.synchronize()
+            m.set_interface_time(mode)
+            if m is got:
+                for _ in range(3):
+                    x = LBM_Manager(other, case, "f16", schedule="fused")
+                    x.fluidSimulate(1)
+                    x.close()
+    for l in range(case.max_level + 1):
+        for a, b in zip(want.populations(l), got.populations(l)):
+            assert np.isfinite(a).all() and np.array_equal(a, b), l
+    want.close()
+    got.close()
+    other.close()
