@@ -940,6 +940,7 @@ int mt_case_set_schedule(mt_ctx *h, int32_t id, int32_t schedule)
         c->primed = false;
         // the fused graphs bake in the pass each level uses
         amr_drop_fused(ctx, *c);
+        drop_batches(ctx, id);
     }
     c->use_bricks = bricks;
     c->schedule = MT_SCHED_FUSED;
@@ -963,6 +964,7 @@ int mt_case_set_interface_scaling(mt_ctx *h, int32_t id, int32_t scaling)
             if (c->fgraph[p]) cudaGraphExecDestroy(c->fgraph[p]);
             c->fgraph[p] = nullptr;
         }
+        drop_batches(ctx, id);
     }
     c->scaling = scaling;
     return MT_OK;
@@ -1007,6 +1009,7 @@ int mt_case_set_face_velocity(mt_ctx *h, int32_t id, int32_t face, const double 
     if (c->dense || !c->built) return set_err(ctx, MT_ERR_STATE, "face velocities need a built multi-level case");
     if (face < 0 || face > 5) return set_err(ctx, MT_ERR_ARG, "face must be 0..5 (West East South North Bot Top)");
     if (!u) return set_err(ctx, MT_ERR_ARG, "null velocity");
+    drop_batches(ctx, id);
     return amr_set_face(ctx, *c, face, u);
 }
 

@@ -216,3 +216,35 @@ def test_tuned_member_steps_in_its_new_forms(ctx):
     assert _pass_forms(batch) == set(v[v >= 0].tolist())
     batch.close()
     m.close()
+
+
+@pytest.mark.parametrize("what", ["scaling", "face", "schedule"])
+def test_member_changed_between_batch_steps(ctx, what):
+    """What a captured step bakes in, changed on a member, reaches the batch."""
+    from mortontrie_amr_b200.case import cavity_case
+    from mortontrie_amr_b200.lbm import Batch, LBM_Manager
+    case = cavity_case(q=19, coarse=(24, 24, 24), max_level=1, re=100.0)
+
+    def change(m):
+        if what == "scaling":
+            m.set_interface_scaling("standard")
+        elif what == "face":
+            m.set_face_velocity(5, (0.02, 0.01, 0.0))
+        else:
+            m.set_schedule("fused_lists")
+
+    alone, member, plain = (LBM_Manager(ctx, case, "f64", schedule="fused") for _ in range(3))
+    batch = Batch(ctx, [member, plain])
+    alone.fluidSimulate(2)
+    batch.step(2)
+    change(alone)
+    change(member)
+    alone.fluidSimulate(2)
+    batch.step(2)
+    ctx.synchronize()
+    _assert_same(_state(alone), _state(member))
+    if what != "schedule":
+        assert not np.array_equal(member.populations(1)[0], plain.populations(1)[0])
+    batch.close()
+    for m in (alone, member, plain):
+        m.close()
