@@ -128,7 +128,9 @@ int mt_case_create(mt_ctx *ctx, const mt_case_desc *desc, int32_t *case_id);
  * key set is generated on the device. */
 int mt_case_create_dense(mt_ctx *ctx, const mt_case_desc *desc, int32_t *case_id);
 int mt_case_destroy(mt_ctx *ctx, int32_t case_id);
-/* add keys to one index set of one level (Lat_Manager::lat_f[l].insert ...) */
+/* add keys to one index set of one level (Lat_Manager::lat_f[l].insert ...): the
+ * cells' Morton codes in finest-cell units, whose lowest 3 (max_level - level)
+ * bits are zero (MT_ERR_MESH from mt_case_build otherwise) */
 int mt_case_add_set(mt_ctx *ctx, int32_t case_id, int32_t level, int32_t set_id, const uint64_t *keys, int64_t n);
 /* Lat_Manager::dis: finest-level keys (ascending) and Q-1 wall distances each */
 int mt_case_set_dis(mt_ctx *ctx, int32_t case_id, const uint64_t *keys, const double *rows, int64_t n);

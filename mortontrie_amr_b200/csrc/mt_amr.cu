@@ -19,15 +19,17 @@ namespace mt {
 // build kernels
 // ----------------------------------------------------------------------------
 // sorted raw keys (with repeats): a cell starts where the key changes (low
-// half), a brick where the key's brick part does (high half)
-__global__ void k_starts(const uint64_t *key, int64_t n, int shift, unsigned long long *flag)
+// half), a brick where the key's brick part does (high half).  A key with bits
+// below the level's cells names no slot.
+__global__ void k_starts(const uint64_t *key, int64_t n, int low, unsigned long long *flag, int *err)
 {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
     unsigned long long v = 0;
     if (i == 0 || key[i] != key[i - 1]) v |= 1ull;
-    if (i == 0 || (key[i] >> shift) != (key[i - 1] >> shift)) v |= 1ull << 32;
+    if (i == 0 || (key[i] >> (low + 6)) != (key[i - 1] >> (low + 6))) v |= 1ull << 32;
     flag[i] = v;
+    if (key[i] & ((1ull << low) - 1ull)) atomicOr(err, DEVERR_KEY_BITS);
 }
 
 // c = inclusive scan of the starts: cell rank and brick of sorted key i
@@ -428,7 +430,7 @@ static int build_level(Ctx &ctx, Case &c, int l)
         void *tmp = nullptr;
         MT_CUDA(ctx, cudaMallocAsync(&tmp, std::max(t1, t2), ctx.stream));
         MT_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, t1, d_raw, d_sorted, (int)nraw, 0, 64, ctx.stream));
-        k_starts<<<grid_for(nraw, 256), 256, 0, ctx.stream>>>(d_sorted, nraw, lv.low + 6, d_start);
+        k_starts<<<grid_for(nraw, 256), 256, 0, ctx.stream>>>(d_sorted, nraw, lv.low, d_start, c.dev_err);
         MT_LAUNCHED(ctx);
         MT_CUDA(ctx, cub::DeviceScan::InclusiveSum(tmp, t2, d_start, d_scan, (int)nraw, ctx.stream));
         unsigned long long h_num = 0;
@@ -634,6 +636,8 @@ int amr_build(Ctx &ctx, Case &c)
     }
     MT_CUDA(ctx, cudaMemcpyAsync(herr, c.dev_err, sizeof(herr), cudaMemcpyDeviceToHost, ctx.stream));
     MT_CUDA(ctx, cudaStreamSynchronize(ctx.stream));
+    if (herr[0] & DEVERR_KEY_BITS)
+        return set_err(ctx, MT_ERR_MESH, "a key has bits set below the cells of its level");
     if (herr[0] & DEVERR_MISSING_CHILD)
         return set_err(ctx, MT_ERR_MESH, "a child of an overlap_F2C cell is not stored on the finer level");
     if (herr[0] & DEVERR_DIS_NOT_FINEST) return set_err(ctx, MT_ERR_MESH, "a dis key is not a finest-level cell");

@@ -47,6 +47,7 @@ enum : int {
     DEVERR_MISSING_BC_NBR = 2,    // a boundary cell's reserved neighbour is not stored
     DEVERR_DIS_NOT_FINEST = 4,    // a dis key is not a finest-level cell
     DEVERR_NONFINITE = 8,         // NaN/Inf population found by the guard
+    DEVERR_KEY_BITS = 16,         // a key with bits below its level's cells
 };
 
 // what a child that the explosion writes may be besides (k_expl_children)

@@ -185,3 +185,14 @@ def test_region_arguments(ctx):
     ms.has_refine[1] = 1                                                  # a box beside a region
     assert lib().mt_case_generate(ctx.h, cid.value, C.byref(ms)) == -1
     lib().mt_case_destroy(ctx.h, cid.value)
+
+
+def test_key_below_its_level_is_refused(ctx):
+    """An uploaded key with bits below its level's cells names no cell of it."""
+    from mortontrie_amr_b200.case import sphere_case
+    from mortontrie_amr_b200.lbm import LBM_Manager, MTError
+    case = sphere_case(coarse=(32, 16, 16), refine=[((6, 4, 4), (18, 12, 12))], center=(12, 8, 8), radius=2.0)
+    keys = case.mesh.levels[0]["lat_f"]
+    case.mesh.levels[0]["lat_f"] = np.sort(np.append(keys[1:], keys[0] | np.uint64(1)))
+    with pytest.raises(MTError, match="MT_ERR_MESH.*below"):
+        LBM_Manager(ctx, case)
