@@ -466,8 +466,8 @@ __global__ void k_bc_neq(const int32_t *list, int64_t nl, int b, int64_t n, cons
                 tmp[t * nl + j] = (double)full_sh<S>(sh, T::ld(f, at<Q>(k, i)), k);
                 continue;
             }
-            const C fw = feq_g<Q, C>(k, rho[i], (C)ubx, (C)uby, (C)ubz);
-            const C fn = feq_g<Q, C>(k, rho[nb], u[nb], u[n + nb], u[2 * n + nb]);
+            const C fw = feq_dir<Q, C>(k, rho[i], (C)ubx, (C)uby, (C)ubz);
+            const C fn = feq_dir<Q, C>(k, rho[nb], u[nb], u[n + nb], u[2 * n + nb]);
             tmp[t * nl + j] = (double)(fw + full_sh<S>(sh, T::ld(f, at<Q>(k, nb)), k) - fn);
         } else {
             T::st(f, at<Q>(k, i), stored_sh<S>(sh, (C)tmp[t * nl + j], k));
@@ -509,8 +509,8 @@ __global__ void __launch_bounds__(128) k_bc_neq_all(const int32_t *__restrict__ 
             tmp[t * nl + j] = (double)full_sh<S>(sh, T::cv(f[at<Q>(k, i)]), k);
             return;
         }
-        const C fw = feq_g<Q, C>(k, rho[i], (C)ub.u[b][0], (C)ub.u[b][1], (C)ub.u[b][2]);
-        const C fn = feq_g<Q, C>(k, rho[nb], u[nb], u[n + nb], u[2 * n + nb]);
+        const C fw = feq_dir<Q, C>(k, rho[i], (C)ub.u[b][0], (C)ub.u[b][1], (C)ub.u[b][2]);
+        const C fn = feq_dir<Q, C>(k, rho[nb], u[nb], u[n + nb], u[2 * n + nb]);
         tmp[t * nl + j] = (double)(fw + full_sh<S>(sh, T::cv(f[at<Q>(k, nb)]), k) - fn);
     } else {
         T::st(f, at<Q>(k, i), stored_sh<S>(sh, (C)tmp[t * nl + j], k));

@@ -326,12 +326,20 @@ template <int Q, class R> MT_HD void macros_g(const R *d, R &rho, R &ux, R &uy, 
     uy = vy * is;
     uz = vz * is;
 }
-template <int Q, class R> MT_HD R feq_g(int i, R rho, R ux, R uy, R uz)
+// For a direction known at run time only: the whole product e . u (edot_ref asks
+// for the components one by one, for which the compiler lays the direction
+// table out in every thread's local memory: the boundary sweep of a 96^3 FP64
+// cavity 172 us, 19 us this way).
+template <int Q, class R> MT_HD R feq_dir(int i, R rho, R ux, R uy, R uz)
 {
-    if constexpr (std::is_same<R, double>::value) return feq_ref<Q>(i, rho, ux, uy, uz);
     const R uu = ux * ux + uy * uy + uz * uz;
     const R euv = ex(i) * ux + ey(i) * uy + ez(i) * uz;
     return rho * (R)w<Q>(i) * (R(1) + R(3) * euv + R(4.5) * euv * euv - R(1.5) * uu);
+}
+template <int Q, class R> MT_HD R feq_g(int i, R rho, R ux, R uy, R uz)
+{
+    if constexpr (std::is_same<R, double>::value) return feq_ref<Q>(i, rho, ux, uy, uz);
+    return feq_dir<Q, R>(i, rho, ux, uy, uz);
 }
 template <int Q, class R> MT_HD R feq_heluo_g(int i, R rho, R ux, R uy, R uz)
 {
