@@ -1718,15 +1718,35 @@ __global__ void k_macro_to_f64(const C *rho, const C *u, int64_t n, const int32_
     du[nc + r] = (double)u[n + i];
     du[2 * nc + r] = (double)u[2 * n + i];
 }
-// (slots without a cell hold anything)
+// (slots without a cell hold anything)  A block per brick, whose Q x 64 values of
+// each buffer are contiguous: 16-byte loads, a thread's slots and their share of
+// the brick's occupancy from the position in the row.  (Value by value, each with
+// a division for its brick and its cell's tag, a 96^3 D3Q19 cavity's check took
+// 460 us; FP64 160, FP32 100, FP16 125 us so.)
 template <class S>
-__global__ void k_guard(const S *f, const S *fcol, const uint32_t *__restrict__ tag, int q, int64_t total, int *err)
+__global__ void __launch_bounds__(128) k_guard(const S *__restrict__ f, const S *__restrict__ fcol,
+                                               const unsigned long long *__restrict__ mask, int64_t nb, int q, int *err)
 {
-    int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    constexpr int E = 16 / (int)sizeof(S), ROW = 64 / E;
+    const bool both = f != fcol;
     bool bad = false;
-    for (; j < total; j += (int64_t)gridDim.x * blockDim.x)
-        if (tag[(j / (64 * q)) * 64 + (j & 63)])
-            bad |= !isfinite((double)Store<S>::ld(f, j)) || !isfinite((double)Store<S>::ld(fcol, j));
+    for (int64_t b = blockIdx.x; b < nb; b += gridDim.x) {
+        const unsigned long long m = mask[b];
+        const int64_t base = b * q * ROW;
+        auto check = [&](const uint4 &v, int o) {
+            alignas(16) S w[E];
+            *(uint4 *)w = v;
+#pragma unroll
+            for (int e = 0; e < E; ++e) bad |= ((m >> ((o % ROW) * E + e)) & 1) && !isfinite((double)Store<S>::cv(w[e]));
+        };
+#pragma unroll 4
+        for (int o = threadIdx.x; o < q * ROW; o += blockDim.x) {
+            const uint4 x = __ldg((const uint4 *)f + base + o);
+            const uint4 y = both ? __ldg((const uint4 *)fcol + base + o) : x;
+            check(x, o);
+            if (both) check(y, o);
+        }
+    }
     if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(err, DEVERR_NONFINITE);
 }
 
@@ -2751,9 +2771,9 @@ int AmrOps<S>::guard(Ctx &ctx, Case &c, bool current_only)
     for (int l = 0; l <= c.d.max_level; ++l) {
         Level &lv = c.lv[l];
         if (!lv.n) continue;
-        const int64_t total = lv.n * c.d.q;
-        k_guard<S><<<(unsigned)std::min<int64_t>(grid_for(total, 256), 148 * 16), 256, 0, ctx.stream>>>(
-            (const S *)(current_only ? lv.fcol : lv.f), (const S *)lv.fcol, lv.tag, c.d.q, total, c.dev_err);
+        k_guard<S><<<(unsigned)std::min<int64_t>(lv.nbrick, 148 * 16), 128, 0, ctx.stream>>>(
+            (const S *)(current_only ? lv.fcol : lv.f), (const S *)lv.fcol, (const unsigned long long *)lv.bmask,
+            lv.nbrick, c.d.q, c.dev_err);
         MT_LAUNCHED(ctx);
     }
     return MT_OK;

@@ -671,3 +671,28 @@ def test_checkpoint_resume_equals_continuous(ctx, tmp_path, which, storage):
         other.load_checkpoint(path)
     for m in (a, b, other):
         m.close()
+
+
+@pytest.mark.parametrize("q", [19, 27])
+@pytest.mark.parametrize("storage", ["f64", "f32", "f16", "bf16"])
+def test_guard_sees_every_corner_of_the_buffers(ctx, q, storage):
+    """One non-finite value in the first or last cell of a level of partly filled
+    bricks, first or last direction, either buffer, is found; none is not."""
+    from mortontrie_amr_b200.case import cavity_case
+    from mortontrie_amr_b200.lbm import LBM_Manager, MTError
+    mgr = LBM_Manager(ctx, cavity_case(q=q, coarse=(13, 11, 14), max_level=1, re=50.0), storage)
+    mgr.status()
+    for level in (0, 1):
+        good = mgr.populations(level)
+        for which in (0, 1):
+            for k in (0, q - 1):
+                for cell in (0, -1):
+                    for v in (np.nan, np.inf):
+                        bad = [a.copy() for a in good]
+                        bad[which][k, cell] = v
+                        mgr.set_populations(level, *bad)
+                        with pytest.raises(MTError, match="MT_ERR_NONFINITE"):
+                            mgr.status()
+        mgr.set_populations(level, *good)
+        mgr.status()
+    mgr.close()
