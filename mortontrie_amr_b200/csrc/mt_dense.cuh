@@ -361,12 +361,14 @@ inline Shift dense_shift(int q)
 
 // whether the fused pass works on pairs of cells: 16-bit storage always (its
 // one-cell form loads 2 bytes at a time), FP32 for the cumulant, whose
-// arithmetic bounds the one-cell form; FP32 LBGK runs one cell per thread at
-// the memory's rate.  32-bit element offsets.
+// arithmetic bounds the one-cell form, once its pairs fill a block of 128 on
+// every SM (below that one thread's chain is the time: 16^3 and 32^3 4.7 us a step
+// on pairs, 4.2 cell by cell; 64^3 10.3 / 12.4); FP32 LBGK runs one cell per thread
+// at the memory's rate.  32-bit element offsets.
 template <class S> inline bool dense_pairs(const Case &c)
 {
     if (!Store<S>::shifted || c.N < 2 || (uint64_t)c.d.q * (uint64_t)c.N >= (1ull << 32)) return false;
-    return sizeof(S) == 2 || c.d.collision != MT_COLL_LBGK;
+    return sizeof(S) == 2 || (c.d.collision != MT_COLL_LBGK && c.N >= 2 * 128 * 148);
 }
 
 inline DenseGeom dense_geom(int bits)
