@@ -122,7 +122,7 @@ __device__ __forceinline__ void macros_collide_store(typename Store<S>::C *d, ty
         if constexpr (COLL == MT_COLL_LBGK) {
             p2::lbgk<Q, float>(d, r, x, y, z, om, sh);
         } else {
-            p2::cumulant<float, false>(d, r, x, y, z, om, sh);
+            p2::cumulant(d, r, x, y, z, om, sh);
         }
 #pragma unroll
         for (int k = K0; k < K1; ++k) T::st(out, at<Q>(k, i), d[k]);
@@ -1239,7 +1239,7 @@ __device__ __forceinline__ void brick_warp_pair(int32_t b, int lane, BrickHood &
     if constexpr (COLL == MT_COLL_LBGK)
         p2::lbgk<Q, float2>(d, r, x, y, z, om, sh);
     else
-        p2::cumulant<float2, false>(d, r, x, y, z, om, sh);
+        p2::cumulant(d, r, x, y, z, om, sh);
 #pragma unroll
     for (int k = 0; k < Q; ++k) v[k] = CP::word(d[k]);
     store(fnext + o, k0, k1);

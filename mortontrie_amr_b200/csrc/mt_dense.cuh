@@ -101,7 +101,7 @@ __device__ __forceinline__ void lbgk_dev_pairs(float *s, float omega)
 // -> 236 us (at 80 registers 512 us, at 96 356 us).
 template <int Q, class S, int COLL, int MODE, int CONV, class IDX>
 __global__ void __launch_bounds__(sizeof(S) == 8 ? 256 : 1024, sizeof(S) == 8 ? 2 : 1) k_dense(const S *__restrict__ A, S *__restrict__ B, IDX N, DenseGeom g,
-                                              const Relax tau, const Shift sh)
+                                              const Relax tau)
 {
     using T = Store<S>;
     using C = typename T::C;
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(sizeof(S) == 8 ? 256 : 1024, sizeof(S) == 8 ? 
             if constexpr (COLL == MT_COLL_LBGK)
                 lbgk_dev_pairs<Q>(f, tau.om);
             else
-                p2::cumulant<float, true>(f, r, x, y, z, tau.om, sh);
+                p2::cumulant(f, r, x, y, z, tau.om, p2::NoShift{});
         }
     }
 #pragma unroll
@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(sizeof(S) == 8 ? 256 : 1024, sizeof(S) == 8 ? 
 // the FP16 cumulant is the FP32 pipe.
 template <int Q, class S, int COLL, int CONV>
 __global__ void __launch_bounds__(COLL == MT_COLL_LBGK ? 256 : 128, COLL == MT_COLL_LBGK ? (Q == 19 ? 4 : 3) : (sizeof(S) == 2 ? 7 : 6))
-    k_dense_pair(const S *__restrict__ A, S *__restrict__ B, uint32_t N, DenseGeom g, const Relax tau, const Shift sh)
+    k_dense_pair(const S *__restrict__ A, S *__restrict__ B, uint32_t N, DenseGeom g, const Relax tau)
 {
     using CP = CellPair<S>;
     const uint32_t pidx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(COLL == MT_COLL_LBGK ? 256 : 128, COLL == MT_C
         float2 f[Q], r, x, y, z;
 #pragma unroll
         for (int k = 0; k < Q; ++k) f[k] = CP::f2(w[k]);
-        p2::cumulant<float2, true>(f, r, x, y, z, om, sh);
+        p2::cumulant(f, r, x, y, z, om, p2::NoShift{});
 #pragma unroll
         for (int k = 0; k < Q; ++k) CP::st(B + (size_t)k * N + i0, CP::word(f[k]));
     }
@@ -352,13 +352,6 @@ static __global__ void k_sum_partials(const double *partial, int64_t nb, double 
     }
 }
 
-// the dense path stores f - w_q
-inline Shift dense_shift(int q)
-{
-    const double zero[3] = {0., 0., 0.};
-    return make_shift(q, zero);
-}
-
 // whether the fused pass works on pairs of cells: 16-bit storage always (its
 // one-cell form loads 2 bytes at a time), FP32 for the cumulant, whose
 // arithmetic bounds the one-cell form, once its pairs fill a block of 128 on
@@ -393,7 +386,6 @@ int DenseOps<S>::step(Ctx &ctx, Case &c, int mode)
     S *Bp = (S *)c.B;
     const int tb = c.d.stream_convention;
     const double tau = c.d.tau[0];
-    const Shift sh = dense_shift(c.d.q);
     if constexpr (Store<S>::shifted) {
         if (mode == DM_FUSED && dense_pairs<S>(c)) {
             const int PB = std::min(B, c.d.collision == MT_COLL_LBGK ? 256 : 128);
@@ -402,9 +394,9 @@ int DenseOps<S>::step(Ctx &ctx, Case &c, int mode)
             auto go = [&](auto q, auto coll) {
                 constexpr int QQ = decltype(q)::value, CC = decltype(coll)::value;
                 if (tb)
-                    k_dense_pair<QQ, S, CC, 1><<<pgrid, PB, 0, ctx.stream>>>(A, Bp, n32, g, tau, sh);
+                    k_dense_pair<QQ, S, CC, 1><<<pgrid, PB, 0, ctx.stream>>>(A, Bp, n32, g, tau);
                 else
-                    k_dense_pair<QQ, S, CC, 0><<<pgrid, PB, 0, ctx.stream>>>(A, Bp, n32, g, tau, sh);
+                    k_dense_pair<QQ, S, CC, 0><<<pgrid, PB, 0, ctx.stream>>>(A, Bp, n32, g, tau);
             };
             using Q19 = std::integral_constant<int, 19>;
             using Q27 = std::integral_constant<int, 27>;
@@ -428,11 +420,11 @@ int DenseOps<S>::step(Ctx &ctx, Case &c, int mode)
     do {                                                                                                   \
         const IDX n = (IDX)c.N;                                                                            \
         if (mode == DM_COLLIDE)                                                                            \
-            k_dense<QQ, S, CC, DM_COLLIDE, 0, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau, sh);          \
+            k_dense<QQ, S, CC, DM_COLLIDE, 0, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau);          \
         else if (tb)                                                                                       \
-            k_dense<QQ, S, CC, DM_FUSED, 1, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau, sh);            \
+            k_dense<QQ, S, CC, DM_FUSED, 1, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau);            \
         else                                                                                               \
-            k_dense<QQ, S, CC, DM_FUSED, 0, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau, sh);            \
+            k_dense<QQ, S, CC, DM_FUSED, 0, IDX><<<grid, B, 0, ctx.stream>>>(A, Bp, n, g, tau);            \
     } while (0)
 #define MT_DENSE_LAUNCH(QQ, CC)                      \
     do {                                             \

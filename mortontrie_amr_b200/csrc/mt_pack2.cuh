@@ -133,6 +133,12 @@ __device__ __forceinline__ void lbgk(V *s, V &rho, V &ux, V &uy, V &uz, float om
     }
 }
 
+// a direction's storage shift in FP32; NoShift (u_s = 0) the weight, which takes
+// no kernel parameter (the table made a launch of a 16^3 cube 0.4 us longer)
+struct NoShift {};
+__device__ __forceinline__ float shift_at(const Shift &sh, int k) { return sh.v[k]; }
+__device__ __forceinline__ constexpr float shift_at(const NoShift &, int k) { return (float)w<27>(k); }
+
 // backward chimera step of one line (chim_back's FP32 polynomials); Z0, Z1,
 // Z2 mark inputs known to be zero
 template <bool Z0, bool Z1, bool Z2, class V>
@@ -159,15 +165,16 @@ __device__ __forceinline__ void chim_back(V a0, V a1, V a2, V v, V tv, V v2, V &
 // zero, backward transform (the moments the relaxation zeroes left out).  The
 // (2,1,0), (1,0,2), (0,2,1) moments keep their forward values
 // (Collision_Cumulant.cpp:451-454).
-// DEV (the dense cube, u_s = 0): rho - 1 and the momentum are sums of the
-// deviations in direction order, without cancellation; else they come from the
-// x pass's line sums of the full populations.  (Line sums of the deviations, the
-// shift's own added once, would serve both and spare 60 packed additions of
+// shift_k = w_k (NoShift, the dense cube): rho - 1 and the momentum are sums of
+// the deviations in direction order, without cancellation; else they come from
+// the x pass's line sums of the full populations.  (Line sums of the deviations,
+// the shift's own added once, would serve both and spare 60 packed additions of
 // about 600 a pair, 256^3 FP16 416 -> 405 us, but round otherwise: results of
 // this path do not change with the kernel that computes them.)
-template <class V, bool DEV>
-__device__ __forceinline__ void cumulant(V *s, V &rho, V &ux, V &uy, V &uz, float om1, const Shift &sh)
+template <class V, class SH>
+__device__ __forceinline__ void cumulant(V *s, V &rho, V &ux, V &uy, V &uz, float om1, const SH &sh)
 {
+    constexpr bool DEV = std::is_same<SH, NoShift>::value;
     V g[27];
     if constexpr (DEV) {
         V r = s[0], jx = bc<V>(0.f), jy = bc<V>(0.f), jz = bc<V>(0.f);
@@ -185,7 +192,7 @@ __device__ __forceinline__ void cumulant(V *s, V &rho, V &ux, V &uy, V &uz, floa
         uz = mul(jz, is);
     }
 #pragma unroll
-    for (int i = 0; i < 27; ++i) g[(ex(i) + 1) + 3 * (ey(i) + 1) + 9 * (ez(i) + 1)] = addc(s[i], sh.v[i]);
+    for (int i = 0; i < 27; ++i) g[(ex(i) + 1) + 3 * (ey(i) + 1) + 9 * (ez(i) + 1)] = addc(s[i], shift_at(sh, i));
     {
         // x lines: slot 0 line total k0, slot 1 difference d1, slot 2 sum of the ends s1
         V r, jx, jy, jz;
@@ -306,7 +313,7 @@ __device__ __forceinline__ void cumulant(V *s, V &rho, V &ux, V &uy, V &uz, floa
                                            g[ix + 3 * iy], g[ix + 3 * iy + 9], g[ix + 3 * iy + 18]);
 #undef G
 #pragma unroll
-    for (int i = 0; i < 27; ++i) s[i] = addc(g[(ex(i) + 1) + 3 * (ey(i) + 1) + 9 * (ez(i) + 1)], -sh.v[i]);
+    for (int i = 0; i < 27; ++i) s[i] = addc(g[(ex(i) + 1) + 3 * (ey(i) + 1) + 9 * (ez(i) + 1)], -shift_at(sh, i));
 }
 
 }  // namespace p2
