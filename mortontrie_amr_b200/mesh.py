@@ -144,15 +144,36 @@ class Mesh:
     dis_rows: np.ndarray  # (n, Q-1) float64
     extent: list          # per level: (nx, ny, nz) in that level's cells
     markers: Optional["Markers"] = None
+    # n_slots by the sets' sizes; copies of the mesh (dataclasses.replace) share it
+    slots_of: dict = field(default_factory=dict, repr=False, compare=False)
+
+    def _parts(self, level: int) -> list:
+        parts = [self.levels[level][s] for s in SET_NAMES]
+        return parts + list(self.lat_bc) if level == 0 else parts
 
     def all_keys(self, level: int) -> np.ndarray:
-        parts = [self.levels[level][s] for s in SET_NAMES]
-        if level == 0:
-            parts += list(self.lat_bc)
+        parts = self._parts(level)
         return _sorted_unique(np.concatenate(parts)) if parts else np.zeros(0, np.uint64)
 
     def n_cells(self) -> list:
         return [int(self.all_keys(l).size) for l in range(self.spec.max_level + 1)]
+
+    def n_slots(self) -> list:
+        """Device slots per level: 64 for each aligned 4x4x4 brick that holds a
+        cell.  Counted once for sets of these sizes: a request loop asks for
+        every request (a radius-6 sphere's 1.6 M keys take 5 ms)."""
+        top = self.spec.max_level
+        sizes = tuple(int(v.size) for l in range(top + 1) for v in self._parts(l))
+        if sizes not in self.slots_of:
+            out = []
+            for l in range(top + 1):
+                bricks = []
+                for v in self._parts(l):
+                    b = v >> np.uint64(3 * (top - l) + 6)
+                    bricks.append(b[np.append(True, b[1:] != b[:-1])] if b.size else b)
+                out.append(64 * int(np.unique(np.concatenate(bricks)).size))
+            self.slots_of[sizes] = out
+        return self.slots_of[sizes]
 
 
 @dataclass
@@ -222,11 +243,9 @@ def estimate_slots(spec: MeshSpec) -> list:
         regions = octree_regions(spec)
         out = [64 * bricks((0, 0, 0), tuple(-(-n // 4) for n in spec.coarse))]
         for l in range(1, spec.max_level + 1):
-            d = regions[l].children().dilate(1)
-            c = (np.argwhere(d.mask) + d.lo) >> 2
-            c -= c.min(axis=0)
-            shape = c.max(axis=0) + 1
-            out.append(64 * int(np.unique(np.ravel_multi_index(c.T, shape)).size))
+            # a brick is 2x2x2 cells of the coarser level, the region's own, and
+            # the children's one-cell layer lies in the cells around it
+            out.append(64 * int(regions[l].dilate(1).parents().mask.sum()))
         return out
     out = []
     lo, hi = (0, 0, 0), tuple(spec.coarse)

@@ -174,9 +174,7 @@ def footprint_bytes(case, storage: str) -> int:
     if isinstance(case.mesh, SpecMesh):
         slots = estimate_slots(case.mesh.spec)
     else:
-        top = case.mesh.spec.max_level
-        slots = [64 * int(np.unique(case.mesh.all_keys(l) >> np.uint64(3 * (top - l) + 6)).size)
-                 for l in range(top + 1)]
+        slots = case.mesh.n_slots()
     for n in slots:
         total += n * (3 * q * sb + 4 * (q - 1) + 4 * 4 + 8 + 4 + 16 + 8 + 20)
     total += int(case.mesh.markers.dv.size) * 80 if case.mesh.markers is not None else 0

@@ -21,3 +21,19 @@ def test_estimate_slots_bounds_the_bricks(make):
     assert len(est) == L + 1
     for r, e in zip(real, est):
         assert r <= e <= 1.1 * r
+
+
+def test_slots_of_a_mesh_are_counted_once_for_its_copies():
+    """A request's mesh is its template's with other markers: the count of its
+    bricks is the template's, and sets of other sizes are counted anew."""
+    import dataclasses
+    mesh = sphere_case().mesh
+    L = mesh.spec.max_level
+    count = lambda m: [64 * np.unique(m.all_keys(l) >> np.uint64(3 * (L - l) + 6)).size for l in range(L + 1)]  # noqa: E731
+    copy = dataclasses.replace(mesh, markers=None)
+    assert copy.n_slots() == count(mesh)
+    assert mesh.n_slots() is copy.n_slots()
+    levels = [dict(d) for d in mesh.levels]
+    levels[L]["lat_f"] = levels[L]["lat_f"][:1000]
+    less = dataclasses.replace(mesh, levels=levels)
+    assert less.n_slots() == count(less) and mesh.n_slots() == count(mesh)
