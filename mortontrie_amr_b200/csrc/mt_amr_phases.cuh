@@ -2165,22 +2165,6 @@ int amr_phase_q(Ctx &ctx, Case &c, int phase, int l)
         MT_LAUNCHED(ctx);
         return MT_OK;
     }
-    case PH_F2C_COLLIDE:
-        // the F2C share of collide(level) in the fused schedule: their f comes from coalescence
-        if (lv.nlist[1]) {
-            if (c.d.collision == MT_COLL_LBGK) {
-                k_collide<Q, S, MT_COLL_LBGK><<<grid_for(lv.nlist[1], B), B, 0, s>>>(
-                    lv.list[1], lv.nlist[1], nullptr, 0, n, c.d.tau[l], A::f(lv), A::rho(lv), A::u(lv), A::fcol(lv),
-                    c.shift[l]);
-            } else {
-                if constexpr (Q == 27)
-                    k_collide<Q, S, MT_COLL_CUMULANT><<<grid_for(lv.nlist[1], 64), 64, 0, s>>>(
-                        lv.list[1], lv.nlist[1], nullptr, 0, n, c.d.tau[l], A::f(lv), A::rho(lv), A::u(lv), A::fcol(lv),
-                    c.shift[l]);
-            }
-            MT_LAUNCHED(ctx);
-        }
-        return MT_OK;
     case PH_COAL_COLLIDE: {
         if (l >= c.d.max_level || !lv.nlist[1]) return MT_OK;
         Level &fl = c.lv[l + 1];

@@ -24,7 +24,7 @@ constexpr int kNumSets = 6;  // lat_f, F2C, C2F, ghost C2F, ghost F2C, solid
 // phases of the multi-level step (amr_phase): the reference's strategy calls,
 // then the fused schedule's own passes
 enum { PH_MACROS = 0, PH_COLLIDE, PH_STREAM, PH_EXPLOSION, PH_COALESCENCE, PH_BC, PH_IB, PH_BC_INOUT,
-       PH_BC_FACE0 = 8, PH_F2C_COLLIDE = 16, PH_PULL_COLLIDE, PH_PRIME, PH_COAL_COLLIDE,
+       PH_BC_FACE0 = 8, PH_PULL_COLLIDE = 16, PH_PRIME, PH_COAL_COLLIDE,
        PH_SYNC_F, PH_DF, PH_BAND_GRID, PH_FACE_EQ0 = 24, PH_BC_HH = 32, PH_EXPLOSION_B, PH_EXPL_SAVE, PH_MACROS_ALL,
        PH_IB_SUM };
 

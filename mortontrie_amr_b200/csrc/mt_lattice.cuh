@@ -300,8 +300,6 @@ template <int Q> MT_HD double feq_heluo_ref(int i, double rho, double ux, double
     return w<Q>(i) * (rho + 1.0 * (3. * euv + 4.5 * euv * euv - 1.5 * uu));
 }
 
-MT_HD double safe_irho_ref(double r) { return 1.0 / ((r > -1e-6 && r < 1e-6) ? ((r < 0.0) ? -1e-6 : 1e-6) : r); }
-
 // The same three functions for any real type R: with R = double they are
 // the reference-order versions above, with R = float the reduced-precision
 // path's arithmetic.
