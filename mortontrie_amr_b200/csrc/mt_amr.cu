@@ -2,9 +2,11 @@
 // driver of the reference's recursive time step (the phase kernels live in
 // mt_amr_phases.cuh, one instantiation per storage type).
 //
-// Layout per level: cells sorted by Morton key; populations f/fcol as
-// [Q][n] in the storage type; nbr as [(Q-1)][n] int32 (index of key + e_k
-// or -1); index lists (int32) for each reference set in ascending key order.
+// Layout per level: 64 slots for each 4x4x4 Morton brick that holds a cell,
+// bricks in key order (Level in mt_internal.hpp); populations f/fcol as
+// [brick][Q][64] in the storage type; nbr as [(Q-1)][n] int32 (slot of the cell
+// at key + e_k or -1); index lists (int32 slots) for each reference set in
+// ascending key order.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -1153,8 +1155,8 @@ int amr_prime(Ctx &ctx, Case &c)
 // captured graph of its own, from the step's fork to its end.  (Members in
 // lockstep, joined after every phase, with one kernel over all members' bricks
 // per level and model, waited for the slowest member at each phase: 8 mid-sized
-// members 1.63 ms a coarse step against 1.36, 16 small ones 1.83 / 1.47, 4 of
-// 32^3 0.217 / 0.144, 48 up to 128x64x64 16.4 / 15.9.)
+// members 1.63 ms a coarse step against 1.38, 16 small ones 1.83 / 1.48, 4 of
+// 32^3 0.217 / 0.125, 48 up to 128x64x64 16.4 / 16.2.)
 namespace {
 
 int record_batch_step(Ctx &ctx, Batch &B, const std::vector<Case *> &cases)

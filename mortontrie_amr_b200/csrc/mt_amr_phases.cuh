@@ -1185,10 +1185,10 @@ __device__ __forceinline__ void pair_missing(int lane, int textbook, const Brick
 // source pair are constant offsets) for 54, half the stores and conversions
 // and half the arithmetic's issue slots: 79 M instructions for the finest
 // level of the 4-level cumulant sphere where the cell-by-cell pass over a
-// [Q][n] array had 133 M, 128 us for 215 us (108 B of populations per cell:
-// 72 us at the measured copy rate), FP32 167 us for 310 us.  What bounds it
-// now: the FP32 pipe (65 % active) and the gathers' latency at 24 warps per SM
-// side by side, DRAM at 46 % of its peak.
+// [Q][n] array had 133 M, 124 us for 215 us (108 B of populations per cell:
+// 72 us at the measured copy rate), FP32 168 us for 310 us.  What bounds it
+// now: the FP32 pipe (65 % active) and the gathers' latency at 28 warps per SM
+// side by side, DRAM at 46 % of its peak (both of a capture at 24).
 template <int Q, class S, int COLL>
 __device__ __forceinline__ void brick_warp_pair(int32_t b, int lane, BrickHood &h, const BrickTab &t, uint32_t n,
                                                 int textbook, const S *__restrict__ fcol, S *__restrict__ f,

@@ -98,7 +98,7 @@ __device__ __forceinline__ void lbgk_dev_pairs(float *s, float omega)
 // had 64 and spilled (D3Q19 80 B, the cumulant 2.3 KB a thread); per step, with
 // the quotients of mt_lattice.cuh: 128^3 D3Q19 123 -> 103 us, 256^3 916 -> 779 us
 // (6.5 TB/s, the measured copy rate), D3Q27 LBGK 128^3 225 -> 150 us, cumulant 924
-// -> 236 us (at 80 registers 512 us, at 96 356 us).
+// -> 223 us (at 80 registers 512 us, at 96 356 us).
 template <int Q, class S, int COLL, int MODE, int CONV, class IDX>
 __global__ void __launch_bounds__(sizeof(S) == 8 ? 256 : 1024, sizeof(S) == 8 ? 2 : 1) k_dense(const S *__restrict__ A, S *__restrict__ B, IDX N, DenseGeom g,
                                               const Relax tau)
@@ -156,10 +156,10 @@ __global__ void __launch_bounds__(sizeof(S) == 8 ? 256 : 1024, sizeof(S) == 8 ? 
 // pair.  LBGK collides the two cells one after the other at 64 registers (the
 // packed form holds both cells' FP32 values: 80 or more); the cumulant, whose
 // arithmetic bounds the one-cell form, collides both in packed FP32 in blocks of
-// 128 threads, 7 per SM at 16 bits (72 registers: 256^3 416 us), 6 at FP32 (128^3
-// 77.3 us, 64^3 11.5 us).  Cell by cell: FP16 256^3 550 us, FP32 128^3 79.7 us,
-// 64^3 13.7 us.  What bounds
-// the FP16 cumulant is the FP32 pipe.
+// 128 threads, 7 per SM at 16 bits (72 registers; a step of 256^3 FP16 / BF16 414 /
+// 416 us, with 6 414 / 422), 6 at FP32 (128^3 76.1 us, with 7 77.2).  Cell by cell
+// 128^3 FP16 73.7 us (pairs 57.4), FP32 81.8, 64^3 12.4 (10.3).  What bounds the
+// FP16 cumulant is the FP32 pipe.
 template <int Q, class S, int COLL, int CONV>
 __global__ void __launch_bounds__(COLL == MT_COLL_LBGK ? 256 : 128, COLL == MT_COLL_LBGK ? (Q == 19 ? 4 : 3) : (sizeof(S) == 2 ? 7 : 6))
     k_dense_pair(const S *__restrict__ A, S *__restrict__ B, uint32_t N, DenseGeom g, const Relax tau)

@@ -169,7 +169,7 @@ __device__ __forceinline__ void chim_back(V a0, V a1, V a2, V v, V tv, V v2, V &
 // the deviations in direction order, without cancellation; else they come from
 // the x pass's line sums of the full populations.  (Line sums of the deviations,
 // the shift's own added once, would serve both and spare 60 packed additions of
-// about 600 a pair, 256^3 FP16 416 -> 405 us, but round otherwise: results of
+// about 600 a pair, 256^3 FP16 414 -> 402 us, but round otherwise: results of
 // this path do not change with the kernel that computes them.)
 template <class V, class SH>
 __device__ __forceinline__ void cumulant(V *s, V &rho, V &ux, V &uy, V &uz, float om1, const SH &sh)
