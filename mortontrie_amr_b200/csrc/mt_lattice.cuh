@@ -252,9 +252,12 @@ template <int Q> MT_HD void macros_ref(const double *d, double &rho, double &ux,
         uy = quot(vy, s, rs);
         uz = quot(vz, s, rs);
     } else {
-        ux = vx / s;
-        uy = vy / s;
-        uz = vz / s;
+        // an infinite population makes every component NaN: the products with
+        // its zero components that the sums leave out do
+        const double z = 0. * vx + 0. * vy + 0. * vz;
+        ux = vx / s + z;
+        uy = vy / s + z;
+        uz = vz / s + z;
     }
 }
 // e_i . u, zero components left out

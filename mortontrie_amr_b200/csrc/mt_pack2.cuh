@@ -131,6 +131,12 @@ __device__ __forceinline__ void lbgk(V *s, V &rho, V &ux, V &uy, V &uz, float om
         relax(s[k], fma(bc<V>(-1.5f), u2, fma(bc<V>(3.f), e, q)), k);
         relax(s[k + 1], fma(bc<V>(-1.5f), u2, fma(bc<V>(-3.f), e, q)), k + 1);
     }
+    // an infinite population leaves no component of the macros finite (the sums
+    // leave its zero components out; the collision has NaN from u2)
+    const V z = mul(add(add(ux, uy), uz), bc<V>(0.f));
+    ux = add(ux, z);
+    uy = add(uy, z);
+    uz = add(uz, z);
 }
 
 // a direction's storage shift in FP32; NoShift (u_s = 0) the weight, which takes

@@ -83,3 +83,49 @@ def test_cells_outside_slots(ctx):
         d = xyz[:, j[ok]] - xyz[:, ok]
         assert (d[0] == 1 << (1 - l)).all() and (d[1:] == 0).all()
     m.close()
+
+
+def test_macros_of_an_infinite_population_f64(ctx):
+    """calculateMacros multiplies every population by its direction, zero
+    components included: an infinite one leaves no component finite."""
+    from mortontrie_amr_b200.lattice import directions
+    from mortontrie_amr_b200.lbm import LBM_Manager
+    m = LBM_Manager(ctx, _case("q19", "reference"))
+    f, fcol = m.populations(1)
+    cells = np.flatnonzero(m.keys(1)[1] & 1)[5::41]
+    for j, c in enumerate(cells):
+        f[j % 19, c] = (np.inf, -np.inf)[j % 2]
+    m.set_populations(1, f, fcol)
+    m.calculateMacros(1)
+    rho, u = m.macros(1)
+    with np.errstate(invalid="ignore"):
+        e = np.array(directions(19)[:3], float).T
+        r, v = f[0, cells].copy(), np.zeros((3, cells.size))
+        for k in range(1, 19):
+            r += f[k, cells]
+            v += e[k][:, None] * f[k, cells]
+        v /= r
+    assert np.array_equal(rho[cells], r) and np.array_equal(u[:, cells], v, equal_nan=True)
+    assert np.isnan(v).all(axis=0).sum() >= cells.size * 17 // 19
+    m.close()
+
+
+@pytest.mark.parametrize("which", ["q19", "q27_lbgk", "df"])
+def test_macros_of_overflowed_16_bit_populations(ctx, which):
+    """Collisions that overflow FP16 storage: the fused passes write the macros
+    that the phase order's calculateMacros gives, NaN in the same places."""
+    from mortontrie_amr_b200.lbm import LBM_Manager
+    got = []
+    for schedule in ("phases", "fused", "fused_lists"):
+        m = LBM_Manager(ctx, _case(which, "reference"), "f16", schedule=schedule)
+        f, fcol = m.populations(0)
+        for c in np.flatnonzero(m.keys(0)[1] & 1)[3::29]:
+            f[[1, 7, 9, 11, 13], c] = 6e4  # 7/18 of their sum goes on in direction 1
+        m.set_populations(0, f, fcol)
+        m.fluidSimulate(1)
+        got.append(m.macros(0) + m.populations(0))
+        m.close()
+    assert np.isinf(got[0][2]).any() and np.isnan(got[0][1]).any()
+    for other in got[1:]:
+        for a, b in zip(got[0][:3], other[:3]):
+            assert np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(np.isinf(a), np.isinf(b))
