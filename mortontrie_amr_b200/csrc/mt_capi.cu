@@ -823,8 +823,10 @@ int mt_lbm_kernel(mt_ctx *h, int32_t id, int32_t level)
     if (level < 0 || level > c->d.max_level) return set_err(ctx, MT_ERR_ARG, "bad level");
     if ((rc = amr_sync_f(ctx, *c))) return rc;
     c->primed = false;
-    if ((rc = amr_lbm_kernel(ctx, *c, level))) return rc;
-    return amr_phase(ctx, *c, PH_IB_SUM, 0);
+    rc = amr_lbm_kernel(ctx, *c, level);
+    // (after an error too: the force of the calls of treat() that ran counts)
+    const int sum = amr_phase(ctx, *c, PH_IB_SUM, 0);
+    return rc ? rc : sum;
 }
 
 int mt_step(mt_ctx *h, int32_t id, int32_t n)

@@ -153,3 +153,21 @@ def test_interface_option_changed_while_steps_run(ctx):
     want.close()
     got.close()
     other.close()
+
+
+def test_force_of_a_step_that_failed(ctx):
+    """mt_lbm_kernel that stops half way (extrapolated explosion without saved
+    sources, in the second substep): the force of its first substep counts, now
+    and not with some later call."""
+    from mortontrie_amr_b200.lbm import LBM_Manager, MTError
+    case = _sphere(1)
+    mgr = LBM_Manager(ctx, case, interface_time="extrap")
+    with pytest.raises(MTError, match="MT_ERR_STATE"):
+        mgr.LBMkernel(0)
+    f = mgr.force()
+    assert f[3] == 1 and f[0] != 0
+    mgr.reset_force()
+    mgr.set_interface_time("hold")
+    mgr.LBMkernel(0)
+    assert mgr.force()[3] == 2
+    mgr.close()
