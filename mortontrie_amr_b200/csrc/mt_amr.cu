@@ -1222,7 +1222,7 @@ int batch_step(Ctx &ctx, Batch &B, const std::vector<Case *> &cases, int n)
         B.side.emplace_back(new Side);
     }
     if (!B.ev_fork) MT_CUDA(ctx, cudaEventCreateWithFlags(&B.ev_fork, cudaEventDisableTiming));
-    // capture graph g (0/1: one step from that parity, 2: two steps)
+    // capture graph g (0/1: one step from that parity, 2: two steps from parity 0)
     auto record = [&](int g) -> int {
         const int steps = g == 2 ? 2 : 1;
         const int64_t before = ctx.launches;
@@ -1253,7 +1253,9 @@ int batch_step(Ctx &ctx, Batch &B, const std::vector<Case *> &cases, int n)
     };
     int s = 0;
     while (s < n) {
-        const int g = (n - s >= 2) ? 2 : B.par;
+        // (from parity 1 a single step leads to where the two start: the buffers
+        // a graph reads are those of the parity it was recorded from)
+        const int g = (n - s >= 2 && B.par == 0) ? 2 : B.par;
         if (!B.graph[g] && (rc = record(g))) return rc;
         MT_CUDA(ctx, cudaGraphLaunch(B.graph[g], ctx.stream));
         ctx.launches += B.graph_launches[g];

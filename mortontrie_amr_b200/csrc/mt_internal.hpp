@@ -224,12 +224,13 @@ struct Case {
 
 // Cases stepped together (mt_batch_*): every member's step is a parallel branch
 // of one captured graph.  Level 0 of every member swaps buffers once per coarse
-// step, so two captured graphs alternate (par).
+// step: par counts the steps since the graphs were dropped, and a graph serves
+// the parity it was recorded from.
 constexpr size_t kBatchStreams = 32;  // members beyond share a branch
 struct Batch {
     std::vector<int32_t> ids;
-    // [0], [1]: one coarse step from level-0 parity 0 / 1; [2]: two coarse
-    // steps (back to the same parity, valid from either)
+    // [0], [1]: one coarse step from parity 0 / 1; [2]: two coarse steps from
+    // parity 0 and back to it
     cudaGraphExec_t graph[3] = {nullptr, nullptr, nullptr};
     int64_t graph_launches[3] = {0, 0, 0};
     int par = 0;

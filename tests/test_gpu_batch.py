@@ -248,3 +248,25 @@ def test_member_changed_between_batch_steps(ctx, what):
     batch.close()
     for m in (alone, member, plain):
         m.close()
+
+
+@pytest.mark.parametrize("storage", ["f64", "f16"])
+@pytest.mark.parametrize("counts", [(3, 3, 2), (1, 4, 1, 2), (2, 1, 5), (4, 3, 2, 2, 1, 3)])
+def test_step_counts_of_any_parity(ctx, storage, counts):
+    """Two steps in one graph and single ones, from either buffer parity."""
+    from mortontrie_amr_b200.lbm import Batch, LBM_Manager
+    # (FP16: the flows that stay finite)
+    cases = [_mix()[k] for k in ((0, 2, 4, 5) if storage == "f64" else (2, 3))]
+    alone = [LBM_Manager(ctx, c, storage, schedule="fused") for c in cases]
+    members = [LBM_Manager(ctx, c, storage) for c in cases]
+    batch = Batch(ctx, members)
+    for n in counts:
+        batch.step(n)
+        for m in alone:
+            m.fluidSimulate(n)
+        ctx.synchronize()
+        for a, m in zip(alone, members):
+            _assert_same(_state(a), _state(m))
+    batch.close()
+    for m in alone + members:
+        m.close()
